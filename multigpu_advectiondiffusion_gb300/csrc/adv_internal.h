@@ -113,6 +113,7 @@ int heat_tune_variant(const adv_heat_desc& d);
 // --------------------------------------------------------------- Burgers launchers
 struct BurgersLaunch {
   bool tma = false;
+  int mode = 0;  // BurgersMode: the kernel's load path and problem class
   int occ = 0;  // resident CTAs per SM of the stage kernel (before any tuning cap)
   int tiles_x = 0, tiles_y = 0;  // 32 x 16 column tiles; the grid is one wave sharing the tile-planes
   dim3 grid, block;

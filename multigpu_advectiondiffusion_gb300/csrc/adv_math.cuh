@@ -26,6 +26,9 @@ __device__ __forceinline__ float2 div_rn(float2 a, float2 b) {
 }
 __device__ __forceinline__ float2 operator-(float2 a) { return make_float2(-a.x, -a.y); }
 
+__device__ __forceinline__ float fma_rn_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn_(double a, double b, double c) { return __fma_rn(a, b, c); }
+
 // A constant of type T (both lanes for float2).
 template <class T> __device__ __forceinline__ T bc(double v) { return T(v); }
 template <> __device__ __forceinline__ float2 bc<float2>(double v) { return make_float2((float)v, (float)v); }

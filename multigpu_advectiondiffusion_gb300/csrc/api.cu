@@ -24,7 +24,7 @@ adv_status burgers_launch_f64(const adv_burgers_desc& d, const BurgersLaunch& L,
 size_t burgers_smem_f32();
 size_t burgers_smem_f64();
 template <class T>
-void* burgers_kernel_for(const adv_burgers_desc& d);
+void* burgers_kernel_for(const adv_burgers_desc& d, int mode);
 
 // ---------------------------------------------------------------------------- errors
 static thread_local std::string g_last_error;
@@ -110,26 +110,29 @@ adv_status burgers_prepare(const adv_burgers_desc& d, const void* u_in, BurgersL
   L->block = dim3(256, 1, 1);
   const int tiles_x = (d.nx + 31) / 32, tiles_y = (d.ny + 15) / 16;
   L->smem = d.dtype == ADV_F32 ? burgers_smem_f32() : burgers_smem_f64();
-  void* k = d.dtype == ADV_F32 ? burgers_kernel_for<float>(d) : burgers_kernel_for<double>(d);
+  L->mode = d.nz == 1 ? 2 : aligned ? 0 : 1;  // BurgersMode
+  void* k = d.dtype == ADV_F32 ? burgers_kernel_for<float>(d, L->mode) : burgers_kernel_for<double>(d, L->mode);
   if (!k) return set_error(ADV_ERR_UNSUPPORTED, "burgers: no kernel for this configuration");
   ADV_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->smem));
   int occ = 0;
   ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 256, L->smem));
   occ = std::max(occ, 1);
   L->occ = occ;
-  // CTAs with equal shares of the (tile, plane) pairs (at least 8 planes, or
-  // what the autotuner picked).
+  // CTAs with equal shares of the (tile, plane) pairs: one wave of them, so that no last wave is
+  // nearly empty (FP64 121 x 101 x 97: 339 CTAs of 8 planes on 304 resident ones ran 3293 us a stage,
+  // 304 run 2646; FP32 128^3: 46.2 -> 41.3), also when that leaves fewer than 8 planes each (FP32 64^3
+  // 24.6 -> 14.7, 61 x 53 x 47 22.1 -> 12.8: a segment's six extra planes cost less than idle SMs), but
+  // at least 2 planes in 3D. Two waves from 48 planes a CTA on: the cost of a (tile, plane) pair varies
+  // (edge tiles patch their halo) and the second wave evens it out (256^3: 242 -> 234; four: 237).
   const int64_t total = (int64_t)tiles_x * tiles_y * d.nz;
-  int64_t min_share = 8;
+  int64_t min_share = d.nz == 1 ? 1 : 2;
   const TuneParams tp = tune_lookup(TUNE_BURGERS, burgers_tune_variant(d), d.nx, d.ny, d.nz);
   if (tp.set) {
     occ = std::max(1, std::min(occ, tp.a));
     min_share = std::max(1, tp.b);
   }
-  // four waves of CTAs rather than one: the cost of a (tile, plane) pair varies (edge tiles patch
-  // their halo, segments restart the pipeline), and later waves fill the SMs whose CTAs finished
-  // early (measured at 256^3: 456 us per stage with one wave, 403 with four, 414 with eight)
-  const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>(4 * (int64_t)di.sms * occ, total / min_share));
+  const int64_t wave = (int64_t)di.sms * occ;
+  const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>(total >= 48 * wave ? 2 * wave : wave, total / min_share));
   L->tiles_x = tiles_x;
   L->tiles_y = tiles_y;
   L->grid = dim3((unsigned)ctas, 1, 1);

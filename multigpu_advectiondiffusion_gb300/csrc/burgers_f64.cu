@@ -6,17 +6,11 @@
 namespace adv {
 
 template <>
-void* burgers_kernel_for<double>(const adv_burgers_desc& d) {
-  const bool z = d.weno == ADV_WENO5_Z;
-  const bool visc = d.kx != 0.0 || d.ky != 0.0 || d.kz != 0.0;
-#define K(Z, D, V) reinterpret_cast<void*>(&burgers_stage_kernel<double, Z, D, V>)
-  if (d.div == ADV_DIV_FAST) {  // common-denominator form, one division per side
-    if (z) return visc ? K(true, FastDiv, true) : K(true, FastDiv, false);
-    return visc ? K(false, FastDiv, true) : K(false, FastDiv, false);
-  }
-  if (z) return visc ? K(true, double, true) : K(true, double, false);
-  return visc ? K(false, double, true) : K(false, double, false);
+void* burgers_kernel_for<double>(const adv_burgers_desc& d, int mode) {
+#define K(Z, D, V, M) reinterpret_cast<void*>(&burgers_stage_kernel<double, Z, D, V, M>)
+  ADV_BURGERS_PICK(d, mode, double, K);
 #undef K
+  return nullptr;
 }
 
 adv_status burgers_launch_f64(const adv_burgers_desc& d, const BurgersLaunch& L, const BurgersStageArgs& a,

@@ -4,17 +4,28 @@
 // Compute_Laplace_Async, Compute_RK: SingleGPU/Burgers3d_WENO5/kernels.cu:197-530, driven by
 // main.cpp:143-149) and its per-step device copy.
 //
-// Work layout: a CTA owns a 32 x 16 tile of x-y columns (256 threads, two rows per thread) and
-// marches through a chunk of z planes. Each plane of the tile plus a 3-cell halo is staged in a
-// 6-slot shared-memory ring by TMA (x start rounded down to a 16-byte boundary; periodic tiles
-// at a domain edge patch their wrapped halo after the copy lands). For the output plane k:
-//   * f+- of the staged plane go to shared memory once (Lax-Friedrichs split);
-//   * the 33x16 x-faces and 32x17 y-faces are reconstructed by all threads in a flat loop;
-//   * each thread's z-faces come from per-column register windows of f+- sliding along z;
+// Work layout: a CTA owns a 32 x 16 tile of x-y columns (256 threads, two columns adjacent in x per
+// thread) and marches through a chunk of z planes. Each plane of the tile plus a 3-cell halo is
+// staged in an 8-slot shared-memory ring by TMA (x start rounded down to a 16-byte boundary; periodic
+// tiles at a domain edge patch their wrapped halo after the copy lands). Per streamed plane q:
+//   * f+- of the output plane (q - 3) go to shared memory once (Lax-Friedrichs split), in two
+//     layouts: rows for the y-faces, pairs of rows interleaved for the x-faces, so that every
+//     operand pair of the two-value arithmetic is one load and needs no packing;
+//   * each thread's two z-faces come from its columns' line state (WenoLine: what neighbouring faces
+//     share is computed once per cell), advanced by plane q;
+//   * the 33x16 x-faces and 32x17 y-faces are reconstructed by all threads, two at a time;
 //   * L = -(dF/dx + dG/dy + dH/dz) (+ viscous O4 term), the SSP-RK3 combine, the store and a
 //     warp-shuffle max|u_out| reduction (one atomicMax per warp) for the next stage's
 //     Lax-Friedrichs constant and time step all happen in the same pass.
-// Every node is read from HBM once per stage and written once.
+// Two barriers per plane: the one after the split also releases the ring slot of the output plane
+// (nothing reads it later), the one after the faces hands them to their cells.
+// Every node is read from HBM once per stage and written once. Bound by issue: at 256^3 FP32 WENO5-Z
+// a plane takes 612 issue slots per pair of cells, 280 of them paired FP32 instructions (832 and 290
+// before neighbouring faces shared their differences, pairs were loaded instead of packed, and the six
+// quotients per cell went through the paired correction of vnquot): 334 -> 234 us per stage back to
+// back, 50.3 -> 71.8 Gcell-stage/s; the FMA pipe is 55% busy. A 2D problem (nz == 1) streams its one
+// plane alone: no z faces, no z halo (1000 x 900 FP32: 61 -> 14.5 us per stage against streaming the
+// plane seven times).
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -39,8 +50,10 @@ struct BurgersParams {
   int tiles_x, tiles_y;
   int tma;
   int un_is_uin;
+  int vec_ok;  // u_n and u_out: pairs of nodes aligned for one access
   int lf_global;
-  double dx, dy, dz;
+  T dx, dy, dz;
+  T rdx, rdy, rdz;  // 1/h, divided in FP64
   T kx, ky, kz;
   double dt_host, alpha_host;
   const double* dt_dev;
@@ -58,71 +71,89 @@ struct BurgersTile {
   static constexpr int SW = BX + 2 * PADX;  // 40
   static constexpr int SH = BY + 2 * R;     // 22
   static constexpr int PLANE = SW * SH;     // 880
-  // ring: 7 slots; while plane q is consumed the slot of plane q-4 (the previous centre plane)
-  // is refilled with plane q+3, so two planes stay in flight ahead of the one awaited
-  static constexpr int NS = 7;
-  static constexpr int P = 2;
-  static constexpr int NXF = (BX + 1) * BY;  // x-faces
-  static constexpr int NYF = BX * (BY + 1);  // y-faces
+  // ring: 8 slots (a power of two: slot and phase parity of a stream entry are bits of its number);
+  // once plane q-3 (the output plane) has been split, plane q+4 is requested, so three planes stay in
+  // flight ahead of the one awaited
+  static constexpr int NS = 8;
+  static constexpr int P = 3;
+  static constexpr int PX = BX / 2;      // column pairs per row
+  static constexpr int XS = BX + 8;      // x-face operands: cells x0-3 .. x0+34 of a row pair (38 used)
+  static constexpr int XF = BX + 2;      // x-faces per row (33 used)
 };
 
 template <class T>
 struct BurgersSmem {
   static constexpr int SLOT_ELEMS = ((BurgersTile::PLANE * (int)sizeof(T) + 127) / 128 * 128) / (int)sizeof(T);
   static constexpr size_t RING = (size_t)BurgersTile::NS * SLOT_ELEMS * sizeof(T);
-  static constexpr size_t FPM = (size_t)BurgersTile::PLANE * sizeof(T);
-  static constexpr size_t FACES = (size_t)(BurgersTile::NXF + BurgersTile::NYF) * sizeof(T);
-  static constexpr size_t TOTAL = RING + 2 * FPM + FACES;
+  // one split part, in pairs: by row pairs for the x-faces [BY/2][XS], by rows for the y-faces [SH][PX]
+  static constexpr int PART = (BurgersTile::BY / 2) * BurgersTile::XS + BurgersTile::SH * BurgersTile::PX;
+  static constexpr int NFY = (BurgersTile::BY + 1) * BurgersTile::PX;  // pairs of y-faces
+  static constexpr size_t TOTAL = RING + (2 * PART + NFY) * 2 * sizeof(T) + (size_t)BurgersTile::BY * BurgersTile::XF * sizeof(T);
 };
-
-template <class T> __device__ __forceinline__ T absval(T v) { return fabs(v); }
-template <> __device__ __forceinline__ float absval<float>(float v) { return fabsf(v); }
 
 __device__ __forceinline__ int wrapi(int i, int n) {
   i %= n;
   return i < 0 ? i + n : i;
 }
 
-// Face reconstruction and Lax-Friedrichs split for state type T: FP32 takes the fast forms (one
-// division per side, of kind D), FP64 the reference's literal operand order.
+// Face reconstruction and Lax-Friedrichs split of two values at once (V = float2 or double2): FP32,
+// and FP64 with ADV_DIV_FAST, take the common-denominator form (one division per side, of kind D);
+// FP64 otherwise the reference's literal operand order. Line: the z-face of a column pair, advanced
+// one plane at a time; u_a, u_b: the states on both sides of the face (planes q-3 and q-2).
 template <class T, bool Z, class D>
-struct Face;
-template <bool Z, class D>
-struct Face<float, Z, D> {
-  __device__ __forceinline__ static float f(float p0, float p1, float p2, float p3, float p4, float m0, float m1,
-                                            float m2, float m3, float m4) {
-    return weno_face_fast<Z, D>(p0, p1, p2, p3, p4, m0, m1, m2, m3, m4);
+struct Face {
+  using V = typename Vec2<T>::type;
+  __device__ __forceinline__ static V f(V p0, V p1, V p2, V p3, V p4, V m0, V m1, V m2, V m3, V m4) {
+    return weno_face2<Z, D>(p0, p1, p2, p3, p4, m0, m1, m2, m3, m4);
   }
-  __device__ __forceinline__ static void split(float u, float a, float& fp, float& fm) { lf_split_fast(u, a, fp, fm); }
-  // two faces / two splits at once with paired FP32 instructions (bit-identical to the above)
-  __device__ __forceinline__ static float2 f2(float2 p0, float2 p1, float2 p2, float2 p3, float2 p4, float2 m0,
-                                              float2 m1, float2 m2, float2 m3, float2 m4) {
-    return weno_face_fast2<Z, D>(p0, p1, p2, p3, p4, m0, m1, m2, m3, m4);
-  }
-  __device__ __forceinline__ static void split2(float2 u, float2 a, float2& fp, float2& fm) { lf_split_fast2(u, a, fp, fm); }
+  __device__ __forceinline__ static void split(V u, V a, V& fp, V& fm) { lf_split2(u, a, fp, fm); }
+  struct Line {
+    WenoLine<V> p, m;
+    V fp_new;  // f+ of the newest plane, one plane behind f- (its stencil ends one cell lower)
+    __device__ __forceinline__ void clear() { p.clear(); m.clear(); fp_new = vc<V>(0); }
+    __device__ __forceinline__ V push(V fp, V fm, V u_a, V u_b, bool want) {
+      V tp, tm;
+      const V qp = p.template push<Z, D, true>(fp_new, want, tp);
+      const V qm = m.template push<Z, D, false>(fm, want, tm);
+      fp_new = fp;
+      // both sides' linear parts: (f_i + f_{i+1})/2 with f+ + f- = u^2/2
+      const V lin = vmul(vc<V>(0.25), vfma(u_a, u_a, vmul(u_b, u_b)));
+      return vfma(vc<V>(0.5), vsub(qp, qm), vfma(vc<V>(-1.0 / 6.0), vadd(tp, tm), lin));
+    }
+  };
 };
-template <bool Z, class D>
-struct Face<double, Z, D> {
-  __device__ __forceinline__ static double f(double p0, double p1, double p2, double p3, double p4, double m0,
-                                             double m1, double m2, double m3, double m4) {
-    return weno_face_ref<Z, double>(p0, p1, p2, p3, p4, m0, m1, m2, m3, m4);
-  }
-  __device__ __forceinline__ static void split(double u, double a, double& fp, double& fm) { lf_split<double>(u, a, fp, fm); }
-};
-// FP64 state with ADV_DIV_FAST: the common-denominator form, one division per side.
 template <bool Z>
-struct Face<double, Z, FastDiv> {
-  __device__ __forceinline__ static double f(double p0, double p1, double p2, double p3, double p4, double m0,
-                                             double m1, double m2, double m3, double m4) {
-    return weno_face_fast64<Z>(p0, p1, p2, p3, p4, m0, m1, m2, m3, m4);
+struct Face<double, Z, double> {
+  using V = double2;
+  __device__ __forceinline__ static V f(V p0, V p1, V p2, V p3, V p4, V m0, V m1, V m2, V m3, V m4) {
+    return make_double2(weno_face_ref<Z, double>(p0.x, p1.x, p2.x, p3.x, p4.x, m0.x, m1.x, m2.x, m3.x, m4.x),
+                        weno_face_ref<Z, double>(p0.y, p1.y, p2.y, p3.y, p4.y, m0.y, m1.y, m2.y, m3.y, m4.y));
   }
-  __device__ __forceinline__ static void split(double u, double a, double& fp, double& fm) { lf_split_fast64(u, a, fp, fm); }
+  __device__ __forceinline__ static void split(V u, V a, V& fp, V& fm) {
+    lf_split<double>(u.x, a.x, fp.x, fm.x);
+    lf_split<double>(u.y, a.y, fp.y, fm.y);
+  }
+  struct Line {
+    V fp[5], fm[5], fp_new;  // f+ at q-5 .. q-1, f- at q-4 .. q
+    __device__ __forceinline__ void clear() {
+      fp_new = vc<V>(0);
+#pragma unroll
+      for (int s = 0; s < 5; ++s) fp[s] = fm[s] = vc<V>(0);
+    }
+    __device__ __forceinline__ V push(V fpq, V fmq, V, V, bool want) {
+#pragma unroll
+      for (int s = 0; s < 4; ++s) { fp[s] = fp[s + 1]; fm[s] = fm[s + 1]; }
+      fp[4] = fp_new;
+      fp_new = fpq;
+      fm[4] = fmq;
+      return want ? f(fp[0], fp[1], fp[2], fp[3], fp[4], fm[0], fm[1], fm[2], fm[3], fm[4]) : vc<V>(0);
+    }
+  };
 };
 
-struct BurgersPipe {
-  int s_issue, s_wait;  // ring slots of the next plane to issue / to wait for
-  unsigned parity;      // per-slot phase parity of the next wait
-};
+// Stream entries a CTA has waited for so far (entry n lives in slot n % NS and is that slot's phase
+// n / NS); kPipeAborted after a wait that timed out.
+constexpr unsigned kPipeAborted = 0xffffffffu;
 
 // Shared-memory objects of the Burgers pipeline (one set per CTA, whichever kernel runs it).
 __device__ __forceinline__ uint64_t* burgers_bars() {
@@ -133,8 +164,9 @@ __device__ __forceinline__ int* burgers_abort_flag() {
   __shared__ int flag;
   return &flag;
 }
-// A periodic edge tile's patch list: the staged plane's elements that lie outside the domain
-// (slot index) and the in-plane offset of the wrapped node each takes.
+// TMA: a periodic edge tile's patch list, the staged plane's elements that lie outside the domain
+// (slot index) and the in-plane offset of the wrapped node each takes. cp.async loads: the in-plane
+// offset of every element of the staged plane (wrapped when periodic), -1 outside the domain.
 struct BurgersPatch {
   int n;
   uint16_t slot[BurgersTile::PLANE];
@@ -160,25 +192,52 @@ __device__ __forceinline__ void burgers_cta_init(const CUtensorMap* tmap, bool t
   __syncthreads();
 }
 
+// How a kernel loads its planes and which problems it takes: 3D with TMA loads, 3D with element copies
+// (cp.async: rows or bases TMA cannot describe), or any (2D problems, nz == 1, with either load).
+// The common modes carry none of the others' tests in their plane loop.
+enum BurgersMode { BURGERS_3D_TMA = 0, BURGERS_3D_COPY = 1, BURGERS_ANY = 2 };
+
+// |u| or the global constant as one bit operation: (u & m) | o.
+__device__ __forceinline__ float bits_and_or(float u, unsigned m, float o) {
+  return __uint_as_float((__float_as_uint(u) & m) | __float_as_uint(o));
+}
+__device__ __forceinline__ double bits_and_or(double u, unsigned m, double o) {
+  return __hiloint2double((__double2hiint(u) & (int)m) | __double2hiint(o),
+                          (__double2loint(u) & ((int)m >> 30 & 1 ? -1 : 0)) | __double2loint(o));
+}
+
+// Stage combination of a pair, the operations of stage_combine in its order (FP32: paired).
+__device__ __forceinline__ double2 combine2(int stage, double2 un, double2 u, double dt, double2 L) {
+  return make_double2(stage_combine<double>(stage, un.x, u.x, dt, L.x), stage_combine<double>(stage, un.y, u.y, dt, L.y));
+}
+__device__ __forceinline__ float2 combine2(int stage, float2 un, float2 u, float dt, float2 L) {
+  const float2 dL = vmul(make_float2(dt, dt), L);
+  if (stage == 2) return vadd(vmul(vc<float2>(0.75), un), vmul(vc<float2>(0.25), vadd(u, dL)));
+  if (stage == 3) return div_rn(vadd(un, vmul(vc<float2>(2), vadd(u, dL))), vc<float2>(3));
+  return vadd(un, dL);
+}
+
 // One segment: output planes [zs, ze) of the column tile at (x0, y0), streamed through the
-// ring. Flushes this segment's max|u_out| into p.maxabs_key. Returns the pipeline state for the
-// next segment (by value, so it stays in registers), with s_issue = -1 if a wait timed out (the
-// CTA must then return).
-template <class T, bool Z, class D, bool VISC>
-__device__ __forceinline__ BurgersPipe burgers_segment(const CUtensorMap* tmap, const BurgersParams<T>& p, int x0,
-                                                       int y0, int zs, int ze, BurgersPipe pipe) {
+// ring, whose first entry is number n0. Flushes this segment's max|u_out| into p.maxabs_key. Returns
+// the next segment's first entry number, kPipeAborted if a wait timed out (the CTA must then return).
+template <class T, bool Z, class D, bool VISC, int MODE>
+__device__ __forceinline__ unsigned burgers_segment(const CUtensorMap* tmap, const BurgersParams<T>& p, int x0, int y0,
+                                                    int zs, int ze, unsigned n0) {
   using TL = BurgersTile;
   using SM = BurgersSmem<T>;
   using K = typename KeyOf<T>::type;
+  using V = typename Vec2<T>::type;
+  using F = Face<T, Z, D>;
   // FP64 (unless ADV_DIV_FAST): reference operand order, correctly rounded
   constexpr bool EXACT = sizeof(T) == 8 && !std::is_same<D, FastDiv>::value;
+  constexpr int PX = TL::PX, R = TL::R, SW = TL::SW, XS = TL::XS, PART = SM::PART;
+  constexpr int YP = (TL::BY / 2) * XS;  // the y-face operands of a part, after its x-face operands
 
   extern __shared__ __align__(128) unsigned char smem_raw[];
   T* ring = reinterpret_cast<T*>(smem_raw);
-  T* fpS = reinterpret_cast<T*>(smem_raw + SM::RING);
-  T* fmS = fpS + TL::PLANE;
-  T* fxS = fmS + TL::PLANE;
-  // fxS[f] for f < NXF: x-faces [BY][BX+1]; fxS[NXF + g]: y-faces [BY+1][BX]
+  V* const part = reinterpret_cast<V*>(smem_raw + SM::RING);  // f+; f- follows PART pairs later
+  V* const fyS = part + 2 * PART;                             // y-faces [BY+1][PX]
+  T* const fxS = reinterpret_cast<T*>(fyS + SM::NFY);         // x-faces [BY][XF]
   uint64_t* bars = burgers_bars();
   int* abort_flag = burgers_abort_flag();
 
@@ -186,6 +245,11 @@ __device__ __forceinline__ BurgersPipe burgers_segment(const CUtensorMap* tmap, 
   const int nx = p.nx, ny = p.ny, nz = p.nz;
   const size_t sxy = (size_t)nx * ny;
   const bool per = p.periodic != 0;
+  const bool tma = MODE == BURGERS_3D_TMA || (MODE == BURGERS_ANY && p.tma);
+  // 2D (nz == 1): the one plane is streamed alone; its z faces would be equal and their difference
+  // exactly zero, and no z layer is frozen. 3D: the output plane runs `lag` planes behind.
+  const bool twod = MODE == BURGERS_ANY && nz == 1;
+  const int lag = twod ? 0 : R;
 
   // Lax-Friedrichs constant and dt for this stage.
   T alpha;
@@ -193,58 +257,58 @@ __device__ __forceinline__ BurgersPipe burgers_segment(const CUtensorMap* tmap, 
   else if (p.alpha_key) alpha = (T)key_to_value(*static_cast<const K*>(p.alpha_key));
   else alpha = (T)p.alpha_host;
   const T dt = (T)(p.dt_dev ? *p.dt_dev : p.dt_host);
-  const bool glob = p.lf_global != 0;
+  const unsigned speed_m = p.lf_global ? 0u : 0x7fffffffu;
+  const T speed_o = p.lf_global ? alpha : T(0);
+  auto split = [&](V u, V& fp, V& fm) {
+    F::split(u, V{bits_and_or(u.x, speed_m, speed_o), bits_and_or(u.y, speed_m, speed_o)}, fp, fm);
+  };
 
-  // This thread's share of the 1072 x/y faces of a plane: x-faces tid and tid + 256 (of 528:
-  // face row f / 33, face f % 33), y-faces tid and tid + 256 (of 544: face row g / 32, column
-  // g % 32), and one of the 48 left over (x-faces 512..527 in warp 0, y-faces 512..543 in warp
-  // 1). base: shared-memory index of the face's first stencil value; the others follow at stride
-  // 1 (x) or SW (y), known at compile time per slot, so the loads take immediate offsets.
-  static_assert(TL::NXF - 2 * TL::NT == 16 && TL::NYF - 2 * TL::NT == 32, "face slots");
-  auto xbase = [](int f) {
-    const int row = f / (TL::BX + 1), fi = f - row * (TL::BX + 1);
-    return (row + TL::R) * TL::SW + fi + 1;  // column of x0+fi-3
-  };
-  auto ybase = [](int g) {
-    const int fj = g / TL::BX, c = g - fj * TL::BX;
-    return fj * TL::SW + TL::PADX + c;  // row of y0+fj-3
-  };
-  const int fbx0 = xbase(tid), fbx1 = xbase(tid + TL::NT), fby0 = ybase(tid), fby1 = ybase(tid + TL::NT);
-#ifdef ADV_BOUNDS_CHECK
-  // every face slot's stencil (base .. base + 5 strides) inside the staged plane (CTA-uniform
-  // decision, before any copy of this segment is issued)
-  if (__syncthreads_or(!ADV_IN_RANGE(fbx1 + 5, TL::PLANE, p.status) ||
-                       !ADV_IN_RANGE(fby1 + 5 * TL::SW, TL::PLANE, p.status)))
-    return BurgersPipe{-1, -1, 0u};
-#endif
-  // (Reconstructing the 48 as 24 pairs in one warp, with a run-time stride, measured 2% slower:
-  // one warp then carries three paired reconstructions while the others wait at the barrier.)
-  const bool left_x = tid < 16, left_y = tid >= 32 && tid < 64;
-  const int fbl = left_x ? xbase(2 * TL::NT + tid) : ybase(2 * TL::NT + (left_y ? tid - 32 : 0));
-  // Per-thread columns: (lane, warp) and (lane, warp + 8).
-  const int cx = lane;
-  const int cy0 = warp, cy1 = warp + 8;
+  // This thread's columns: 2 cp, 2 cp + 1 of row `row` (a warp holds two rows, one row pair).
+  const int cp = tid & (PX - 1), row = tid / PX;
+  const int own = (row + R) * SW + TL::PADX + 2 * cp;  // its place in a staged plane
+  const int x = x0 + 2 * cp, y = y0 + row;
+  const bool in0 = x < nx && y < ny, in1 = x + 1 < nx && y < ny;  // partial tiles extend past the domain
+  const int FR = per ? 0 : 3;
+  const bool yok = per || (y >= FR && y < ny - FR);
+  const bool upd0 = in0 && yok && (per || (x >= FR && x < nx - FR));
+  const bool upd1 = in1 && yok && (per || (x + 1 >= FR && x + 1 < nx - FR));
+  const bool vec = p.vec_ok && in1;
   K kmax = 0;
-  const T rdx = T(1.0 / p.dx), rdy = T(1.0 / p.dy), rdz = T(1.0 / p.dz);
-  const int F = per ? 0 : 3;
+  // Operand places of this thread's share of the splits and faces.
+  T* const xw = reinterpret_cast<T*>(part + warp * XS + 2 * cp + R) + (row & 1);  // its cells, x layout
+  V* const yw = part + YP + R * PX + tid;                                        // its cells, y layout
+  const V* const xr = part + warp * XS + lane;  // x-face `lane` (between cells lane-1 and lane) of its row pair
+  const V* const yr = part + YP + tid;          // the y-faces below its cells
+  // halo splits, two values each: threads [0, 96) the six halo rows, pairs of columns; [96, 144) the
+  // six halo columns, pairs of rows
+  const bool halo = tid < 6 * PX + 6 * (TL::BY / 2);
+  int h_src, h_step;
+  V* h_dst;
+  if (tid < 6 * PX) {
+    const int h = tid / PX, r = h < R ? h : h + TL::BY;
+    h_src = r * SW + TL::PADX + 2 * cp;
+    h_step = 1;
+    h_dst = part + YP + r * PX + cp;
+  } else {
+    const int i = tid - 6 * PX, rp = (i / 6) % (TL::BY / 2), h = i % 6, c = h < R ? h : h + TL::BX;
+    h_src = (2 * rp + R) * SW + c + TL::PADX - R;
+    h_step = SW;
+    h_dst = part + rp * XS + c;
+  }
+  // the last x-face of each row pair (lanes [0, 8)) and the top row of y-faces (lanes [8, 24)): one
+  // warp, another each plane
+  const bool l_x = lane < TL::BY / 2;
+  const int l_st = l_x ? 1 : PX;
+  const int l_src = l_x ? lane * XS + TL::BX : YP + TL::BY * PX + (lane - TL::BY / 2);
 
-  int s_issue = pipe.s_issue, s_wait = pipe.s_wait;
-  unsigned parity = pipe.parity;
-  // z windows per column: f+ at k-2..k+2, f- at k-1..k+3, the f+ of the newest plane held back
-  // one step, u at k-3..k+3 (viscous variant only).
-  T fpw[2][5], fmw[2][5], fpn[2], uw[2][VISC ? 7 : 1];
-
-  const int Q = (ze - zs) + 2 * TL::R;
-  const int p0 = zs - TL::R;
-  const bool edge = per && (x0 - TL::PADX < 0 || x0 + TL::BX + TL::PADX > nx || y0 - TL::R < 0 || y0 + TL::BY + TL::R > ny);
-  // 2D (nz == 1): every streamed plane is the one plane, so the z faces of each column are equal
-  // and their difference is exactly zero; no z layer is frozen.
-  const bool twod = nz == 1;
+  const int Q = (ze - zs) + 2 * lag;
+  const int p0 = zs - lag;
+  const bool edge = per && (x0 - TL::PADX < 0 || x0 + TL::BX + TL::PADX > nx || y0 - R < 0 || y0 + TL::BY + R > ny);
   // Periodic plane index: within one period of the domain (the usual case) a conditional add or
   // subtract, not the integer division of wrapi (5% of the stage at 256^3).
   auto plane_z = [&](int q) {
     int z = p0 + q;
-    if (per || twod) {
+    if (per) {
       if (z < 0) z += nz;
       else if (z >= nz) z -= nz;
       if ((unsigned)z >= (unsigned)nz) z = wrapi(z, nz);
@@ -253,14 +317,24 @@ __device__ __forceinline__ BurgersPipe burgers_segment(const CUtensorMap* tmap, 
   };
   // Periodic edge tile: the TMA box zero-fills what lies outside the domain. The elements to
   // patch with their wrapped neighbours are listed once per segment (CTA-uniform branch), so a
-  // plane's patch is one load and one store per listed element.
+  // plane's patch is one load and one store per listed element. Element copies (cp.async) take every
+  // element's place in its plane from the same list, so a plane's staging has no index arithmetic.
   BurgersPatch* patch = burgers_patch();
-  if (edge) {
-    if (tid == 0) patch->n = 0;
+  if (!tma) {
+    for (int e = tid; e < TL::PLANE; e += TL::NT) {
+      const int r = e / SW, c = e - r * SW;
+      int gx = x0 - TL::PADX + c, gy = y0 - R + r;
+      if (per) { gx = wrapi(gx, nx); gy = wrapi(gy, ny); }
+      const bool ok = gx >= 0 && gx < nx && gy >= 0 && gy < ny;
+      patch->src[e] = ok ? (int64_t)gy * nx + gx : -1;
+    }
+    // each thread reads back only what it wrote: no barrier
+  } else if (edge) {
+    if (tid == 0) patch->n = 0;  // (the previous segment's list was last read before its last barrier)
     __syncthreads();
     for (int e = tid; e < TL::PLANE; e += TL::NT) {
-      const int r = e / TL::SW, c = e - r * TL::SW;
-      const int gx = x0 - TL::PADX + c, gy = y0 - TL::R + r;
+      const int r = e / SW, c = e - r * SW;
+      const int gx = x0 - TL::PADX + c, gy = y0 - R + r;
       if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) {
         const int k = atomicAdd(&patch->n, 1);
         patch->slot[k] = (uint16_t)e;
@@ -269,278 +343,206 @@ __device__ __forceinline__ BurgersPipe burgers_segment(const CUtensorMap* tmap, 
     }
     __syncthreads();
   }
+  auto slot = [&](int q) { return ring + ((n0 + (unsigned)q) % TL::NS) * SM::SLOT_ELEMS; };  // of stream entry q
   auto issue = [&](int q) {
-    T* dst = ring + s_issue * SM::SLOT_ELEMS;
-    const int z = plane_z(q);
-    if (p.tma) {
+    if (tma) {
       if (tid == 0) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        uint64_t* bar = &bars[s_issue];
+        uint64_t* bar = &bars[(n0 + (unsigned)q) % TL::NS];
         mbar_arrive_expect_tx(bar, TL::PLANE * (unsigned)sizeof(T));
-        tma_load_3d(dst, tmap, x0 - TL::PADX, y0 - TL::R, z, bar);
+        tma_load_3d(slot(q), tmap, x0 - TL::PADX, y0 - R, plane_z(q), bar);
       }
     } else {
+      T* dst = slot(q);
+      const int z = plane_z(q);
       const bool zok = z >= 0 && z < nz;
+      const T* plane = p.uin + (zok ? (size_t)z * sxy : 0);
       for (int e = tid; e < TL::PLANE; e += TL::NT) {
-        const int r = e / TL::SW, c = e - r * TL::SW;
-        int gx = x0 - TL::PADX + c, gy = y0 - TL::R + r;
-        if (per) { gx = wrapi(gx, nx); gy = wrapi(gy, ny); }
-        const bool ok = zok && gx >= 0 && gx < nx && gy >= 0 && gy < ny;
-        const T* src = ok ? p.uin + (size_t)z * sxy + (size_t)gy * nx + gx : p.uin;
+        const int64_t o = patch->src[e];
+        const bool ok = zok && o >= 0;
+        const T* src = ok ? plane + o : p.uin;
         cp_async_zfill<sizeof(T)>(dst + e, src, ok && ADV_IN_RANGE(src - p.uin, sxy * nz, p.status));
       }
       cp_async_commit();
     }
-    s_issue = s_issue + 1 == TL::NS ? 0 : s_issue + 1;
+  };
+  auto wait = [&](int q) {
+    const unsigned n = n0 + (unsigned)q;
+    return mbar_wait_bounded(&bars[n % TL::NS], (n / TL::NS) & 1u, p.status);
   };
 
   for (int q = 0; q <= TL::P && q < Q; ++q) issue(q);
-  if (!p.tma)
-    for (int q = Q; q <= TL::P; ++q) cp_async_commit();
+  if (!tma)
+    for (int q = Q; q <= TL::P; ++q) cp_async_commit();  // one group per plane index
 
-  T fz_prev[2] = {T(0), T(0)};
-#pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    fpn[c] = T(0);
-#pragma unroll
-    for (int s = 0; s < 5; ++s) { fpw[c][s] = T(0); fmw[c][s] = T(0); }
-#pragma unroll
-    for (int s = 0; s < (VISC ? 7 : 1); ++s) uw[c][s] = T(0);
-  }
+  typename F::Line line;
+  line.clear();
+  V fz_prev = vc<V>(0), uc = vc<V>(0);  // z-face below the output plane; u of plane q-3
+  V ub = vc<V>(0), ua = vc<V>(0);       // viscous variant: u of planes q-4, q-5
+  size_t gi = (size_t)zs * sxy + (size_t)y * nx + x;  // this thread's nodes of the output plane
+#pragma unroll 1
   for (int q = 0; q < Q; ++q) {
-    T* plq = ring + s_wait * SM::SLOT_ELEMS;
-    const int s_cent = s_wait >= 3 ? s_wait - 3 : s_wait - 3 + TL::NS;  // slot of stream entry q - 3
-    if (p.tma) {
-      if (!mbar_wait_bounded(&bars[s_wait], (parity >> s_wait) & 1u, p.status)) *abort_flag = 1;  // every lane waits (converged)
+    T* plq = slot(q);
+    const T* plc = slot(q - lag);  // the output plane
+    if (tma) {
+      if (!wait(q)) *abort_flag = 1;  // every lane waits (converged)
       if (edge) {
-        // the listed elements of plane q take their wrapped neighbours; written here, read only
-        // after the next barrier
+        // the listed elements of plane q take their wrapped neighbours; outside this thread's own
+        // columns they are read only by the split three planes later (2D: after this barrier)
         const size_t zo = (size_t)plane_z(q) * sxy;
         for (int k = tid; k < patch->n; k += TL::NT) {
-          const size_t gi = zo + (size_t)patch->src[k];
+          const size_t gs = zo + (size_t)patch->src[k];
           const int e = patch->slot[k];
-          if (ADV_IN_RANGE(gi, sxy * nz, p.status) && ADV_IN_RANGE(e, TL::PLANE, p.status)) plq[e] = p.uin[gi];
+          if (ADV_IN_RANGE(gs, sxy * nz, p.status) && ADV_IN_RANGE(e, TL::PLANE, p.status)) plq[e] = p.uin[gs];
         }
+        if (twod) __syncthreads();
       }
     } else {
       cp_async_wait<TL::P>();
+      __syncthreads();  // the other threads' copies of plane q
     }
-    // plane q visible to all threads; abort_flag uniform; and every read of stream entry q - 4
-    // (the centre plane of the previous iteration) is done, so its slot can be refilled
-    __syncthreads();
-    const bool aborted = *abort_flag != 0;
-    parity ^= 1u << s_wait;
-    s_wait = s_wait + 1 == TL::NS ? 0 : s_wait + 1;
-    if (p.tma) {
-      if (aborted) {
-        // A wait expired: let the copies already issued (planes q+1 .. q+P) land before returning.
-        if (tid == 0) {
-          int sl = s_wait;
-          for (int m = q + 1; m < Q && m <= q + TL::P; ++m) {
-            mbar_wait_bounded(&bars[sl], (parity >> sl) & 1u, p.status);
-            sl = sl + 1 == TL::NS ? 0 : sl + 1;
-          }
-        }
-        return BurgersPipe{-1, -1, 0u};
+    const int k = zs + q - 2 * lag;  // output plane (q >= 2 lag)
+    const bool out = q >= 2 * lag;
+    const bool any_upd = out && (per || twod || (k >= FR && k < nz - FR));  // CTA-uniform
+    V visc = vc<V>(0);
+    if (twod) uc = *reinterpret_cast<const V*>(plc + own);
+    if (any_upd) {
+      // f+- of the output plane into shared memory: this thread's cells in both layouts, and the halos
+      V fp, fm;
+      split(uc, fp, fm);
+      yw[0] = fp;
+      yw[PART] = fm;
+      xw[0] = fp.x; xw[2] = fp.y;
+      xw[2 * PART] = fm.x; xw[2 * PART + 2] = fm.y;
+      if (halo) {
+        split(V{plc[h_src], plc[h_src + h_step]}, fp, fm);
+        h_dst[0] = fp;
+        h_dst[PART] = fm;
       }
-      if (q + TL::P + 1 < Q) issue(q + TL::P + 1);  // into the slot of entry q - 4
-    }
-    // ---- z windows: push plane q for this thread's two columns
-    {
-      const T uq[2] = {plq[(cy0 + TL::R) * TL::SW + TL::PADX + cx], plq[(cy1 + TL::R) * TL::SW + TL::PADX + cx]};
-      T fpq[2], fmq[2];
-      if constexpr (sizeof(T) == 4) {
-        const float2 u2 = make_float2(uq[0], uq[1]);
-        const float2 a2 = glob ? f2(alpha) : make_float2(absval(uq[0]), absval(uq[1]));
-        float2 fp2, fm2;
-        Face<T, Z, D>::split2(u2, a2, fp2, fm2);
-        fpq[0] = fp2.x; fpq[1] = fp2.y; fmq[0] = fm2.x; fmq[1] = fm2.y;
-      } else {
-#pragma unroll
-        for (int c = 0; c < 2; ++c) Face<T, Z, D>::split(uq[c], glob ? alpha : absval(uq[c]), fpq[c], fmq[c]);
-      }
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-#pragma unroll
-        for (int s = 0; s < 4; ++s) { fpw[c][s] = fpw[c][s + 1]; fmw[c][s] = fmw[c][s + 1]; }
-        fpw[c][4] = fpn[c];
-        fpn[c] = fpq[c];
-        fmw[c][4] = fmq[c];
-        if (VISC) {
-#pragma unroll
-          for (int s = 0; s < 6; ++s) uw[c][s] = uw[c][s + 1];
-          uw[c][VISC ? 6 : 0] = uq[c];
-        }
-      }
-    }
-    // z-face at (newest plane - 3) + 1/2 once the windows hold planes newest-5 .. newest.
-    T fz_new[2] = {T(0), T(0)};
-    if (q >= 5 && !twod) {  // 2D: both z faces would be equal; their difference stays exactly 0
-      if constexpr (sizeof(T) == 4) {
-        auto pk = [&](const T (&w)[2][5], int s) { return make_float2(w[0][s], w[1][s]); };
-        const float2 fz = Face<T, Z, D>::f2(pk(fpw, 0), pk(fpw, 1), pk(fpw, 2), pk(fpw, 3), pk(fpw, 4), pk(fmw, 0),
-                                            pk(fmw, 1), pk(fmw, 2), pk(fmw, 3), pk(fmw, 4));
-        fz_new[0] = fz.x;
-        fz_new[1] = fz.y;
-      } else {
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-          fz_new[c] = Face<T, Z, D>::f(fpw[c][0], fpw[c][1], fpw[c][2], fpw[c][3], fpw[c][4], fmw[c][0], fmw[c][1],
-                                      fmw[c][2], fmw[c][3], fmw[c][4]);
-      }
-    }
-    if (q >= 6) {
-      const int k = zs + q - 6;  // output plane; its staged copy is stream entry q - 3
-      const T* plc = ring + s_cent * SM::SLOT_ELEMS;
-      const bool kin = per || twod || (k >= F && k < nz - F);
-      const bool any_upd = kin && !aborted;
-      if (any_upd) {
-        // f+- of the output plane into shared memory
-        if constexpr (sizeof(T) == 4) {
-          // elements tid + 256 j, j = 0..3 (880 = 3 * 256 + 112), in pairs (0, 1) and (2, 3)
-          static_assert(TL::PLANE > 3 * TL::NT && TL::PLANE <= 4 * TL::NT, "split pairing assumes 3..4 rounds");
-#pragma unroll
-          for (int j = 0; j < 4; j += 2) {
-            const int e0 = tid + TL::NT * j, e1 = e0 + TL::NT;
-            if (e0 >= TL::PLANE) break;
-            const bool two = e1 < TL::PLANE;
-            const float2 u2 = make_float2(plc[e0], two ? plc[e1] : plc[e0]);
-            const float2 a2 = glob ? f2(alpha) : make_float2(absval(u2.x), absval(u2.y));
-            float2 fp2, fm2;
-            Face<T, Z, D>::split2(u2, a2, fp2, fm2);
-            fpS[e0] = fp2.x;
-            fmS[e0] = fm2.x;
-            if (two) {
-              fpS[e1] = fp2.y;
-              fmS[e1] = fm2.y;
-            }
-          }
-        } else {
-          for (int e = tid; e < TL::PLANE; e += TL::NT) {
-            const T u = plc[e];
-            T fp, fm;
-            Face<T, Z, D>::split(u, glob ? alpha : absval(u), fp, fm);
-            fpS[e] = fp;
-            fmS[e] = fm;
-          }
-        }
-        __syncthreads();
-        // x- and y-faces of the plane, this thread's precomputed share
-        auto face1 = [&](int b, auto stride) {
-          constexpr int st = decltype(stride)::value;
-          return Face<T, Z, D>::f(fpS[b], fpS[b + st], fpS[b + 2 * st], fpS[b + 3 * st], fpS[b + 4 * st],
-                                  fmS[b + st], fmS[b + 2 * st], fmS[b + 3 * st], fmS[b + 4 * st], fmS[b + 5 * st]);
+      if (VISC) {
+        const T* const r0 = plc + own;
+        const V xl = *reinterpret_cast<const V*>(r0 - 2), xh = *reinterpret_cast<const V*>(r0 + 2);
+        const V ym2 = *reinterpret_cast<const V*>(r0 - 2 * SW), ym1 = *reinterpret_cast<const V*>(r0 - SW);
+        const V yp1 = *reinterpret_cast<const V*>(r0 + SW), yp2 = *reinterpret_cast<const V*>(r0 + 2 * SW);
+        auto o4 = [](T m2, T m1, T c, T p1, T p2) {
+          return sub_rn(add_rn(sub_rn(add_rn(-m2, mul_rn(T(16), m1)), mul_rn(T(30), c)), mul_rn(T(16), p1)), p2);
         };
-        using X1 = std::integral_constant<int, 1>;
-        using YS = std::integral_constant<int, TL::SW>;
-        if constexpr (sizeof(T) == 4) {
-          // two faces per paired FP32 instruction: (x tid, x tid + 256), (y tid, y tid + 256)
-          auto face2 = [&](int b0, int b1, auto stride) {
-            constexpr int st = decltype(stride)::value;
-            auto P = [&](int k) { return make_float2(fpS[b0 + k * st], fpS[b1 + k * st]); };
-            auto M = [&](int k) { return make_float2(fmS[b0 + k * st], fmS[b1 + k * st]); };
-            return Face<T, Z, D>::f2(P(0), P(1), P(2), P(3), P(4), M(1), M(2), M(3), M(4), M(5));
-          };
-          const float2 fx = face2(fbx0, fbx1, X1{});
-          fxS[tid] = fx.x;
-          fxS[tid + TL::NT] = fx.y;
-          const float2 fy = face2(fby0, fby1, YS{});
-          fxS[TL::NXF + tid] = fy.x;
-          fxS[TL::NXF + tid + TL::NT] = fy.y;
-        } else {
-          fxS[tid] = face1(fbx0, X1{});
-          fxS[tid + TL::NT] = face1(fbx1, X1{});
-          fxS[TL::NXF + tid] = face1(fby0, YS{});
-          fxS[TL::NXF + tid + TL::NT] = face1(fby1, YS{});
+        V vz = vc<V>(0);
+        if (!twod) {
+          const V up1 = *reinterpret_cast<const V*>(slot(q - 2) + own), up2 = *reinterpret_cast<const V*>(slot(q - 1) + own);
+          vz.x = o4(ua.x, ub.x, uc.x, up1.x, up2.x);
+          vz.y = o4(ua.y, ub.y, uc.y, up1.y, up2.y);
         }
-        if (left_x) fxS[2 * TL::NT + tid] = face1(fbl, X1{});
-        else if (left_y) fxS[TL::NXF + 2 * TL::NT + (tid - 32)] = face1(fbl, YS{});
-        __syncthreads();
+        visc.x = add_rn(add_rn(mul_rn(p.kx, o4(xl.x, xl.y, uc.x, uc.y, xh.x)),
+                               mul_rn(p.ky, o4(ym2.x, ym1.x, uc.x, yp1.x, yp2.x))), mul_rn(p.kz, vz.x));
+        visc.y = add_rn(add_rn(mul_rn(p.kx, o4(xl.y, uc.x, uc.y, xh.x, xh.y)),
+                               mul_rn(p.ky, o4(ym2.y, ym1.y, uc.y, yp1.y, yp2.y))), mul_rn(p.kz, vz.y));
       }
-      // ---- RHS, stage combine, store, max|u_out|
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int cy = c ? cy1 : cy0;
-        const int x = x0 + cx, y = y0 + cy;
-        const T uo = VISC ? uw[c][VISC ? 3 : 0] : plc[(cy + TL::R) * TL::SW + TL::PADX + cx];
-        T res = uo;
-        const bool inside = x < nx && y < ny;  // partial tiles extend past the domain
-        const bool upd = any_upd && inside && (per || (x >= F && x < nx - F && y >= F && y < ny - F));
-        if (upd) {
-          const T fxp = fxS[cy * (TL::BX + 1) + cx + 1], fxm = fxS[cy * (TL::BX + 1) + cx];
-          const T fyp = fxS[TL::NXF + (cy + 1) * TL::BX + cx], fym = fxS[TL::NXF + cy * TL::BX + cx];
-          T L;
-          if (EXACT) {
-            L = div_rn(-sub_rn(fxp, fxm), T(p.dx));
-            L = sub_rn(L, div_rn(sub_rn(fyp, fym), T(p.dy)));
-            L = sub_rn(L, div_rn(sub_rn(fz_new[c], fz_prev[c]), T(p.dz)));
+    }
+    // ---- the z-face between planes q-3 and q-2, once the line holds planes q-5 .. q
+    V fz = vc<V>(0), u2 = uc;
+    if (!twod) {
+      const V uq = *reinterpret_cast<const V*>(plq + own);
+      u2 = *reinterpret_cast<const V*>(slot(q - 2) + own);  // (before plane 2: a stale slot, not used)
+      V fp, fm;
+      split(uq, fp, fm);
+      fz = line.push(fp, fm, uc, u2, q >= 2 * R - 1);
+    }
+    __syncthreads();  // f+- in place; every read of the output plane's slot is done
+    if (tma && *abort_flag != 0) {
+      // A wait expired: let the copies already issued (planes q+1 .. q+P) land before returning.
+      if (tid == 0)
+        for (int m = q + 1; m < Q && m <= q + TL::P; ++m) wait(m);
+      return kPipeAborted;
+    }
+    if (q + TL::P + 1 < Q) issue(q + TL::P + 1);
+    else if (!tma) cp_async_commit();
+    if (out) {
+      V un = uc, res = uc;
+      if (any_upd) {
+        if (!p.un_is_uin) {  // requested before the faces, used after them
+          if (vec) {
+            if (ADV_IN_RANGE(gi + 1, sxy * nz, p.status)) un = *reinterpret_cast<const V*>(p.un + gi);
           } else {
-            L = -(fxp - fxm) * rdx - (fyp - fym) * rdy - (fz_new[c] - fz_prev[c]) * rdz;
+            if (in0 && ADV_IN_RANGE(gi, sxy * nz, p.status)) un.x = p.un[gi];
+            if (in1 && ADV_IN_RANGE(gi + 1, sxy * nz, p.status)) un.y = p.un[gi + 1];
           }
-          if (VISC) {
-            const T* row = plc + (cy + TL::R) * TL::SW + TL::PADX + cx;
-            constexpr int W = TL::SW;
-            const T vx = sub_rn(add_rn(sub_rn(add_rn(-row[-2], mul_rn(T(16), row[-1])), mul_rn(T(30), uo)),
-                                       mul_rn(T(16), row[1])), row[2]);
-            const T vy = sub_rn(add_rn(sub_rn(add_rn(-row[-2 * W], mul_rn(T(16), row[-W])), mul_rn(T(30), uo)),
-                                       mul_rn(T(16), row[W])), row[2 * W]);
-            constexpr int Z1 = VISC ? 1 : 0, Z2 = VISC ? 2 : 0, Z4 = VISC ? 4 : 0, Z5 = VISC ? 5 : 0;
-            const T vz = sub_rn(add_rn(sub_rn(add_rn(-uw[c][Z1], mul_rn(T(16), uw[c][Z2])), mul_rn(T(30), uo)),
-                                       mul_rn(T(16), uw[c][Z4])), uw[c][Z5]);
-            const T v = add_rn(add_rn(mul_rn(p.kx, vx), mul_rn(p.ky, vy)), mul_rn(p.kz, vz));
-            L = add_rn(L, v);
-            // The reference's first viscous z-block starts at slab 3 yet runs 16 slabs, adding
-            // slabs 16..18 twice (kernels.cu:464-491); reproduced only on request.
-            if (p.bug_b2 && !per && k >= 16 && k <= 18 && k <= nz - 3) L = add_rn(L, v);
-          }
-          T un;
-          if (p.un_is_uin) un = uo;
-          else {
-            const size_t gi = (size_t)k * sxy + (size_t)y * nx + x;
-            un = ADV_IN_RANGE(gi, sxy * nz, p.status) ? p.un[gi] : T(0);
-          }
-          res = stage_combine<T>(p.stage, un, uo, dt, L);
         }
-        if (inside) {
-          if (ADV_IN_RANGE((size_t)k * sxy + (size_t)y * nx + x, sxy * nz, p.status))
-            p.out[(size_t)k * sxy + (size_t)y * nx + x] = res;
-          const K kk = abs_key(res);
-          kmax = kk > kmax ? kk : kmax;
+        auto face = [](const V* a, int st) {
+          const V* const m = a + PART;
+          return F::f(a[0], a[st], a[2 * st], a[3 * st], a[4 * st], m[st], m[2 * st], m[3 * st], m[4 * st], m[5 * st]);
+        };
+        const V fx = face(xr, 1);
+        fxS[(2 * warp) * TL::XF + lane] = fx.x;
+        fxS[(2 * warp + 1) * TL::XF + lane] = fx.y;
+        const V fym = face(yr, PX);
+        fyS[tid] = fym;
+        if (warp == (q & 7) && lane < TL::BY / 2 + PX) {
+          const V f = face(part + l_src, l_st);
+          if (l_x) {
+            fxS[(2 * lane) * TL::XF + TL::BX] = f.x;
+            fxS[(2 * lane + 1) * TL::XF + TL::BX] = f.y;
+          } else {
+            fyS[TL::BY * PX + lane - TL::BY / 2] = f;
+          }
         }
+        __syncthreads();
+        // ---- RHS, stage combine
+        const V fx0 = *reinterpret_cast<const V*>(fxS + row * TL::XF + 2 * cp);  // faces 2 cp, 2 cp + 1
+        const V fx1 = {fx0.y, fxS[row * TL::XF + 2 * cp + 2]};
+        const V fyp = fyS[tid + PX];
+        V L;
+        if constexpr (EXACT) {
+          auto rhs = [&](T fxm, T fxp, T fym1, T fyp1, T fzm, T fzp) {
+            return sub_rn(sub_rn(div_rn(-sub_rn(fxp, fxm), p.dx), div_rn(sub_rn(fyp1, fym1), p.dy)),
+                          div_rn(sub_rn(fzp, fzm), p.dz));
+          };
+          L = {rhs(fx0.x, fx1.x, fym.x, fyp.x, fz_prev.x, fz.x), rhs(fx0.y, fx1.y, fym.y, fyp.y, fz_prev.y, fz.y)};
+        } else {
+          L = vfma(vsub(fz_prev, fz), V{p.rdz, p.rdz},
+                   vfma(vsub(fym, fyp), V{p.rdy, p.rdy}, vmul(vsub(fx0, fx1), V{p.rdx, p.rdx})));
+        }
+        if (VISC) {
+          L = vadd(L, visc);
+          // The reference's first viscous z-block starts at slab 3 yet runs 16 slabs, adding
+          // slabs 16..18 twice (kernels.cu:464-491); reproduced only on request.
+          if (p.bug_b2 && !per && k >= 16 && k <= 18 && k <= nz - 3) L = vadd(L, visc);
+        }
+        const V c = combine2(p.stage, un, uc, dt, L);
+        if (upd0) res.x = c.x;
+        if (upd1) res.y = c.y;
       }
+      if (vec) {
+        if (ADV_IN_RANGE(gi + 1, sxy * nz, p.status)) *reinterpret_cast<V*>(p.out + gi) = res;
+      } else {
+        if (in0 && ADV_IN_RANGE(gi, sxy * nz, p.status)) p.out[gi] = res.x;
+        if (in1 && ADV_IN_RANGE(gi + 1, sxy * nz, p.status)) p.out[gi + 1] = res.y;
+      }
+      const K k0 = in0 ? abs_key(res.x) : K(0), k1 = in1 ? abs_key(res.y) : K(0);
+      kmax = k0 > kmax ? k0 : kmax;
+      kmax = k1 > kmax ? k1 : kmax;
+      gi += sxy;
     }
-    if (q >= 5) {
-      fz_prev[0] = fz_new[0];
-      fz_prev[1] = fz_new[1];
-    }
-    if (!p.tma) {
-      // cp.async: one commit group per plane index; the refill of entry q - 3's slot waits here
-      __syncthreads();  // stream entry q - 3 fully consumed
-      if (aborted) return BurgersPipe{-1, -1, 0u};
-      if (q + TL::P + 1 < Q) issue(q + TL::P + 1);
-      else cp_async_commit();
-    }
+    fz_prev = fz;
+    if (VISC) { ua = ub; ub = uc; }
+    uc = u2;
   }
   if (p.maxabs_key) {
     kmax = warp_max(kmax);
     if (lane == 0 && kmax) atomicMax(static_cast<K*>(p.maxabs_key), kmax);
   }
-  return BurgersPipe{s_issue, s_wait, parity};
+  return n0 + (unsigned)Q;
 }
 
-// Minimum resident CTAs per SM the compiler must allow for (it caps registers accordingly).
-// FP32 inviscid with the IEEE or FP64 weight division: asking for 2 lets the compiler pick its
-// own schedule, which lands at 78-80 registers -- still three CTAs (24 warps) per SM -- and
-// measured 3-4% faster than the schedule it picks under a 3-CTA bound (76 registers); the grid
-// follows the occupancy it reports. FP32 with the reciprocal division and FP32 viscous: 3 (under
-// a 2-CTA bound they take 86-90 registers and only two CTAs fit). FP64: 2.
-template <class T, bool VISC, class D>
+// Minimum resident CTAs per SM the compiler must allow for (it caps registers accordingly): three for
+// FP32 (80 registers; without the bound it takes 108 and two CTAs fit), two for FP64.
+template <class T>
 constexpr int burgers_min_ctas() {
-  return sizeof(T) == 4 && (VISC || std::is_same<D, FastDiv>::value) ? 3 : 2;
+  return sizeof(T) == 4 ? 3 : 2;
 }
 
-template <class T, bool Z, class D, bool VISC>
-__global__ void __launch_bounds__(256, burgers_min_ctas<T, VISC, D>())
+template <class T, bool Z, class D, bool VISC, int MODE>
+__global__ void __launch_bounds__(256, burgers_min_ctas<T>())
 burgers_stage_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ BurgersParams<T> p) {
   using TL = BurgersTile;
   if (p.active && *p.active == 0) return;
@@ -550,15 +552,15 @@ burgers_stage_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_cons
   const int64_t total = (int64_t)p.tiles_x * p.tiles_y * nz;
   const int64_t seg_a = total * blockIdx.x / gridDim.x, seg_b = total * (blockIdx.x + 1) / gridDim.x;
   burgers_cta_init<T>(&tmap, p.tma != 0);
-  BurgersPipe pipe{0, 0, 0u};
+  unsigned entries = 0;
   for (int64_t pos = seg_a; pos < seg_b;) {
     const int64_t tile = pos / nz;
     const int zs = (int)(pos - tile * nz);
     const int ze = (int)min((int64_t)nz, zs + (seg_b - pos));
     pos += ze - zs;
     const int x0 = (int)(tile % p.tiles_x) * TL::BX, y0 = (int)(tile / p.tiles_x) * TL::BY;
-    pipe = burgers_segment<T, Z, D, VISC>(&tmap, p, x0, y0, zs, ze, pipe);
-    if (pipe.s_issue < 0) return;
+    entries = burgers_segment<T, Z, D, VISC, MODE>(&tmap, p, x0, y0, zs, ze, entries);
+    if (entries == kPipeAborted) return;
   }
 }
 
@@ -575,14 +577,13 @@ struct alignas(64) BurgersBatchInst {
 // Batched stage over many instances: the units (instance, tile, z-plane) of all instances,
 // instance-major then tile-major, are cut into gridDim.x equal contiguous ranges. Instances
 // whose active flag is 0 are skipped (the choice is per segment, so uniform over the CTA).
-// (The batched kernel keeps three CTAs for FP32: under a 2-CTA bound it takes 120 registers.)
-template <class T, bool Z, class D, bool VISC>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2)
+template <class T, bool Z, class D, bool VISC, int MODE>
+__global__ void __launch_bounds__(256, burgers_min_ctas<T>())
 burgers_batch_kernel(const BurgersBatchInst<T>* __restrict__ inst, int n_inst, int64_t total_units, int tma) {
   using TL = BurgersTile;
   const int64_t seg_a = total_units * blockIdx.x / gridDim.x, seg_b = total_units * (blockIdx.x + 1) / gridDim.x;
   burgers_cta_init<T>(nullptr, tma != 0);
-  BurgersPipe pipe{0, 0, 0u};
+  unsigned entries = 0;
   int i = 0;
   {
     int lo = 0, hi = n_inst - 1;
@@ -613,8 +614,8 @@ burgers_batch_kernel(const BurgersBatchInst<T>* __restrict__ inst, int n_inst, i
     const int x0 = (int)(tile % p.tiles_x) * TL::BX, y0 = (int)(tile / p.tiles_x) * TL::BY;
     const CUtensorMap* tm = &inst[i].tmap;
     if (tma && threadIdx.x == 0) tma_prefetch_desc(tm);
-    pipe = burgers_segment<T, Z, D, VISC>(tm, p, x0, y0, zs, ze, pipe);
-    if (pipe.s_issue < 0) return;
+    entries = burgers_segment<T, Z, D, VISC, MODE>(tm, p, x0, y0, zs, ze, entries);
+    if (entries == kPipeAborted) return;
   }
 }
 

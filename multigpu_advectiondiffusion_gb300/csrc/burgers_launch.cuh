@@ -7,7 +7,25 @@
 namespace adv {
 
 template <class T>
-void* burgers_kernel_for(const adv_burgers_desc& d);
+void* burgers_kernel_for(const adv_burgers_desc& d, int mode);
+
+// The kernel of a scheme and mode among all instantiations of K<Z, D, VISC, MODE>. FP32 divides alike
+// for ADV_DIV_F32 and ADV_DIV_F64 (an FP64 quotient rounded to FP32 is the correctly rounded one).
+#define ADV_BURGERS_PICK(d, mode, D, K)                                                                        \
+  do {                                                                                                         \
+    const bool z_ = (d).weno == ADV_WENO5_Z, fast_ = (d).div == ADV_DIV_FAST;                                  \
+    const bool visc_ = (d).kx != 0.0 || (d).ky != 0.0 || (d).kz != 0.0;                                        \
+    ADV_BURGERS_PICK_MODE(BURGERS_3D_TMA, mode, D, K)                                                          \
+    ADV_BURGERS_PICK_MODE(BURGERS_3D_COPY, mode, D, K)                                                         \
+    ADV_BURGERS_PICK_MODE(BURGERS_ANY, mode, D, K)                                                             \
+  } while (0)
+#define ADV_BURGERS_PICK_MODE(M, mode, D, K)                                                                   \
+  if ((mode) == M) {                                                                                           \
+    if (z_) return fast_ ? (visc_ ? K(true, FastDiv, true, M) : K(true, FastDiv, false, M))                    \
+                         : (visc_ ? K(true, D, true, M) : K(true, D, false, M));                               \
+    return fast_ ? (visc_ ? K(false, FastDiv, true, M) : K(false, FastDiv, false, M))                          \
+                 : (visc_ ? K(false, D, true, M) : K(false, D, false, M));                                     \
+  }
 
 // Stage parameters of one launch (or of one instance of a batched launch).
 template <class T>
@@ -24,8 +42,11 @@ BurgersParams<T> burgers_params(const adv_burgers_desc& d, const BurgersLaunch& 
   p.tiles_y = L.tiles_y;
   p.tma = L.tma ? 1 : 0;
   p.un_is_uin = a.u_n == a.u_in ? 1 : 0;
+  const uintptr_t pair = 2 * sizeof(T);
+  p.vec_ok = d.nx % 2 == 0 && (uintptr_t)a.u_n % pair == 0 && (uintptr_t)a.u_out % pair == 0 ? 1 : 0;
   p.lf_global = d.lf == ADV_LF_GLOBAL ? 1 : 0;
-  p.dx = d.dx; p.dy = d.dy; p.dz = d.dz;
+  p.dx = (T)d.dx; p.dy = (T)d.dy; p.dz = (T)d.dz;
+  p.rdx = (T)(1.0 / d.dx); p.rdy = (T)(1.0 / d.dy); p.rdz = (T)(1.0 / d.dz);
   p.kx = (T)d.kx; p.ky = (T)d.ky; p.kz = (T)d.kz;
   p.dt_host = a.dt_host;
   p.alpha_host = a.alpha_host;
@@ -42,7 +63,7 @@ template <class T>
 adv_status burgers_launch_t(const adv_burgers_desc& d, const BurgersLaunch& L, const BurgersStageArgs& a,
                             cudaStream_t s) {
   BurgersParams<T> p = burgers_params<T>(d, L, a);
-  void* k = burgers_kernel_for<T>(d);
+  void* k = burgers_kernel_for<T>(d, L.mode);
   if (!k) return set_error(ADV_ERR_UNSUPPORTED, "burgers: no kernel for this configuration");
   void* args[] = {const_cast<CUtensorMap*>(&L.tmap_in), &p};
   ADV_CUDA_TRY(cudaLaunchKernel(k, L.grid, L.block, args, L.smem, s));

@@ -3,7 +3,7 @@
 //
 // Each member contributes its (tile, z-plane) units to one flat range per kind; a batched stage
 // launch cuts that range into equal contiguous shares, one per CTA (two waves of CTAs for heat,
-// eight for Burgers), so small members neither leave SMs idle nor pay a launch each
+// one for Burgers), so small members neither leave SMs idle nor pay a launch each
 // (heat_batch_kernel, burgers_batch_kernel). The
 // device tables hold, per member and per stage slot, the stage parameters and the tensor map of
 // the stage input. A run is one graph with two while-nodes that run concurrently: the heat loop
@@ -23,7 +23,7 @@ namespace adv {
 void* heat_batch_kernel_for(int dtype, int order, bool tma, int stage_kind, int rows, int lanes);
 void* heat_batch_mixed_kernel_for(int stage_kind);
 template <class T>
-void* burgers_batch_kernel_for(const adv_burgers_desc& d);
+void* burgers_batch_kernel_for(const adv_burgers_desc& d, int mode);
 size_t burgers_smem_f32();
 size_t burgers_smem_f64();
 }  // namespace adv
@@ -415,17 +415,18 @@ adv_status create_impl(const adv_heat_member* heat, int n_heat, int scheme, cons
     if (st != ADV_OK) return st;
     for (int s = 0; s < 3; ++s)
       ADV_CUDA_TRY(cudaMemcpy(e->burg_tab[s], bytes[s].data(), bytes[s].size(), cudaMemcpyHostToDevice));
-    e->burg_k = e->burg_dtype == ADV_F32 ? burgers_batch_kernel_for<float>(burgers[0].desc)
-                                         : burgers_batch_kernel_for<double>(burgers[0].desc);
+    int mode = e->burg_tma ? BURGERS_3D_TMA : BURGERS_3D_COPY;
+    for (int i = 0; i < n_burgers; ++i)
+      if (burgers[i].desc.nz == 1) mode = BURGERS_ANY;
+    e->burg_k = e->burg_dtype == ADV_F32 ? burgers_batch_kernel_for<float>(burgers[0].desc, mode)
+                                         : burgers_batch_kernel_for<double>(burgers[0].desc, mode);
     if (!e->burg_k) return set_error(ADV_ERR_UNSUPPORTED, "ensemble: no batched Burgers kernel");
     e->burg_smem = e->burg_dtype == ADV_F32 ? burgers_smem_f32() : burgers_smem_f64();
     ADV_CUDA_TRY(cudaFuncSetAttribute(e->burg_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->burg_smem));
+    // one wave of equal shares (16 heat + 8 Burgers members, 20 steps: 17.97 ms with one wave, 18.65 with
+    // two, 18.85 with four, 20.82 with eight)
     e->burg_ctas = one_wave_ctas(e->burg_k, 256, e->burg_smem, e->sms, e->burg_units, &st);
     if (st != ADV_OK) return st;
-    // eight waves of equal shares: the batched WENO stage's per-pair cost varies across members
-    // and segments, and later waves balance it (measured on the 32-member Burgers batch: 198 ms
-    // per 30 steps with one wave, 177 with four, 169 with eight, 170 with sixteen)
-    e->burg_ctas = (int)std::max<int64_t>(1, std::min<int64_t>(8 * (int64_t)e->burg_ctas, e->burg_units / 4));
     e->h_states.resize((size_t)n_burgers);
   }
   return ADV_OK;

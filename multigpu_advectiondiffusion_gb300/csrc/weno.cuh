@@ -8,23 +8,19 @@
 // Two forms:
 //  * weno_face_ref<double>: the reference's own expression, operand for operand, with
 //    correctly rounded intrinsics -> equal to the FP64 oracle bit for bit.
-//  * weno_side_fast<D>: the same weights with the common denominator b0*b1*b2 (WENO5-Z) or
-//    (b0*b1*b2)^2 (WENO5-JS) multiplied through, leaving ONE division per side instead of four;
-//    D selects that division: float (IEEE), double (FP64) or FastDiv (reciprocal based,
-//    at most 2 ulp). Used for the FP32 state.
+//  * weno_face2 / WenoLine: the same weights with the common denominator b0*b1*b2 (WENO5-Z) or
+//    (b0*b1*b2)^2 (WENO5-JS) multiplied through, leaving ONE division per side instead of four,
+//    and everything expressed in the cells' first and second differences, on two faces at once.
+//    Used for the FP32 state and for an FP64 state with ADV_DIV_FAST.
 #pragma once
+#include <type_traits>
+
 #include "adv_math.cuh"
 
 namespace adv {
 
 // Lax-Friedrichs split of f(u) = u^2/2 (kernels.cu:224-238): f+- = (f +- a u)/2.
 // lf_split: the reference's operand order, correctly rounded (FP64 path, reference operators).
-// lf_split_fast: u * (u/4 +- a/2), the FP32 path.
-__device__ __forceinline__ void lf_split_fast(float u, float a, float& fp, float& fm) {
-  const float hu = 0.25f * u, ha = 0.5f * a;
-  fp = u * (hu + ha);
-  fm = u * (hu - ha);
-}
 template <class T>
 __device__ __forceinline__ void lf_split(T u, T a, T& fp, T& fm) {
   const T f = mul_rn(mul_rn(T(0.5), u), u);
@@ -33,159 +29,157 @@ __device__ __forceinline__ void lf_split(T u, T a, T& fp, T& fm) {
   fm = mul_rn(T(0.5), sub_rn(f, au));
 }
 
-// ---------------------------------------------------------------- fast FP32 form
-struct FastDiv {};  // division tag: __fdividef (reciprocal approximation, <= 2 ulp)
+// ------------------------------------------------------------------ two values at once
+// A pair of values: float2 operations are Blackwell's paired FP32 instructions (FFMA2 / FADD2 /
+// FMUL2: one instruction, each lane rounded like the scalar operation), double2 operations two
+// scalar ones. Every operation is explicit, so the single-grid and the batched kernels round alike.
+template <class T> struct Vec2;
+template <> struct Vec2<float> { using type = float2; };
+template <> struct Vec2<double> { using type = double2; };
+
+__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 vsub(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 a, b, r;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tsub.rn.f32x2 r, a, b;\n\tmov.b64 {%0, %1}, r;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 vabs(float2 a) { return make_float2(fabsf(a.x), fabsf(a.y)); }
+__device__ __forceinline__ double2 vadd(double2 a, double2 b) { return make_double2(__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y)); }
+__device__ __forceinline__ double2 vsub(double2 a, double2 b) { return make_double2(__dsub_rn(a.x, b.x), __dsub_rn(a.y, b.y)); }
+__device__ __forceinline__ double2 vmul(double2 a, double2 b) { return make_double2(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y)); }
+__device__ __forceinline__ double2 vfma(double2 a, double2 b, double2 c) {
+  return make_double2(__fma_rn(a.x, b.x, c.x), __fma_rn(a.y, b.y, c.y));
+}
+__device__ __forceinline__ double2 vabs(double2 a) { return make_double2(fabs(a.x), fabs(a.y)); }
+template <class V> __device__ __forceinline__ V vc(double v);  // a constant in both lanes
+template <> __device__ __forceinline__ float2 vc<float2>(double v) { return make_float2((float)v, (float)v); }
+template <> __device__ __forceinline__ double2 vc<double2>(double v) { return make_double2(v, v); }
+
+// f+- = u (u/4 +- a/2).
+template <class V>
+__device__ __forceinline__ void lf_split2(V u, V a, V& fp, V& fm) {
+  const V hu = vmul(vc<V>(0.25), u), ha = vmul(vc<V>(0.5), a);
+  fp = vmul(u, vadd(hu, ha));
+  fm = vmul(u, vsub(hu, ha));
+}
+
+struct FastDiv {};  // division tag: reciprocal approximation, <= 2 ulp (FP32 state)
+
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+// Negated quotient -num / den of the weight sums (den > 0 and far from the subnormals: at least
+// (4e-6)^3). FP32: FastDiv multiplies by the reciprocal approximation; otherwise one Newton step on
+// the reciprocal and one residual correction of the quotient in fused multiply-adds (Markstein,
+// IBM J. Res. Dev. 34 (1990) 111-119), which returns the correctly rounded quotient -- what an
+// FP64 division rounded to FP32 also returns, so both division kinds of an FP32 state share it.
+// Compiled IEEE divisions took about 10 issue slots per quotient, six quotients per cell; this
+// takes 3.5 in paired instructions. (Negated: the reciprocal of -den makes both corrections plain
+// multiply-adds.)
 template <class D>
-__device__ __forceinline__ float side_div(float num, float den) { return (float)((D)num / (D)den); }
-template <>
-__device__ __forceinline__ float side_div<FastDiv>(float num, float den) { return __fdividef(num, den); }
+__device__ __forceinline__ float2 vnquot(float2 num, float2 den) {
+  const float2 r0 = make_float2(rcp_approx(-den.x), rcp_approx(-den.y));
+  if constexpr (std::is_same<D, FastDiv>::value) return vmul(num, r0);
+  const float2 r = vfma(vfma(den, r0, vc<float2>(1)), r0, r0);
+  const float2 q = vmul(num, r);
+  return vfma(vfma(den, q, num), r, q);
+}
+template <class D>
+__device__ __forceinline__ double2 vnquot(double2 num, double2 den) {
+  return make_double2(-num.x / den.x, -num.y / den.y);
+}
 
-// Left-biased side of one face from a..e = f at i-2..i+2. With the second differences
-// t0 = a-2b+c, t1 = b-2c+d, t2 = c-2d+e and first differences s0 = a-4b+3c, s1 = b-d,
-// s2 = 3c-4d+e, the reference's quantities are
-//   beta_k = 13/12 t_k^2 + 1/4 s_k^2,   q_k/6 = c + t_k/12 + s0/4 | - s1/4 | - s2/4
-// (q_0 = 2a-7b+11c, q_1 = -b+5c+2d, q_2 = 2c+5d-e). The kernel uses 4 beta_k and 4 eps (the
-// factor cancels in the normalised weights), linear weights times 10 (1, 6, 3), and the
-// weighted mean of q_k/6, so each side costs one division and no separate scaling.
-template <bool Z, class D>
-__device__ __forceinline__ float weno_side_fast(float a, float b, float c, float d, float e) {
-  const float t0 = fmaf(-2.f, b, a) + c, t1 = fmaf(-2.f, c, b) + d, t2 = fmaf(-2.f, d, c) + e;
-  const float s0 = fmaf(3.f, c, fmaf(-4.f, b, a)), s1 = b - d, s2 = fmaf(3.f, c, fmaf(-4.f, d, e));
-  const float k = 13.f / 3.f;
-  const float b0 = fmaf(k * t0, t0, fmaf(s0, s0, 4e-6f));  // 4 (beta_k + eps)
-  const float b1 = fmaf(k * t1, t1, fmaf(s1, s1, 4e-6f));
-  const float b2 = fmaf(k * t2, t2, fmaf(s2, s2, 4e-6f));
-  const float r12 = 1.f / 12.f;
-  const float q0 = fmaf(0.25f, s0, fmaf(r12, t0, c));
-  const float q1 = fmaf(-0.25f, s1, fmaf(r12, t1, c));
-  const float q2 = fmaf(-0.25f, s2, fmaf(r12, t2, c));
-  float w0, w1, w2;
+// One side of a face. With f at i-2..i+2 called a..e, first differences A = b-a .. Dd = e-d and
+// second differences t0 = B-A, t1 = C-B, t2 = Dd-C, the reference's quantities are
+//   4 beta_k = 13/3 t_k^2 + s_k^2,  s0 = t0 + 2B, s1 = B + C, s2 = t2 - 2C
+//   q_k/6 = c + C/2 + { t0/3 - t1/2 | -t1/6 | -t2/6 }
+// so the weighted mean of the q_k/6 is
+//   c + C/2 - t1/6 - 1/2 [ (2/3) w0 (t1-t0) + 3 w2' (t2-t1)/3 ] / (w0 + w1 + w2),  w2 = 3 w2'
+// A constant part and one quotient. b0..b2 are 4 (beta_k + eps); the weights are taken times 10 and
+// times the common denominator. Against the form that weighs the three q_k this needs a quarter
+// fewer operations, and its quotient only corrects the (exact in the mean) linear part, so the FP32
+// rounding error of a face falls (rms 6.2e-8 -> 4.3e-8 on smooth data, 6.4e-8 -> 4.8e-8 on noise).
+// Returns the negated quotient -[..]; d_a = t1-t0, d_b = t2-t1 (both negated give the quotient).
+template <bool Z, class D, class V>
+__device__ __forceinline__ V weno_nl(V b0, V b1, V b2, V d_a, V d_b) {
+  const V p12 = vmul(b1, b2);
+  V e0, e1, e2;
   if (Z) {  // alpha_k = d_k (1 + tau/b_k), times 10 b0 b1 b2: d_k (P + tau P/b_k), P = b0 b1 b2
-    const float tau = fabsf(b0 - b2);
-    const float p12 = b1 * b2, P = b0 * p12;
-    w0 = fmaf(tau, p12, P);
-    w1 = 6.f * fmaf(tau, b0 * b2, P);
-    w2 = 3.f * fmaf(tau, b0 * b1, P);
+    const V tau = vabs(vsub(b0, b2)), P = vmul(b0, p12);
+    e0 = vfma(tau, p12, P);
+    e1 = vfma(tau, vmul(b0, b2), P);
+    e2 = vfma(tau, vmul(b0, b1), P);
   } else {  // alpha_k = d_k / b_k^2, times 10 (b0 b1 b2)^2
-    const float p12 = b1 * b2, p02 = b0 * b2, p01 = b0 * b1;
-    w0 = p12 * p12;
-    w1 = (6.f * p02) * p02;
-    w2 = (3.f * p01) * p01;
+    const V p02 = vmul(b0, b2), p01 = vmul(b0, b1);
+    e0 = vmul(p12, p12);
+    e1 = vmul(p02, p02);
+    e2 = vmul(p01, p01);
   }
-  const float num = fmaf(w2, q2, fmaf(w1, q1, w0 * q0));
-  const float den = w0 + w1 + w2;
-  return side_div<D>(num, den);
+  const V den = vfma(vc<V>(3), e2, vfma(vc<V>(6), e1, e0));
+  const V num = vfma(e2, d_b, vmul(vc<V>(2.0 / 3.0), vmul(e0, d_a)));
+  return vnquot<D>(num, den);
 }
 
-// f+ at i-2..i+2 (p0..p4) and f- at i-1..i+3 (m0..m4).
-template <bool Z, class D>
-__device__ __forceinline__ float weno_face_fast(float p0, float p1, float p2, float p3, float p4, float m0, float m1,
-                                                float m2, float m3, float m4) {
-  return weno_side_fast<Z, D>(p0, p1, p2, p3, p4) + weno_side_fast<Z, D>(m4, m3, m2, m1, m0);
+// 4 (beta + eps) from the second difference's share T = 13/3 t^2 + 4 eps and s.
+template <class V>
+__device__ __forceinline__ V weno_T(V t) {
+  return vfma(vmul(vc<V>(13.0 / 3.0), t), t, vc<V>(4e-6));
 }
 
-// ------------------------------------------------------- packed FP32 (two faces at once)
-// The same operations as weno_side_fast / weno_face_fast / lf_split_fast on two independent
-// inputs, issued as Blackwell's paired FP32 instructions (FFMA2 / FADD2 / FMUL2, one
-// instruction for both lanes, each lane rounded exactly as the scalar form): the results are the
-// scalar results bit for bit at half the FP32 instruction count. a - b is issued as
-// fma(b, -1, a), which rounds the exact difference once, like a subtraction.
-__device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-
-__device__ __forceinline__ void lf_split_fast2(float2 u, float2 a, float2& fp, float2& fm) {
-  const float2 hu = mul2(f2(0.25f), u), ha = mul2(f2(0.5f), a);
-  fp = mul2(u, add2(hu, ha));
-  fm = mul2(u, sub2(hu, ha));
+// Side from a..e: lin = c (the caller adds C/2 and t1/6 of both sides together), C, t1, quotient.
+template <bool Z, class D, class V>
+__device__ __forceinline__ V weno_side2(V a, V b, V c, V d, V e, V& C, V& t1) {
+  const V A = vsub(b, a), B = vsub(c, b), E = vsub(e, d);
+  C = vsub(d, c);
+  const V t0 = vsub(B, A), t2 = vsub(E, C);
+  t1 = vsub(C, B);
+  const V two = vc<V>(2);
+  const V s0 = vfma(two, B, t0), s1 = vadd(B, C), s2 = vfma(vc<V>(-2), C, t2);
+  return weno_nl<Z, D>(vfma(s0, s0, weno_T(t0)), vfma(s1, s1, weno_T(t1)), vfma(s2, s2, weno_T(t2)), vsub(t1, t0),
+                       vsub(t2, t1));
 }
 
-template <bool Z, class D>
-__device__ __forceinline__ float2 weno_side_fast2(float2 a, float2 b, float2 c, float2 d, float2 e) {
-  const float2 t0 = add2(fma2(f2(-2.f), b, a), c), t1 = add2(fma2(f2(-2.f), c, b), d),
-               t2 = add2(fma2(f2(-2.f), d, c), e);
-  const float2 s0 = fma2(f2(3.f), c, fma2(f2(-4.f), b, a)), s1 = sub2(b, d),
-               s2 = fma2(f2(3.f), c, fma2(f2(-4.f), d, e));
-  const float2 k = f2(13.f / 3.f);
-  const float2 b0 = fma2(mul2(k, t0), t0, fma2(s0, s0, f2(4e-6f)));
-  const float2 b1 = fma2(mul2(k, t1), t1, fma2(s1, s1, f2(4e-6f)));
-  const float2 b2 = fma2(mul2(k, t2), t2, fma2(s2, s2, f2(4e-6f)));
-  const float2 r12 = f2(1.f / 12.f);
-  const float2 q0 = fma2(f2(0.25f), s0, fma2(r12, t0, c));
-  const float2 q1 = fma2(f2(-0.25f), s1, fma2(r12, t1, c));
-  const float2 q2 = fma2(f2(-0.25f), s2, fma2(r12, t2, c));
-  float2 w0, w1, w2;
-  if (Z) {
-    const float2 dd = sub2(b0, b2);
-    const float2 tau = make_float2(fabsf(dd.x), fabsf(dd.y));
-    const float2 p12 = mul2(b1, b2), P = mul2(b0, p12);
-    w0 = fma2(tau, p12, P);
-    w1 = mul2(f2(6.f), fma2(tau, mul2(b0, b2), P));
-    w2 = mul2(f2(3.f), fma2(tau, mul2(b0, b1), P));
-  } else {
-    const float2 p12 = mul2(b1, b2), p02 = mul2(b0, b2), p01 = mul2(b0, b1);
-    w0 = mul2(p12, p12);
-    w1 = mul2(mul2(f2(6.f), p02), p02);
-    w2 = mul2(mul2(f2(3.f), p01), p01);
+// Two faces i+1/2: f+ at i-2..i+2 (p0..p4) and f- at i-1..i+3 (m0..m4) of each.
+template <bool Z, class D, class V>
+__device__ __forceinline__ V weno_face2(V p0, V p1, V p2, V p3, V p4, V m0, V m1, V m2, V m3, V m4) {
+  V Cp, tp, Cm, tm;
+  const V qp = weno_side2<Z, D>(p0, p1, p2, p3, p4, Cp, tp);
+  const V qm = weno_side2<Z, D>(m4, m3, m2, m1, m0, Cm, tm);
+  const V lin = vfma(vc<V>(-1.0 / 6.0), vadd(tp, tm), vfma(vc<V>(0.5), vadd(Cp, Cm), vadd(p2, m2)));
+  return vfma(vc<V>(0.5), vadd(qp, qm), lin);
+}
+
+// One split part along a line walked cell by cell: what neighbouring faces share (differences, the
+// three indicators of a triple of cells) is computed once per cell. After push(f_n) the state holds
+// f_n, D_n = f_n - f_{n-1}, t_{n-1} = D_n - D_{n-1}, d_{n-1} = t_{n-1} - t_{n-2}; of the triple
+// around m = n-1 the central indicator, and the right-sided ones of n-1 and n-2. push returns the
+// negated quotient of the side whose upwind cell is n-2 (PLUS: the face above it, f+) or of the side whose
+// downwind cell is n-2 (the face below it, f-), and t_{n-2}.
+template <class V>
+struct WenoLine {
+  V f, D, t, d, bc, br1, br2;
+  __device__ __forceinline__ void clear() { f = D = t = d = bc = br1 = br2 = vc<V>(0); }
+  // (want false: the state alone, while a segment's first planes fill it)
+  template <bool Z, class DIV, bool PLUS>
+  __device__ __forceinline__ V push(V fn, bool want, V& t_mid) {
+    const V Dn = vsub(fn, f), tn = vsub(Dn, D), dn = vsub(tn, t), T = weno_T(tn);
+    const V sl = vfma(vc<V>(-2), D, tn), sc = vadd(D, Dn), sr = vfma(vc<V>(2), Dn, tn);
+    const V bl = vfma(sl, sl, T);
+    t_mid = t;
+    V q = vc<V>(0);
+    if (want) q = PLUS ? weno_nl<Z, DIV>(br2, bc, bl, d, dn) : weno_nl<Z, DIV>(bl, bc, br2, dn, d);
+    f = fn; D = Dn; t = tn; d = dn;
+    bc = vfma(sc, sc, T);
+    br2 = br1;
+    br1 = vfma(sr, sr, T);
+    return q;
   }
-  const float2 num = fma2(w2, q2, fma2(w1, q1, mul2(w0, q0)));
-  const float2 den = add2(add2(w0, w1), w2);
-  return make_float2(side_div<D>(num.x, den.x), side_div<D>(num.y, den.y));
-}
-
-template <bool Z, class D>
-__device__ __forceinline__ float2 weno_face_fast2(float2 p0, float2 p1, float2 p2, float2 p3, float2 p4, float2 m0,
-                                                  float2 m1, float2 m2, float2 m3, float2 m4) {
-  return add2(weno_side_fast2<Z, D>(p0, p1, p2, p3, p4), weno_side_fast2<Z, D>(m4, m3, m2, m1, m0));
-}
-
-// ------------------------------------------------------------------- fast FP64 form
-// weno_side_fast's common-denominator weights and contracted products for an FP64 state: one
-// IEEE division per side instead of the reference form's four, and fused multiply-adds. The
-// same function of the inputs as the reference form, rounded differently (a few ulps of the
-// face value); selected for FP64 states with ADV_DIV_FAST.
-template <bool Z>
-__device__ __forceinline__ double weno_side_fast64(double a, double b, double c, double d, double e) {
-  const double t0 = fma(-2.0, b, a) + c, t1 = fma(-2.0, c, b) + d, t2 = fma(-2.0, d, c) + e;
-  const double s0 = fma(3.0, c, fma(-4.0, b, a)), s1 = b - d, s2 = fma(3.0, c, fma(-4.0, d, e));
-  const double k = 13.0 / 3.0;
-  const double b0 = fma(k * t0, t0, fma(s0, s0, 4e-6));  // 4 (beta_k + eps)
-  const double b1 = fma(k * t1, t1, fma(s1, s1, 4e-6));
-  const double b2 = fma(k * t2, t2, fma(s2, s2, 4e-6));
-  const double r12 = 1.0 / 12.0;
-  const double q0 = fma(0.25, s0, fma(r12, t0, c));
-  const double q1 = fma(-0.25, s1, fma(r12, t1, c));
-  const double q2 = fma(-0.25, s2, fma(r12, t2, c));
-  double w0, w1, w2;
-  if (Z) {
-    const double tau = fabs(b0 - b2);
-    w0 = (b0 + tau) * (b1 * b2);
-    w1 = (6.0 * (b1 + tau)) * (b0 * b2);
-    w2 = (3.0 * (b2 + tau)) * (b0 * b1);
-  } else {
-    const double p12 = b1 * b2, p02 = b0 * b2, p01 = b0 * b1;
-    w0 = p12 * p12;
-    w1 = (6.0 * p02) * p02;
-    w2 = (3.0 * p01) * p01;
-  }
-  const double num = fma(w2, q2, fma(w1, q1, w0 * q0));
-  const double den = w0 + w1 + w2;
-  return num / den;
-}
-
-template <bool Z>
-__device__ __forceinline__ double weno_face_fast64(double p0, double p1, double p2, double p3, double p4, double m0,
-                                                   double m1, double m2, double m3, double m4) {
-  return weno_side_fast64<Z>(p0, p1, p2, p3, p4) + weno_side_fast64<Z>(m4, m3, m2, m1, m0);
-}
-
-__device__ __forceinline__ void lf_split_fast64(double u, double a, double& fp, double& fm) {
-  const double hu = 0.25 * u, ha = 0.5 * a;
-  fp = u * (hu + ha);
-  fm = u * (hu - ha);
-}
+};
 
 // ---------------------------------------------------------- reference literal form
 // Operand order of kernels.cu:142-192 / :92-140 (and of the CPU oracle), correctly rounded.

@@ -167,6 +167,11 @@ constexpr int TR = 8;   // rows per tile, AX = 0
 constexpr int TL = 32;  // faces along the line per tile, AX = 1, 2
 }  // namespace w7f
 
+__device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return vadd(a, b); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return vmul(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return vfma(a, b, c); }
+
 template <int K>
 __device__ __forceinline__ float2 w7_beta2(const float2* x) {  // x: the candidate's cells 0..3
   constexpr W7B B = kBeta[K];
