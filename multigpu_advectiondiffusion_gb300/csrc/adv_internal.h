@@ -53,7 +53,8 @@ int* device_status_ptr();
 // ------------------------------------------------------------------ launch-shape tuning
 // Parameters picked by the autotuner (autotune.cu) per device and problem; `set` is false when the
 // problem was never tuned (launchers then use their defaults). Kinds and parameters:
-//   TUNE_HEAT, TUNE_BURGERS: a = CTAs per SM (<= occupancy), b = minimum planes per CTA share
+//   TUNE_HEAT, TUNE_BURGERS: a = CTAs per SM (<= occupancy), b = minimum planes per CTA share; all
+//     resident CTAs with b = 8 (the tuner's default candidate) stands for the launcher's own rule
 //   TUNE_HEATK_STEP, TUNE_HEATK_ADJ: a = block height (threads in y), b = z planes per CTA
 //   TUNE_HEAT_STEPS: a = forward-Euler time steps per launch of adv_heat_run (1, or 2 with the
 //     two-step kernel where it measured faster), b = 1
@@ -62,6 +63,7 @@ struct TuneParams {
   int a = 0, b = 0;
   bool set = false;
 };
+inline bool tune_is_shape(const TuneParams& t, int occ) { return t.set && !(t.a >= occ && t.b == 8); }
 TuneParams tune_lookup(int kind, int variant, int nx, int ny, int nz);
 void tune_store(int kind, int variant, int nx, int ny, int nz, TuneParams p);
 void tune_clear();

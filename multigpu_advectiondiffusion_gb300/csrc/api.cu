@@ -127,7 +127,7 @@ adv_status burgers_prepare(const adv_burgers_desc& d, const void* u_in, BurgersL
   const int64_t total = (int64_t)tiles_x * tiles_y * d.nz;
   int64_t min_share = d.nz == 1 ? 1 : 2;
   const TuneParams tp = tune_lookup(TUNE_BURGERS, burgers_tune_variant(d), d.nx, d.ny, d.nz);
-  if (tp.set) {
+  if (tune_is_shape(tp, occ)) {
     occ = std::max(1, std::min(occ, tp.a));
     min_share = std::max(1, tp.b);
   }

@@ -341,7 +341,7 @@ adv_status adv_autotune_heat(const adv_heat_desc* d, const void* u, void* stream
   const int shares3[] = {4, 8, 16, 32};
   for (int a = 1; a <= std::max(occ, 1); ++a)
     for (int b : (d->ndim == 3 ? shares3 : shares2)) cands.push_back({a, b});
-  const Candidate dflt{occ, d->ndim == 3 ? 8 : 1};
+  const Candidate dflt{occ, d->ndim == 3 ? 8 : 1};  // 3D: the launcher's own rule (tune_is_shape)
   const size_t cells = (size_t)d->nx * d->ny * nz;
   const int reps = (int)std::max<size_t>(10, std::min<size_t>(200, ((size_t)256 << 20) / std::max<size_t>(cells, 1)));
   HeatLaunch La, Lb;
@@ -398,7 +398,7 @@ adv_status adv_autotune_burgers(const adv_burgers_desc* d, const void* u, void* 
   std::vector<Candidate> cands;
   for (int a = 1; a <= occ; ++a)
     for (int b : {4, 8, 16, 32}) cands.push_back({a, b});
-  const Candidate dflt{occ, 8};
+  const Candidate dflt{occ, 8};  // the launcher's own rule (tune_is_shape)
   const int reps = (int)std::max<size_t>(3, std::min<size_t>(20, ((size_t)32 << 20) / std::max<size_t>(cells, 1)));
   BurgersLaunch Lc;
   BurgersStageArgs a{};

@@ -95,12 +95,16 @@ adv_status heat_prepare(const adv_heat_desc& d, const void* u_in, HeatLaunch* L,
   ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k0, 32 * L->warps, smem));
   occ = std::max(occ, 1);
   L->occ = occ;
-  // One wave: every CTA resident at once, each with an equal share of the (tile, plane) pairs,
-  // at least 8 planes each in 3D so the z halo stays small (or what the autotuner picked).
+  // One wave: every CTA resident at once, each with an equal share of the (tile, plane) pairs (or what
+  // the autotuner picked), one plane at least. A share's z halo is read again by its neighbours, but
+  // the grids whose shares get short are the small ones, which the L2 holds: at least 8 planes a share
+  // left a 64^3 grid on 16 SMs. us per step, 8 planes -> 1: FP32 O2 32^3 11.4 -> 3.3, 64^3 8.9 -> 3.1,
+  // 96^3 11.5 -> 4.5, 128^3 8.9 -> 5.4; O4 SSP-RK3 64^3 FP32 51 -> 17, FP64 233 -> 65; the same from
+  // 192^3 on, where every share is longer than that anyway.
   const int64_t total = (int64_t)tiles_x * tiles_y * nz;
-  int64_t min_share = d.ndim == 3 ? 8 : 1;
+  int64_t min_share = 1;
   const TuneParams tp = tune_lookup(TUNE_HEAT, heat_tune_variant(d), d.nx, d.ny, nz);
-  if (tp.set) {
+  if (d.ndim == 3 ? tune_is_shape(tp, occ) : tp.set) {
     occ = std::max(1, std::min(occ, tp.a));
     min_share = std::max(1, tp.b);
   }
