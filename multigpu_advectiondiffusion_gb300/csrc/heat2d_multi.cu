@@ -1,17 +1,23 @@
-// heat2d_multi.cu -- 2D forward-Euler heat, several time steps per launch (overlapped temporal
-// tiling) for adv_heat_run.
+// heat2d_multi.cu -- 2D FP32 heat, several time steps per launch (overlapped temporal tiling) for
+// adv_heat_run.
 //
 // A 2D grid of the reference's sizes (SingleGPU/Diffusion2d: 512^2 .. 1001^2 nodes, 1-4 MB per
-// array) is too small to hide a launch per step: the single-step stage spends most of its time
-// in launch gaps and in the load -> compute -> store latency of one plane. Here a CTA copies a
-// 32 x 32 tile of outputs plus a halo of K * R nodes (R the stencil radius) into shared memory
-// once, advances it K steps in place -- after step s the values are valid on the tile grown by
-// (K - s) * R, so the halo's recomputation shrinks step by step -- and writes the tile once:
-// one launch and one pass over memory per K steps (FP32; in FP64 the recomputed halo costs more on
-// the FP64 pipe than the launches it saves, so FP64 keeps one step per launch). Each node's
-// update is the fused single-step
-// stage's expression (lap / combine of heat_stage.cuh, the fused multiply-add form), applied to
-// the same neighbour values, so the result equals K single steps bit for bit.
+// array) is too small to hide a launch per stage: a single-stage launch spends most of its time
+// in launch gaps and in the load -> compute -> store latency of one plane. Here a CTA loads a
+// 64 x 64 block of nodes into registers once, advances it K steps in place -- after each stage the
+// values are valid on a block smaller by the stencil radius R on every side, so the tile it writes
+// is what is left after the last one -- and writes that tile once: one launch and one pass over
+// memory per K steps (FP32; in FP64 the recomputed halo costs more on the FP64 pipe than the
+// launches it saves, so FP64 keeps one stage per launch).
+//
+// Layout: a warp owns 8 whole rows, a lane two adjacent nodes of each, so y neighbours are the
+// thread's own registers, x neighbours one shuffle per side, the arithmetic runs two nodes at a time
+// in paired FP32 instructions, and only a warp's outermost R rows go through shared memory (double
+// buffered: one barrier per stage). The form before this kept the block in shared memory (six
+// accesses per node and step, scalar arithmetic) at 14.5 us per 8 steps of a 512^2 grid.
+// Each node's update is the fused single-stage kernel's expression (lap / combine of
+// heat_stage.cuh, the fused multiply-add form), applied to the same neighbour values, so the result
+// equals the single-stage launches bit for bit.
 #include <algorithm>
 
 #include "adv_device.cuh"
@@ -20,133 +26,204 @@
 
 namespace adv {
 
+template <int ORDER, bool RK3, int STEPS>
 struct Heat2Multi {
-  static constexpr int BX = 32, BY = 32;  // outputs per CTA
-  static constexpr int K = 8;             // steps per launch at most (4: 118, 16: 138 Gcell/s)
-  static constexpr int TX = 32, TY = 16;  // 512 threads (256: 122 vs 145 Gcell/s at 512^2)
+  static constexpr int WARPS = 8, RY = 8;          // warps per CTA, rows per warp
+  static constexpr int EX = 64, EY = WARPS * RY;   // block held in registers
+  static constexpr int R = ORDER / 2;
+  static constexpr int K = STEPS;                  // steps per launch at most
+  static constexpr int H = K * (RK3 ? 3 : 1) * R;  // halo: one radius per stage
+  static constexpr int BX = EX - 2 * H, BY = EY - 2 * H;  // nodes written
+  static_assert(BX >= 32 && BY >= 32 && H % 2 == 0, "tile");
 };
 
-template <class T>
 struct Heat2MultiParams {
-  const T* in;
-  T* out;
+  const float* in;
+  float* out;
   int nx, ny, frozen, zero_boundary, steps;
-  T kx, ky, dt;
+  int vec_ok;  // pairs of nodes aligned for one access
+  float kx, ky, dt;
   int* status;  // device status word (bounds-checked build)
 };
 
-template <class T, int ORDER, bool FAST>
-__global__ void __launch_bounds__(512) heat2d_multi_kernel(const __grid_constant__ Heat2MultiParams<T> p) {
-  using M = Heat2Multi;
-  constexpr int R = ORDER / 2, H = M::K * R;
-  constexpr int EX = M::BX + 2 * H, EY = M::BY + 2 * H;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* bufA = reinterpret_cast<T*>(smem_raw);
-  T* bufB = bufA + EX * EY;
-  const int x0 = blockIdx.x * M::BX - H, y0 = blockIdx.y * M::BY - H;  // grid coordinates of buffer (0, 0)
+template <int ORDER, bool RK3, int STEPS>
+__global__ void __launch_bounds__(256) heat2d_multi_kernel(const __grid_constant__ Heat2MultiParams p) {
+  using M = Heat2Multi<ORDER, RK3, STEPS>;
+  constexpr int R = M::R, RY = M::RY, WARPS = M::WARPS;
+  // [parity][warp][its first R rows, its last R rows]
+  __shared__ float2 rows[2][WARPS][2 * R][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nx = p.nx, ny = p.ny, F = p.frozen;
-  // load the grown tile (nodes off the grid read as 0; no update ever reads them)
-  for (int j = threadIdx.y; j < EY; j += M::TY) {
-    const int gy = y0 + j;
-    for (int i = threadIdx.x; i < EX; i += M::TX) {
-      const int gx = x0 + i;
-      const size_t gi = (size_t)gy * nx + gx;
-      bufA[j * EX + i] = (gx >= 0 && gx < nx && gy >= 0 && gy < ny && ADV_IN_RANGE(gi, (size_t)nx * ny, p.status))
-                             ? p.in[gi]
-                             : T(0);
+  const int x = (int)blockIdx.x * M::BX - M::H + 2 * lane;          // grid coordinates of this thread's
+  const int y = (int)blockIdx.y * M::BY - M::H + RY * warp;          // first node
+  const size_t total = (size_t)nx * ny;
+  // nodes off the grid read as 0; no update of a node that is written ever reads them
+  float2 u[RY];
+#pragma unroll
+  for (int r = 0; r < RY; ++r) {
+    const size_t o = (size_t)(y + r) * nx + x;
+    const bool row = y + r >= 0 && y + r < ny;
+    if (p.vec_ok) {  // x is even, and so is nx: both nodes on the grid or neither
+      u[r] = row && x >= 0 && x < nx && ADV_IN_RANGE(o + 1, total, p.status)
+                 ? *reinterpret_cast<const float2*>(p.in + o) : make_float2(0.f, 0.f);
+    } else {
+      u[r].x = row && x >= 0 && x < nx && ADV_IN_RANGE(o, total, p.status) ? p.in[o] : 0.f;
+      u[r].y = row && x + 1 >= 0 && x + 1 < nx && ADV_IN_RANGE(o + 1, total, p.status) ? p.in[o + 1] : 0.f;
     }
   }
-  __syncthreads();
-  T* src = bufA;
-  T* dst = bufB;
-  // Every step updates the whole buffer but its outer R nodes with the interior formula, without
-  // per-node domain tests: values that are no longer valid after step s (a ring that grows by R
-  // per step), and values of nodes off the grid, are never read by a valid interior node (those
-  // are at least F >= R nodes inside the grid). Frozen nodes of the grid then take their own rule
-  // (kept, or 0 on the outermost layer with zero_boundary); only CTAs whose grown tile reaches
-  // into the frozen layers test for them.
-  const bool inner = x0 >= F && x0 + EX <= nx - F && y0 >= F && y0 + EY <= ny - F;
-  const bool zero = p.zero_boundary != 0;
-  for (int s = 1; s <= p.steps; ++s) {
-    for (int j = R + threadIdx.y; j < EY - R; j += M::TY) {
-      const int gy = y0 + j;
-      const bool rowF = gy < F || gy >= ny - F, rowO = gy == 0 || gy == ny - 1;
-      const T* row = src + j * EX;
-      T* drow = dst + j * EX;
-      for (int i = R + threadIdx.x; i < EX - R; i += M::TX) {
-        const T* c = row + i;
-        const T L = lap<T, ORDER, 2, FAST>(R > 1 ? c[-2] : T(0), c[-1], c[0], c[1], R > 1 ? c[2] : T(0),
-                                           R > 1 ? c[-2 * EX] : T(0), c[-EX], c[EX], R > 1 ? c[2 * EX] : T(0),
-                                           T(0), T(0), T(0), T(0), p.kx, p.ky, T(0));
-        T v = combine<T, FAST>(1, c[0], c[0], p.dt, L);
-        if (!inner) {
-          const int gx = x0 + i;
-          if (rowF || gx < F || gx >= nx - F) v = (zero && (rowO || gx == 0 || gx == nx - 1)) ? T(0) : c[0];
-        }
-        drow[i] = v;
-      }
+  // Every stage updates the whole block with the interior formula, without per-node domain tests:
+  // values that are no longer valid (a ring that grows by R per stage, fed at the block's edges by
+  // whatever the shuffle or the clamped row gives), and values of nodes off the grid, are never read
+  // by a valid interior node (those are at least F >= R nodes inside the grid). Frozen nodes of the
+  // grid then take their own rule (kept, or 0 on the outermost layer with zero_boundary); only CTAs
+  // whose block reaches into the frozen layers test for them.
+  const int bx0 = (int)blockIdx.x * M::BX - M::H, by0 = (int)blockIdx.y * M::BY - M::H;
+  const bool inner = bx0 >= F && bx0 + M::EX <= nx - F && by0 >= F && by0 + M::EY <= ny - F;
+  // frozen columns of this thread (the same in every row) and rows of this warp (bit r)
+  const bool fx0 = x < F || x >= nx - F, fx1 = x + 1 < F || x + 1 >= nx - F;
+  const bool zx0 = p.zero_boundary && (x == 0 || x == nx - 1), zx1 = p.zero_boundary && (x + 1 == 0 || x + 1 == nx - 1);
+  unsigned frow = 0, zrow = 0;
+#pragma unroll
+  for (int r = 0; r < RY; ++r) {
+    if (y + r < F || y + r >= ny - F) frow |= 1u << r;
+    if (p.zero_boundary && (y + r == 0 || y + r == ny - 1)) zrow |= 1u << r;
+  }
+  const float2 kx = make_float2(p.kx, p.kx), ky = make_float2(p.ky, p.ky), dt = make_float2(p.dt, p.dt);
+  float2 un[RK3 ? RY : 1];
+  int par = 0;
+  auto stage = [&](auto stage_c) {
+    constexpr int STAGE = decltype(stage_c)::value;
+#pragma unroll
+    for (int d = 0; d < R; ++d) {
+      rows[par][warp][d][lane] = u[d];
+      rows[par][warp][R + d][lane] = u[RY - R + d];
     }
     __syncthreads();
-    T* t = src;
-    src = dst;
-    dst = t;
+    float2 up[R], dn[R];  // the R rows above (nearest last) and below (nearest first)
+    const int wu = warp > 0 ? warp - 1 : 0, wd = warp < WARPS - 1 ? warp + 1 : warp;
+#pragma unroll
+    for (int d = 0; d < R; ++d) {
+      up[d] = rows[par][wu][R + d][lane];
+      dn[d] = rows[par][wd][d][lane];
+    }
+    par ^= 1;
+    // FROZEN: 0 no frozen node in the block, 1 frozen columns only in this warp's rows, 2 any
+    auto update = [&](auto frozen_c) {
+      constexpr int FROZEN = decltype(frozen_c)::value;
+      float2 m1 = up[R - 1], m2 = up[0];  // old rows r-1 and r-2
+#pragma unroll
+      for (int r = 0; r < RY; ++r) {
+        const float2 c = u[r];
+        auto below = [&](int d) {  // old row r + d
+          const int j = r + d;
+          return j < RY ? u[j < RY ? j : 0] : dn[j < RY ? 0 : j - RY < R ? j - RY : 0];
+        };
+        const float2 p1 = below(1);
+        const float ly = __shfl_up_sync(0xffffffffu, c.y, 1), rx = __shfl_down_sync(0xffffffffu, c.x, 1);
+        float2 L;
+        if constexpr (ORDER == 2) {
+          // lap's operations; the x part node by node (as pairs its neighbours would straddle the
+          // register pairs: packing them cost 13% at 2048^2)
+          const float2 Sx = make_float2(add_rn(fma_rn(-2.f, c.x, c.y), ly), add_rn(fma_rn(-2.f, c.y, rx), c.x));
+          const float2 Sy = add_rn(fma_rn(make_float2(-2.f, -2.f), c, p1), m1);
+          L = fma_rn(ky, Sy, mul_rn(kx, Sx));
+        } else {
+          const float lx = __shfl_up_sync(0xffffffffu, c.x, 1), ry = __shfl_down_sync(0xffffffffu, c.y, 1);
+          L = lap<float2, ORDER, 2, true>(make_float2(lx, ly), make_float2(ly, c.x), c, make_float2(c.y, rx),
+                                          make_float2(rx, ry), m2, m1, p1, below(2), c, c, c, c, kx, ky, kx);
+        }
+        float2 v = combine<float2, true>(STAGE, STAGE == 1 ? c : un[RK3 ? r : 0], c, dt, L);
+        if (FROZEN) {
+          const bool fr = FROZEN == 2 && (frow >> r & 1u), zr = FROZEN == 2 && (zrow >> r & 1u);
+          if (fx0 || fr) v.x = zx0 || zr ? 0.f : c.x;
+          if (fx1 || fr) v.y = zx1 || zr ? 0.f : c.y;
+        }
+        u[r] = v;
+        m2 = m1;
+        m1 = c;
+      }
+    };
+    if (inner) update(std::integral_constant<int, 0>{});
+    else if (frow == 0) update(std::integral_constant<int, 1>{});  // (the same choice in all lanes of a warp)
+    else update(std::integral_constant<int, 2>{});
+  };
+#pragma unroll 1
+  for (int s = 0; s < p.steps; ++s) {
+    if constexpr (RK3) {
+#pragma unroll
+      for (int r = 0; r < RY; ++r) un[r] = u[r];
+      stage(std::integral_constant<int, 1>{});
+      stage(std::integral_constant<int, 2>{});
+      stage(std::integral_constant<int, 3>{});
+    } else {
+      stage(std::integral_constant<int, 1>{});
+    }
   }
-  // the tile itself
-  for (int j = threadIdx.y; j < M::BY; j += M::TY) {
-    const int gy = y0 + H + j;
-    if (gy >= ny) break;
-    for (int i = threadIdx.x; i < M::BX; i += M::TX) {
-      const int gx = x0 + H + i;
-      if (gx < nx && ADV_IN_RANGE((size_t)gy * nx + gx, (size_t)nx * ny, p.status))
-        p.out[(size_t)gy * nx + gx] = src[(j + H) * EX + i + H];
+  // the tile itself: lanes and rows H nodes inside the block
+  if (2 * lane < M::H || 2 * lane >= M::H + M::BX) return;
+#pragma unroll
+  for (int r = 0; r < RY; ++r) {
+    const int j = RY * warp + r;
+    if (j < M::H || j >= M::H + M::BY || y + r >= ny) continue;
+    const size_t o = (size_t)(y + r) * nx + x;
+    if (p.vec_ok) {
+      if (x < nx && ADV_IN_RANGE(o + 1, total, p.status)) *reinterpret_cast<float2*>(p.out + o) = u[r];
+    } else {
+      if (x < nx && ADV_IN_RANGE(o, total, p.status)) p.out[o] = u[r].x;
+      if (x + 1 < nx && ADV_IN_RANGE(o + 1, total, p.status)) p.out[o + 1] = u[r].y;
     }
   }
 }
 
 namespace {
-template <class T, int ORDER, bool FAST>
-constexpr size_t heat2d_multi_smem() {
-  constexpr int H = Heat2Multi::K * (ORDER / 2);
-  return 2 * (size_t)(Heat2Multi::BX + 2 * H) * (Heat2Multi::BY + 2 * H) * sizeof(T);
-}
-
-template <class T, int ORDER, bool FAST>
+template <int ORDER, bool RK3, int STEPS>
 adv_status launch_t(const adv_heat_desc& d, const void* in, void* out, int steps, cudaStream_t s) {
-  constexpr size_t smem = heat2d_multi_smem<T, ORDER, FAST>();
-  static bool attr = false;  // 18 KB (O2) or 32 KB (O4) per CTA: under the default 48 KB, set anyway
-  if (!attr) {
-    ADV_CUDA_TRY(cudaFuncSetAttribute(heat2d_multi_kernel<T, ORDER, FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-    attr = true;
-  }
-  Heat2MultiParams<T> p;
-  p.in = static_cast<const T*>(in);
-  p.out = static_cast<T*>(out);
+  using M = Heat2Multi<ORDER, RK3, STEPS>;
+  Heat2MultiParams p;
+  p.in = static_cast<const float*>(in);
+  p.out = static_cast<float*>(out);
   p.nx = d.nx;
   p.ny = d.ny;
   p.frozen = d.frozen;
   p.zero_boundary = d.zero_boundary;
   p.steps = steps;
-  p.kx = (T)d.kx;
-  p.ky = (T)d.ky;
-  p.dt = (T)d.dt;
+  p.vec_ok = d.nx % 2 == 0 && (uintptr_t)in % 8 == 0 && (uintptr_t)out % 8 == 0 ? 1 : 0;
+  p.kx = (float)d.kx;
+  p.ky = (float)d.ky;
+  p.dt = (float)d.dt;
   p.status = device_status_ptr();
-  const dim3 grid((unsigned)((d.nx + Heat2Multi::BX - 1) / Heat2Multi::BX),
-                  (unsigned)((d.ny + Heat2Multi::BY - 1) / Heat2Multi::BY));
-  heat2d_multi_kernel<T, ORDER, FAST><<<grid, dim3(Heat2Multi::TX, Heat2Multi::TY), smem, s>>>(p);
+  const dim3 grid((unsigned)((d.nx + M::BX - 1) / M::BX), (unsigned)((d.ny + M::BY - 1) / M::BY));
+  heat2d_multi_kernel<ORDER, RK3, STEPS><<<grid, 32 * M::WARPS, 0, s>>>(p);
   ADV_CUDA_TRY(cudaGetLastError());
   count_launches(1);
   return ADV_OK;
 }
 }  // namespace
 
-int heat2d_multi_steps() { return Heat2Multi::K; }
+bool heat2d_multi_eligible(const adv_heat_desc& d) {
+  // grid.y of the launch (at least 32 rows per CTA)
+  return d.ndim == 2 && d.dtype == ADV_F32 && (d.ny + 31) / 32 <= 65535;
+}
 
-adv_status heat2d_multi_launch(const adv_heat_desc& d, const void* in, void* out, int steps, cudaStream_t s) {
-  if (d.ndim != 2 || steps < 1 || steps > Heat2Multi::K || in == out)
+// Steps per launch: SSP-RK3 2 (six stages); O4 forward Euler 8; O2 16 where the 32-node tiles it leaves
+// still give every CTA an SM of its own, else 8 (48-node tiles: fewer nodes computed twice).
+int heat2d_multi_steps(const adv_heat_desc& d, int time_scheme) {
+  if (time_scheme == ADV_SSPRK3) return 2;
+  if (d.order != 2) return 8;
+  DeviceInfo di;
+  const int sms = device_info(&di) == ADV_OK ? di.sms : 152;
+  return (int64_t)((d.nx + 31) / 32) * ((d.ny + 31) / 32) <= sms ? 16 : 8;
+}
+
+adv_status heat2d_multi_launch(const adv_heat_desc& d, int time_scheme, const void* in, void* out, int steps,
+                               cudaStream_t s) {
+  const int most = heat2d_multi_steps(d, time_scheme);
+  if (!heat2d_multi_eligible(d) || steps < 1 || steps > most || in == out)
     return set_error(ADV_ERR_INVALID_ARG, "heat2d multi-step: bad arguments");
-  if (d.dtype != ADV_F32) return set_error(ADV_ERR_UNSUPPORTED, "heat2d multi-step: FP32 only");
-  return d.order == 2 ? launch_t<float, 2, true>(d, in, out, steps, s) : launch_t<float, 4, true>(d, in, out, steps, s);
+  if (time_scheme == ADV_SSPRK3)
+    return d.order == 2 ? launch_t<2, true, 2>(d, in, out, steps, s) : launch_t<4, true, 2>(d, in, out, steps, s);
+  if (d.order == 4) return launch_t<4, false, 8>(d, in, out, steps, s);
+  return most == 16 ? launch_t<2, false, 16>(d, in, out, steps, s) : launch_t<2, false, 8>(d, in, out, steps, s);
 }
 
 }  // namespace adv
