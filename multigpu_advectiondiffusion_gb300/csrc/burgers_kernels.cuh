@@ -213,7 +213,7 @@ __device__ __forceinline__ double2 combine2(int stage, double2 un, double2 u, do
 __device__ __forceinline__ float2 combine2(int stage, float2 un, float2 u, float dt, float2 L) {
   const float2 dL = vmul(make_float2(dt, dt), L);
   if (stage == 2) return vadd(vmul(vc<float2>(0.75), un), vmul(vc<float2>(0.25), vadd(u, dL)));
-  if (stage == 3) return div_rn(vadd(un, vmul(vc<float2>(2), vadd(u, dL))), vc<float2>(3));
+  if (stage == 3) return div3(vfma(vc<float2>(2), vadd(u, dL), un));
   return vadd(un, dL);
 }
 

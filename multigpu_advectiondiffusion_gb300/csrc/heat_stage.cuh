@@ -87,7 +87,8 @@ struct HeatParams {
 
 // Laplacian at one node from its neighbours along each axis (m2, m1, centre, p1, p2).
 // EXACT: the reference's operand order (3D east first, kernels.cu:95-97; 2D west first,
-// Diffusion2d/kernels.cu:82-83; O2 e - 2o + w, kernels.cu:58-60), correctly rounded.
+// Diffusion2d/kernels.cu:82-83; O2 e - 2o + w, kernels.cu:58-60), every operation rounded on its own
+// (products by powers of two are exact short of overflow and go into fused multiply-adds).
 // FAST (FP32): O2 fma(-2, c, p1) + m1 per axis; O4 fma(16, far-side neighbour,
 // fma(-30, c, fma(16, near-side neighbour, -near-side outer))) - far-side outer with the same
 // near/far sides as the reference; L = fma(kz, Sz, fma(ky, Sy, kx * Sx)).
@@ -100,10 +101,10 @@ __device__ __forceinline__ T lap(T xm2, T xm1, T c, T xp1, T xp2, T ym2, T ym1, 
       Sx = add_rn(fma_rn(bc<T>(-2), c, xp1), xm1);
       Sy = add_rn(fma_rn(bc<T>(-2), c, yp1), ym1);
       if (NDIM == 3) Sz = add_rn(fma_rn(bc<T>(-2), c, zp1), zm1);
-    } else {
-      Sx = add_rn(sub_rn(xp1, mul_rn(bc<T>(2), c)), xm1);
-      Sy = add_rn(sub_rn(yp1, mul_rn(bc<T>(2), c)), ym1);
-      if (NDIM == 3) Sz = add_rn(sub_rn(zp1, mul_rn(bc<T>(2), c)), zm1);
+    } else {  // p1 - 2c: 2c is exact, so the fused form rounds alike
+      Sx = add_rn(fma_rn(bc<T>(-2), c, xp1), xm1);
+      Sy = add_rn(fma_rn(bc<T>(-2), c, yp1), ym1);
+      if (NDIM == 3) Sz = add_rn(fma_rn(bc<T>(-2), c, zp1), zm1);
     }
   } else {
     // near side first: +1 in 3D, -1 in 2D
@@ -114,9 +115,12 @@ __device__ __forceinline__ T lap(T xm2, T xm1, T c, T xp1, T xp2, T ym2, T ym1, 
       Sy = sub_rn(fma_rn(bc<T>(16), by1, fma_rn(bc<T>(-30), c, fma_rn(bc<T>(16), ay1, -ay2))), by2);
       if (NDIM == 3) Sz = sub_rn(fma_rn(bc<T>(16), zm1, fma_rn(bc<T>(-30), c, fma_rn(bc<T>(16), zp1, -zp2))), zm2);
     } else {
-      Sx = sub_rn(add_rn(sub_rn(add_rn(-ax2, mul_rn(bc<T>(16), ax1)), mul_rn(bc<T>(30), c)), mul_rn(bc<T>(16), bx1)), bx2);
-      Sy = sub_rn(add_rn(sub_rn(add_rn(-ay2, mul_rn(bc<T>(16), ay1)), mul_rn(bc<T>(30), c)), mul_rn(bc<T>(16), by1)), by2);
-      if (NDIM == 3) Sz = sub_rn(add_rn(sub_rn(add_rn(-zp2, mul_rn(bc<T>(16), zp1)), mul_rn(bc<T>(30), c)), mul_rn(bc<T>(16), zm1)), zm2);
+      // -a2 + 16 a1 - 30 c + 16 b1 - b2: 16 a1 and 16 b1 are exact, so the fused forms round alike
+      // (19 -> 13 FP64 operations for the three axes with 30 c shared)
+      const T c30 = mul_rn(bc<T>(30), c);
+      Sx = sub_rn(fma_rn(bc<T>(16), bx1, sub_rn(fma_rn(bc<T>(16), ax1, -ax2), c30)), bx2);
+      Sy = sub_rn(fma_rn(bc<T>(16), by1, sub_rn(fma_rn(bc<T>(16), ay1, -ay2), c30)), by2);
+      if (NDIM == 3) Sz = sub_rn(fma_rn(bc<T>(16), zm1, sub_rn(fma_rn(bc<T>(16), zp1, -zp2), c30)), zm2);
     }
   }
   if (FAST) {
@@ -135,7 +139,7 @@ template <class T, bool FAST>
 __device__ __forceinline__ T combine(int stage, T un, T uin, T dt, T L) {
   if constexpr (!FAST) return stage_combine<T>(stage, un, uin, dt, L);
   if (stage == 2) return fma_rn(bc<T>(0.25), fma_rn(dt, L, uin), mul_rn(bc<T>(0.75), un));
-  if (stage == 3) return div_rn(fma_rn(bc<T>(2), fma_rn(dt, L, uin), un), bc<T>(3));
+  if (stage == 3) return div3(fma_rn(bc<T>(2), fma_rn(dt, L, uin), un));
   return fma_rn(dt, L, un);
 }
 
