@@ -77,6 +77,7 @@ struct HeatLaunch {
   bool tma = false;
   int occ = 0;                   // resident CTAs per SM of the stage kernel (before any tuning cap)
   int rows = 2;                  // rows per thread
+  int nodes = 4;                 // nodes per thread along x (a 16-byte vector, or 1)
   int warps = 8;                 // warps per CTA
   int lanes = 32;                // lanes per row (16: two rows per warp); tile lanes*vector x (32*warps/lanes)*rows
   int tiles_x = 0, tiles_y = 0;  // x-y tiles; the grid is one wave of CTAs sharing the tile-planes
@@ -89,8 +90,8 @@ struct HeatLaunch {
   int withheld_plane = kNoWithheldPlane;
   unsigned long long wait_limit_ns = 0;
 };
-// rows: rows per thread of the stage kernel (2 or 4), lanes: lanes per row (32 or 16); 0 = the
-// library's choice.
+// rows: rows per thread of a batched kernel's tile (2 or 4), lanes: lanes per row (32 or 16); 0 = the
+// single-grid stage kernel, its tile the library's choice.
 adv_status heat_prepare(const adv_heat_desc& d, const void* u_in, HeatLaunch* L, int rows = 0, int lanes = 0);
 // Lanes per row of the 4-row FP32 tile for rows of nx nodes: 16 (64-wide tiles) where 128-wide
 // tiles leave clearly more lanes idle, else 32.

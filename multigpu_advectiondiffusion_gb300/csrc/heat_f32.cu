@@ -4,9 +4,30 @@
 namespace adv {
 
 // Kernel for (order, ndim, TMA or cp.async loads, stage specialisation, rows per thread, warps
-// per CTA, lanes per row). Four rows per thread with 4 warps exist for the 3D O2 stencil with TMA
+// per CTA, lanes per row, nodes per thread along x). One node per thread with element copies
+// (HeatTile1). Four rows per thread with 4 warps exist for the 3D O2 stencil with TMA
 // loads, in rows of 32 lanes (tile 128 x 16) or 16 lanes (tile 64 x 32).
-void* heat_kernel_f32(int order, int ndim, bool tma, int stage_kind, int rows, int warps, int lanes) {
+void* heat_kernel_f32(int order, int ndim, bool tma, int stage_kind, int rows, int warps, int lanes, int nodes) {
+  if (nodes == 1) {
+    if (tma) return nullptr;
+#define H1(O, N, S)                                                                                                   \
+  reinterpret_cast<void*>(&heat_stage_kernel<float, O, N, false, S, HeatTile1<float, O>::ROWS, HeatTile1<float, O>::WARPS, \
+                                             HeatTile1<float, O>::LANES, false, false, 1>)
+#define HS1(O, N)                  \
+  switch (stage_kind) {            \
+    case 1: return H1(O, N, 1);    \
+    case 2: return H1(O, N, 2);    \
+    case 3: return H1(O, N, 3);    \
+    default: return H1(O, N, 0);   \
+  }
+    if (order == 2 && ndim == 3) { HS1(2, 3) }
+    if (order == 4 && ndim == 3) { HS1(4, 3) }
+    if (order == 2 && ndim == 2) { HS1(2, 2) }
+    if (order == 4 && ndim == 2) { HS1(4, 2) }
+#undef HS1
+#undef H1
+    return nullptr;
+  }
   if (rows == 4) {
     if (order != 2 || ndim != 3 || !tma || warps != 4) return nullptr;
 #define R4(L)                                                                                  \
@@ -20,7 +41,7 @@ void* heat_kernel_f32(int order, int ndim, bool tma, int stage_kind, int rows, i
     R4(32)
 #undef R4
   }
-  if (warps != 8 || lanes != 32) return nullptr;
+  if (warps != 8 || lanes != 32 || !tma) return nullptr;
 #define HK(O, N, M, S) reinterpret_cast<void*>(&heat_stage_kernel<float, O, N, M, S>)
 #define HS(O, N, M)                                            \
   switch (stage_kind) {                                        \
@@ -29,10 +50,10 @@ void* heat_kernel_f32(int order, int ndim, bool tma, int stage_kind, int rows, i
     case 3: return HK(O, N, M, 3);                             \
     default: return HK(O, N, M, 0);                            \
   }
-  if (order == 2 && ndim == 3) { if (tma) { HS(2, 3, true) } else { HS(2, 3, false) } }
-  if (order == 4 && ndim == 3) { if (tma) { HS(4, 3, true) } else { HS(4, 3, false) } }
-  if (order == 2 && ndim == 2) { if (tma) { HS(2, 2, true) } else { HS(2, 2, false) } }
-  if (order == 4 && ndim == 2) { if (tma) { HS(4, 2, true) } else { HS(4, 2, false) } }
+  if (order == 2 && ndim == 3) { HS(2, 3, true) }
+  if (order == 4 && ndim == 3) { HS(4, 3, true) }
+  if (order == 2 && ndim == 2) { HS(2, 2, true) }
+  if (order == 4 && ndim == 2) { HS(4, 2, true) }
 #undef HS
 #undef HK
   return nullptr;

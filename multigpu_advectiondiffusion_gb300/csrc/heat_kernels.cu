@@ -7,8 +7,8 @@
 
 namespace adv {
 
-void* heat_kernel_f32(int order, int ndim, bool tma, int stage_kind, int rows, int warps, int lanes);
-void* heat_kernel_f64(int order, int ndim, bool tma, int stage_kind, int rows, int warps, int lanes, bool contract);
+void* heat_kernel_f32(int order, int ndim, bool tma, int stage_kind, int rows, int warps, int lanes, int nodes);
+void* heat_kernel_f64(int order, int ndim, bool tma, int stage_kind, int nodes, bool contract);
 
 adv_status heat_validate(const adv_heat_desc* d) {
   if (!d) return set_error(ADV_ERR_INVALID_ARG, "heat: null descriptor");
@@ -30,19 +30,29 @@ adv_status heat_validate(const adv_heat_desc* d) {
 namespace {
 
 void* pick_kernel(const adv_heat_desc& d, bool tma, int stage_kind, const HeatLaunch& L) {
-  return d.dtype == ADV_F32 ? heat_kernel_f32(d.order, d.ndim, tma, stage_kind, L.rows, L.warps, L.lanes)
-                            : heat_kernel_f64(d.order, d.ndim, tma, stage_kind, L.rows, L.warps, L.lanes,
-                                              d.contract != 0);
+  return d.dtype == ADV_F32 ? heat_kernel_f32(d.order, d.ndim, tma, stage_kind, L.rows, L.warps, L.lanes, L.nodes)
+                            : heat_kernel_f64(d.order, d.ndim, tma, stage_kind, L.nodes, d.contract != 0);
 }
 
-template <class T, int ORDER, int NDIM, int ROWS, int WARPS = 8, int LANES = 32>
+template <class T, int ORDER, int NDIM, int ROWS, int WARPS = 8, int LANES = 32, int NODES = 16 / (int)sizeof(T)>
 void tile_dims(int* bx, int* by, int* sw, int* sh, int* padx, int* r, size_t* smem) {
-  using C = HeatTile<T, ORDER, NDIM, ROWS, WARPS, LANES>;
+  using C = HeatTile<T, ORDER, NDIM, ROWS, WARPS, LANES, NODES>;
   *bx = C::BX; *by = C::BY; *sw = C::SW; *sh = C::SH; *padx = C::PADX; *r = C::R; *smem = C::SMEM;
 }
+template <class T, int ORDER, int NDIM>
+void tile_dims1(int* bx, int* by, int* sw, int* sh, int* padx, int* r, size_t* smem) {
+  using T1 = HeatTile1<T, ORDER>;
+  tile_dims<T, ORDER, NDIM, T1::ROWS, T1::WARPS, T1::LANES, 1>(bx, by, sw, sh, padx, r, smem);
+}
 
-void tile_for(int dtype, int order, int ndim, int rows, int lanes, int* bx, int* by, int* sw, int* sh, int* padx,
+void tile_for(int dtype, int order, int ndim, int rows, int lanes, int nodes, int* bx, int* by, int* sw, int* sh, int* padx,
               int* r, size_t* smem) {
+  if (nodes == 1) {
+#define TD(T, O, N) if (order == O && ndim == N) return tile_dims1<T, O, N>(bx, by, sw, sh, padx, r, smem);
+    if (dtype == ADV_F32) { TD(float, 2, 3) TD(float, 4, 3) TD(float, 2, 2) TD(float, 4, 2) }
+    else { TD(double, 2, 3) TD(double, 4, 3) TD(double, 2, 2) TD(double, 4, 2) }
+#undef TD
+  }
   if (rows == 4 && lanes == 16) return tile_dims<float, 2, 3, 4, 4, 16>(bx, by, sw, sh, padx, r, smem);
   if (rows == 4) return tile_dims<float, 2, 3, 4, 4, 32>(bx, by, sw, sh, padx, r, smem);
 #define TD(T, O, N) if (order == O && ndim == N) return tile_dims<T, O, N, 2>(bx, by, sw, sh, padx, r, smem);
@@ -77,24 +87,35 @@ adv_status heat_prepare(const adv_heat_desc& d, const void* u_in, HeatLaunch* L,
   // 16 nodes instead of 8 (FP32 3D O2 with TMA loads).
   const bool rows4_ok = aligned && d.dtype == ADV_F32 && d.order == 2 && d.ndim == 3;
   if (rows == 4 && !rows4_ok) return set_error(ADV_ERR_UNSUPPORTED, "heat: 4 rows per thread need FP32 3D O2 with TMA");
-  L->rows = rows == 0 ? (rows4_ok ? 4 : 2) : rows;
-  L->warps = L->rows == 4 ? 4 : 8;
-  L->lanes = L->rows == 4 ? (lanes != 0 ? lanes : heat_row_lanes(d.nx)) : 32;
+  L->nodes = 16 / es;
+  if (rows == 0 && (d.dtype == ADV_F64 || !aligned)) {  // HeatTile1
+    L->nodes = 1;
+    L->rows = d.dtype == ADV_F64 ? HeatTile1<double, 2>::ROWS : d.order == 2 ? HeatTile1<float, 2>::ROWS : HeatTile1<float, 4>::ROWS;
+    L->warps = d.dtype == ADV_F64 ? HeatTile1<double, 2>::WARPS : d.order == 2 ? HeatTile1<float, 2>::WARPS : HeatTile1<float, 4>::WARPS;
+    L->lanes = d.dtype == ADV_F64 ? HeatTile1<double, 2>::LANES : HeatTile1<float, 2>::LANES;
+  } else {
+    L->rows = rows == 0 ? (rows4_ok ? 4 : 2) : rows;
+    L->warps = L->rows == 4 ? 4 : 8;
+    L->lanes = L->rows == 4 ? (lanes != 0 ? lanes : heat_row_lanes(d.nx)) : 32;
+  }
   int bx, by, sw, sh, padx, r;
   size_t smem;
-  tile_for(d.dtype, d.order, d.ndim, L->rows, L->lanes, &bx, &by, &sw, &sh, &padx, &r, &smem);
+  tile_for(d.dtype, d.order, d.ndim, L->rows, L->lanes, L->nodes, &bx, &by, &sw, &sh, &padx, &r, &smem);
   L->block = dim3((unsigned)L->lanes, (unsigned)(32 * L->warps / L->lanes), 1);
   const int tiles_x = (d.nx + bx - 1) / bx, tiles_y = (d.ny + by - 1) / by;
-  for (int sk = 0; sk <= 3; ++sk) {
-    void* k = pick_kernel(d, L->tma, sk, *L);
-    if (!k) return set_error(ADV_ERR_UNSUPPORTED, "heat: no kernel for this configuration");
-    ADV_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int occ = 1;
+  L->occ = 0;
+  if (rows == 0) {  // (with explicit rows the caller runs a batched kernel of its own over this tile)
+    for (int sk = 0; sk <= 3; ++sk) {
+      void* k = pick_kernel(d, L->tma, sk, *L);
+      if (!k) return set_error(ADV_ERR_UNSUPPORTED, "heat: no kernel for this configuration");
+      ADV_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    }
+    void* k0 = pick_kernel(d, L->tma, 1, *L);
+    ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k0, 32 * L->warps, smem));
+    occ = std::max(occ, 1);
+    L->occ = occ;
   }
-  void* k0 = pick_kernel(d, L->tma, 1, *L);
-  int occ = 0;
-  ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k0, 32 * L->warps, smem));
-  occ = std::max(occ, 1);
-  L->occ = occ;
   // One wave: every CTA resident at once, each with an equal share of the (tile, plane) pairs (or what
   // the autotuner picked), one plane at least. A share's z halo is read again by its neighbours, but
   // the grids whose shares get short are the small ones, which the L2 holds: at least 8 planes a share

@@ -43,11 +43,11 @@ __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fm
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float2 fma_rn(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
-// Tile: TX lanes per row (32, or 16 with two rows per warp) x one 16-byte vector each, RY rows per
-// thread, WARPS warps.
-template <class T, int ORDER, int NDIM, int ROWS = 2, int WARPS = 8, int LANES = 32>
+// Tile: TX lanes per row (32, or 16 with two rows per warp) x VX nodes each (one 16-byte vector, or one
+// node), RY rows per thread, WARPS warps.
+template <class T, int ORDER, int NDIM, int ROWS = 2, int WARPS = 8, int LANES = 32, int NODES = 16 / (int)sizeof(T)>
 struct HeatTile {
-  static constexpr int VX = 16 / (int)sizeof(T);  // nodes per thread along x (one 16-byte vector)
+  static constexpr int VX = NODES;  // nodes per thread along x
   static constexpr int TX = LANES, NT = 32 * WARPS, TY = NT / TX;
   static_assert(LANES == 32 || LANES == 16, "rows of 32 or 16 lanes");
   static constexpr int RY = ROWS;  // rows per thread
@@ -55,7 +55,8 @@ struct HeatTile {
   static constexpr int BX = TX * VX, BY = TY * RY;
   static constexpr int R = ORDER / 2;
   static constexpr int RZ = NDIM == 3 ? R : 0;
-  static constexpr int PADX = VX;  // shared column 0 holds x0 - PADX (16-byte aligned start)
+  static constexpr int PADX = 16 / (int)sizeof(T);  // shared column 0 holds x0 - PADX (16-byte aligned start)
+  static_assert(PADX >= R, "x halo");
   static constexpr int SW = BX + 2 * PADX;
   static constexpr int SH = BY + 2 * R;
   static constexpr int PLANE = SW * SH;
@@ -64,6 +65,20 @@ struct HeatTile {
   static constexpr int P = NDIM == 3 ? 3 : 0;  // planes prefetched ahead of the one consumed
   static constexpr int NS = RZ + 1 + P;         // ring slots
   static constexpr size_t SMEM = (size_t)NS * SLOT_ELEMS * sizeof(T);
+};
+
+// The single-grid launches' tiles outside the FP32 TMA path: one node per thread along x.
+//  * FP32 rows TMA cannot describe (element copies): 32 lanes; rows stay coalesced whatever their
+//    alignment, and a copied row costs a thread one cp.async and no index division.
+//  * FP64 (either load): 16 x 16 nodes. FP64 is bound by its pipe, which runs a whole warp's lanes
+//    whether their nodes are on the grid or not: a 201 x 199 plane fills 92% of the lanes of 16 x 16
+//    tiles against 76% of 64 x 16 ones.
+template <class T, int ORDER> struct HeatTile1;
+template <int ORDER> struct HeatTile1<float, ORDER> {
+  static constexpr int ROWS = ORDER == 2 ? 8 : 4, WARPS = ORDER == 2 ? 4 : 8, LANES = 32;
+};
+template <int ORDER> struct HeatTile1<double, ORDER> {
+  static constexpr int ROWS = 2, WARPS = 4, LANES = 16;
 };
 
 template <class T>
@@ -191,12 +206,12 @@ __device__ __forceinline__ int* heat_abort_flag() {
 // segment (by value, so it stays in registers), with s_issue = -1 if a wait timed out (the CTA
 // must then return).
 template <class T, int ORDER, int NDIM, bool TMA, int STAGE, int ROWS = 2, int WARPS = 8, int LANES = 32,
-          bool CONTRACT = false, bool HOOK = false>
+          bool CONTRACT = false, bool HOOK = false, int NODES = 16 / (int)sizeof(T)>
 __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const HeatParams<T>& p, int x0, int y0, int zs,
                                              int ze, HeatPipe pipe) {
-  using C = HeatTile<T, ORDER, NDIM, ROWS, WARPS, LANES>;
+  using C = HeatTile<T, ORDER, NDIM, ROWS, WARPS, LANES, NODES>;
   constexpr int RY = C::RY;
-  using V = typename Vec16<T>::type;
+  using V = std::conditional_t<NODES == 1, T, typename Vec16<T>::type>;
   // FP32 always, FP64 on request: the fused multiply-add pattern instead of the reference's
   // separately rounded operations
   constexpr bool FAST = sizeof(T) == 4 || CONTRACT;
@@ -228,6 +243,33 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
         mbar_arrive_expect_tx(&bars[s_issue], C::PLANE_BYTES);
         tma_load_3d(dst, tmap, x0 - C::PADX, y0 - R, z, &bars[s_issue]);
       }
+    } else if constexpr (VX == 1) {
+      // column tx of rows ty, ty + TY, ..; then the 2 R halo columns, one element per thread
+      const bool zok = z >= 0 && z < nz;
+      const T* const plane = p.uin + (zok ? (size_t)z * sxy : 0);
+      const T* src = plane + (int64_t)(y0 - R + ty) * nx + (x0 + tx);
+      T* d = dst + ty * SW + C::PADX + tx;
+      const bool xok = zok && x0 + tx < nx;
+#pragma unroll
+      for (int j = 0; j < (C::SH + C::TY - 1) / C::TY; ++j) {
+        const int r = ty + j * C::TY;
+        if ((C::SH % C::TY == 0 || r < C::SH)) {
+          const bool ok = xok && (unsigned)(y0 - R + r) < (unsigned)ny;
+          cp_async_zfill<sizeof(T)>(d, ok ? src : p.uin, ok && ADV_IN_RANGE(src - p.uin, sxy * nz, p.status));
+        }
+        src += (size_t)C::TY * nx;
+        d += C::TY * SW;
+      }
+      static_assert(2 * R * C::SH <= 2 * C::NT, "halo columns: at most two elements per thread");
+#pragma unroll
+      for (int e = tid; e < 2 * R * C::SH; e += C::NT) {
+        const int r = e / (2 * R), k = e % (2 * R), c = k < R ? C::PADX - R + k : C::PADX + C::BX - R + k;
+        const int gx = x0 - C::PADX + c, gy = y0 - R + r;
+        const bool ok = zok && gx >= 0 && gx < nx && gy >= 0 && gy < ny;
+        const T* const h = ok ? plane + (size_t)gy * nx + gx : p.uin;
+        cp_async_zfill<sizeof(T)>(dst + r * SW + c, h, ok && ADV_IN_RANGE(h - p.uin, sxy * nz, p.status));
+      }
+      cp_async_commit();
     } else {
       const bool zok = z >= 0 && z < nz;
       for (int e = tid; e < C::PLANE; e += C::NT) {
@@ -288,7 +330,7 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
   bool row_ok[RY];
 #pragma unroll
   for (int r = 0; r < RY; ++r) row_ok[r] = ya + r < ny;
-  const bool vec_rows = p.vec_ok && xb + VX <= nx;
+  const bool vec_rows = (VX == 1 || p.vec_ok) && xb + VX <= nx;
   // every lane stores whole vectors of existing rows: one uniform branch instead of one per row
   const bool warp_vec_store = __all_sync(0xffffffffu, vec_rows && ya + RY - 1 < ny);
   T* obase = p.out + (size_t)zs * sxy + (size_t)ya * nx + xb;  // output row pointer, plane zs
@@ -337,12 +379,17 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
         for (int e = 0; e < VX; ++e) xr[r][R + e] = WS(RZ)[r][e];
 #pragma unroll
         for (int d = 1; d <= R; ++d) {
+          if constexpr (VX == 1) {  // (a shuffle and its edge lanes would cost more than the load)
+            xr[r][R - d] = row0[r * SW - d];
+            xr[r][R + d] = row0[r * SW + d];
+          } else {
           T lft = __shfl_up_sync(0xffffffffu, WS(RZ)[r][VX - d], 1, C::TX);
           T rgt = __shfl_down_sync(0xffffffffu, WS(RZ)[r][d - 1], 1, C::TX);
           if (tx == 0) lft = row0[r * SW - d];
           if (tx == C::TX - 1) rgt = row0[r * SW + VX - 1 + d];
           xr[r][R - d] = lft;
           xr[r][R + VX - 1 + d] = rgt;
+          }
         }
       }
       // y-neighbourhood: yv[j][e] holds row ya - R + j (j = 0 .. 2R+RY-1); rows ya .. ya+RY-1
@@ -366,38 +413,41 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
       // Every lane evaluates the stencil (halo values outside the grid are finite zero fill);
       // nodes that are not updated are fixed up afterwards with warp-uniform branches.
       T res[RY][VX];
-      if constexpr (sizeof(T) == 4 && ORDER == 2) {
-        // FP32 O2: node pairs (e, e+1) in paired instructions, the same operations lane by lane
-        // (the O4 stencil stays scalar: paired it needs more registers than its occupancy allows)
-        static_assert(VX % 2 == 0, "node pairs");
+      if constexpr (sizeof(T) == 4 && (ORDER == 2 || VX == 1)) {
+        // FP32: nodes in paired instructions, the same operations lane by lane: (e, e+1) of a row, or
+        // rows (r, r+1) with one node per thread (the O4 stencil on vectors stays scalar: paired it
+        // needs more registers than its occupancy allows)
+        constexpr int DR = VX == 1 ? 1 : 0, DE = 1 - DR;
+        static_assert(VX == 1 ? RY % 2 == 0 : VX % 2 == 0, "node pairs");
         constexpr int O1 = R >= 2 ? 2 : 1;
         const float2 kx2 = make_float2(kx, kx), ky2 = make_float2(ky, ky), kz2 = make_float2(kz, kz);
         const float2 dt2 = make_float2(dt, dt);
 #pragma unroll
-        for (int r = 0; r < RY; ++r)
+        for (int r = 0; r < RY; r += 1 + DR)
 #pragma unroll
-          for (int e = 0; e < VX; e += 2) {
-            auto X = [&](int j) { return make_float2(xr[r][j], xr[r][j + 1]); };
-            auto Y = [&](int j) { return make_float2(yv[j][e], yv[j][e + 1]); };
-            auto W = [&](int j) { return make_float2(WS(j)[r][e], WS(j)[r][e + 1]); };
+          for (int e = 0; e < VX; e += 1 + DE) {
+            auto X = [&](int j) { return make_float2(xr[r][e + j], xr[r + DR][e + DE + j]); };
+            auto Y = [&](int j) { return make_float2(yv[r + j][e], yv[r + DR + j][e + DE]); };
+            auto W = [&](int j) { return make_float2(WS(j)[r][e], WS(j)[r + DR][e + DE]); };
             const float2 c = W(RZ);
             const float2 L = lap<float2, ORDER, NDIM, true>(
-                X(R + e - O1), X(R + e - 1), c, X(R + e + 1), X(R + e + O1), Y(R + r - O1), Y(R + r - 1),
-                Y(R + r + 1), Y(R + r + O1), W(RZ >= 2 ? RZ - 2 : 0), W(RZ >= 1 ? RZ - 1 : 0),
-                W(RZ + (RZ >= 1 ? 1 : 0)), W(RZ + (RZ >= 2 ? 2 : 0)), kx2, ky2, kz2);
+                X(R - O1), X(R - 1), c, X(R + 1), X(R + O1), Y(R - O1), Y(R - 1), Y(R + 1), Y(R + O1),
+                W(RZ >= 2 ? RZ - 2 : 0), W(RZ >= 1 ? RZ - 1 : 0), W(RZ + (RZ >= 1 ? 1 : 0)),
+                W(RZ + (RZ >= 2 ? 2 : 0)), kx2, ky2, kz2);
             float2 un = c;
             if (STAGE != 1) {
               const size_t off = (size_t)(q - 2 * RZ) * sxy + (size_t)r * nx + e;
               const T* src = p.un + (obase - p.out) + off;
+              const T* src1 = src + (DR ? (size_t)nx : (size_t)1);
               const bool i0 = (warp_inside || ((inside >> (r * VX + e)) & 1u)) &&
                               ADV_IN_RANGE(src - p.un, sxy * nz, p.status);
-              const bool i1 = (warp_inside || ((inside >> (r * VX + e + 1)) & 1u)) &&
-                              ADV_IN_RANGE(src - p.un + 1, sxy * nz, p.status);
-              un = make_float2(i0 ? src[0] : T(0), i1 ? src[1] : T(0));
+              const bool i1 = (warp_inside || ((inside >> ((r + DR) * VX + e + DE)) & 1u)) &&
+                              ADV_IN_RANGE(src1 - p.un, sxy * nz, p.status);
+              un = make_float2(i0 ? *src : T(0), i1 ? *src1 : T(0));
             }
             const float2 v = combine<float2, true>(stage, un, c, dt2, L);
             res[r][e] = v.x;
-            res[r][e + 1] = v.y;
+            res[r + DR][e + DE] = v.y;
           }
       } else {
 #pragma unroll
@@ -525,18 +575,19 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
 }
 
 // Resident CTAs per SM the register budget is sized for.
-template <class T, int ORDER, int ROWS, int WARPS>
+template <class T, int ORDER, int ROWS, int WARPS, int NODES = 16 / (int)sizeof(T)>
 constexpr int heat_min_ctas() {
+  if (NODES == 1) return sizeof(T) == 8 ? 4 : ORDER == 2 ? 5 : 3;
   return ROWS > 2 ? 16 / WARPS : (ORDER == 2 ? 4 : (sizeof(T) == 4 ? 3 : 2));
 }
 
 // HOOK: the failure-path test's variant (adv_test_heat_stage_withheld); every other launch runs the
 // kernels without it.
 template <class T, int ORDER, int NDIM, bool TMA, int STAGE, int ROWS = 2, int WARPS = 8, int LANES = 32,
-          bool CONTRACT = false, bool HOOK = false>
-__global__ void __launch_bounds__(32 * WARPS, heat_min_ctas<T, ORDER, ROWS, WARPS>())
+          bool CONTRACT = false, bool HOOK = false, int NODES = 16 / (int)sizeof(T)>
+__global__ void __launch_bounds__(32 * WARPS, heat_min_ctas<T, ORDER, ROWS, WARPS, NODES>())
 heat_stage_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ HeatParams<T> p) {
-  using C = HeatTile<T, ORDER, NDIM, ROWS, WARPS, LANES>;
+  using C = HeatTile<T, ORDER, NDIM, ROWS, WARPS, LANES, NODES>;
   uint64_t* bars = heat_bars<T, ORDER, NDIM>();
   int& abort_flag = *heat_abort_flag();
   const int tid = threadIdx.y * C::TX + threadIdx.x;
@@ -560,7 +611,7 @@ heat_stage_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
     const int ze = (int)min((int64_t)p.nz, zs + (seg_b - pos));
     pos += ze - zs;
     const int x0 = (int)(tile % p.tiles_x) * C::BX, y0 = (int)(tile / p.tiles_x) * C::BY;
-    pipe = heat_segment<T, ORDER, NDIM, TMA, STAGE, ROWS, WARPS, LANES, CONTRACT, HOOK>(&tmap, p, x0, y0, zs, ze, pipe);
+    pipe = heat_segment<T, ORDER, NDIM, TMA, STAGE, ROWS, WARPS, LANES, CONTRACT, HOOK, NODES>(&tmap, p, x0, y0, zs, ze, pipe);
     if (pipe.s_issue < 0) return;
   }
 }
