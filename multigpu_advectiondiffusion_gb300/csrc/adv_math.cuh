@@ -55,6 +55,18 @@ __device__ __forceinline__ float2 div3(float2 x) {
 }
 __device__ __forceinline__ float div3(float x) { return __fdiv_rn(x, 3.f); }
 
+// x / h, correctly rounded, from the correctly rounded reciprocal r = RN(1/h) (an IEEE division on the
+// host): one correction makes the quotient faithful, the second rounds it exactly (Markstein, as above);
+// five operations instead of a compiled division's ten. Other ranges (zeros apart) divide.
+__device__ __forceinline__ double div_by(double x, double h, double r) {
+  const double q0 = __dmul_rn(x, r);
+  const double q1 = __fma_rn(__fma_rn(-h, q0, x), r, q0);
+  const double q = __fma_rn(__fma_rn(-h, q1, x), r, q1);
+  const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu, eh = ((unsigned)__double2hiint(h) >> 20) & 0x7ffu;
+  if (ex - 512u < 1024u && eh - 768u < 512u) return q;
+  return x == 0.0 ? x : __ddiv_rn(x, h);
+}
+
 // SSP-RK3 stage combination (stage 1 is forward Euler), operand order of
 // SingleGPU/Diffusion3d_baselineCode/kernels.cu:130-138:
 //   1: un + dt*L;  2: 0.75*un + 0.25*(uin + dt*L);  3: (un + 2*(uin + dt*L)) / 3

@@ -134,19 +134,14 @@ struct Face<double, Z, double> {
     lf_split<double>(u.y, a.y, fp.y, fm.y);
   }
   struct Line {
-    V fp[5], fm[5], fp_new;  // f+ at q-5 .. q-1, f- at q-4 .. q
-    __device__ __forceinline__ void clear() {
-      fp_new = vc<V>(0);
-#pragma unroll
-      for (int s = 0; s < 5; ++s) fp[s] = fm[s] = vc<V>(0);
-    }
-    __device__ __forceinline__ V push(V fpq, V fmq, V, V, bool want) {
-#pragma unroll
-      for (int s = 0; s < 4; ++s) { fp[s] = fp[s + 1]; fm[s] = fm[s + 1]; }
-      fp[4] = fp_new;
-      fp_new = fpq;
-      fm[4] = fmq;
-      return want ? f(fp[0], fp[1], fp[2], fp[3], fp[4], fm[0], fm[1], fm[2], fm[3], fm[4]) : vc<V>(0);
+    WenoRefLine<Z, true> p;
+    WenoRefLine<Z, false> m;
+    V fp_new;  // f+ of the newest plane, one plane behind f-
+    __device__ __forceinline__ void clear() { p.clear(); m.clear(); fp_new = vc<V>(0); }
+    __device__ __forceinline__ V push(V fp, V fm, V, V, bool want) {
+      const V qp = p.push(fp_new, want), qm = m.push(fm, want);
+      fp_new = fp;
+      return vadd(qp, qm);
     }
   };
 };
@@ -494,8 +489,8 @@ __device__ __forceinline__ unsigned burgers_segment(const CUtensorMap* tmap, con
         V L;
         if constexpr (EXACT) {
           auto rhs = [&](T fxm, T fxp, T fym1, T fyp1, T fzm, T fzp) {
-            return sub_rn(sub_rn(div_rn(-sub_rn(fxp, fxm), p.dx), div_rn(sub_rn(fyp1, fym1), p.dy)),
-                          div_rn(sub_rn(fzp, fzm), p.dz));
+            return sub_rn(sub_rn(div_by(-sub_rn(fxp, fxm), p.dx, p.rdx), div_by(sub_rn(fyp1, fym1), p.dy, p.rdy)),
+                          div_by(sub_rn(fzp, fzm), p.dz, p.rdz));
           };
           L = {rhs(fx0.x, fx1.x, fym.x, fyp.x, fz_prev.x, fz.x), rhs(fx0.y, fx1.y, fym.y, fyp.y, fz_prev.y, fz.y)};
         } else {

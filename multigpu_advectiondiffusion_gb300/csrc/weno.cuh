@@ -182,55 +182,88 @@ struct WenoLine {
 };
 
 // ---------------------------------------------------------- reference literal form
-// Operand order of kernels.cu:142-192 / :92-140 (and of the CPU oracle), correctly rounded.
+// Operand order of kernels.cu:142-192 / :92-140 (and of the CPU oracle), every operation rounded on
+// its own. Products by powers of two are exact (short of overflow; the quarter of C*C only ever meets
+// eps = 1e-6 or a tau of the same size), so they go into fused multiply-adds without changing a bit:
+// 52 operations and four divisions per side instead of 66 and four. FP64 is bound by its pipe (two lanes
+// per SM and cycle), so a stage's time follows this count.
 // RECIP: the normalisation of SingleGPU/Burgers3d_WENO5_SharedMem/kernels.cu:51-198, which takes
 // alphasum = 1/(a0 + a1 + a2) and multiplies by (1/6)*alphasum instead of dividing by 6*alphasum.
+
+// The second difference's share of an indicator, 13/12 (a - 2b + c)^2: the same for the three sides
+// that use the triple (a, b, c), always in ascending cell order.
+template <class T>
+__device__ __forceinline__ T weno_ref_k(T a, T b, T c) {
+  const T A = add_rn(fma_rn_(T(-2), b, a), c);
+  return mul_rn(mul_rn(T(13. / 12.), A), A);
+}
+
+// One side from its five cells in ascending order and their three triples' shares. PLUS: f+ (weights
+// 1/10, 6/10, 3/10), else f- on the mirrored candidates (3/10, 6/10, 1/10).
+template <bool Z, class T, bool RECIP, bool PLUS>
+__device__ __forceinline__ T weno_side_ref(T a, T b, T c, T d, T e, T K0, T K1, T K2) {
+  const T eps = T(1e-6);
+  const T c3 = mul_rn(T(3), c);
+  const T C0 = add_rn(fma_rn_(T(-4), b, a), c3), C1 = sub_rn(b, d), C2 = add_rn(fma_rn_(T(-4), d, c3), e);
+  const T B0 = fma_rn_(T(0.25), mul_rn(C0, C0), K0), B1 = fma_rn_(T(0.25), mul_rn(C1, C1), K1),
+          B2 = fma_rn_(T(0.25), mul_rn(C2, C2), K2);
+  const T d0 = T(PLUS ? 1. / 10. : 3. / 10.), d1 = T(6. / 10.), d2 = T(PLUS ? 3. / 10. : 1. / 10.);
+  T a0, a1, a2;
+  if (Z) {
+    const T tau5 = fabs(sub_rn(B0, B2));
+    a0 = mul_rn(d0, add_rn(T(1), div_rn(tau5, add_rn(B0, eps))));
+    a1 = mul_rn(d1, add_rn(T(1), div_rn(tau5, add_rn(B1, eps))));
+    a2 = mul_rn(d2, add_rn(T(1), div_rn(tau5, add_rn(B2, eps))));
+  } else {
+    const T e0 = add_rn(eps, B0), e1 = add_rn(eps, B1), e2 = add_rn(eps, B2);
+    a0 = div_rn(d0, mul_rn(e0, e0));
+    a1 = div_rn(d1, mul_rn(e1, e1));
+    a2 = div_rn(d2, mul_rn(e2, e2));
+  }
+  T q0, q1, q2;
+  if (PLUS) {
+    q0 = add_rn(fma_rn_(T(2), a, -mul_rn(T(7), b)), mul_rn(T(11), c));  // (2a - 7b) + 11c
+    q1 = fma_rn_(T(2), d, add_rn(-b, mul_rn(T(5), c)));                 // (-b + 5c) + 2d
+    q2 = sub_rn(fma_rn_(T(2), c, mul_rn(T(5), d)), e);                  // (2c + 5d) - e
+  } else {
+    q0 = fma_rn_(T(2), c, add_rn(-a, mul_rn(T(5), b)));                 // (-a + 5b) + 2c
+    q1 = sub_rn(fma_rn_(T(2), b, mul_rn(T(5), c)), d);                  // (2b + 5c) - d
+    q2 = fma_rn_(T(2), e, sub_rn(mul_rn(T(11), c), mul_rn(T(7), d)));   // (11c - 7d) + 2e
+  }
+  const T num = add_rn(add_rn(mul_rn(a0, q0), mul_rn(a1, q1)), mul_rn(a2, q2)), sum = add_rn(add_rn(a0, a1), a2);
+  return RECIP ? mul_rn(num, mul_rn(T(1. / 6.), div_rn(T(1), sum))) : div_rn(num, mul_rn(T(6), sum));
+}
+
 template <bool Z, class T, bool RECIP = false>
 __device__ __forceinline__ T weno_face_ref(T vmm, T vm, T v, T vp, T vpp, T umm, T um, T u, T up, T upp) {
-  const T c1312 = T(13. / 12.), c14 = T(1. / 4.), eps = T(1e-6);
-  auto beta = [&](T a, T b, T c, T d, T e, T& B0, T& B1, T& B2) {
-    const T A0 = add_rn(sub_rn(a, mul_rn(T(2), b)), c);
-    const T C0 = add_rn(sub_rn(a, mul_rn(T(4), b)), mul_rn(T(3), c));
-    B0 = add_rn(mul_rn(mul_rn(c1312, A0), A0), mul_rn(mul_rn(c14, C0), C0));
-    const T A1 = add_rn(sub_rn(b, mul_rn(T(2), c)), d);
-    const T C1 = sub_rn(b, d);
-    B1 = add_rn(mul_rn(mul_rn(c1312, A1), A1), mul_rn(mul_rn(c14, C1), C1));
-    const T A2 = add_rn(sub_rn(c, mul_rn(T(2), d)), e);
-    const T C2 = add_rn(sub_rn(mul_rn(T(3), c), mul_rn(T(4), d)), e);
-    B2 = add_rn(mul_rn(mul_rn(c1312, A2), A2), mul_rn(mul_rn(c14, C2), C2));
-  };
-  auto weights = [&](T B0, T B1, T B2, T d0, T d1, T d2, T& a0, T& a1, T& a2) {
-    if (Z) {
-      const T tau5 = fabs(sub_rn(B0, B2));
-      a0 = mul_rn(d0, add_rn(T(1), div_rn(tau5, add_rn(B0, eps))));
-      a1 = mul_rn(d1, add_rn(T(1), div_rn(tau5, add_rn(B1, eps))));
-      a2 = mul_rn(d2, add_rn(T(1), div_rn(tau5, add_rn(B2, eps))));
-    } else {
-      a0 = div_rn(d0, mul_rn(add_rn(eps, B0), add_rn(eps, B0)));
-      a1 = div_rn(d1, mul_rn(add_rn(eps, B1), add_rn(eps, B1)));
-      a2 = div_rn(d2, mul_rn(add_rn(eps, B2), add_rn(eps, B2)));
-    }
-  };
-  T B0, B1, B2, a0, a1, a2;
-  beta(vmm, vm, v, vp, vpp, B0, B1, B2);
-  weights(B0, B1, B2, T(1. / 10.), T(6. / 10.), T(3. / 10.), a0, a1, a2);
-  T asum = add_rn(add_rn(a0, a1), a2);
-  const T q0m = add_rn(sub_rn(mul_rn(T(2), vmm), mul_rn(T(7), vm)), mul_rn(T(11), v));
-  const T q1m = add_rn(add_rn(-vm, mul_rn(T(5), v)), mul_rn(T(2), vp));
-  const T q2m = sub_rn(add_rn(mul_rn(T(2), v), mul_rn(T(5), vp)), vpp);
-  auto normalise = [&](T num, T sum) {
-    return RECIP ? mul_rn(num, mul_rn(T(1. / 6.), div_rn(T(1), sum))) : div_rn(num, mul_rn(T(6), sum));
-  };
-  const T fm = normalise(add_rn(add_rn(mul_rn(a0, q0m), mul_rn(a1, q1m)), mul_rn(a2, q2m)), asum);
-
-  beta(umm, um, u, up, upp, B0, B1, B2);
-  weights(B0, B1, B2, T(3. / 10.), T(6. / 10.), T(1. / 10.), a0, a1, a2);
-  asum = add_rn(add_rn(a0, a1), a2);
-  const T q0p = add_rn(add_rn(-umm, mul_rn(T(5), um)), mul_rn(T(2), u));
-  const T q1p = sub_rn(add_rn(mul_rn(T(2), um), mul_rn(T(5), u)), up);
-  const T q2p = add_rn(sub_rn(mul_rn(T(11), u), mul_rn(T(7), up)), mul_rn(T(2), upp));
-  const T fp = normalise(add_rn(add_rn(mul_rn(a0, q0p), mul_rn(a1, q1p)), mul_rn(a2, q2p)), asum);
+  const T fm = weno_side_ref<Z, T, RECIP, true>(vmm, vm, v, vp, vpp, weno_ref_k(vmm, vm, v), weno_ref_k(vm, v, vp),
+                                                weno_ref_k(v, vp, vpp));
+  const T fp = weno_side_ref<Z, T, RECIP, false>(umm, um, u, up, upp, weno_ref_k(umm, um, u), weno_ref_k(um, u, up),
+                                                 weno_ref_k(u, up, upp));
   return add_rn(fm, fp);
 }
+
+// The literal form along a line: the triples' shares are computed once per cell (K0, K1: of the two
+// triples before the newest). push returns the side of the newest five cells.
+template <bool Z, bool PLUS>
+struct WenoRefLine {
+  double2 f[4], K0, K1;  // the last four cells
+  __device__ __forceinline__ void clear() {
+    const double2 zero = make_double2(0.0, 0.0);
+    K0 = K1 = f[0] = f[1] = f[2] = f[3] = zero;
+  }
+  __device__ __forceinline__ double2 push(double2 n, bool want) {
+    const double2 K2 = make_double2(weno_ref_k(f[2].x, f[3].x, n.x), weno_ref_k(f[2].y, f[3].y, n.y));
+    double2 r = make_double2(0.0, 0.0);
+    if (want) {
+      r.x = weno_side_ref<Z, double, false, PLUS>(f[0].x, f[1].x, f[2].x, f[3].x, n.x, K0.x, K1.x, K2.x);
+      r.y = weno_side_ref<Z, double, false, PLUS>(f[0].y, f[1].y, f[2].y, f[3].y, n.y, K0.y, K1.y, K2.y);
+    }
+    K0 = K1;
+    K1 = K2;
+    f[0] = f[1]; f[1] = f[2]; f[2] = f[3]; f[3] = n;
+    return r;
+  }
+};
 
 }  // namespace adv
