@@ -15,25 +15,31 @@
 // (each face coefficient k_ij = (k_i + k_j)/2 feeds half its derivative to each end). Neighbours
 // outside the domain contribute nothing.
 //
-// Kernels: one thread per (x, y) column over a chunk of z planes, z neighbours from a register
-// window, x/y neighbours from global loads that hit L1 (adjacent threads share them). Every
-// operation is an explicit correctly rounded add/mul/fma, mirrored by the oracle.
+// Kernels (heatk_step_kernel, heatk_adjoint_kernel): a thread owns VX nodes along x (one 16- or 8-byte
+// vector where rows allow it, else one) by RY rows and marches through a chunk of z planes; loads run one
+// plane ahead of their use. What a face needs -- its coefficient, the difference across it and one
+// rounded product -- is computed once and serves both its ends: along z it is carried from plane to
+// plane, along y and x between the thread's own nodes. x neighbours of a vector come from shuffles, y
+// neighbours beyond the thread's rows from global loads that hit L1. No node tests any neighbour: mu is
+// masked when it is loaded, absent neighbours are the centre's own values (the boundary's mu is 0, so
+// their terms vanish as the formulas ask), and boundary nodes are fixed up afterwards in the warps that
+// hold any. Every operation is an explicit correctly rounded add/mul/fma in the oracle's order, FP32 in
+// pairs. Bound by the latency of the loads in flight (192^3 FP32: 12 B per node and step in 16.0 us,
+// 5.3 TB/s out of HBM and L2 together; 24 B per adjoint step in 37.6 us, 4.5 TB/s). The form before this,
+// one thread per column with its neighbours' tests and products per node, was issue bound in its selects:
+// 59 and 171 instructions per node, 20.8 and 48.5 us (191^3, scalar rows: 26.6 -> 20.2 and 78 -> 40.2).
 #include <algorithm>
 #include <cstring>
 #include <initializer_list>
 
+#include "adv_device.cuh"
 #include "adv_internal.h"
-#include "nvtx_range.h"
 #include "adv_math.cuh"
+#include "nvtx_range.h"
 
 namespace adv {
 
 namespace {
-
-constexpr int KX = 32;  // block width; the height (4..16 threads) and the z planes per CTA are tunable
-
-__device__ __forceinline__ float fma_k(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fma_k(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 template <class T>
 struct HeatKArgs {
@@ -45,284 +51,448 @@ struct HeatKArgs {
   int nx, ny, nz, zero_boundary;
   int zc;  // z planes per CTA
   T cx, cy, cz;
+  int* status;
 };
 
-template <class T>
-__global__ void __launch_bounds__(512) heatk_step_kernel(const __grid_constant__ HeatKArgs<T> a) {
-  const int x = blockIdx.x * KX + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= a.nx || y >= a.ny) return;
-  const int z0 = blockIdx.z * a.zc, z1 = min(a.nz, z0 + a.zc);
-  const size_t sx = 1, sy = (size_t)a.nx, sz = (size_t)a.nx * a.ny;
-  const bool col_in = x > 0 && x < a.nx - 1 && y > 0 && y < a.ny - 1;
-  const T h = T(0.5);
-  size_t o = (size_t)x + sy * y + sz * z0;
-  T uc = a.u[o], kc = a.k[o];
-  T um = z0 > 0 ? a.u[o - sz] : uc, km = z0 > 0 ? a.k[o - sz] : kc;
-  for (int z = z0; z < z1; ++z, o += sz) {
-    const T up = z + 1 < a.nz ? a.u[o + sz] : uc, kp = z + 1 < a.nz ? a.k[o + sz] : kc;
-    T res;
-    if (col_in && z > 0 && z < a.nz - 1) {
-      auto flux = [&](T u_p, T u_m, T k_p, T k_m) {
-        const T fp = mul_rn(h, add_rn(kc, k_p)), fm = mul_rn(h, add_rn(kc, k_m));
-        return fma_k(fp, sub_rn(u_p, uc), -mul_rn(fm, sub_rn(uc, u_m)));
-      };
-      const T Fx = flux(a.u[o + sx], a.u[o - sx], a.k[o + sx], a.k[o - sx]);
-      const T Fy = flux(a.u[o + sy], a.u[o - sy], a.k[o + sy], a.k[o - sy]);
-      const T Fz = flux(up, um, kp, km);
-      res = add_rn(uc, fma_k(a.cz, Fz, fma_k(a.cy, Fy, mul_rn(a.cx, Fx))));
-    } else {
-      res = a.zero_boundary ? T(0) : uc;
-    }
-    a.out[o] = res;
-    um = uc; uc = up; km = kc; kc = kp;
+// Resident 256-thread CTAs the register budget is sized for. FP32 adjoint on vectors: two (126
+// registers; three spill and run 81 us at 192^3 against 38).
+template <class T, int VX, bool ADJOINT>
+constexpr int heatk_min_ctas() {
+  return ADJOINT ? (sizeof(T) == 4 && VX == 1 ? 3 : 2) : (sizeof(T) == 4 ? 4 : 3);
+}
+// N values; elementwise operations, FP32 two at a time in paired instructions (each lane rounded like
+// the scalar operation).
+template <class T, int N> struct VN { T v[N]; };
+template <class T, int N, class F2, class F1>
+__device__ __forceinline__ void each(F2 f2, F1 f1) {
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int i = 0; i + 1 < N; i += 2) f2(i);
+    if constexpr (N % 2) f1(N - 1);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) f1(i);
   }
 }
-
-template <class T>
-__global__ void __launch_bounds__(512) heatk_adjoint_kernel(const __grid_constant__ HeatKArgs<T> a) {
-  const int x = blockIdx.x * KX + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= a.nx || y >= a.ny) return;
-  const int z0 = blockIdx.z * a.zc, z1 = min(a.nz, z0 + a.zc);
-  const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const size_t sy = (size_t)nx, sz = (size_t)nx * ny;
-  const T h = T(0.5);
-  // interior tests of this column and of its x / y neighbours' columns
-  auto in1 = [](int i, int n) { return i > 0 && i < n - 1; };
-  const bool xin = in1(x, nx), yin = in1(y, ny);
-  const bool hxp = x + 1 < nx, hxm = x > 0, hyp = y + 1 < ny, hym = y > 0;
-  const bool cxp = in1(x + 1, nx) && yin, cxm = in1(x - 1, nx) && yin;
-  const bool cyp = xin && in1(y + 1, ny), cym = xin && in1(y - 1, ny);
-  const bool ccol = xin && yin;
-  // one axis from the neighbours' values (an absent neighbour passes the centre's values)
-  auto axis = [&](bool hp, bool hm, bool inp, bool inm, T lp, T lm, T up, T um, T kp, T km, T muc, T uc, T kc, T& S,
-                  T& G) {
-    const T mup = hp && inp ? lp : T(0), mum = hm && inm ? lm : T(0);
-    const T kfp = mul_rn(h, add_rn(kc, kp)), kfm = mul_rn(h, add_rn(kc, km));
-    const T dmp = hp ? sub_rn(mup, muc) : T(0), dmm = hm ? sub_rn(mum, muc) : T(0);
-    const T dup = sub_rn(up, uc), dum = sub_rn(um, uc);
-    S = fma_k(kfm, dmm, mul_rn(kfp, dmp));
-    G = fma_k(dum, -dmm, mul_rn(dup, -dmp));
-  };
-  size_t o = (size_t)x + sy * y + sz * z0;
-  // z windows of lam, u, k at z-1, z, z+1
-  T lc = a.lam[o], uc = a.u[o], kc = a.k[o];
-  T lm = z0 > 0 ? a.lam[o - sz] : lc, um = z0 > 0 ? a.u[o - sz] : uc, km = z0 > 0 ? a.k[o - sz] : kc;
-  for (int z = z0; z < z1; ++z, o += sz) {
-    const bool hzp = z + 1 < nz, hzm = z > 0;
-    const T lp = hzp ? a.lam[o + sz] : lc, up = hzp ? a.u[o + sz] : uc, kp = hzp ? a.k[o + sz] : kc;
-    const bool zin = in1(z, nz);
-    const bool in_c = ccol && zin;
-    const T muc = in_c ? lc : T(0);
-    const size_t ox = hxp ? o + 1 : o, oxm = hxm ? o - 1 : o, oy = hyp ? o + sy : o, oym = hym ? o - sy : o;
-    T Sx, Gx, Sy, Gy, Sz, Gz;
-    axis(hxp, hxm, cxp && zin, cxm && zin, a.lam[ox], a.lam[oxm], a.u[ox], a.u[oxm], a.k[ox], a.k[oxm], muc, uc, kc,
-         Sx, Gx);
-    axis(hyp, hym, cyp && zin, cym && zin, a.lam[oy], a.lam[oym], a.u[oy], a.u[oym], a.k[oy], a.k[oym], muc, uc, kc,
-         Sy, Gy);
-    axis(hzp, hzm, ccol && in1(z + 1, nz), ccol && in1(z - 1, nz), lp, lm, up, um, kp, km, muc, uc, kc, Sz, Gz);
-    const T keep = (in_c || !a.zero_boundary) ? lc : T(0);
-    a.out[o] = add_rn(keep, fma_k(a.cz, Sz, fma_k(a.cy, Sy, mul_rn(a.cx, Sx))));
-    a.grad[o] = fma_k(h, fma_k(a.cz, Gz, fma_k(a.cy, Gy, mul_rn(a.cx, Gx))), a.grad[o]);
-    lm = lc; lc = lp; um = uc; uc = up; km = kc; kc = kp;
-  }
+template <class T, int N> __device__ __forceinline__ float2 pr(const VN<T, N>& a, int i) { return make_float2(a.v[i], a.v[i + 1]); }
+#define ADV_VN_PUT(r, i, w) do { const float2 w_ = (w); r.v[i] = w_.x; r.v[(i) + 1] = w_.y; } while (0)
+template <class T, int N>
+__device__ __forceinline__ VN<T, N> vadd(const VN<T, N>& a, const VN<T, N>& b) {
+  VN<T, N> r;
+  each<T, N>([&](int i) { ADV_VN_PUT(r, i, add_rn(pr(a, i), pr(b, i))); }, [&](int i) { r.v[i] = add_rn(a.v[i], b.v[i]); });
+  return r;
 }
+template <class T, int N>
+__device__ __forceinline__ VN<T, N> vsub(const VN<T, N>& a, const VN<T, N>& b) {
+  VN<T, N> r;
+  each<T, N>([&](int i) { ADV_VN_PUT(r, i, sub_rn(pr(a, i), pr(b, i))); }, [&](int i) { r.v[i] = sub_rn(a.v[i], b.v[i]); });
+  return r;
+}
+template <class T, int N>
+__device__ __forceinline__ VN<T, N> vmul(const VN<T, N>& a, const VN<T, N>& b) {
+  VN<T, N> r;
+  each<T, N>([&](int i) { ADV_VN_PUT(r, i, mul_rn(pr(a, i), pr(b, i))); }, [&](int i) { r.v[i] = mul_rn(a.v[i], b.v[i]); });
+  return r;
+}
+template <class T, int N>
+__device__ __forceinline__ VN<T, N> vscale(T s, const VN<T, N>& a) {
+  VN<T, N> r;
+  each<T, N>([&](int i) { ADV_VN_PUT(r, i, mul_rn(make_float2(s, s), pr(a, i))); }, [&](int i) { r.v[i] = mul_rn(s, a.v[i]); });
+  return r;
+}
+template <class T, int N>
+__device__ __forceinline__ VN<T, N> vfma(const VN<T, N>& a, const VN<T, N>& b, const VN<T, N>& c) {
+  VN<T, N> r;
+  each<T, N>([&](int i) { ADV_VN_PUT(r, i, __ffma2_rn(pr(a, i), pr(b, i), pr(c, i))); },
+             [&](int i) { r.v[i] = fma_rn_(a.v[i], b.v[i], c.v[i]); });
+  return r;
+}
+template <class T, int N>
+__device__ __forceinline__ VN<T, N> vaxpy(T s, const VN<T, N>& a, const VN<T, N>& c) {
+  VN<T, N> r;
+  each<T, N>([&](int i) { ADV_VN_PUT(r, i, __ffma2_rn(make_float2(s, s), pr(a, i), pr(c, i))); },
+             [&](int i) { r.v[i] = fma_rn_(s, a.v[i], c.v[i]); });
+  return r;
+}
+#undef ADV_VN_PUT
 
-// ------------------------------------------------------------ vector kernels (16-byte rows)
-// The same per-node arithmetic as the kernels above (so the same bits), with each thread owning
-// VX = 16 / sizeof(T) consecutive nodes of a row: one 16-byte load per field and row instead of
-// one per node, the nodes' x neighbours from the thread's own vector plus one scalar per side.
-// Used when nx is a multiple of VX and every array is 16-byte aligned.
-template <class T> struct V16;
-template <> struct V16<float> { using type = float4; static constexpr int N = 4; };
-template <> struct V16<double> { using type = double2; static constexpr int N = 2; };
-constexpr int KXV = 16;  // threads per block row
-// FP32 adjoint rows in 8-byte vectors (two nodes per thread): half the registers of 16-byte
-// vectors (56 instead of 101), so twice the resident warps to cover the latency of its seven
-// input streams (measured 11% faster at 192^3)
-constexpr int kAdjVxF32 = 2;
-
-// vector of N elements of T in one load / store (N * sizeof(T) = 8 or 16 bytes)
-template <class T, int N> struct VecN;
+// VX nodes in one access (VX * sizeof(T) = 16 or 8 bytes, or one node).
+template <class T, int N> struct VecN { using type = T; };
 template <> struct VecN<float, 4> { using type = float4; };
 template <> struct VecN<float, 2> { using type = float2; };
 template <> struct VecN<double, 2> { using type = double2; };
 template <class T, int N>
-__device__ __forceinline__ void ldvn(const T* p, T (&v)[N]) {
+__device__ __forceinline__ VN<T, N> ldv(const T* p) {
   const typename VecN<T, N>::type w = *reinterpret_cast<const typename VecN<T, N>::type*>(p);
+  VN<T, N> r;
 #pragma unroll
-  for (int e = 0; e < N; ++e) v[e] = reinterpret_cast<const T*>(&w)[e];
+  for (int e = 0; e < N; ++e) r.v[e] = reinterpret_cast<const T*>(&w)[e];
+  return r;
 }
 template <class T, int N>
-__device__ __forceinline__ void stvn(T* p, const T (&v)[N]) {
+__device__ __forceinline__ void stv(T* p, const VN<T, N>& v) {
   typename VecN<T, N>::type w;
 #pragma unroll
-  for (int e = 0; e < N; ++e) reinterpret_cast<T*>(&w)[e] = v[e];
+  for (int e = 0; e < N; ++e) reinterpret_cast<T*>(&w)[e] = v.v[e];
   *reinterpret_cast<typename VecN<T, N>::type*>(p) = w;
 }
 
-template <class T>
-__device__ __forceinline__ void ldv(const T* p, T (&v)[V16<T>::N]) {
-  const typename V16<T>::type w = *reinterpret_cast<const typename V16<T>::type*>(p);
+// A thread's nodes and what its neighbours are. LX: threads per block row.
+template <class T, int VX, int RY, int LX>
+struct HeatKThread {
+  static constexpr int N = RY * VX;
+  int x, y, z0, z1;
+  int nx, ny, nz;
+  int64_t sz;
+  int64_t first;     // offset of its first node in the grid's first plane (clamped to the grid)
+  int dr[RY];        // its rows' offsets from the first (rows past the grid: the last one) ..
+  int above, below;  // .. and those of the rows y-1 and y+RY (clamped to its own first / last)
+  bool ok[RY];       // the row is on the grid (and so are all VX nodes)
+  int left, right;   // offsets of the nodes x-1 and x+VX (clamped)
+  int tx;
+  __device__ __forceinline__ bool init(int gnx, int gny, int gnz, int zc) {
+    tx = threadIdx.x;
+    nx = gnx; ny = gny; nz = gnz;
+    x = (blockIdx.x * LX + tx) * VX;
+    y = (blockIdx.y * blockDim.y + threadIdx.y) * RY;
+    z0 = blockIdx.z * zc;
+    z1 = min(nz, z0 + zc);
+    sz = (int64_t)nx * ny;
+    const bool any = x < nx && y < ny;
+    const int xc = min(x, nx - VX), yc = min(y, ny - 1);  // threads past the grid read its last nodes (shuffles)
+    first = (int64_t)yc * nx + xc;
 #pragma unroll
-  for (int e = 0; e < V16<T>::N; ++e) v[e] = reinterpret_cast<const T*>(&w)[e];
-}
-template <class T>
-__device__ __forceinline__ void stv(T* p, const T (&v)[V16<T>::N]) {
-  typename V16<T>::type w;
-#pragma unroll
-  for (int e = 0; e < V16<T>::N; ++e) reinterpret_cast<T*>(&w)[e] = v[e];
-  *reinterpret_cast<typename V16<T>::type*>(p) = w;
-}
-
-template <class T>
-__global__ void __launch_bounds__(256) heatk_step_vec_kernel(const __grid_constant__ HeatKArgs<T> a) {
-  constexpr int VX = V16<T>::N;
-  const int xb = (blockIdx.x * KXV + threadIdx.x) * VX, y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (xb >= a.nx || y >= a.ny) return;
-  const int z0 = blockIdx.z * a.zc, z1 = min(a.nz, z0 + a.zc);
-  const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const size_t sy = (size_t)nx, sz = (size_t)nx * ny;
-  const T h = T(0.5);
-  const bool yin = y > 0 && y < ny - 1;
-  const bool hl = xb > 0, hr = xb + VX < nx;
-  size_t o = (size_t)xb + sy * y + sz * z0;
-  T uc[VX], kc[VX], um[VX], km[VX];
-  ldv(a.u + o, uc);
-  ldv(a.k + o, kc);
-  if (z0 > 0) { ldv(a.u + o - sz, um); ldv(a.k + o - sz, km); }
-  else {
-#pragma unroll
-    for (int e = 0; e < VX; ++e) { um[e] = uc[e]; km[e] = kc[e]; }
-  }
-  for (int z = z0; z < z1; ++z, o += sz) {
-    T up[VX], kp[VX];
-    if (z + 1 < nz) { ldv(a.u + o + sz, up); ldv(a.k + o + sz, kp); }
-    else {
-#pragma unroll
-      for (int e = 0; e < VX; ++e) { up[e] = uc[e]; kp[e] = kc[e]; }
+    for (int r = 0; r < RY; ++r) {
+      ok[r] = any && y + r < ny;
+      dr[r] = (min(yc + r, ny - 1) - yc) * nx;
     }
-    T res[VX];
-    const bool zin = z > 0 && z < nz - 1;
-    if (yin && zin) {
-      T uyp[VX], uym[VX], kyp[VX], kym[VX];
-      ldv(a.u + o + sy, uyp); ldv(a.u + o - sy, uym); ldv(a.k + o + sy, kyp); ldv(a.k + o - sy, kym);
-      const T ul = hl ? a.u[o - 1] : T(0), kl = hl ? a.k[o - 1] : T(0);
-      const T ur = hr ? a.u[o + VX] : T(0), kr = hr ? a.k[o + VX] : T(0);
+    above = yc > 0 ? -nx : 0;
+    below = (min(yc + RY, ny - 1) - yc) * nx;
+    left = xc > 0 ? -1 : 0;
+    right = xc + VX < nx ? VX : VX - 1;
+    return any;
+  }
+  // a field's pointer at this thread's first node of plane z (at most the last plane)
+  __device__ __forceinline__ const T* at(const T* f, int z) const { return f + (int64_t)min(z, nz - 1) * sz + first; }
+  __device__ __forceinline__ VN<T, N> plane(const T* p) const {  // its nodes of a plane
+    VN<T, N> a;
 #pragma unroll
-      for (int e = 0; e < VX; ++e) {
-        const int x = xb + e;
-        if (x > 0 && x < nx - 1) {
-          const T c = uc[e], kce = kc[e];
-          auto flux = [&](T u_p, T u_m, T k_p, T k_m) {
-            const T fp = mul_rn(h, add_rn(kce, k_p)), fm = mul_rn(h, add_rn(kce, k_m));
-            return fma_k(fp, sub_rn(u_p, c), -mul_rn(fm, sub_rn(c, u_m)));
-          };
-          const T uxp = e + 1 < VX ? uc[e + 1 < VX ? e + 1 : 0] : ur, kxp = e + 1 < VX ? kc[e + 1 < VX ? e + 1 : 0] : kr;
-          const T uxm = e > 0 ? uc[e > 0 ? e - 1 : 0] : ul, kxm = e > 0 ? kc[e > 0 ? e - 1 : 0] : kl;
-          const T Fx = flux(uxp, uxm, kxp, kxm);
-          const T Fy = flux(uyp[e], uym[e], kyp[e], kym[e]);
-          const T Fz = flux(up[e], um[e], kp[e], km[e]);
-          res[e] = add_rn(c, fma_k(a.cz, Fz, fma_k(a.cy, Fy, mul_rn(a.cx, Fx))));
-        } else {
-          res[e] = a.zero_boundary ? T(0) : uc[e];
-        }
+    for (int r = 0; r < RY; ++r) {
+      const VN<T, VX> w = ldv<T, VX>(p + dr[r]);
+#pragma unroll
+      for (int e = 0; e < VX; ++e) a.v[r * VX + e] = w.v[e];
+    }
+    return a;
+  }
+  // the values left and right of each of its rows (at the ends of the grid: its own end nodes)
+  __device__ __forceinline__ void sides(const T* p, const VN<T, N>& c, T (&l)[RY], T (&r)[RY]) const {
+#pragma unroll
+    for (int j = 0; j < RY; ++j) {
+      if constexpr (VX == 1) {
+        l[j] = p[dr[j] + left];
+        r[j] = p[dr[j] + right];
+      } else {
+        l[j] = __shfl_up_sync(0xffffffffu, c.v[j * VX + VX - 1], 1, LX);
+        r[j] = __shfl_down_sync(0xffffffffu, c.v[j * VX], 1, LX);
+        if (tx == 0) l[j] = p[dr[j] + left];
+        if (tx == LX - 1) r[j] = p[dr[j] + right];
       }
+    }
+  }
+};
+
+template <class T, int VX, int RY, int LX>
+__global__ void __launch_bounds__(256, heatk_min_ctas<T, VX, false>()) heatk_step_kernel(const __grid_constant__ HeatKArgs<T> a) {
+  using Th = HeatKThread<T, VX, RY, LX>;
+  constexpr int N = Th::N;
+  using V = VN<T, N>;
+  Th t;
+  const bool any = t.init(a.nx, a.ny, a.nz, a.zc);
+  const T h = T(0.5);
+  const int nx = a.nx, ny = a.ny, nz = a.nz;
+  bool fixed = false;  // some node of this thread on the x or y boundary
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int gx = t.x + i % VX, gy = t.y + i / VX;
+    fixed |= gx <= 0 || gx >= nx - 1 || gy <= 0 || gy >= ny - 1;
+  }
+  const bool warp_fixed = __any_sync(0xffffffffu, fixed);
+  const T* pu = t.at(a.u, t.z0);  // plane z, and two planes ahead
+  const T* pk = t.at(a.k, t.z0);
+  const T* pu2 = t.at(a.u, t.z0 + 2);
+  const T* pk2 = t.at(a.k, t.z0 + 2);
+  T* po = a.out + (pu - a.u);
+  V uc = t.plane(pu), kc = t.plane(pk);
+  V up = t.plane(t.at(a.u, t.z0 + 1)), kp = t.plane(t.at(a.k, t.z0 + 1));
+  V npz;  // negated rounded product of the face below the plane
+  {
+    const int zm = max(t.z0 - 1, 0);
+    const V um = t.plane(t.at(a.u, zm)), km = t.plane(t.at(a.k, zm));
+    npz = vmul(vscale(h, vadd(kc, km)), vsub(um, uc));
+  }
+  for (int z = t.z0; z < t.z1; ++z) {
+    const V un = t.plane(pu2), kn = t.plane(pk2);  // used by the next plane
+    const VN<T, VX> ua = ldv<T, VX>(pu + t.above), ub = ldv<T, VX>(pu + t.below);
+    const VN<T, VX> ka = ldv<T, VX>(pk + t.above), kb = ldv<T, VX>(pk + t.below);
+    T ul[RY], ur[RY], kl[RY], kr[RY];
+    t.sides(pu, uc, ul, ur);
+    t.sides(pk, kc, kl, kr);
+    // per axis F = kf_p (u_p - u) - rn(kf_m (u - u_m)), the second term negated as kf_m (u_m - u)
+    V Fx, Fy, Fz;
+    {
+      const V kf = vscale(h, vadd(kc, kp));
+      Fz = vfma(kf, vsub(up, uc), npz);
+      npz = vmul(kf, vsub(uc, up));
+    }
+    if constexpr (VX == 1) {
+      V L, R, KL, KR;
+#pragma unroll
+      for (int j = 0; j < RY; ++j) { L.v[j] = ul[j]; R.v[j] = ur[j]; KL.v[j] = kl[j]; KR.v[j] = kr[j]; }
+      Fx = vfma(vscale(h, vadd(kc, KR)), vsub(R, uc), vmul(vscale(h, vadd(kc, KL)), vsub(L, uc)));
     } else {
 #pragma unroll
-      for (int e = 0; e < VX; ++e) res[e] = a.zero_boundary ? T(0) : uc[e];
-    }
-    stv(a.out + o, res);
+      for (int j = 0; j < RY; ++j) {
+        T np = mul_rn(mul_rn(h, add_rn(kc.v[j * VX], kl[j])), sub_rn(ul[j], uc.v[j * VX]));
 #pragma unroll
-    for (int e = 0; e < VX; ++e) { um[e] = uc[e]; uc[e] = up[e]; km[e] = kc[e]; kc[e] = kp[e]; }
+        for (int e = 0; e < VX; ++e) {
+          const int i = j * VX + e;
+          const T u1 = e + 1 < VX ? uc.v[e + 1 < VX ? i + 1 : i] : ur[j], k1 = e + 1 < VX ? kc.v[e + 1 < VX ? i + 1 : i] : kr[j];
+          const T kf = mul_rn(h, add_rn(kc.v[i], k1)), d = sub_rn(u1, uc.v[i]);
+          Fx.v[i] = fma_rn_(kf, d, np);
+          np = mul_rn(kf, -d);
+        }
+      }
+    }
+    {
+      VN<T, VX> u0, k0;  // the row above
+      auto rowv = [&](const V& f, int j) {
+        VN<T, VX> w;
+#pragma unroll
+        for (int e = 0; e < VX; ++e) w.v[e] = f.v[j * VX + e];
+        return w;
+      };
+      u0 = rowv(uc, 0); k0 = rowv(kc, 0);
+      VN<T, VX> np = vmul(vscale(h, vadd(k0, ka)), vsub(ua, u0));
+#pragma unroll
+      for (int j = 0; j < RY; ++j) {
+        const VN<T, VX> u1 = j + 1 < RY ? rowv(uc, j + 1 < RY ? j + 1 : j) : ub, k1 = j + 1 < RY ? rowv(kc, j + 1 < RY ? j + 1 : j) : kb;
+        const VN<T, VX> kf = vscale(h, vadd(k0, k1));
+        const VN<T, VX> F = vfma(kf, vsub(u1, u0), np);
+        np = vmul(kf, vsub(u0, u1));
+#pragma unroll
+        for (int e = 0; e < VX; ++e) Fy.v[j * VX + e] = F.v[e];
+        u0 = u1; k0 = k1;
+      }
+    }
+    V res = vadd(uc, vaxpy(a.cz, Fz, vaxpy(a.cy, Fy, vscale(a.cx, Fx))));
+    const bool zfix = z == 0 || z == nz - 1;
+    if (warp_fixed || zfix) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const int gx = t.x + i % VX, gy = t.y + i / VX;
+        if (zfix || gx <= 0 || gx >= nx - 1 || gy <= 0 || gy >= ny - 1) res.v[i] = a.zero_boundary ? T(0) : uc.v[i];
+      }
+    }
+    if (any) {
+#pragma unroll
+      for (int j = 0; j < RY; ++j)
+        if (t.ok[j]) {
+          VN<T, VX> w;
+#pragma unroll
+          for (int e = 0; e < VX; ++e) w.v[e] = res.v[j * VX + e];
+          if (ADV_IN_RANGE(po - a.out + t.dr[j] + VX - 1, t.sz * nz, a.status)) stv<T, VX>(po + t.dr[j], w);
+        }
+    }
+    uc = up; up = un; kc = kp; kp = kn;
+    pu += t.sz; pk += t.sz; po += t.sz;
+    if (z + 3 < nz) { pu2 += t.sz; pk2 += t.sz; }
   }
 }
 
-template <class T, int VXN = V16<T>::N>
-__global__ void __launch_bounds__(256) heatk_adjoint_vec_kernel(const __grid_constant__ HeatKArgs<T> a) {
-  constexpr int VX = VXN;
-  const int xb = (blockIdx.x * blockDim.x + threadIdx.x) * VX, y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (xb >= a.nx || y >= a.ny) return;
-  const int z0 = blockIdx.z * a.zc, z1 = min(a.nz, z0 + a.zc);
-  const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const size_t sy = (size_t)nx, sz = (size_t)nx * ny;
+template <class T, int VX, int RY, int LX>
+__global__ void __launch_bounds__(256, heatk_min_ctas<T, VX, true>()) heatk_adjoint_kernel(const __grid_constant__ HeatKArgs<T> a) {
+  using Th = HeatKThread<T, VX, RY, LX>;
+  constexpr int N = Th::N;
+  using V = VN<T, N>;
+  Th t;
+  const bool any = t.init(a.nx, a.ny, a.nz, a.zc);
   const T h = T(0.5);
+  const int nx = a.nx, ny = a.ny, nz = a.nz;
   auto in1 = [](int i, int n) { return i > 0 && i < n - 1; };
-  const bool yin = in1(y, ny), hyp = y + 1 < ny, hym = y > 0;
-  const bool hl = xb > 0, hr = xb + VX < nx;
-  auto axis = [&](bool hp, bool hm, bool inp, bool inm, T lp, T lm, T up, T um, T kp, T km, T muc, T uc, T kc, T& S,
-                  T& G) {
-    const T mup = hp && inp ? lp : T(0), mum = hm && inm ? lm : T(0);
-    const T kfp = mul_rn(h, add_rn(kc, kp)), kfm = mul_rn(h, add_rn(kc, km));
-    const T dmp = hp ? sub_rn(mup, muc) : T(0), dmm = hm ? sub_rn(mum, muc) : T(0);
-    const T dup = sub_rn(up, uc), dum = sub_rn(um, uc);
-    S = fma_k(kfm, dmm, mul_rn(kfp, dmp));
-    G = fma_k(dum, -dmm, mul_rn(dup, -dmp));
-  };
-  size_t o = (size_t)xb + sy * y + sz * z0;
-  T lc[VX], uc[VX], kc[VX], lm[VX], um[VX], km[VX];
-  ldvn<T, VX>(a.lam + o, lc); ldvn<T, VX>(a.u + o, uc); ldvn<T, VX>(a.k + o, kc);
-  if (z0 > 0) { ldvn<T, VX>(a.lam + o - sz, lm); ldvn<T, VX>(a.u + o - sz, um); ldvn<T, VX>(a.k + o - sz, km); }
-  else {
+  // which nodes of this thread (bit i), of the rows beside it and of the columns beside it lie off the
+  // x and y boundary; warps without a boundary node anywhere near need no masks
+  unsigned inb = 0, ina = 0, inl = 0, inr = 0, inbl = 0;
 #pragma unroll
-    for (int e = 0; e < VX; ++e) { lm[e] = lc[e]; um[e] = uc[e]; km[e] = kc[e]; }
+  for (int i = 0; i < N; ++i)
+    if (in1(t.x + i % VX, nx) && in1(t.y + i / VX, ny)) inb |= 1u << i;
+#pragma unroll
+  for (int e = 0; e < VX; ++e) {
+    if (in1(t.x + e, nx) && in1(t.y - 1, ny)) ina |= 1u << e;
+    if (in1(t.x + e, nx) && in1(t.y + RY, ny)) inbl |= 1u << e;
   }
-  for (int z = z0; z < z1; ++z, o += sz) {
-    const bool hzp = z + 1 < nz, hzm = z > 0;
-    T lp[VX], up[VX], kp[VX];
-    if (hzp) { ldvn<T, VX>(a.lam + o + sz, lp); ldvn<T, VX>(a.u + o + sz, up); ldvn<T, VX>(a.k + o + sz, kp); }
-    else {
 #pragma unroll
-      for (int e = 0; e < VX; ++e) { lp[e] = lc[e]; up[e] = uc[e]; kp[e] = kc[e]; }
-    }
-    // y neighbours (an absent one passes the centre's values, as in the scalar kernel)
-    T lyp[VX], uyp[VX], kyp[VX], lym[VX], uym[VX], kym[VX];
-    if (hyp) { ldvn<T, VX>(a.lam + o + sy, lyp); ldvn<T, VX>(a.u + o + sy, uyp); ldvn<T, VX>(a.k + o + sy, kyp); }
-    else {
+  for (int j = 0; j < RY; ++j) {
+    if (in1(t.x - 1, nx) && in1(t.y + j, ny)) inl |= 1u << j;
+    if (in1(t.x + VX, nx) && in1(t.y + j, ny)) inr |= 1u << j;
+  }
+  constexpr unsigned ALL = (1u << N) - 1u, ROW = (1u << VX) - 1u, COL = (1u << RY) - 1u;
+  const bool warp_masked = __any_sync(0xffffffffu, inb != ALL || ina != ROW || inbl != ROW || inl != COL || inr != COL);
+  auto mask = [&](V m, int z) {  // lam of plane z -> mu
+    if (warp_masked || !in1(z, nz)) {
+      const unsigned b = in1(z, nz) ? inb : 0u;
 #pragma unroll
-      for (int e = 0; e < VX; ++e) { lyp[e] = lc[e]; uyp[e] = uc[e]; kyp[e] = kc[e]; }
+      for (int i = 0; i < N; ++i) m.v[i] = (b >> i) & 1u ? m.v[i] : T(0);
     }
-    if (hym) { ldvn<T, VX>(a.lam + o - sy, lym); ldvn<T, VX>(a.u + o - sy, uym); ldvn<T, VX>(a.k + o - sy, kym); }
-    else {
+    return m;
+  };
+  const T* pu = t.at(a.u, t.z0);  // plane z, and two planes ahead
+  const T* pk = t.at(a.k, t.z0);
+  const T* pl = t.at(a.lam, t.z0);
+  const T* pu2 = t.at(a.u, t.z0 + 2);
+  const T* pk2 = t.at(a.k, t.z0 + 2);
+  const T* pl2 = t.at(a.lam, t.z0 + 2);
+  T* po = a.out + (pu - a.u);
+  T* pg = a.grad + (pu - a.u);
+  V uc = t.plane(pu), kc = t.plane(pk), mc = mask(t.plane(pl), t.z0);
+  V kfz, dmz, duz;  // the face below the plane: coefficient, mu and u differences (upper - lower)
+  {
+    const int zm = max(t.z0 - 1, 0);
+    const V um = t.plane(t.at(a.u, zm)), km = t.plane(t.at(a.k, zm));
+    const V mm = t.z0 > 0 ? mask(t.plane(t.at(a.lam, zm)), zm) : mc;
+    kfz = vscale(h, vadd(kc, km));
+    dmz = vsub(mc, mm);
+    duz = vsub(uc, um);
+  }
+  V up, kp, mp;
+  {
+    const int zp = min(t.z0 + 1, nz - 1);
+    up = t.plane(t.at(a.u, zp)); kp = t.plane(t.at(a.k, zp));
+    mp = mask(t.plane(t.at(a.lam, zp)), zp);
+  }
+  for (int z = t.z0; z < t.z1; ++z) {
+    const int z2 = min(z + 2, nz - 1);
+    const V un = t.plane(pu2), kn = t.plane(pk2), ln = t.plane(pl2);  // used by the next plane
+    const V g = t.plane(pg);
+    const VN<T, VX> ua = ldv<T, VX>(pu + t.above), ub = ldv<T, VX>(pu + t.below);
+    const VN<T, VX> ka = ldv<T, VX>(pk + t.above), kb = ldv<T, VX>(pk + t.below);
+    VN<T, VX> ma = ldv<T, VX>(pl + t.above), mb = ldv<T, VX>(pl + t.below);
+    T ul[RY], ur[RY], kl[RY], kr[RY], ml[RY], mr[RY];
+    t.sides(pu, uc, ul, ur);
+    t.sides(pk, kc, kl, kr);
+    t.sides(pl, mc, ml, mr);
+    const bool zin = in1(z, nz);
+    if (warp_masked || !zin) {
 #pragma unroll
-      for (int e = 0; e < VX; ++e) { lym[e] = lc[e]; uym[e] = uc[e]; kym[e] = kc[e]; }
-    }
-    const T ll = hl ? a.lam[o - 1] : T(0), ul = hl ? a.u[o - 1] : T(0), kl = hl ? a.k[o - 1] : T(0);
-    const T lr = hr ? a.lam[o + VX] : T(0), ur = hr ? a.u[o + VX] : T(0), kr = hr ? a.k[o + VX] : T(0);
-    T g[VX], out[VX];
-    ldvn<T, VX>(a.grad + o, g);
-    const bool zin = in1(z, nz), zinp = in1(z + 1, nz), zinm = in1(z - 1, nz);
+      for (int e = 0; e < VX; ++e) {
+        if (!zin || !((ina >> e) & 1u)) ma.v[e] = T(0);
+        if (!zin || !((inbl >> e) & 1u)) mb.v[e] = T(0);
+      }
 #pragma unroll
-    for (int e = 0; e < VX; ++e) {
-      const int x = xb + e;
-      const bool xin = in1(x, nx), hxp = x + 1 < nx, hxm = x > 0;
-      const bool ccol = xin && yin;
-      const bool in_c = ccol && zin;
-      const T muc = in_c ? lc[e] : T(0);
-      // x neighbours of node e: inside the vector, or the scalars past its ends
-      const T lxp = hxp ? (e + 1 < VX ? lc[e + 1 < VX ? e + 1 : 0] : lr) : lc[e];
-      const T uxp = hxp ? (e + 1 < VX ? uc[e + 1 < VX ? e + 1 : 0] : ur) : uc[e];
-      const T kxp = hxp ? (e + 1 < VX ? kc[e + 1 < VX ? e + 1 : 0] : kr) : kc[e];
-      const T lxm = hxm ? (e > 0 ? lc[e > 0 ? e - 1 : 0] : ll) : lc[e];
-      const T uxm = hxm ? (e > 0 ? uc[e > 0 ? e - 1 : 0] : ul) : uc[e];
-      const T kxm = hxm ? (e > 0 ? kc[e > 0 ? e - 1 : 0] : kl) : kc[e];
-      T Sx, Gx, Sy, Gy, Sz, Gz;
-      axis(hxp, hxm, in1(x + 1, nx) && yin && zin, in1(x - 1, nx) && yin && zin, lxp, lxm, uxp, uxm, kxp, kxm, muc,
-           uc[e], kc[e], Sx, Gx);
-      axis(hyp, hym, xin && in1(y + 1, ny) && zin, xin && in1(y - 1, ny) && zin, lyp[e], lym[e], uyp[e], uym[e],
-           kyp[e], kym[e], muc, uc[e], kc[e], Sy, Gy);
-      axis(hzp, hzm, ccol && zinp, ccol && zinm, lp[e], lm[e], up[e], um[e], kp[e], km[e], muc, uc[e], kc[e], Sz, Gz);
-      const T keep = (in_c || !a.zero_boundary) ? lc[e] : T(0);
-      out[e] = add_rn(keep, fma_k(a.cz, Sz, fma_k(a.cy, Sy, mul_rn(a.cx, Sx))));
-      g[e] = fma_k(h, fma_k(a.cz, Gz, fma_k(a.cy, Gy, mul_rn(a.cx, Gx))), g[e]);
+      for (int j = 0; j < RY; ++j) {
+        if (!zin || !((inl >> j) & 1u)) ml[j] = T(0);
+        if (!zin || !((inr >> j) & 1u)) mr[j] = T(0);
+      }
     }
-    stvn<T, VX>(a.out + o, out);
-    stvn<T, VX>(a.grad + o, g);
+    // Per axis S = kf_m (mu_m - mu) + rn(kf_p (mu_p - mu)), G = (u_m - u) (mu - mu_m) + rn((u_p - u)(mu - mu_p)):
+    // a face with differences dm, du (upper - lower) gives its lower end rn(kf dm) and rn(du (-dm)),
+    // its upper end kf (-dm) and (-du) dm, all in the signs of the formulas.
+    V Sx, Gx, Sy, Gy, Sz, Gz;
+    auto ends = [&](auto kf0, auto dm0, auto du0, auto kf1, auto dm1, auto du1, auto& S, auto& G) {
+      auto neg = [](auto v) {
 #pragma unroll
-    for (int e = 0; e < VX; ++e) {
-      lm[e] = lc[e]; lc[e] = lp[e]; um[e] = uc[e]; uc[e] = up[e]; km[e] = kc[e]; kc[e] = kp[e];
+        for (auto& e : v.v) e = -e;
+        return v;
+      };
+      S = vfma(kf0, neg(dm0), vmul(kf1, dm1));
+      G = vfma(neg(du0), dm0, vmul(du1, neg(dm1)));
+    };
+    {
+      const V kf = vscale(h, vadd(kc, kp)), dm = vsub(mp, mc), du = vsub(up, uc);
+      ends(kfz, dmz, duz, kf, dm, du, Sz, Gz);
+      kfz = kf; dmz = dm; duz = du;
     }
+    if constexpr (VX == 1) {
+      V L, R, KL, KR, ML, MR;
+#pragma unroll
+      for (int j = 0; j < RY; ++j) {
+        L.v[j] = ul[j]; R.v[j] = ur[j]; KL.v[j] = kl[j]; KR.v[j] = kr[j]; ML.v[j] = ml[j]; MR.v[j] = mr[j];
+      }
+      ends(vscale(h, vadd(kc, KL)), vsub(mc, ML), vsub(uc, L), vscale(h, vadd(kc, KR)), vsub(MR, mc), vsub(R, uc), Sx, Gx);
+    } else {
+#pragma unroll
+      for (int j = 0; j < RY; ++j) {
+        const int i0 = j * VX;
+        T kf0 = mul_rn(h, add_rn(kc.v[i0], kl[j])), dm0 = sub_rn(mc.v[i0], ml[j]), du0 = sub_rn(uc.v[i0], ul[j]);
+#pragma unroll
+        for (int e = 0; e < VX; ++e) {
+          const int i = i0 + e, n = e + 1 < VX ? i + 1 : i;
+          const T u1 = e + 1 < VX ? uc.v[n] : ur[j], k1 = e + 1 < VX ? kc.v[n] : kr[j], m1 = e + 1 < VX ? mc.v[n] : mr[j];
+          const T kf = mul_rn(h, add_rn(kc.v[i], k1)), dm = sub_rn(m1, mc.v[i]), du = sub_rn(u1, uc.v[i]);
+          Sx.v[i] = fma_rn_(kf0, -dm0, mul_rn(kf, dm));
+          Gx.v[i] = fma_rn_(-du0, dm0, mul_rn(du, -dm));
+          kf0 = kf; dm0 = dm; du0 = du;
+        }
+      }
+    }
+    {
+      auto rowv = [&](const V& f, int j) {
+        VN<T, VX> w;
+#pragma unroll
+        for (int e = 0; e < VX; ++e) w.v[e] = f.v[j * VX + e];
+        return w;
+      };
+      VN<T, VX> u0 = rowv(uc, 0), k0 = rowv(kc, 0), m0 = rowv(mc, 0);
+      VN<T, VX> kf0 = vscale(h, vadd(k0, ka)), dm0 = vsub(m0, ma), du0 = vsub(u0, ua);
+#pragma unroll
+      for (int j = 0; j < RY; ++j) {
+        const int n = j + 1 < RY ? j + 1 : j;
+        const VN<T, VX> u1 = j + 1 < RY ? rowv(uc, n) : ub, k1 = j + 1 < RY ? rowv(kc, n) : kb, m1 = j + 1 < RY ? rowv(mc, n) : mb;
+        const VN<T, VX> kf = vscale(h, vadd(k0, k1)), dm = vsub(m1, m0), du = vsub(u1, u0);
+        VN<T, VX> S, G;
+        ends(kf0, dm0, du0, kf, dm, du, S, G);
+#pragma unroll
+        for (int e = 0; e < VX; ++e) { Sy.v[j * VX + e] = S.v[e]; Gy.v[j * VX + e] = G.v[e]; }
+        u0 = u1; k0 = k1; m0 = m1; kf0 = kf; dm0 = dm; du0 = du;
+      }
+    }
+    V keep = mc;
+    if (!a.zero_boundary && (warp_masked || !zin)) {
+      const V l = t.plane(pl);
+#pragma unroll
+      for (int i = 0; i < N; ++i) keep.v[i] = l.v[i];
+    }
+    const V out = vadd(keep, vaxpy(a.cz, Sz, vaxpy(a.cy, Sy, vscale(a.cx, Sx))));
+    const V gn = vaxpy(h, vaxpy(a.cz, Gz, vaxpy(a.cy, Gy, vscale(a.cx, Gx))), g);
+    if (any) {
+#pragma unroll
+      for (int j = 0; j < RY; ++j)
+        if (t.ok[j]) {
+          VN<T, VX> w, q;
+#pragma unroll
+          for (int e = 0; e < VX; ++e) { w.v[e] = out.v[j * VX + e]; q.v[e] = gn.v[j * VX + e]; }
+          if (ADV_IN_RANGE(po - a.out + t.dr[j] + VX - 1, t.sz * nz, a.status)) {
+            stv<T, VX>(po + t.dr[j], w);
+            stv<T, VX>(pg + t.dr[j], q);
+          }
+        }
+    }
+    uc = up; up = un; kc = kp; kp = kn; mc = mp;
+    mp = mask(ln, z2);
+    pu += t.sz; pk += t.sz; pl += t.sz; po += t.sz; pg += t.sz;
+    if (z + 3 < nz) { pu2 += t.sz; pk2 += t.sz; pl2 += t.sz; }
   }
 }
+
+// Launch forms: rows of whole vectors in aligned arrays, or one node per thread along x.
+template <class T> struct HeatKForm;
+template <> struct HeatKForm<float> {
+  static constexpr int STEP_VX = 4, STEP_RY = 1, ADJ_VX = 2, ADJ_RY = 2;
+};
+template <> struct HeatKForm<double> {
+  static constexpr int STEP_VX = 2, STEP_RY = 1, ADJ_VX = 2, ADJ_RY = 1;
+};
+constexpr int kLxVec = 16, kLxOne = 32;  // threads per block row
+constexpr int kRyOne = 2;                // rows per thread, one node along x
 
 adv_status heatk_validate(const adv_heatk_desc* d) {
   if (!d) return set_error(ADV_ERR_INVALID_ARG, "heatk: null descriptor");
@@ -345,6 +515,7 @@ HeatKArgs<T> make_args(const adv_heatk_desc& d, const void* k, const void* u, co
   a.nx = d.nx; a.ny = d.ny; a.nz = d.nz;
   a.zero_boundary = d.zero_boundary;
   a.cx = (T)d.cx; a.cy = (T)d.cy; a.cz = (T)d.cz;
+  a.status = device_status_ptr();
   return a;
 }
 
@@ -357,58 +528,87 @@ bool vec_ok(const adv_heatk_desc& d, std::initializer_list<const void*> ptrs) {
   return true;
 }
 
-// Block height and z planes per CTA: the autotuner's choice for this problem, else 8 and 16.
-void heatk_shape(const adv_heatk_desc& d, int kind, int* ky, int* zc) {
+// Block height and z planes per CTA: the autotuner's choice for this problem, else (its default
+// candidate, 8 and 16, included) 8 and what gives one wave of CTAs: a chunk's two extra planes are cheap
+// against idle SMs (16 planes left a 64^3 grid 2 CTAs per SM at 12.6 us per step, one wave runs 2.5) and
+// against a second, nearly empty wave (192^3 step: 16.0 us; 8 planes, 1.1 waves: 21). bx, by: nodes per
+// CTA at height 8.
+void heatk_shape(const adv_heatk_desc& d, int kind, const void* kernel, int lx, int bx, int by, int* ky, int* zc) {
   const TuneParams tp = tune_lookup(kind, d.dtype, d.nx, d.ny, d.nz);
-  *ky = tp.set ? tp.a : 8;
-  *zc = tp.set ? tp.b : 16;
+  if (tp.set && !(tp.a == 8 && tp.b == 16)) {
+    *ky = tp.a;
+    *zc = tp.b;
+    return;
+  }
+  *ky = 8;
+  DeviceInfo di;
+  const int sms = device_info(&di) == ADV_OK ? di.sms : 152;
+  int occ = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, lx * 8, 0) != cudaSuccess || occ < 1) occ = 4;
+  const int64_t tiles = (int64_t)((d.nx + bx - 1) / bx) * ((d.ny + by - 1) / by);
+  const int64_t chunks = std::max<int64_t>(1, std::min<int64_t>(d.nz, (int64_t)sms * occ / tiles));
+  *zc = (int)((d.nz + chunks - 1) / chunks);
 }
 
-adv_status heatk_step_launch(const adv_heatk_desc& d, const void* k, const void* u_in, void* u_out, cudaStream_t s) {
+// Grid of a kernel with vx x ry nodes per thread and lx threads per block row.
+dim3 heatk_grid(const adv_heatk_desc& d, int vx, int ry, int lx, int ky, int zc) {
+  const int bx = vx * lx, by = ry * ky;
+  return dim3((unsigned)((d.nx + bx - 1) / bx), (unsigned)((d.ny + by - 1) / by), (unsigned)((d.nz + zc - 1) / zc));
+}
+
+template <class T, int VX, int RY, int LX>
+adv_status heatk_step_t(const adv_heatk_desc& d, const void* k, const void* u_in, void* u_out, cudaStream_t s) {
   int ky, zc;
-  heatk_shape(d, TUNE_HEATK_STEP, &ky, &zc);
-  const int vx = d.dtype == ADV_F32 ? 4 : 2;
-  const bool vec = vec_ok(d, {k, u_in, u_out});
-  const int bx = vec ? KXV : KX, xs = vec ? KXV * vx : KX;
-  const dim3 grid((unsigned)((d.nx + xs - 1) / xs), (unsigned)((d.ny + ky - 1) / ky), (unsigned)((d.nz + zc - 1) / zc));
-  if (d.dtype == ADV_F32) {
-    HeatKArgs<float> a = make_args<float>(d, k, u_in, nullptr, u_out, nullptr);
-    a.zc = zc;
-    if (vec) heatk_step_vec_kernel<float><<<grid, dim3(bx, ky), 0, s>>>(a);
-    else heatk_step_kernel<float><<<grid, dim3(bx, ky), 0, s>>>(a);
-  } else {
-    HeatKArgs<double> a = make_args<double>(d, k, u_in, nullptr, u_out, nullptr);
-    a.zc = zc;
-    if (vec) heatk_step_vec_kernel<double><<<grid, dim3(bx, ky), 0, s>>>(a);
-    else heatk_step_kernel<double><<<grid, dim3(bx, ky), 0, s>>>(a);
-  }
+  const auto kernel = &heatk_step_kernel<T, VX, RY, LX>;
+  heatk_shape(d, TUNE_HEATK_STEP, reinterpret_cast<const void*>(kernel), LX, VX * LX, RY * 8, &ky, &zc);
+  if (LX > 16) ky = std::min(ky, 8);  // 256 threads at most
+  HeatKArgs<T> a = make_args<T>(d, k, u_in, nullptr, u_out, nullptr);
+  a.zc = zc;
+  kernel<<<heatk_grid(d, VX, RY, LX, ky, zc), dim3(LX, ky), 0, s>>>(a);
   ADV_CUDA_TRY(cudaGetLastError());
   count_launches(1);
   return ADV_OK;
+}
+
+template <class T, int VX, int RY, int LX>
+adv_status heatk_adjoint_t(const adv_heatk_desc& d, const void* k, const void* u_n, const void* lam_next, void* lam_out,
+                           void* grad_k, cudaStream_t s) {
+  int ky, zc;
+  const auto kernel = &heatk_adjoint_kernel<T, VX, RY, LX>;
+  heatk_shape(d, TUNE_HEATK_ADJ, reinterpret_cast<const void*>(kernel), LX, VX * LX, RY * 8, &ky, &zc);
+  if (LX > 16) ky = std::min(ky, 8);
+  HeatKArgs<T> a = make_args<T>(d, k, u_n, lam_next, lam_out, grad_k);
+  a.zc = zc;
+  kernel<<<heatk_grid(d, VX, RY, LX, ky, zc), dim3(LX, ky), 0, s>>>(a);
+  ADV_CUDA_TRY(cudaGetLastError());
+  count_launches(1);
+  return ADV_OK;
+}
+
+template <class T>
+adv_status heatk_step_any(const adv_heatk_desc& d, const void* k, const void* u_in, void* u_out, cudaStream_t s) {
+  using Fm = HeatKForm<T>;
+  return vec_ok(d, {k, u_in, u_out}) ? heatk_step_t<T, Fm::STEP_VX, Fm::STEP_RY, kLxVec>(d, k, u_in, u_out, s)
+                                     : heatk_step_t<T, 1, kRyOne, kLxOne>(d, k, u_in, u_out, s);
+}
+
+template <class T>
+adv_status heatk_adjoint_any(const adv_heatk_desc& d, const void* k, const void* u_n, const void* lam_next, void* lam_out,
+                             void* grad_k, cudaStream_t s) {
+  using Fm = HeatKForm<T>;
+  return vec_ok(d, {k, u_n, lam_next, lam_out, grad_k})
+             ? heatk_adjoint_t<T, Fm::ADJ_VX, Fm::ADJ_RY, kLxVec>(d, k, u_n, lam_next, lam_out, grad_k, s)
+             : heatk_adjoint_t<T, 1, kRyOne, kLxOne>(d, k, u_n, lam_next, lam_out, grad_k, s);
+}
+
+adv_status heatk_step_launch(const adv_heatk_desc& d, const void* k, const void* u_in, void* u_out, cudaStream_t s) {
+  return d.dtype == ADV_F32 ? heatk_step_any<float>(d, k, u_in, u_out, s) : heatk_step_any<double>(d, k, u_in, u_out, s);
 }
 
 adv_status heatk_adjoint_launch(const adv_heatk_desc& d, const void* k, const void* u_n, const void* lam_next,
                                 void* lam_out, void* grad_k, cudaStream_t s) {
-  int ky, zc;
-  heatk_shape(d, TUNE_HEATK_ADJ, &ky, &zc);
-  const int vx = d.dtype == ADV_F32 ? kAdjVxF32 : 2;
-  const bool vec = vec_ok(d, {k, u_n, lam_next, lam_out, grad_k});
-  const int bx = vec ? KXV : KX, xs = vec ? KXV * vx : KX;
-  const dim3 grid((unsigned)((d.nx + xs - 1) / xs), (unsigned)((d.ny + ky - 1) / ky), (unsigned)((d.nz + zc - 1) / zc));
-  if (d.dtype == ADV_F32) {
-    HeatKArgs<float> a = make_args<float>(d, k, u_n, lam_next, lam_out, grad_k);
-    a.zc = zc;
-    if (vec) heatk_adjoint_vec_kernel<float, kAdjVxF32><<<grid, dim3(bx, ky), 0, s>>>(a);
-    else heatk_adjoint_kernel<float><<<grid, dim3(bx, ky), 0, s>>>(a);
-  } else {
-    HeatKArgs<double> a = make_args<double>(d, k, u_n, lam_next, lam_out, grad_k);
-    a.zc = zc;
-    if (vec) heatk_adjoint_vec_kernel<double><<<grid, dim3(bx, ky), 0, s>>>(a);
-    else heatk_adjoint_kernel<double><<<grid, dim3(bx, ky), 0, s>>>(a);
-  }
-  ADV_CUDA_TRY(cudaGetLastError());
-  count_launches(1);
-  return ADV_OK;
+  return d.dtype == ADV_F32 ? heatk_adjoint_any<float>(d, k, u_n, lam_next, lam_out, grad_k, s)
+                            : heatk_adjoint_any<double>(d, k, u_n, lam_next, lam_out, grad_k, s);
 }
 
 size_t array_bytes(const adv_heatk_desc& d) {
