@@ -13,46 +13,56 @@
 // and 3 for lam.
 //
 // Work layout (one wave of CTAs, balanced (tile, z-plane) segments as in the forward stage): a
-// CTA owns 32 x 16 columns and streams the planes z-5 .. z+4 of its segment through an 8-slot
-// shared ring (v and lam with a 5-cell periodic halo, cp.async). Per streamed plane p each
-// thread advances its two columns' z windows and differentiates the z-face p-3+1/2, pushing the
-// partials into per-column accumulators for cells p-5..p; cell p-5 is then complete in z. For
-// that plane the x- and y-faces of the tile (37 x 16 and 32 x 21) are differentiated by all
-// threads into shared memory (structure of arrays), each cell gathers its ten partials per axis,
-// and the stage output is written. Every face is differentiated once per pass.
+// CTA owns 32 x 16 columns, two adjacent in x per thread, and streams the planes z-5 .. z+4 of its
+// segment through shared-memory rings (cp.async; v with a 5-cell periodic halo, lam with 3 cells, two
+// planes behind). Per streamed plane p each thread advances its columns' f+- windows and differentiates
+// the z-faces p-3+1/2, pushing the partials into per-column accumulators for cells p-5..p; cell p-5 is
+// then complete in z. For that plane f+- go to shared memory in two layouts (pairs of rows for the
+// x-faces, pairs of columns for the y-faces, as in the forward stage: an operand pair is one load), the
+// 37 x 16 x-faces and 32 x 21 y-faces of the tile are differentiated two at a time into shared memory
+// (structure of arrays), each cell gathers its ten partials per axis, and the stage output is written.
+// Every face is differentiated once per pass. Bound by issue, as the forward stage: 128^3 FP32 WENO5-Z
+// 146.6 -> 91.7 us per stage back to back, FP64 64^3 1326 -> 630, against one face per thread with its two
+// sides packed into a pair, the weights' full form (about 125 paired instructions a side against 84) and
+// an index division per staged element.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 
 #include "adv_device.cuh"
 #include "adv_internal.h"
-#include "nvtx_range.h"
 #include "adv_math.cuh"
+#include "nvtx_range.h"
+#include "weno.cuh"
 
 namespace adv {
 
 namespace {
 
 struct AdjTile {
-  static constexpr int BX = 32, BY = 16, NT = 256;
-  static constexpr int H = 5;                  // halo of the staged region (v needs 5, lam 3)
-  static constexpr int SW = BX + 2 * H;        // 42
-  static constexpr int SH = BY + 2 * H;        // 26
-  static constexpr int PLANE = SW * SH;        // 1092
-  static constexpr int NS = 8;                 // ring slots: planes p-5 .. p+2
-  static constexpr int P = 2;                  // planes prefetched ahead
-  static constexpr int NFX = (BX + 5) * BY;    // x-faces i+1/2, i = -3 .. 33, per row: 592
-  static constexpr int NFY = BX * (BY + 5);    // y-faces: 672
+  static constexpr int BX = 32, BY = 16, NT = 256, PX = BX / 2;
+  static constexpr int H = 5, HL = 3;                    // halos of v and lam
+  static constexpr int PADX = 6, SW = BX + 2 * PADX;     // v: shared column 0 holds x0 - 6 (pairs aligned)
+  static constexpr int SH = BY + 2 * H, PLANE = SW * SH;
+  static constexpr int PADL = 4, SWL = BX + 2 * PADL;    // lam: column 0 holds x0 - 4
+  static constexpr int SHL = BY + 2 * HL, PLANEL = SWL * SHL;
+  static constexpr int NS = 8, NSL = 6;                  // ring slots: v p-5 .. p+2, lam p-5 .. p
+  static constexpr int FX = BX + 5, NFX = FX * BY / 2;   // x-faces i+1/2, i = -3 .. 33, per pair of rows
+  static constexpr int FY = BY + 5, NFY = FY * PX;       // y-faces, pairs of columns
   static constexpr int NF = NFY > NFX ? NFY : NFX;
+  static constexpr int XS = BX + 2 * H;                  // x-face operands per pair of rows: cells x0-5 .. x0+36
 };
 
 template <class T>
 struct AdjSmem {
-  static constexpr int SLOT = ((AdjTile::PLANE * (int)sizeof(T) + 127) / 128 * 128) / (int)sizeof(T);
-  static constexpr size_t RING = (size_t)AdjTile::NS * 2 * SLOT * sizeof(T);  // v and lam per slot
-  static constexpr size_t FPM = (size_t)2 * SLOT * sizeof(T);                 // f+ and f- of a plane
-  static constexpr size_t FB = (size_t)10 * AdjTile::NF * sizeof(T);          // face partials (SoA)
-  static constexpr size_t TOTAL = RING + FPM + FB;
+  using TL = AdjTile;
+  static constexpr int SLOT = ((TL::PLANE * (int)sizeof(T) + 127) / 128 * 128) / (int)sizeof(T);
+  static constexpr int SLOTL = ((TL::PLANEL * (int)sizeof(T) + 127) / 128 * 128) / (int)sizeof(T);
+  static constexpr size_t RING = (size_t)(TL::NS * SLOT + TL::NSL * SLOTL) * sizeof(T);
+  static constexpr int PART = TL::BY / 2 * TL::XS + TL::SH * TL::PX;            // pairs of one split part
+  static constexpr size_t FB = (size_t)10 * TL::NF * 2 * sizeof(T);             // face partials (SoA)
+  static constexpr size_t JX = (size_t)TL::BX * TL::BY * sizeof(T);             // x part of J^T lam per cell
+  static constexpr size_t TOTAL = RING + (size_t)2 * PART * 2 * sizeof(T) + FB + JX + TL::PLANE * sizeof(int64_t);
 };
 
 template <class T>
@@ -64,13 +74,10 @@ struct AdjArgs {
   T* acc_out;       // accumulated adjoint of u^n (stages 3, 2); may equal acc_in
   int nx, ny, nz, stage;
   int tiles_x, tiles_y;
+  int vec_ok;  // outputs and acc_in: pairs of nodes aligned for one access
   T dt, rdx, rdy, rdz;
+  int* status;
 };
-
-template <class T> __device__ __forceinline__ T absv(T x) { return fabs(x); }
-template <> __device__ __forceinline__ float absv<float>(float x) { return fabsf(x); }
-__device__ __forceinline__ float rcp(float x) { return __frcp_rn(x); }
-__device__ __forceinline__ double rcp(double x) { return 1.0 / x; }
 
 // Periodic index. Inside the domain (every element of an interior tile) it is the index itself,
 // without the integer division of the general case.
@@ -80,199 +87,118 @@ __device__ __forceinline__ int wrap(int i, int n) {
   return i < 0 ? i + n : i;
 }
 
-template <class T> __device__ __forceinline__ T fplus(T u) { return u * (T(0.25) * u + T(0.5) * absv(u)); }
-template <class T> __device__ __forceinline__ T fminus(T u) { return u * (T(0.25) * u - T(0.5) * absv(u)); }
+__device__ __forceinline__ float2 vrcp(float2 x) {  // one Newton step on the approximation: 1 ulp
+  const float2 r = make_float2(rcp_approx(-x.x), rcp_approx(-x.y));
+  const float2 n = vfma(vfma(x, r, vc<float2>(1)), r, r);
+  return make_float2(-n.x, -n.y);
+}
+__device__ __forceinline__ double2 vrcp(double2 x) { return make_double2(1.0 / x.x, 1.0 / x.y); }
+// sign(d) t, 0 where d is 0
+__device__ __forceinline__ float sgn_mul(float d, float t) { return d == 0.f ? 0.f : __uint_as_float(__float_as_uint(t) ^ (__float_as_uint(d) & 0x80000000u)); }
+__device__ __forceinline__ double sgn_mul(double d, double t) { return d > 0.0 ? t : d < 0.0 ? -t : 0.0; }
 
-// d side(a..e) / d(a..e) times ybar, for the common-denominator weights (see the header).
-template <class T, bool Z>
-__device__ __forceinline__ void side_rev(T a, T b, T c, T d, T e, T ybar, T& ga, T& gb, T& gc, T& gd, T& ge) {
-  const T t0 = a - T(2) * b + c, t1 = b - T(2) * c + d, t2 = c - T(2) * d + e;
-  const T s0 = a - T(4) * b + T(3) * c, s1 = b - d, s2 = T(3) * c - T(4) * d + e;
-  const T K = T(13.0 / 3.0), E = T(4e-6);
-  const T B0 = K * t0 * t0 + s0 * s0 + E, B1 = K * t1 * t1 + s1 * s1 + E, B2 = K * t2 * t2 + s2 * s2 + E;
-  const T q0 = c + t0 * T(1.0 / 12.0) + s0 * T(0.25), q1 = c + t1 * T(1.0 / 12.0) - s1 * T(0.25),
-          q2 = c + t2 * T(1.0 / 12.0) - s2 * T(0.25);
-  T w0, w1, w2, tau = T(0);
-  T Bb0, Bb1, Bb2;
+// Reverse mode of one WENO side (weno_side2 in weno.cuh) for two faces at once: g[k] = psi d side / d f_k
+// of f = a..e at i-2 .. i+2. The side is c + C/2 - t1/6 - q/2, q = num / den, num = 2/3 e0 (t1-t0) +
+// e2 (t2-t1), den = e0 + 6 e1 + 3 e2; bars of e, b, s, t and of the first differences follow in turn (the
+// bars of e and b carry a factor 2).
+template <bool Z, class V>
+__device__ __forceinline__ void side_rev(V a, V b, V c, V d, V e, V psi, V (&g)[5]) {
+  const V A = vsub(b, a), B = vsub(c, b), C = vsub(d, c), E = vsub(e, d);
+  const V t0 = vsub(B, A), t1 = vsub(C, B), t2 = vsub(E, C);
+  const V s0 = vfma(vc<V>(2), B, t0), s1 = vadd(B, C), s2 = vfma(vc<V>(-2), C, t2);
+  const V K = vc<V>(13.0 / 3.0), eps = vc<V>(4e-6);
+  const V k0 = vmul(K, t0), k1 = vmul(K, t1), k2 = vmul(K, t2);
+  const V b0 = vfma(k0, t0, vfma(s0, s0, eps)), b1 = vfma(k1, t1, vfma(s1, s1, eps)), b2 = vfma(k2, t2, vfma(s2, s2, eps));
+  const V p12 = vmul(b1, b2), p02 = vmul(b0, b2), p01 = vmul(b0, b1);
+  const V da = vsub(t1, t0), db = vsub(t2, t1);
+  V e0, e1, e2, d02, tau;
   if (Z) {
-    tau = absv(B0 - B2);
-    const T P0 = B0 + tau, P1 = B1 + tau, P2 = B2 + tau;
-    const T b12 = B1 * B2, b02 = B0 * B2, b01 = B0 * B1;
-    w0 = P0 * b12;
-    w1 = T(6) * P1 * b02;
-    w2 = T(3) * P2 * b01;
-    const T rD = rcp(w0 + w1 + w2);
-    const T side = (w0 * q0 + w1 * q1 + w2 * q2) * rD;
-    const T Nb = ybar * rD;
-    const T wb0 = Nb * (q0 - side), wb1 = T(6) * Nb * (q1 - side), wb2 = T(3) * Nb * (q2 - side);
-    const T taub = wb0 * b12 + wb1 * b02 + wb2 * b01;
-    Bb0 = wb0 * b12 + wb1 * P1 * B2 + wb2 * P2 * B1;
-    Bb1 = wb0 * P0 * B2 + wb1 * b02 + wb2 * P2 * B0;
-    Bb2 = wb0 * P0 * B1 + wb1 * P1 * B0 + wb2 * b01;
-    const T sg = B0 > B2 ? T(1) : (B0 < B2 ? T(-1) : T(0));
-    Bb0 += sg * taub;
-    Bb2 -= sg * taub;
-    const T qb0 = Nb * w0, qb1 = Nb * w1, qb2 = Nb * w2;
-    const T tb0 = T(2) * K * t0 * Bb0 + qb0 * T(1.0 / 12.0), tb1 = T(2) * K * t1 * Bb1 + qb1 * T(1.0 / 12.0),
-            tb2 = T(2) * K * t2 * Bb2 + qb2 * T(1.0 / 12.0);
-    const T sb0 = T(2) * s0 * Bb0 + qb0 * T(0.25), sb1 = T(2) * s1 * Bb1 - qb1 * T(0.25),
-            sb2 = T(2) * s2 * Bb2 - qb2 * T(0.25);
-    const T cb = qb0 + qb1 + qb2;
-    ga = tb0 + sb0;
-    gb = T(-2) * tb0 + tb1 - T(4) * sb0 + sb1;
-    gc = tb0 - T(2) * tb1 + tb2 + T(3) * sb0 + T(3) * sb2 + cb;
-    gd = tb1 - T(2) * tb2 - sb1 - T(4) * sb2;
-    ge = tb2 + sb2;
+    d02 = vsub(b0, b2);
+    tau = vabs(d02);
+    const V P = vmul(b0, p12);
+    e0 = vfma(tau, p12, P);
+    e1 = vfma(tau, p02, P);
+    e2 = vfma(tau, p01, P);
   } else {
-    const T p12 = B1 * B2, p02 = B0 * B2, p01 = B0 * B1;
-    w0 = p12 * p12;
-    w1 = T(6) * p02 * p02;
-    w2 = T(3) * p01 * p01;
-    const T rD = rcp(w0 + w1 + w2);
-    const T side = (w0 * q0 + w1 * q1 + w2 * q2) * rD;
-    const T Nb = ybar * rD;
-    const T wb0 = Nb * (q0 - side), wb1 = Nb * (q1 - side), wb2 = Nb * (q2 - side);
-    Bb0 = T(12) * wb1 * p02 * B2 + T(6) * wb2 * p01 * B1;
-    Bb1 = T(2) * wb0 * p12 * B2 + T(6) * wb2 * p01 * B0;
-    Bb2 = T(2) * wb0 * p12 * B1 + T(12) * wb1 * p02 * B0;
-    const T qb0 = Nb * w0, qb1 = Nb * w1, qb2 = Nb * w2;
-    const T tb0 = T(2) * K * t0 * Bb0 + qb0 * T(1.0 / 12.0), tb1 = T(2) * K * t1 * Bb1 + qb1 * T(1.0 / 12.0),
-            tb2 = T(2) * K * t2 * Bb2 + qb2 * T(1.0 / 12.0);
-    const T sb0 = T(2) * s0 * Bb0 + qb0 * T(0.25), sb1 = T(2) * s1 * Bb1 - qb1 * T(0.25),
-            sb2 = T(2) * s2 * Bb2 - qb2 * T(0.25);
-    const T cb = qb0 + qb1 + qb2;
-    ga = tb0 + sb0;
-    gb = T(-2) * tb0 + tb1 - T(4) * sb0 + sb1;
-    gc = tb0 - T(2) * tb1 + tb2 + T(3) * sb0 + T(3) * sb2 + cb;
-    gd = tb1 - T(2) * tb2 - sb1 - T(4) * sb2;
-    ge = tb2 + sb2;
+    e0 = vmul(p12, p12);
+    e1 = vmul(p02, p02);
+    e2 = vmul(p01, p01);
   }
-}
-
-// FP32: the two sides of one face (f+ in lane x, f- in lane y) differentiated together with
-// Blackwell's paired FP32 instructions (FFMA2 / FADD2 / FMUL2), the same algebra as side_rev.
-__device__ __forceinline__ float2 c2(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float2 ad2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 sb2(float2 a, float2 b) { return __ffma2_rn(b, c2(-1.f), a); }
-__device__ __forceinline__ float2 ml2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fm2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-
-template <bool Z>
-__device__ __forceinline__ void side_rev2(float2 a, float2 b, float2 c, float2 d, float2 e, float2 ybar, float2 (&g)[5]) {
-  const float2 m2 = c2(-2.f), m4 = c2(-4.f), p3 = c2(3.f), r12 = c2(1.f / 12.f), qt = c2(0.25f);
-  const float2 t0 = ad2(fm2(m2, b, a), c), t1 = ad2(fm2(m2, c, b), d), t2 = ad2(fm2(m2, d, c), e);
-  const float2 s0 = fm2(p3, c, fm2(m4, b, a)), s1 = sb2(b, d), s2 = fm2(p3, c, fm2(m4, d, e));
-  const float2 K = c2(13.f / 3.f), E = c2(4e-6f);
-  const float2 B0 = fm2(ml2(K, t0), t0, fm2(s0, s0, E)), B1 = fm2(ml2(K, t1), t1, fm2(s1, s1, E)),
-               B2 = fm2(ml2(K, t2), t2, fm2(s2, s2, E));
-  const float2 q0 = fm2(qt, s0, fm2(r12, t0, c)), q1 = fm2(c2(-0.25f), s1, fm2(r12, t1, c)),
-               q2 = fm2(c2(-0.25f), s2, fm2(r12, t2, c));
-  float2 w0, w1, w2, Bb0, Bb1, Bb2;
+  const V r = vrcp(vfma(vc<V>(3), e2, vfma(vc<V>(6), e1, e0)));
+  const V da3 = vmul(vc<V>(2.0 / 3.0), da);
+  const V q = vmul(vfma(e2, db, vmul(e0, da3)), r);
+  const V gr = vmul(vmul(vc<V>(-1), psi), r);  // 2 x the bar of num
+  const V x0 = vmul(gr, vsub(da3, q)), x1 = vmul(vmul(vc<V>(-6), gr), q), x2 = vmul(gr, vfma(vc<V>(-3), q, db));
+  V y0, y1, y2;  // 2 x the bars of b0, b1, b2
   if (Z) {
-    const float2 d02 = sb2(B0, B2);
-    const float2 tau = make_float2(fabsf(d02.x), fabsf(d02.y));
-    const float2 sg = make_float2(d02.x > 0.f ? 1.f : (d02.x < 0.f ? -1.f : 0.f),
-                                  d02.y > 0.f ? 1.f : (d02.y < 0.f ? -1.f : 0.f));
-    const float2 P0 = ad2(B0, tau), P1 = ad2(B1, tau), P2 = ad2(B2, tau);
-    const float2 b12 = ml2(B1, B2), b02 = ml2(B0, B2), b01 = ml2(B0, B1);
-    w0 = ml2(P0, b12);
-    w1 = ml2(ml2(c2(6.f), P1), b02);
-    w2 = ml2(ml2(p3, P2), b01);
-    const float2 den = ad2(ad2(w0, w1), w2);
-    const float2 rD = make_float2(__frcp_rn(den.x), __frcp_rn(den.y));
-    const float2 side = ml2(fm2(w2, q2, fm2(w1, q1, ml2(w0, q0))), rD);
-    const float2 Nb = ml2(ybar, rD);
-    const float2 wb0 = ml2(Nb, sb2(q0, side)), wb1 = ml2(ml2(c2(6.f), Nb), sb2(q1, side)),
-                 wb2 = ml2(ml2(p3, Nb), sb2(q2, side));
-    const float2 taub = fm2(wb2, b01, fm2(wb1, b02, ml2(wb0, b12)));
-    Bb0 = fm2(wb2, ml2(P2, B1), fm2(wb1, ml2(P1, B2), ml2(wb0, b12)));
-    Bb1 = fm2(wb2, ml2(P2, B0), fm2(wb1, b02, ml2(wb0, ml2(P0, B2))));
-    Bb2 = fm2(wb2, b01, fm2(wb1, ml2(P1, B0), ml2(wb0, ml2(P0, B1))));
-    Bb0 = fm2(sg, taub, Bb0);
-    Bb2 = fm2(make_float2(-sg.x, -sg.y), taub, Bb2);
-    const float2 qb0 = ml2(Nb, w0), qb1 = ml2(Nb, w1), qb2 = ml2(Nb, w2);
-    const float2 K2 = c2(26.f / 3.f);
-    const float2 tb0 = fm2(ml2(K2, t0), Bb0, ml2(qb0, r12)), tb1 = fm2(ml2(K2, t1), Bb1, ml2(qb1, r12)),
-                 tb2 = fm2(ml2(K2, t2), Bb2, ml2(qb2, r12));
-    const float2 sv0 = fm2(ml2(c2(2.f), s0), Bb0, ml2(qb0, qt)), sv1 = fm2(ml2(c2(2.f), s1), Bb1, ml2(qb1, c2(-0.25f))),
-                 sv2 = fm2(ml2(c2(2.f), s2), Bb2, ml2(qb2, c2(-0.25f)));
-    const float2 cb = ad2(ad2(qb0, qb1), qb2);
-    g[0] = ad2(tb0, sv0);
-    g[1] = ad2(fm2(m2, tb0, tb1), fm2(m4, sv0, sv1));
-    g[2] = ad2(fm2(m2, tb1, ad2(tb0, tb2)), fm2(p3, ad2(sv0, sv2), cb));
-    g[3] = fm2(m4, sv2, sb2(fm2(m2, tb2, tb1), sv1));
-    g[4] = ad2(tb2, sv2);
+    const V X = vadd(vadd(x0, x1), x2);
+    const V z0 = vmul(tau, x0), z1 = vmul(tau, x1), z2 = vmul(tau, x2);
+    const V tb = vfma(x2, p01, vfma(x1, p02, vmul(x0, p12)));
+    const V st = {sgn_mul(d02.x, tb.x), sgn_mul(d02.y, tb.y)};
+    y0 = vadd(vfma(z1, b2, vfma(z2, b1, vmul(X, p12))), st);
+    y1 = vfma(z0, b2, vfma(z2, b0, vmul(X, p02)));
+    y2 = vsub(vfma(z0, b1, vfma(z1, b0, vmul(X, p01))), st);
   } else {
-    const float2 p12 = ml2(B1, B2), p02 = ml2(B0, B2), p01 = ml2(B0, B1);
-    w0 = ml2(p12, p12);
-    w1 = ml2(ml2(c2(6.f), p02), p02);
-    w2 = ml2(ml2(p3, p01), p01);
-    const float2 den = ad2(ad2(w0, w1), w2);
-    const float2 rD = make_float2(__frcp_rn(den.x), __frcp_rn(den.y));
-    const float2 side = ml2(fm2(w2, q2, fm2(w1, q1, ml2(w0, q0))), rD);
-    const float2 Nb = ml2(ybar, rD);
-    const float2 wb0 = ml2(Nb, sb2(q0, side)), wb1 = ml2(Nb, sb2(q1, side)), wb2 = ml2(Nb, sb2(q2, side));
-    Bb0 = fm2(ml2(c2(12.f), wb1), ml2(p02, B2), ml2(ml2(c2(6.f), wb2), ml2(p01, B1)));
-    Bb1 = fm2(ml2(c2(2.f), wb0), ml2(p12, B2), ml2(ml2(c2(6.f), wb2), ml2(p01, B0)));
-    Bb2 = fm2(ml2(c2(2.f), wb0), ml2(p12, B1), ml2(ml2(c2(12.f), wb1), ml2(p02, B0)));
-    const float2 qb0 = ml2(Nb, w0), qb1 = ml2(Nb, w1), qb2 = ml2(Nb, w2);
-    const float2 K2 = c2(26.f / 3.f);
-    const float2 tb0 = fm2(ml2(K2, t0), Bb0, ml2(qb0, r12)), tb1 = fm2(ml2(K2, t1), Bb1, ml2(qb1, r12)),
-                 tb2 = fm2(ml2(K2, t2), Bb2, ml2(qb2, r12));
-    const float2 sv0 = fm2(ml2(c2(2.f), s0), Bb0, ml2(qb0, qt)), sv1 = fm2(ml2(c2(2.f), s1), Bb1, ml2(qb1, c2(-0.25f))),
-                 sv2 = fm2(ml2(c2(2.f), s2), Bb2, ml2(qb2, c2(-0.25f)));
-    const float2 cb = ad2(ad2(qb0, qb1), qb2);
-    g[0] = ad2(tb0, sv0);
-    g[1] = ad2(fm2(m2, tb0, tb1), fm2(m4, sv0, sv1));
-    g[2] = ad2(fm2(m2, tb1, ad2(tb0, tb2)), fm2(p3, ad2(sv0, sv2), cb));
-    g[3] = fm2(m4, sv2, sb2(fm2(m2, tb2, tb1), sv1));
-    g[4] = ad2(tb2, sv2);
+    const V two = vc<V>(2);
+    const V z0 = vmul(vmul(two, p12), x0), z1 = vmul(vmul(two, p02), x1), z2 = vmul(vmul(two, p01), x2);
+    y0 = vfma(z1, b2, vmul(z2, b1));
+    y1 = vfma(z0, b2, vmul(z2, b0));
+    y2 = vfma(z0, b1, vmul(z1, b0));
   }
-}
-
-// Both sides of one face: gp[k] = d side(pv) / d pv[k] * psi and gm[k] = d side(mv) / d mv[k] * psi.
-template <class T, bool Z>
-__device__ __forceinline__ void sides_rev(const T (&pv)[5], const T (&mv)[5], T psi, T (&gp)[5], T (&gm)[5]) {
-  if constexpr (sizeof(T) == 4) {
-    float2 g[5];
-    side_rev2<Z>(make_float2(pv[0], mv[0]), make_float2(pv[1], mv[1]), make_float2(pv[2], mv[2]),
-                 make_float2(pv[3], mv[3]), make_float2(pv[4], mv[4]), c2(psi), g);
-#pragma unroll
-    for (int k = 0; k < 5; ++k) { gp[k] = g[k].x; gm[k] = g[k].y; }
-  } else {
-    side_rev<T, Z>(pv[0], pv[1], pv[2], pv[3], pv[4], psi, gp[0], gp[1], gp[2], gp[3], gp[4]);
-    side_rev<T, Z>(mv[0], mv[1], mv[2], mv[3], mv[4], psi, gm[0], gm[1], gm[2], gm[3], gm[4]);
-  }
-}
-
-// Partials of one face from the six cells v[0..5] = v at i-2 .. i+3 (split inside) and its
-// weight psi: P[k] for f+ at i-2+k, M[k] for f- at i-1+k.
-template <class T, bool Z>
-__device__ __forceinline__ void face_rev(const T* v, T psi, T* P, T* M) {
-  const T pv[5] = {fplus(v[0]), fplus(v[1]), fplus(v[2]), fplus(v[3]), fplus(v[4])};
-  const T mv[5] = {fminus(v[5]), fminus(v[4]), fminus(v[3]), fminus(v[2]), fminus(v[1])};
-  T gp[5], gm[5];
-  sides_rev<T, Z>(pv, mv, psi, gp, gm);
-#pragma unroll
-  for (int k = 0; k < 5; ++k) { P[k] = gp[k]; M[4 - k] = gm[k]; }
+  const V dab = vmul(vmul(vc<V>(1.0 / 3.0), e0), gr), dbb = vmul(vmul(vc<V>(0.5), e2), gr);  // bars of t1-t0, t2-t1
+  const V u0 = vmul(s0, y0), u1 = vmul(s1, y1), u2 = vmul(s2, y2);                            // bars of s0, s1, s2
+  const V T0 = vsub(vfma(k0, y0, u0), dab);
+  const V T1 = vfma(vc<V>(-1.0 / 6.0), psi, vfma(k1, y1, vsub(dab, dbb)));
+  const V T2 = vadd(vfma(k2, y2, u2), dbb);
+  const V Bb = vadd(vfma(vc<V>(2), u0, u1), vsub(T0, T1));
+  const V Cb = vadd(vfma(vc<V>(-2), u2, u1), vfma(vc<V>(0.5), psi, vsub(T1, T2)));
+  g[0] = T0;
+  g[1] = vsub(vmul(vc<V>(-1), T0), Bb);
+  g[2] = vadd(vsub(Bb, Cb), psi);
+  g[3] = vsub(Cb, T2);
+  g[4] = T2;
 }
 
 template <class T, bool Z>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) burgers_adjoint_kernel(const __grid_constant__ AdjArgs<T> a) {
   using TL = AdjTile;
   using SM = AdjSmem<T>;
+  using V = typename Vec2<T>::type;
+  constexpr int H = TL::H, SW = TL::SW, SWL = TL::SWL, PX = TL::PX, XS = TL::XS, PART = SM::PART, NF = TL::NF;
+  constexpr int YP = TL::BY / 2 * XS;  // y-face operands of a part, after its x-face operands
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  T* ring = reinterpret_cast<T*>(smem_raw);  // slot s: v at ring + 2 s SLOT, lam at + SLOT
-  T* fpS = reinterpret_cast<T*>(smem_raw + SM::RING);
-  T* fmS = fpS + SM::SLOT;
-  T* FB = reinterpret_cast<T*>(smem_raw + SM::RING + SM::FPM);  // [10][NF]: P0..P4, M0..M4
+  T* const ring = reinterpret_cast<T*>(smem_raw);
+  T* const ringl = ring + TL::NS * SM::SLOT;
+  V* const part = reinterpret_cast<V*>(smem_raw + SM::RING);  // f+; f- follows PART pairs later
+  V* const FB = part + 2 * PART;                              // [10][NF]: P0..P4, M0..M4
+  T* const jx = reinterpret_cast<T*>(FB + 10 * NF);           // [BY][BX]
+  int64_t* const src = reinterpret_cast<int64_t*>(jx + TL::BX * TL::BY);  // in-plane offsets of v's staged elements
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int cp = tid & (PX - 1), row = tid / PX;
   const int nx = a.nx, ny = a.ny, nz = a.nz;
   const size_t sxy = (size_t)nx * ny;
+  const int own = (row + H) * SW + TL::PADX + 2 * cp;           // this thread's cells in a plane of v ..
+  const int ownl = (row + TL::HL) * SWL + TL::PADL + 2 * cp;    // .. and of lam
+  // halo splits, two values each: threads [0, 160) the ten halo rows, pairs of columns; [160, 240) the ten
+  // halo columns, pairs of rows
+  const bool halo = tid < 10 * PX + 10 * (TL::BY / 2);
+  int h_src, h_step;
+  V* h_dst;
+  if (tid < 10 * PX) {
+    const int h = tid / PX, r = h < H ? h : h + TL::BY;
+    h_src = r * SW + TL::PADX + 2 * cp;
+    h_step = 1;
+    h_dst = part + YP + r * PX + cp;
+  } else {
+    const int i = tid - 10 * PX, rp = (i / 10) % (TL::BY / 2), h = i % 10, c = h < H ? h : h + TL::BX;
+    h_src = (2 * rp + H) * SW + c + TL::PADX - H;
+    h_step = SW;
+    h_dst = part + rp * XS + c;
+  }
+  auto split = [](V u, V& fp, V& fm) { lf_split2(u, vabs(u), fp, fm); };
   const int64_t total = (int64_t)a.tiles_x * a.tiles_y * nz;
   const int64_t seg_a = total * blockIdx.x / gridDim.x, seg_b = total * (blockIdx.x + 1) / gridDim.x;
-  const int cx = lane, cy0 = warp, cy1 = warp + 8;
 
   for (int64_t pos = seg_a; pos < seg_b;) {
     const int64_t tile = pos / nz;
@@ -281,154 +207,188 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) burgers_adjoint_k
     pos += ze - zs;
     const int x0 = (int)(tile % a.tiles_x) * TL::BX, y0 = (int)(tile / a.tiles_x) * TL::BY;
     const int Q = (ze - zs) + 10;  // planes zs-5 .. ze+4
-    int s_issue = 0;
+    __syncthreads();  // the previous segment's copies have all been issued, its planes read
+    for (int e = tid; e < TL::PLANE; e += TL::NT) {
+      const int r = e / SW, c = e - r * SW;
+      src[e] = (int64_t)wrap(y0 - H + r, ny) * nx + wrap(x0 - TL::PADX + c, nx);
+    }
+    __syncthreads();
+    // stream entry q: v of plane zs-5+q and lam of the plane two before it
     auto issue = [&](int q) {
-      T* dv = ring + (size_t)(2 * s_issue) * SM::SLOT;
-      T* dl = dv + SM::SLOT;
-      const int z = wrap(zs - 5 + q, nz);
-      const size_t zo = (size_t)z * sxy;
-      for (int e = tid; e < TL::PLANE; e += TL::NT) {
-        const int r = e / TL::SW, c = e - r * TL::SW;
-        const size_t o = zo + (size_t)wrap(y0 - TL::H + r, ny) * nx + wrap(x0 - TL::H + c, nx);
-        cp_async_zfill<sizeof(T)>(dv + e, a.v + o, true);
-        cp_async_zfill<sizeof(T)>(dl + e, a.lam + o, true);
+      if (q < Q) {
+        T* const dv = ring + (q % TL::NS) * SM::SLOT;
+        const T* const pv = a.v + (size_t)wrap(zs - 5 + q, nz) * sxy;
+#pragma unroll 2
+        for (int e = tid; e < TL::PLANE; e += TL::NT)
+          cp_async_zfill<sizeof(T)>(dv + e, pv + src[e], ADV_IN_RANGE(pv + src[e] - a.v, sxy * nz, a.status));
+        if (q >= 2) {
+          T* const dl = ringl + ((q - 2) % TL::NSL) * SM::SLOTL;
+          const T* const pl = a.lam + (size_t)wrap(zs - 7 + q, nz) * sxy;
+#pragma unroll 2
+          for (int e = tid; e < TL::PLANEL; e += TL::NT) {
+            const int r = e / SWL, c = e - r * SWL;
+            const int64_t o = src[(r + H - TL::HL) * SW + c + TL::PADX - TL::PADL];
+            cp_async_zfill<sizeof(T)>(dl + e, pl + o, ADV_IN_RANGE(pl + o - a.lam, sxy * nz, a.status));
+          }
+        }
       }
       cp_async_commit();
-      s_issue = s_issue + 1 == TL::NS ? 0 : s_issue + 1;
     };
-    auto slot_of = [&](int q) { return q % TL::NS; };
-    for (int q = 0; q <= TL::P; ++q) issue(q);  // Q >= 11 > P
+    issue(0);
+    issue(1);
 
-    T vw[2][6];                 // v at p-5 .. p per column
-    T accP[2][6], accM[2][6];   // partial sums for cells p-5 .. p
+    V fpw[5], fmw[5], fp_new = vc<V>(0);  // f+ at p-5 .. p-1, f- at p-4 .. p, f+ at p
+    V accP[6], accM[6];                   // partial sums for cells p-5 .. p
 #pragma unroll
-    for (int c = 0; c < 2; ++c)
+    for (int k = 0; k < 6; ++k) { accP[k] = vc<V>(0); accM[k] = vc<V>(0); }
 #pragma unroll
-      for (int k = 0; k < 6; ++k) { vw[c][k] = T(0); accP[c][k] = T(0); accM[c][k] = T(0); }
+    for (int k = 0; k < 5; ++k) { fpw[k] = vc<V>(0); fmw[k] = vc<V>(0); }
 
+#pragma unroll 1
     for (int q = 0; q < Q; ++q) {
-      cp_async_wait<TL::P>();
-      __syncthreads();  // plane q visible
-      const T* vq = ring + (size_t)(2 * slot_of(q)) * SM::SLOT;
-      // ---- z: windows and the face p-3+1/2 (p = plane q)
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int cy = c ? cy1 : cy0;
-        const int ci = (cy + TL::H) * TL::SW + TL::H + cx;
-#pragma unroll
-        for (int k = 0; k < 5; ++k) vw[c][k] = vw[c][k + 1];
-        vw[c][5] = vq[ci];
-        if (q >= 5) {
-          const T* l3 = ring + (size_t)(2 * slot_of(q - 3)) * SM::SLOT + SM::SLOT;
-          const T* l2 = ring + (size_t)(2 * slot_of(q - 2)) * SM::SLOT + SM::SLOT;
-          const T psi = a.rdz * (l2[ci] - l3[ci]);
-          T P[5], M[5];
-          face_rev<T, Z>(vw[c], psi, P, M);
-#pragma unroll
-          for (int k = 0; k < 5; ++k) { accP[c][k] += P[k]; accM[c][k + 1] += M[k]; }
+      cp_async_wait<1>();
+      __syncthreads();  // entry q visible; entry q - 6's slots and the face buffers free
+      issue(q + 2);
+      const T* const vq = ring + (q % TL::NS) * SM::SLOT;
+      const T* const vo = ring + ((q + 3) % TL::NS) * SM::SLOT;            // plane q - 5
+      const T* const lo = ringl + ((q + 1) % TL::NSL) * SM::SLOTL;         // lam of plane q - 5
+      const bool out = q >= 10;
+      if (out) {
+        V fp, fm;
+        split(*reinterpret_cast<const V*>(vo + own), fp, fm);
+        V* const yw = part + YP + H * PX + tid;
+        yw[0] = fp;
+        yw[PART] = fm;
+        T* const xw = reinterpret_cast<T*>(part + warp * XS + 2 * cp + H) + (row & 1);
+        xw[0] = fp.x; xw[2] = fp.y;
+        xw[2 * PART] = fm.x; xw[2 * PART + 2] = fm.y;
+        if (halo) {
+          split(V{vo[h_src], vo[h_src + h_step]}, fp, fm);
+          h_dst[0] = fp;
+          h_dst[PART] = fm;
         }
       }
-      if (q >= 10) {
-        // ---- output plane o = plane q-5: its x- and y-faces
-        const int so = slot_of(q - 5);
-        const T* vo = ring + (size_t)(2 * so) * SM::SLOT;
-        const T* lo = vo + SM::SLOT;
-        for (int e = tid; e < TL::PLANE; e += TL::NT) {
-          const T u = vo[e];
-          fpS[e] = fplus(u);
-          fmS[e] = fminus(u);
+      // ---- z: windows and the face p-3+1/2 (p = plane q)
+      {
+        V fp, fm;
+        split(*reinterpret_cast<const V*>(vq + own), fp, fm);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { fpw[k] = fpw[k + 1]; fmw[k] = fmw[k + 1]; }
+        fpw[4] = fp_new;
+        fp_new = fp;
+        fmw[4] = fm;
+      }
+      if (q >= 5) {
+        const V l3 = *reinterpret_cast<const V*>(ringl + ((q + 3) % TL::NSL) * SM::SLOTL + ownl);
+        const V l2 = *reinterpret_cast<const V*>(ringl + ((q + 4) % TL::NSL) * SM::SLOTL + ownl);
+        const V psi = vmul(V{a.rdz, a.rdz}, vsub(l2, l3));
+        V g[5];
+        side_rev<Z>(fpw[0], fpw[1], fpw[2], fpw[3], fpw[4], psi, g);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) accP[k] = vadd(accP[k], g[k]);
+        side_rev<Z>(fmw[4], fmw[3], fmw[2], fmw[1], fmw[0], psi, g);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) accM[k + 1] = vadd(accM[k + 1], g[4 - k]);
+      }
+      if (out) {
+        __syncthreads();  // f+- in place
+        // one face pair: operands at p (f+; f- PART later) with stride st, partials into FB[.][f]
+        auto face = [&](const V* p, int st, V psi, int f) {
+          V g[5];
+          side_rev<Z>(p[0], p[st], p[2 * st], p[3 * st], p[4 * st], psi, g);
+#pragma unroll
+          for (int k = 0; k < 5; ++k) FB[k * NF + f] = g[k];
+          const V* const m = p + PART;
+          side_rev<Z>(m[5 * st], m[4 * st], m[3 * st], m[2 * st], m[st], psi, g);
+#pragma unroll
+          for (int k = 0; k < 5; ++k) FB[(5 + k) * NF + f] = g[4 - k];
+        };
+        // x-faces: f = 37 rp + i + 3; rows 2 rp, 2 rp + 1
+        auto xface = [&](int rp, int fi) {
+          const T* const l = lo + (2 * rp + TL::HL) * SWL + TL::PADL + fi - 3;  // lam of cell i, both rows
+          const V psi = vmul(V{a.rdx, a.rdx}, vsub(V{l[1], l[SWL + 1]}, V{l[0], l[SWL]}));
+          face(part + rp * XS + fi, 1, psi, rp * TL::FX + fi);
+        };
+        xface(warp, lane);
+        {  // the five faces past lane 31 of every row pair: 40, in two warps (others each plane)
+          const int e = ((warp - q) & 7) * 32 + lane;
+          if (e < 5 * (TL::BY / 2)) xface(e / 5, 32 + e % 5);
         }
         __syncthreads();
-        T gP[2], gM[2];
-        // x-faces: face f = r * 37 + (i + 3), i = -3 .. 33, of row r
-        for (int f = tid; f < TL::NFX; f += TL::NT) {
-          const int r = f / (TL::BX + 5), i = f - r * (TL::BX + 5) - 3;
-          const int b = (r + TL::H) * TL::SW + TL::H + i;  // region index of cell i
-          const T psi = a.rdx * (lo[b + 1] - lo[b]);
-          const T pv[5] = {fpS[b - 2], fpS[b - 1], fpS[b], fpS[b + 1], fpS[b + 2]};
-          const T mv[5] = {fmS[b + 3], fmS[b + 2], fmS[b + 1], fmS[b], fmS[b - 1]};
-          T gp[5], gm[5];
-          sides_rev<T, Z>(pv, mv, psi, gp, gm);
-#pragma unroll
-          for (int k = 0; k < 5; ++k) {
-            FB[k * TL::NF + f] = gp[k];
-            FB[(5 + k) * TL::NF + f] = gm[4 - k];
+        {
+          // x part of J^T lam: rows 2 warp, 2 warp + 1 of column `lane`
+          const V* const P = FB + warp * TL::FX + lane + 3;
+          V sp = vadd(P[2 * NF], vadd(vadd(P[4 * NF - 2], P[3 * NF - 1]), vadd(P[NF + 1], P[2])));
+          const V* const M = P + 5 * NF;
+          V sm = vadd(M[NF], vadd(vadd(M[4 * NF - 3], M[3 * NF - 2]), vadd(M[2 * NF - 1], M[1])));
+          const T* const uu = vo + (2 * warp + H) * SW + TL::PADX + lane;
+          const V u = {uu[0], uu[SW]};
+          const V hu = vmul(vc<V>(0.5), u), au = vabs(u);
+          const V j = vfma(vadd(hu, au), sp, vmul(vsub(hu, au), sm));
+          jx[(2 * warp) * TL::BX + lane] = j.x;
+          jx[(2 * warp + 1) * TL::BX + lane] = j.y;
+        }
+        __syncthreads();
+        // y-faces: f = 16 (j + 3) + column pair
+        auto yface = [&](int fj, int c) {
+          const T* const l = lo + (fj - 3 + TL::HL) * SWL + TL::PADL + 2 * c;  // lam of row j
+          const V psi = vmul(V{a.rdy, a.rdy}, vsub(*reinterpret_cast<const V*>(l + SWL), *reinterpret_cast<const V*>(l)));
+          face(part + YP + fj * PX + c, PX, psi, fj * PX + c);
+        };
+        yface(row, cp);
+        {  // the five rows of faces past row 15: 80, in three warps
+          const int e = ((warp - q - 3) & 7) * 32 + lane;
+          if (e < 5 * PX) yface(TL::BY + e / PX, e % PX);
+        }
+        __syncthreads();
+        const int ko = wrap(zs - 10 + q, nz);
+        const V* const P = FB + (row + 3) * PX + cp;
+        const V sp = vadd(accP[0], vadd(P[2 * NF], vadd(vadd(P[4 * NF - 2 * PX], P[3 * NF - PX]), vadd(P[NF + PX], P[2 * PX]))));
+        const V* const M = P + 5 * NF;
+        const V sm = vadd(accM[0], vadd(M[NF], vadd(vadd(M[4 * NF - 3 * PX], M[3 * NF - 2 * PX]), vadd(M[2 * NF - PX], M[PX]))));
+        const V u = *reinterpret_cast<const V*>(vo + own), lam = *reinterpret_cast<const V*>(lo + ownl);
+        const V hu = vmul(vc<V>(0.5), u), au = vabs(u);
+        const V jt = vadd(*reinterpret_cast<const V*>(jx + row * TL::BX + 2 * cp),
+                          vfma(vadd(hu, au), sp, vmul(vsub(hu, au), sm)));
+        const V t = vfma(V{a.dt, a.dt}, jt, lam);
+        const int x = x0 + 2 * cp, y = y0 + row;
+        const bool in0 = x < nx && y < ny, in1 = x + 1 < nx && y < ny;
+        const size_t o = (size_t)ko * sxy + (size_t)y * nx + x;
+        const bool vec = a.vec_ok && in1;
+        V acc = vc<V>(0);
+        if (a.stage != 3) {
+          if (vec) {
+            if (ADV_IN_RANGE(o + 1, sxy * nz, a.status)) acc = *reinterpret_cast<const V*>(a.acc_in + o);
+          } else {
+            if (in0 && ADV_IN_RANGE(o, sxy * nz, a.status)) acc.x = a.acc_in[o];
+            if (in1 && ADV_IN_RANGE(o + 1, sxy * nz, a.status)) acc.y = a.acc_in[o + 1];
           }
         }
-        __syncthreads();
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int cy = c ? cy1 : cy0;
-          const int fr = cy * (TL::BX + 5) + 3;  // face index of i = 0 in row cy
-          T sp = T(0), sm = T(0);
-#pragma unroll
-          for (int d = -2; d <= 2; ++d) sp += FB[(2 - d) * TL::NF + fr + cx + d];       // faces cx-2 .. cx+2
-#pragma unroll
-          for (int d = -3; d <= 1; ++d) sm += FB[(5 + 1 - d) * TL::NF + fr + cx + d];   // faces cx-3 .. cx+1
-          gP[c] = sp;
-          gM[c] = sm;
-        }
-        __syncthreads();
-        // y-faces: face f = (j + 3) * 32 + col, j = -3 .. 17
-        for (int f = tid; f < TL::NFY; f += TL::NT) {
-          const int jj = f / TL::BX, col = f - jj * TL::BX, j = jj - 3;
-          const int b = (j + TL::H) * TL::SW + TL::H + col;
-          constexpr int W = TL::SW;
-          const T psi = a.rdy * (lo[b + W] - lo[b]);
-          const T pv[5] = {fpS[b - 2 * W], fpS[b - W], fpS[b], fpS[b + W], fpS[b + 2 * W]};
-          const T mv[5] = {fmS[b + 3 * W], fmS[b + 2 * W], fmS[b + W], fmS[b], fmS[b - W]};
-          T gp[5], gm[5];
-          sides_rev<T, Z>(pv, mv, psi, gp, gm);
-#pragma unroll
-          for (int k = 0; k < 5; ++k) {
-            FB[k * TL::NF + f] = gp[k];
-            FB[(5 + k) * TL::NF + f] = gm[4 - k];
+        auto put = [&](T* dst, V w) {
+          if (vec) {
+            if (ADV_IN_RANGE(o + 1, sxy * nz, a.status)) *reinterpret_cast<V*>(dst + o) = w;
+          } else {
+            if (in0 && ADV_IN_RANGE(o, sxy * nz, a.status)) dst[o] = w.x;
+            if (in1 && ADV_IN_RANGE(o + 1, sxy * nz, a.status)) dst[o + 1] = w.y;
           }
-        }
-        __syncthreads();
-        const int ko = wrap(zs - 5 + q - 5, nz);
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int cy = c ? cy1 : cy0;
-          T sp = T(0), sm = T(0);
-#pragma unroll
-          for (int d = -2; d <= 2; ++d) sp += FB[(2 - d) * TL::NF + (cy + d + 3) * TL::BX + cx];
-#pragma unroll
-          for (int d = -3; d <= 1; ++d) sm += FB[(5 + 1 - d) * TL::NF + (cy + d + 3) * TL::BX + cx];
-          const int x = x0 + cx, y = y0 + cy;
-          if (x < nx && y < ny) {
-            const int ci = (cy + TL::H) * TL::SW + TL::H + cx;
-            const T u = vo[ci], lam_c = lo[ci];
-            const T SP = accP[c][0] + gP[c] + sp, SMM = accM[c][0] + gM[c] + sm;
-            const T au = absv(u), hu = T(0.5) * u;
-            const T jt = (hu + au) * SP + (hu - au) * SMM;
-            const T t = lam_c + a.dt * jt;
-            const size_t o = (size_t)ko * sxy + (size_t)y * nx + x;
-            if (a.stage == 3) {
-              a.out[o] = T(2.0 / 3.0) * t;
-              a.acc_out[o] = lam_c * T(1.0 / 3.0);
-            } else if (a.stage == 2) {
-              a.out[o] = T(0.25) * t;
-              a.acc_out[o] = a.acc_in[o] + T(0.75) * lam_c;
-            } else {
-              a.out[o] = a.acc_in[o] + t;
-            }
-          }
+        };
+        if (a.stage == 3) {
+          put(a.out, vmul(vc<V>(2.0 / 3.0), t));
+          put(a.acc_out, vmul(vc<V>(1.0 / 3.0), lam));
+        } else if (a.stage == 2) {
+          put(a.out, vmul(vc<V>(0.25), t));
+          put(a.acc_out, vfma(vc<V>(0.75), lam, acc));
+        } else {
+          put(a.out, vadd(acc, t));
         }
       }
       // shift the z accumulators: cell p-5 leaves, p+1 enters
       if (q >= 5) {
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-#pragma unroll
-          for (int k = 0; k < 5; ++k) { accP[c][k] = accP[c][k + 1]; accM[c][k] = accM[c][k + 1]; }
-          accP[c][5] = T(0);
-          accM[c][5] = T(0);
-        }
+        for (int k = 0; k < 5; ++k) { accP[k] = accP[k + 1]; accM[k] = accM[k + 1]; }
+        accP[5] = vc<V>(0);
+        accM[5] = vc<V>(0);
       }
-      __syncthreads();  // slot of plane q-5 (and the face buffer) free for reuse
-      if (q + TL::P + 1 < Q) issue(q + TL::P + 1);
-      else cp_async_commit();
     }
   }
 }
@@ -473,7 +433,10 @@ adv_status adjoint_stage_t(const adv_burgers_desc& d, int stage, const void* v, 
   a.stage = stage;
   a.tiles_x = (d.nx + AdjTile::BX - 1) / AdjTile::BX;
   a.tiles_y = (d.ny + AdjTile::BY - 1) / AdjTile::BY;
+  const uintptr_t pair = 2 * sizeof(T);
+  a.vec_ok = d.nx % 2 == 0 && (uintptr_t)out % pair == 0 && (uintptr_t)acc_in % pair == 0 && (uintptr_t)acc_out % pair == 0;
   a.dt = (T)dt;
+  a.status = device_status_ptr();
   a.rdx = (T)(1.0 / d.dx); a.rdy = (T)(1.0 / d.dy); a.rdz = (T)(1.0 / d.dz);
   void* k = adjoint_kernel(d);
   const size_t smem = AdjSmem<T>::TOTAL;
@@ -482,8 +445,9 @@ adv_status adjoint_stage_t(const adv_burgers_desc& d, int stage, const void* v, 
   ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 256, smem));
   occ = std::max(occ, 1);
   const int64_t units = (int64_t)a.tiles_x * a.tiles_y * d.nz;
-  // four waves of equal shares, as the forward stage: later waves balance the uneven pair costs
-  const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>(4 * (int64_t)di.sms * occ, units / 8));
+  // one wave of equal shares (128^3: 91.7 us per stage, two waves 96, four 112: a segment streams ten extra
+  // planes), at least two planes each (48^3: 16.8 us, four 23.1, eight 35.6)
+  const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>((int64_t)di.sms * occ, units / 2));
   void* args[] = {&a};
   ADV_CUDA_TRY(cudaLaunchKernel(k, dim3((unsigned)ctas), dim3(256), args, smem, s));
   count_launches(1);
