@@ -16,16 +16,17 @@
 //     u = u - B_s r.
 // For the FP64 state every operation is evaluated in the prototypes' operand order with correctly
 // rounded intrinsics (no contraction), so its results are those of the prototypes -- and of the
-// CPU oracle that restates them -- bit for bit; the FP32 state's faces take a faster form of the
-// same scheme (the FP32 face kernels below).
+// CPU oracle that restates them -- bit for bit; the FP32 state evaluates the same scheme in a fused
+// kernel of its own (weno7_fused_kernel below).
 //
-// Kernels. Per stage and axis: a face kernel (one thread per face i+1/2, the two split parts'
+// Kernels. FP64, per stage and axis: a face kernel (one thread per face i+1/2, the two split parts'
 // reconstructions hp and hn into two face arrays) and a residual kernel (one thread per node,
 // accumulating the axis's residual into the stage's right-hand side); the last axis's residual
 // kernel also applies the Runge-Kutta update in place and, at the last stage, reduces max|u| for
-// the next step's dt. Threads run along x, so every access of every axis is coalesced. The time
-// loop is one CUDA graph with a device-driven while node (the step-start kernel of the Burgers
-// loop: dt rule, trim, t in FP64).
+// the next step's dt. Threads run along x, so every access of every axis is coalesced. FP32: one launch
+// per stage, the state going u -> a -> b -> a -> b -> u through two work arrays. The time loop is one
+// CUDA graph with a device-driven while node (the step-start kernel of the Burgers loop: dt rule, trim,
+// t in FP64); a run of a few steps at most is launched directly, each step predicated on the device.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -38,6 +39,9 @@
 #include "nvtx_range.h"
 #include "weno.cuh"
 
+#ifndef W7OCC
+#define W7OCC 3
+#endif
 namespace adv {
 namespace {
 
@@ -144,151 +148,286 @@ __global__ void __launch_bounds__(256) weno7_face_kernel(const T* __restrict__ u
   }
 }
 
-// ------------------------------------------------------------------ FP32 face kernels
-// The FP32 state takes a form written for speed rather than the prototype's operand order (the
-// FP64 state keeps that order, bit for bit):
-//  * a tile of faces stages the split parts of its cells in shared memory once -- as 64-bit
-//    pairs (f+ of a cell, f- of the next along the line), one load per operand pair -- instead of
-//    every face re-reading and re-splitting its eight cells;
-//  * both split parts of a face are reconstructed together in paired FP32 instructions (lane x
-//    the part moving towards +x on cells i-3..i+3, lane y the other on cells i-2..i+4: the
-//    smoothness indicators use the same coefficients on both);
-//  * the prototype's weights d_k / (eps + beta_k)^2, normalised, are evaluated from
-//    r_k = e_min / e_k (e_k = eps + beta_k, e_min the smallest): alpha_k = d_k r_k^2 lies in
-//    (0, d_k] and the largest is at least d_min, so no product overflows, underflows or leaves a
-//    zero sum, and the face value sum_k alpha_k q_k / (12 sum_k alpha_k) takes one division; the
-//    quotients use the reciprocal-based division (at most 2 ulp each).
-// Tiles: AX = 0, 32 faces along x by 8 rows (one face per thread); AX = 1, 2, 32 x positions by
-// 32 faces along the line (four faces per thread). Cells past a line's ends are its end values
-// (clamped), as in the prototype.
-namespace w7f {
-constexpr int TX = 32;  // x positions (AX = 0: faces) per tile
-constexpr int TR = 8;   // rows per tile, AX = 0
-constexpr int TL = 32;  // faces along the line per tile, AX = 1, 2
-}  // namespace w7f
+// ------------------------------------------------------------------ FP32 fused stage
+// One launch per Runge-Kutta stage: R(u) of all axes, then r = A r + dt R, u_out = u - B r (or R alone for
+// adv_weno7_rhs). 16 bytes per cell and stage (u, r read; r, u_out written) where separate face and
+// residual kernels moved 92.
+//
+// The scheme in differences. With f at i-3 .. i+3, D2_j the second difference at j, c3_k the third
+// difference of candidate k's cells (k = 0: i-3..i, .., 3: i..i+3) and s_j = f_{j+1} - f_{j-1}, the
+// prototype's integer indicators are, for every candidate, the same form of its cubic's derivatives
+// at i:
+//   beta_k / 720 = G_k^2 + 13/3 C_k^2 + 781/180 c3_k^2
+//   G_1 = s_i - c3_1/4, G_2 = s_i - c3_2/4, C_1 = C_2 = D2_i
+//   G_0 = s_{i-1} + 2 D2_{i-1} + 3/4 c3_0, C_0 = D2_{i-1} + c3_0
+//   G_3 = s_{i+1} - 2 D2_{i+1} + 3/4 c3_3, C_3 = D2_{i+1} - c3_3
+// (expanded, the sixteen coefficients of kBeta), and the candidates' face values differ by fourth
+// differences D4: v_1 - v_2 = D4_i/12, v_0 - v_1 = -D4_{i-1}/4, v_3 - v_2 = D4_{i+1}/12. So a side is
+// the symmetric candidate v_2 plus one quotient; both sides' v_2 add up to (7 (w_i + w_{i+1}) -
+// (w_{i-1} + w_{i+2}))/12 with w = f+ + f- = u^2/2. Weights d_k/(eps + beta_k)^2 come from r_k = e_min/e_k
+// (e_k = (eps + beta_k)/720, e_min the smallest): alpha_k = d_k r_k^2 lies in (0, d_k] and the largest is at
+// least d_min, so no product overflows, underflows or leaves a zero sum. Reciprocals are the
+// approximation (1 ulp). No term cancels to less than its own rounding, unlike the integer forms.
+//
+// Layout as the WENO5 stage (burgers_kernels.cuh): 32 x 16 columns per CTA, two adjacent in x per
+// thread; planes with a halo of 4 stream through an 8-slot ring (cp.async from a list of the clamped
+// in-plane offsets); f+- of the output plane go to shared memory in pairs of rows (x-faces) and of
+// columns (y-faces); z-faces come from register windows; two barriers per plane. Bound by the FMA pipe
+// and the barriers (pipe 54% busy, 459 paired FP32 instructions of 922 per pair of cells): right-hand side
+// 256^3 383 us with two CTAs per SM, 371 with three; a run of 3 steps at 160^3 2556 -> 1743 us against
+// six face and residual launches per stage.
+struct W7Tile {
+  static constexpr int BX = 32, BY = 16, NT = 256, PX = BX / 2, R = 4;
+  static constexpr int SW = BX + 2 * R, SH = BY + 2 * R, PLANE = SW * SH;
+  static constexpr int NS = 8, P = 3;
+  static constexpr int XS = SW;                            // x-face operands per pair of rows
+  static constexpr int PART = BY / 2 * XS + SH * PX;       // pairs of one split part
+  static constexpr int XF = BX + 2;
+  static constexpr size_t SMEM = (size_t)NS * PLANE * 4 + (size_t)(2 * PART + (BY + 1) * PX) * 8 + (size_t)BY * XF * 4 +
+                                 (size_t)PLANE * 8;
+};
 
-__device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return vadd(a, b); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return vmul(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return vfma(a, b, c); }
+struct W7Params {
+  const float* u;
+  float* out;  // the new state, or R(u)
+  float* r;    // 2N-storage register; null: R(u) alone
+  int nx, ny, nz, tiles_x, tiles_y;
+  int stage;
+  int vec_ok;  // out and r: pairs of nodes aligned for one access
+  float rhx, rhy, rhz;
+  const double* dt_dev;
+  unsigned* maxkey;
+  const int* active;
+  int* status;
+};
 
-template <int K>
-__device__ __forceinline__ float2 w7_beta2(const float2* x) {  // x: the candidate's cells 0..3
-  constexpr W7B B = kBeta[K];
-  auto c = [](double v) { return f2((float)v); };
-  const float2 a = fma2(c(B.k[1]), x[3], mul2(c(B.k[0]), x[2]));
-  const float2 b = fma2(c(B.k[5]), x[3], fma2(c(B.k[4]), x[B.d], fma2(c(B.k[3]), x[B.c], mul2(c(B.k[2]), x[B.b]))));
-  const float2 t = fma2(c(B.k[9]), x[3], fma2(c(B.k[8]), x[B.t], mul2(c(B.k[7]), x[B.s])));
-  return fma2(x[0], b, fma2(x[1], t, fma2(mul2(c(B.k[6]), x[3]), x[3], mul2(x[2], a))));
-}
-
-template <int K>
-__device__ __forceinline__ float2 w7_cand2(const float2* x) {  // 12 x candidate K, per lane
-  auto c = [](int j) { return make_float2((float)kPolyP[K][j], (float)kPolyM[K][j]); };
-  return fma2(c(3), x[3], fma2(c(2), x[2], fma2(c(1), x[1], mul2(c(0), x[0]))));
-}
-
-// x[j] = (f+ of cell i-3+j, f- of cell i-2+j), j = 0..6. Returns (hn, hp): the +x part on cells
-// i-3..i+3, the -x part on cells i-2..i+4.
-__device__ __forceinline__ float2 w7_face2(const float2 (&x)[7]) {
-  const float2 eps = f2(1e-6f);
-  const float2 e0 = add2(w7_beta2<0>(x + 0), eps), e1 = add2(w7_beta2<1>(x + 1), eps);
-  const float2 e2 = add2(w7_beta2<2>(x + 2), eps), e3 = add2(w7_beta2<3>(x + 3), eps);
+// The nonlinear part of one side for two faces, times 12: 12 (side - v_2); cells i-3 .. i+3.
+__device__ __forceinline__ float2 w7_side2(const float2 (&f)[7]) {
+  auto c = [](double v) { return vc<float2>(v); };
+  float2 D1[6], D2[5], D3[4];
+#pragma unroll
+  for (int j = 0; j < 6; ++j) D1[j] = vsub(f[j + 1], f[j]);
+#pragma unroll
+  for (int j = 0; j < 5; ++j) D2[j] = vsub(D1[j + 1], D1[j]);  // at cells i-2 .. i+2
+#pragma unroll
+  for (int j = 0; j < 4; ++j) D3[j] = vsub(D2[j + 1], D2[j]);
+  const float2 s0 = vadd(D1[1], D1[2]), s1 = vadd(D1[2], D1[3]), s2 = vadd(D1[3], D1[4]);
+  float2 T[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) T[j] = vfma(vmul(c(781.0 / 180.0), D3[j]), D3[j], c(1e-6 / 720.0));
+  const float2 K = vmul(vmul(c(13.0 / 3.0), D2[2]), D2[2]);
+  const float2 C0 = vadd(D2[1], D3[0]), C3 = vsub(D2[3], D3[3]);
+  const float2 G1 = vfma(c(-0.25), D3[1], s1), G2 = vfma(c(-0.25), D3[2], s1);
+  const float2 G0 = vfma(c(0.75), D3[0], vfma(c(2), D2[1], s0)), G3 = vfma(c(0.75), D3[3], vfma(c(-2), D2[3], s2));
+  const float2 e0 = vfma(G0, G0, vfma(vmul(c(13.0 / 3.0), C0), C0, T[0])), e1 = vfma(G1, G1, vadd(K, T[1]));
+  const float2 e2 = vfma(G2, G2, vadd(K, T[2])), e3 = vfma(G3, G3, vfma(vmul(c(13.0 / 3.0), C3), C3, T[3]));
   const float2 em = make_float2(fminf(fminf(e0.x, e1.x), fminf(e2.x, e3.x)), fminf(fminf(e0.y, e1.y), fminf(e2.y, e3.y)));
-  auto alpha = [&](float2 e, int k) {
-    const float2 r = make_float2(__fdividef(em.x, e.x), __fdividef(em.y, e.y));
-    return mul2(mul2(make_float2((float)kLinP[k], (float)kLinM[k]), r), r);
+  auto sq = [&](float2 e) {
+    const float2 r = vmul(em, make_float2(rcp_approx(e.x), rcp_approx(e.y)));
+    return vmul(r, r);
   };
-  const float2 a0 = alpha(e0, 0), a1 = alpha(e1, 1), a2 = alpha(e2, 2), a3 = alpha(e3, 3);
-  const float2 num = fma2(a3, w7_cand2<3>(x + 3), fma2(a2, w7_cand2<2>(x + 2), fma2(a1, w7_cand2<1>(x + 1),
-                                                                                   mul2(a0, w7_cand2<0>(x + 0)))));
-  const float2 den = mul2(f2(12.f), add2(add2(a0, a1), add2(a2, a3)));
-  return make_float2(__fdividef(num.x, den.x), __fdividef(num.y, den.y));
+  const float2 a0 = sq(e0), a1 = sq(e1), a2 = sq(e2), a3 = sq(e3);  // x 1, 12, 18, 4
+  const float2 den = vfma(c(18), a2, vfma(c(12), a1, vfma(c(4), a3, a0)));
+  const float2 q0 = vsub(D3[1], D3[0]), q1 = vsub(D3[2], D3[1]), q2 = vsub(D3[3], D3[2]);  // D4 at i-1, i, i+1
+  const float2 num = vfma(vmul(c(12), a1), q1, vfma(vmul(c(4), a3), q2, vmul(a0, vfma(c(-3), q0, q1))));
+  return vmul(num, make_float2(rcp_approx(den.x), rcp_approx(den.y)));
 }
 
-// (f+, f-) of one node value: f = u^2/2 split with a = |u|.
-__device__ __forceinline__ float2 w7_split_fast(float v) {
-  const float f = 0.5f * v * v, av = fabsf(v) * v;
-  return make_float2(0.5f * (f + av), 0.5f * (f - av));
-}
+__device__ __forceinline__ void w7_split2(float2 u, float2& fp, float2& fm) { lf_split2(u, vabs(u), fp, fm); }
 
-template <int AX>
-__global__ void __launch_bounds__(256) weno7_face_fast_kernel(const float* __restrict__ u, float* __restrict__ hp,
-                                                              float* __restrict__ hn, W7Geom g) {
-  using namespace w7f;
-  constexpr int ROWS = AX == 0 ? TR : TL + 7;  // shared rows: y rows (AX 0) or line cells
-  constexpr int COLS = AX == 0 ? TX + 8 : TX;  // shared columns: x cells (AX 0; 39 used) or x
-  __shared__ float2 fs[ROWS][COLS];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int nx = g.nx, ny = g.ny, nz = g.nz;
-  const int x0 = blockIdx.x * TX;
-  // line position of the tile's first face and the fixed coordinate(s)
-  const int l0 = AX == 0 ? x0 : blockIdx.y * TL;
-  const int N = AX == 0 ? nx : AX == 1 ? ny : nz;
-  const int64_t sxy = (int64_t)nx * ny;
-  auto at = [&](int x, int y, int z) { return (int64_t)z * sxy + (int64_t)y * nx + x; };
-  for (int e = threadIdx.x; e < ROWS * COLS; e += 256) {
-    const int r = e / COLS, c = e - r * COLS;
-    float2 v = make_float2(0.f, 0.f);
-    if (AX == 0) {
-      const int y = blockIdx.y * TR + r, z = blockIdx.z;
-      const int x = min(max(x0 + c - 3, 0), nx - 1);
-      if (c < TX + 7 && y < ny) v = w7_split_fast(u[at(x, y, z)]);
-    } else {
-      const int x = x0 + c, l = min(max(l0 + r - 3, 0), N - 1);
-      if (x < nx) v = w7_split_fast(AX == 1 ? u[at(x, l, blockIdx.z)] : u[at(x, blockIdx.z, l)]);
-    }
-    // element t of a line holds (f+ of cell t, f- of cell t+1): the operand pairs of the paired
-    // reconstruction, loaded as they are (18% faster than packing them from (f+, f-) per cell)
-    float* fsf = reinterpret_cast<float*>(&fs[0][0]);
-    fsf[2 * (r * COLS + c)] = v.x;
-    if (AX == 0 ? c > 0 : r > 0) fsf[2 * (AX == 0 ? r * COLS + c - 1 : (r - 1) * COLS + c) + 1] = v.y;
-  }
-  __syncthreads();
-  if (AX == 0) {
-    const int x = x0 + tx, y = blockIdx.y * TR + ty;
-    if (x < nx && y < ny) {
-      float2 c[7];
-#pragma unroll
-      for (int j = 0; j < 7; ++j) c[j] = fs[ty][tx + j];
-      const float2 h = w7_face2(c);
-      const int64_t o = at(x, y, blockIdx.z);
-      hn[o] = h.x;
-      hp[o] = h.y;
-    }
+__global__ void __launch_bounds__(256, 3) weno7_fused_kernel(const __grid_constant__ W7Params p) {
+  using TL = W7Tile;
+  constexpr int R = TL::R, SW = TL::SW, PX = TL::PX, XS = TL::XS, PART = TL::PART, YP = TL::BY / 2 * XS;
+  if (p.active && *p.active == 0) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float* const ring = reinterpret_cast<float*>(smem_raw);
+  float2* const part = reinterpret_cast<float2*>(ring + TL::NS * TL::PLANE);  // f+; f- PART pairs later
+  float2* const fyS = part + 2 * PART;                                        // y-faces [BY+1][PX]
+  float* const fxS = reinterpret_cast<float*>(fyS + (TL::BY + 1) * PX);       // x-faces [BY][XF]
+  int64_t* const src = reinterpret_cast<int64_t*>(fxS + TL::BY * TL::XF);
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int cp = tid & (PX - 1), row = tid / PX;
+  const int own = (row + R) * SW + R + 2 * cp;
+  const int nx = p.nx, ny = p.ny, nz = p.nz;
+  const size_t sxy = (size_t)nx * ny;
+  const bool twod = nz == 1;
+  const int lag = twod ? 0 : R;
+  const float A = (float)kA[p.stage], B = (float)kB[p.stage];
+  const float dt = p.r ? (float)*p.dt_dev : 0.f;
+  unsigned kmax = 0;
+  // halo splits, two values each: threads [0, 128) the eight halo rows, [128, 192) the eight halo columns
+  const bool halo = tid < 8 * PX + 8 * (TL::BY / 2);
+  int h_src, h_step;
+  float2* h_dst;
+  if (tid < 8 * PX) {
+    const int h = tid / PX, r = h < R ? h : h + TL::BY;
+    h_src = r * SW + R + 2 * cp;
+    h_step = 1;
+    h_dst = part + YP + r * PX + cp;
   } else {
-    const int x = x0 + tx;
-    if (x < nx) {
+    const int i = tid - 8 * PX, rp = (i / 8) % (TL::BY / 2), h = i % 8, c = h < R ? h : h + TL::BX;
+    h_src = (2 * rp + R) * SW + c;
+    h_step = SW;
+    h_dst = part + rp * XS + c;
+  }
+  // the last x-face of each row pair (lanes [0, 8)) and the top row of y-faces (lanes [8, 24))
+  const bool l_x = lane < TL::BY / 2;
+  const int l_st = l_x ? 1 : PX;
+  const int l_src = l_x ? lane * XS + TL::BX : YP + TL::BY * PX + (lane - TL::BY / 2);
+  unsigned n = 0;  // stream entries so far (slot n % NS)
+
+  const int64_t total = (int64_t)p.tiles_x * p.tiles_y * nz;
+  const int64_t seg_a = total * blockIdx.x / gridDim.x, seg_b = total * (blockIdx.x + 1) / gridDim.x;
+  for (int64_t pos = seg_a; pos < seg_b;) {
+    const int64_t tile = pos / nz;
+    const int zs = (int)(pos - tile * nz);
+    const int ze = (int)min((int64_t)nz, zs + (seg_b - pos));
+    pos += ze - zs;
+    const int x0 = (int)(tile % p.tiles_x) * TL::BX, y0 = (int)(tile / p.tiles_x) * TL::BY;
+    const int Q = (ze - zs) + 2 * lag;
+    for (int e = tid; e < TL::PLANE; e += TL::NT) {  // (each thread reads back only what it wrote)
+      const int r = e / SW, c = e - r * SW;
+      src[e] = (int64_t)min(max(y0 - R + r, 0), ny - 1) * nx + min(max(x0 - R + c, 0), nx - 1);
+    }
+    auto slot = [&](int q) { return ring + ((n + (unsigned)q) % TL::NS) * TL::PLANE; };
+    auto issue = [&](int q) {
+      if (q < Q) {
+        float* const dst = slot(q);
+        const float* const plane = p.u + (size_t)min(max(zs - lag + q, 0), nz - 1) * sxy;
+        for (int e = tid; e < TL::PLANE; e += TL::NT)
+          cp_async_zfill<4>(dst + e, plane + src[e], ADV_IN_RANGE(plane + src[e] - p.u, sxy * nz, p.status));
+      }
+      cp_async_commit();
+    };
+    for (int q = 0; q <= TL::P; ++q) issue(q);
+
+    const int x = x0 + 2 * cp, y = y0 + row;
+    const bool in0 = x < nx && y < ny, in1 = x + 1 < nx && y < ny;
+    const bool vec = p.vec_ok && in1;
+    size_t gi = (size_t)zs * sxy + (size_t)y * nx + x;
+    float2 fp[7], fm[7], fp_new = vc<float2>(0);  // f+ at q-7 .. q-1, f- at q-6 .. q
 #pragma unroll
-      for (int j = 0; j < TL / 8; ++j) {
-        const int t = ty + 8 * j, l = l0 + t;
-        if (l < N) {
-          float2 c[7];
-#pragma unroll
-          for (int m = 0; m < 7; ++m) c[m] = fs[t + m][tx];
-          const float2 h = w7_face2(c);
-          const int64_t o = AX == 1 ? at(x, l, blockIdx.z) : at(x, blockIdx.z, l);
-          hn[o] = h.x;
-          hp[o] = h.y;
+    for (int k = 0; k < 7; ++k) fp[k] = fm[k] = vc<float2>(0);
+    float2 w1 = vc<float2>(0), w2 = w1, w3 = w1;  // u^2 at planes q-3, q-4, q-5
+    float2 fz_prev = vc<float2>(0);
+#pragma unroll 1
+    for (int q = 0; q < Q; ++q) {
+      const float* const plq = slot(q);
+      const float* const plc = slot(q - lag);  // the output plane
+      cp_async_wait<TL::P>();
+      __syncthreads();  // plane q visible
+      const bool out = q >= 2 * lag;
+      const float2 uc = *reinterpret_cast<const float2*>(plc + own);
+      if (out) {
+        float2 a, b;
+        w7_split2(uc, a, b);
+        float2* const yw = part + YP + R * PX + tid;
+        yw[0] = a;
+        yw[PART] = b;
+        float* const xw = reinterpret_cast<float*>(part + warp * XS + 2 * cp + R) + (row & 1);
+        xw[0] = a.x; xw[2] = a.y;
+        xw[2 * PART] = b.x; xw[2 * PART + 2] = b.y;
+        if (halo) {
+          w7_split2(make_float2(plc[h_src], plc[h_src + h_step]), a, b);
+          h_dst[0] = a;
+          h_dst[PART] = b;
         }
       }
+      // ---- the z-face between planes q-4 and q-3
+      float2 fz = vc<float2>(0);
+      if (!twod) {
+        float2 a, b;
+        w7_split2(*reinterpret_cast<const float2*>(plq + own), a, b);
+        const float2 u2 = *reinterpret_cast<const float2*>(slot(q - 2) + own);  // (before plane 2: stale, not used)
+        const float2 w0 = vmul(u2, u2);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) { fp[k] = fp[k + 1]; fm[k] = fm[k + 1]; }
+        fp[6] = fp_new;
+        fp_new = a;
+        fm[6] = b;
+        if (q >= 2 * R - 1 && zs - 2 * R + q >= 0) {  // (the face below plane 0 is 0)
+          const float2 qp = w7_side2(fp);
+          const float2 m[7] = {fm[6], fm[5], fm[4], fm[3], fm[2], fm[1], fm[0]};
+          const float2 lin = vfma(vc<float2>(3.5), vadd(w1, w2), vmul(vc<float2>(-0.5), vadd(w0, w3)));
+          fz = vmul(vc<float2>(1.0 / 12.0), vadd(lin, vadd(qp, w7_side2(m))));
+        }
+        w3 = w2; w2 = w1; w1 = w0;
+      }
+      __syncthreads();  // f+- in place; every read of the output plane's slot is done
+      issue(q + TL::P + 1);
+      if (out) {
+        float2 rr = vc<float2>(0);
+        if (p.r && p.stage > 0) {  // requested before the faces, used after them (stage 0: A = 0)
+          if (vec) {
+            if (ADV_IN_RANGE(gi + 1, sxy * nz, p.status)) rr = *reinterpret_cast<const float2*>(p.r + gi);
+          } else {
+            if (in0 && ADV_IN_RANGE(gi, sxy * nz, p.status)) rr.x = p.r[gi];
+            if (in1 && ADV_IN_RANGE(gi + 1, sxy * nz, p.status)) rr.y = p.r[gi + 1];
+          }
+        }
+        auto face = [](const float2* a, int st) {
+          const float2* const b = a + PART;
+          const float2 f[7] = {a[0], a[st], a[2 * st], a[3 * st], a[4 * st], a[5 * st], a[6 * st]};
+          const float2 m[7] = {b[7 * st], b[6 * st], b[5 * st], b[4 * st], b[3 * st], b[2 * st], b[st]};
+          // cells i-1, i, i+1, i+2: f[2..5] and m[5..2]
+          const float2 in = vadd(vadd(f[3], m[4]), vadd(f[4], m[3])), ex = vadd(vadd(f[2], m[5]), vadd(f[5], m[2]));
+          const float2 lin = vfma(vc<float2>(7), in, vmul(vc<float2>(-1), ex));
+          return vmul(vc<float2>(1.0 / 12.0), vadd(lin, vadd(w7_side2(f), w7_side2(m))));
+        };
+        float2 fx = face(part + warp * XS + lane, 1);
+        if (x0 + lane == 0) fx = vc<float2>(0);  // the face left of the first node
+        fxS[(2 * warp) * TL::XF + lane] = fx.x;
+        fxS[(2 * warp + 1) * TL::XF + lane] = fx.y;
+        float2 fym = face(part + YP + tid, PX);
+        if (y == 0) fym = vc<float2>(0);
+        fyS[tid] = fym;
+        if (warp == (q & 7) && lane < TL::BY / 2 + PX) {
+          const float2 f = face(part + l_src, l_st);
+          if (l_x) {
+            fxS[(2 * lane) * TL::XF + TL::BX] = f.x;
+            fxS[(2 * lane + 1) * TL::XF + TL::BX] = f.y;
+          } else {
+            fyS[TL::BY * PX + lane - TL::BY / 2] = f;
+          }
+        }
+        __syncthreads();
+        const float2 fx0 = *reinterpret_cast<const float2*>(fxS + row * TL::XF + 2 * cp);
+        const float2 fx1 = make_float2(fx0.y, fxS[row * TL::XF + 2 * cp + 2]);
+        const float2 fyp = fyS[tid + PX];
+        const float2 L = vfma(vsub(fz, fz_prev), make_float2(p.rhz, p.rhz),
+                              vfma(vsub(fyp, fym), make_float2(p.rhy, p.rhy), vmul(vsub(fx1, fx0), make_float2(p.rhx, p.rhx))));
+        float2 res = L;
+        if (p.r) {
+          rr = vfma(make_float2(A, A), rr, vmul(make_float2(dt, dt), L));
+          res = vfma(make_float2(-B, -B), rr, uc);
+          const unsigned k0 = in0 ? abs_key(res.x) : 0u, k1 = in1 ? abs_key(res.y) : 0u;
+          kmax = max(kmax, max(k0, k1));
+        }
+        auto put = [&](float* dst, float2 v) {
+          if (vec) {
+            if (ADV_IN_RANGE(gi + 1, sxy * nz, p.status)) *reinterpret_cast<float2*>(dst + gi) = v;
+          } else {
+            if (in0 && ADV_IN_RANGE(gi, sxy * nz, p.status)) dst[gi] = v.x;
+            if (in1 && ADV_IN_RANGE(gi + 1, sxy * nz, p.status)) dst[gi + 1] = v.y;
+          }
+        };
+        put(p.out, res);
+        if (p.r) put(p.r, rr);
+        gi += sxy;
+      }
+      fz_prev = fz;
     }
+    n += (unsigned)Q;
+  }
+  if (p.maxkey) {
+    kmax = warp_max(kmax);
+    if (lane == 0 && kmax) atomicMax(p.maxkey, kmax);
   }
 }
 
-// Face launch of axis AX: the tiled FP32 kernel where its grid fits, else the generic kernel.
 template <class T, int AX>
 void weno7_face_launch(const T* u, T* hp, T* hn, const W7Geom& g, int grid, cudaStream_t s) {
-  if constexpr (std::is_same<T, float>::value) {
-    using namespace w7f;
-    const int64_t gx = (g.nx + TX - 1) / TX;
-    const int64_t gy = AX == 0 ? (g.ny + TR - 1) / TR : AX == 1 ? (g.ny + TL - 1) / TL : (g.nz + TL - 1) / TL;
-    const int64_t gz = AX == 2 ? g.ny : g.nz;
-    if (gx <= 0x7fffffff && gy <= 65535 && gz <= 65535) {
-      weno7_face_fast_kernel<AX><<<dim3((unsigned)gx, (unsigned)gy, (unsigned)gz), 256, 0, s>>>(u, hp, hn, g);
-      return;
-    }
-  }
   weno7_face_kernel<T, AX><<<grid, 256, 0, s>>>(u, hp, hn, g);
 }
 
@@ -399,62 +538,91 @@ int weno7_grid(const adv_weno7_desc& d) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)sms * 16));
 }
 
-// The face + residual launches of one stage (stage 0..4), the update fused into the last axis.
-template <class T>
-adv_status weno7_stage_t(const adv_weno7_desc& d, T* u, const W7Work& w, int stage, const double* dt_dev,
+// One FP32 stage (out: the new state; r: the 2N-storage register) or, with r null, R(u) alone.
+adv_status weno7_fused(const adv_weno7_desc& d, const float* u, float* out, float* r, int stage, const double* dt_dev,
+                       void* maxkey, const int* active, bool count, cudaStream_t s) {
+  DeviceInfo di;
+  adv_status st = device_info(&di);
+  if (st != ADV_OK) return st;
+  W7Params p;
+  p.u = u;
+  p.out = out;
+  p.r = r;
+  p.nx = d.nx; p.ny = d.ny; p.nz = d.nz;
+  p.tiles_x = (d.nx + W7Tile::BX - 1) / W7Tile::BX;
+  p.tiles_y = (d.ny + W7Tile::BY - 1) / W7Tile::BY;
+  p.stage = stage;
+  p.vec_ok = d.nx % 2 == 0 && (uintptr_t)out % 8 == 0 && (uintptr_t)r % 8 == 0 ? 1 : 0;
+  p.rhx = (float)(1.0 / d.dx); p.rhy = (float)(1.0 / d.dy); p.rhz = (float)(1.0 / d.dz);
+  p.dt_dev = dt_dev;
+  p.maxkey = static_cast<unsigned*>(maxkey);
+  p.active = active;
+  p.status = device_status_ptr();
+  ADV_CUDA_TRY(cudaFuncSetAttribute(weno7_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)W7Tile::SMEM));
+  int occ = 0;
+  ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, weno7_fused_kernel, W7Tile::NT, W7Tile::SMEM));
+  // one wave of equal shares, at least two planes each (a segment streams eight more)
+  const int64_t units = (int64_t)p.tiles_x * p.tiles_y * d.nz;
+  const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>((int64_t)di.sms * std::max(occ, 1), d.nz == 1 ? units : units / 2));
+  weno7_fused_kernel<<<(unsigned)ctas, W7Tile::NT, W7Tile::SMEM, s>>>(p);
+  ADV_CUDA_TRY(cudaGetLastError());
+  if (count) count_launches(1);
+  return ADV_OK;
+}
+
+// The face + residual launches of one FP64 stage (stage 0..4), the update fused into the last axis.
+adv_status weno7_stage64(const adv_weno7_desc& d, double* u, const W7Work& w, int stage, const double* dt_dev,
                          void* maxkey, const int* active, bool count, cudaStream_t s) {
-  using K = typename KeyOf<T>::type;
+  using K = KeyOf<double>::type;
   const W7Geom g{d.nx, d.ny, d.nz, (int64_t)d.nx * d.ny * d.nz};
   const int grid = weno7_grid(d);
   const int nd = weno7_ndim(d);
-  T* hp = reinterpret_cast<T*>(w.hp);
-  T* hn = reinterpret_cast<T*>(w.hn);
-  T* acc = reinterpret_cast<T*>(w.acc);
-  T* r = reinterpret_cast<T*>(w.r);
+  double* hp = reinterpret_cast<double*>(w.hp);
+  double* hn = reinterpret_cast<double*>(w.hn);
+  double* acc = reinterpret_cast<double*>(w.acc);
+  double* r = reinterpret_cast<double*>(w.r);
   K* mk = static_cast<K*>(maxkey);
-  const T hx = T(d.dx), hy = T(d.dy), hz = T(d.dz);
-  weno7_face_launch<T, 0>(u, hp, hn, g, grid, s);
-  weno7_residual_launch<T, 0, true, false>(hp, hn, acc, r, u, g, hx, stage, dt_dev, mk, active, grid, s);
-  weno7_face_launch<T, 1>(u, hp, hn, g, grid, s);
+  weno7_face_launch<double, 0>(u, hp, hn, g, grid, s);
+  weno7_residual_launch<double, 0, true, false>(hp, hn, acc, r, u, g, d.dx, stage, dt_dev, mk, active, grid, s);
+  weno7_face_launch<double, 1>(u, hp, hn, g, grid, s);
   if (nd == 2) {
-    weno7_residual_launch<T, 1, false, true>(hp, hn, acc, r, u, g, hy, stage, dt_dev, mk, active, grid, s);
+    weno7_residual_launch<double, 1, false, true>(hp, hn, acc, r, u, g, d.dy, stage, dt_dev, mk, active, grid, s);
   } else {
-    weno7_residual_launch<T, 1, false, false>(hp, hn, acc, r, u, g, hy, stage, dt_dev, mk,
-                                                                   active, grid, s);
-    weno7_face_launch<T, 2>(u, hp, hn, g, grid, s);
-    weno7_residual_launch<T, 2, false, true>(hp, hn, acc, r, u, g, hz, stage, dt_dev, mk, active, grid, s);
+    weno7_residual_launch<double, 1, false, false>(hp, hn, acc, r, u, g, d.dy, stage, dt_dev, mk, active, grid, s);
+    weno7_face_launch<double, 2>(u, hp, hn, g, grid, s);
+    weno7_residual_launch<double, 2, false, true>(hp, hn, acc, r, u, g, d.dz, stage, dt_dev, mk, active, grid, s);
   }
   ADV_CUDA_TRY(cudaGetLastError());
   if (count) count_launches(2 * nd);
   return ADV_OK;
 }
 
+// One of a step's five stages. FP32 goes u -> a -> b -> a -> b -> u through the work arrays hp, hn.
 adv_status weno7_stage(const adv_weno7_desc& d, void* u, const W7Work& w, int stage, const double* dt_dev,
                        void* maxkey, const int* active, bool count, cudaStream_t s) {
-  if (d.dtype == ADV_F32)
-    return weno7_stage_t<float>(d, static_cast<float*>(u), w, stage, dt_dev, maxkey, active, count, s);
-  return weno7_stage_t<double>(d, static_cast<double*>(u), w, stage, dt_dev, maxkey, active, count, s);
+  if (d.dtype == ADV_F64) return weno7_stage64(d, static_cast<double*>(u), w, stage, dt_dev, maxkey, active, count, s);
+  float* const a = reinterpret_cast<float*>(w.hp);
+  float* const b = reinterpret_cast<float*>(w.hn);
+  float* const v[6] = {static_cast<float*>(u), a, b, a, b, static_cast<float*>(u)};
+  return weno7_fused(d, v[stage], v[stage + 1], reinterpret_cast<float*>(w.r), stage, dt_dev, maxkey, active, count, s);
 }
 
-// The right-hand side alone (the summed residuals, no update): RHS kernels into acc, then copied
-// to the caller's L.
-template <class T>
-adv_status weno7_rhs_t(const adv_weno7_desc& d, const T* u, T* L, const W7Work& w, cudaStream_t s) {
+int weno7_stage_launches(const adv_weno7_desc& d) { return d.dtype == ADV_F64 ? 2 * weno7_ndim(d) : 1; }
+
+// The right-hand side alone (the summed residuals, no update), FP64.
+adv_status weno7_rhs64(const adv_weno7_desc& d, const double* u, double* L, const W7Work& w, cudaStream_t s) {
   const W7Geom g{d.nx, d.ny, d.nz, (int64_t)d.nx * d.ny * d.nz};
   const int grid = weno7_grid(d);
   const int nd = weno7_ndim(d);
-  T* hp = reinterpret_cast<T*>(w.hp);
-  T* hn = reinterpret_cast<T*>(w.hn);
-  weno7_face_launch<T, 0>(u, hp, hn, g, grid, s);
-  weno7_residual_launch<T, 0, true, false>(hp, hn, L, nullptr, nullptr, g, T(d.dx), 0, nullptr,
-                                                                 nullptr, nullptr, grid, s);
-  weno7_face_launch<T, 1>(u, hp, hn, g, grid, s);
-  weno7_residual_launch<T, 1, false, false>(hp, hn, L, nullptr, nullptr, g, T(d.dy), 0, nullptr,
-                                                                 nullptr, nullptr, grid, s);
+  double* hp = reinterpret_cast<double*>(w.hp);
+  double* hn = reinterpret_cast<double*>(w.hn);
+  weno7_face_launch<double, 0>(u, hp, hn, g, grid, s);
+  weno7_residual_launch<double, 0, true, false>(hp, hn, L, nullptr, nullptr, g, d.dx, 0, nullptr, nullptr, nullptr, grid, s);
+  weno7_face_launch<double, 1>(u, hp, hn, g, grid, s);
+  weno7_residual_launch<double, 1, false, false>(hp, hn, L, nullptr, nullptr, g, d.dy, 0, nullptr, nullptr, nullptr, grid, s);
   if (nd == 3) {
-    weno7_face_launch<T, 2>(u, hp, hn, g, grid, s);
-    weno7_residual_launch<T, 2, false, false>(hp, hn, L, nullptr, nullptr, g, T(d.dz), 0,
-                                                                   nullptr, nullptr, nullptr, grid, s);
+    weno7_face_launch<double, 2>(u, hp, hn, g, grid, s);
+    weno7_residual_launch<double, 2, false, false>(hp, hn, L, nullptr, nullptr, g, d.dz, 0, nullptr, nullptr, nullptr, grid, s);
   }
   ADV_CUDA_TRY(cudaGetLastError());
   count_launches(2 * nd);
@@ -484,8 +652,9 @@ adv_status adv_weno7_rhs(const adv_weno7_desc* d, const void* u, void* L, void* 
   if (u == L) return set_error(ADV_ERR_INVALID_ARG, "weno7: u and L must not alias");
   const W7Work w = weno7_work(*d, workspace);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (d->dtype == ADV_F32) return weno7_rhs_t<float>(*d, static_cast<const float*>(u), static_cast<float*>(L), w, s);
-  return weno7_rhs_t<double>(*d, static_cast<const double*>(u), static_cast<double*>(L), w, s);
+  if (d->dtype == ADV_F32)
+    return weno7_fused(*d, static_cast<const float*>(u), static_cast<float*>(L), nullptr, 0, nullptr, nullptr, nullptr, true, s);
+  return weno7_rhs64(*d, static_cast<const double*>(u), static_cast<double*>(L), w, s);
 }
 
 adv_status adv_weno7_run(const adv_weno7_desc* d, void* u, void* workspace, double tEnd, double cfl,
@@ -511,16 +680,20 @@ adv_status adv_weno7_run(const adv_weno7_desc* d, void* u, void* workspace, doub
   if ((st = max_abs_launch(d->dtype, u, (int64_t)n, key0, s)) != ADV_OK) return st;
   // one time step: the step-start kernel (dt, t, loop condition), then five stages; the last one
   // reduces max|u| for the next step into slot 0
-  const int nd = weno7_ndim(*d);
   auto body = [&](cudaStream_t cs, unsigned long long cond, int use_cond) -> adv_status {
     adv_status r = burgers_loop_begin_step(w.st, d->dtype, cond, use_cond, cs);
     for (int stg = 0; stg < 5 && r == ADV_OK; ++stg)
       r = weno7_stage(*d, u, w, stg, &w.st->dt, stg == 4 ? key0 : nullptr, &w.st->active, !use_cond, cs);
     return r;
   };
-  const int64_t launched_per_step = 1 + 5 * 2 * nd;
+  const int64_t launched_per_step = 1 + 5 * weno7_stage_launches(*d);
   bool graph_ran = false;
-  if (max_steps > 0 && tEnd > 0.0) {
+  // A run of a few steps at most: its launches, predicated on the loop state, cost less than capturing
+  // and instantiating a graph (about 0.2 ms).
+  if (max_steps > 0 && max_steps <= 8 && tEnd > 0.0) {
+    for (int64_t i = 0; i < max_steps; ++i)
+      if ((st = body(s, 0, 0)) != ADV_OK) return st;
+  } else if (max_steps > 0 && tEnd > 0.0) {
     cudaGraph_t g = nullptr;
     cudaGraphExec_t ge = nullptr;
     cudaStream_t cs;
