@@ -173,6 +173,26 @@ __device__ __forceinline__ BurgersPatch* burgers_patch() {
   return &patch;
 }
 
+// The CTA's running max|u_out| key (8 bytes hold either state type's).
+__device__ __forceinline__ unsigned long long* burgers_block_max() {
+  __shared__ unsigned long long m;
+  return &m;
+}
+// Merges every thread's key into *key (nullable) with one global atomic per CTA: one per warp and segment
+// to the same address took longer than a small grid's stage (2D 1000 x 900: 13,000 of them per launch).
+template <class K>
+__device__ __forceinline__ void burgers_flush_max(K kmax, void* key) {
+  if (!key) return;
+  K* const m = reinterpret_cast<K*>(burgers_block_max());
+  __syncthreads();
+  if (threadIdx.x == 0) *m = 0;
+  __syncthreads();
+  kmax = warp_max(kmax);
+  if ((threadIdx.x & 31) == 0 && kmax) atomicMax(m, kmax);
+  __syncthreads();
+  if (threadIdx.x == 0 && *m) atomicMax(static_cast<K*>(key), *m);
+}
+
 template <class T>
 __device__ __forceinline__ void burgers_cta_init(const CUtensorMap* tmap, bool tma) {
   if (threadIdx.x == 0) {
@@ -213,11 +233,11 @@ __device__ __forceinline__ float2 combine2(int stage, float2 un, float2 u, float
 }
 
 // One segment: output planes [zs, ze) of the column tile at (x0, y0), streamed through the
-// ring, whose first entry is number n0. Flushes this segment's max|u_out| into p.maxabs_key. Returns
-// the next segment's first entry number, kPipeAborted if a wait timed out (the CTA must then return).
+// ring, whose first entry is number n0. Raises kmax to this thread's max|u_out| key. Returns the next
+// segment's first entry number, kPipeAborted if a wait timed out (the CTA must then return).
 template <class T, bool Z, class D, bool VISC, int MODE>
 __device__ __forceinline__ unsigned burgers_segment(const CUtensorMap* tmap, const BurgersParams<T>& p, int x0, int y0,
-                                                    int zs, int ze, unsigned n0) {
+                                                    int zs, int ze, unsigned n0, typename KeyOf<T>::type& kmax) {
   using TL = BurgersTile;
   using SM = BurgersSmem<T>;
   using K = typename KeyOf<T>::type;
@@ -268,7 +288,6 @@ __device__ __forceinline__ unsigned burgers_segment(const CUtensorMap* tmap, con
   const bool upd0 = in0 && yok && (per || (x >= FR && x < nx - FR));
   const bool upd1 = in1 && yok && (per || (x + 1 >= FR && x + 1 < nx - FR));
   const bool vec = p.vec_ok && in1;
-  K kmax = 0;
   // Operand places of this thread's share of the splits and faces.
   T* const xw = reinterpret_cast<T*>(part + warp * XS + 2 * cp + R) + (row & 1);  // its cells, x layout
   V* const yw = part + YP + R * PX + tid;                                        // its cells, y layout
@@ -522,10 +541,6 @@ __device__ __forceinline__ unsigned burgers_segment(const CUtensorMap* tmap, con
     if (VISC) { ua = ub; ub = uc; }
     uc = u2;
   }
-  if (p.maxabs_key) {
-    kmax = warp_max(kmax);
-    if (lane == 0 && kmax) atomicMax(static_cast<K*>(p.maxabs_key), kmax);
-  }
   return n0 + (unsigned)Q;
 }
 
@@ -548,15 +563,17 @@ burgers_stage_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_cons
   const int64_t seg_a = total * blockIdx.x / gridDim.x, seg_b = total * (blockIdx.x + 1) / gridDim.x;
   burgers_cta_init<T>(&tmap, p.tma != 0);
   unsigned entries = 0;
+  typename KeyOf<T>::type kmax = 0;
   for (int64_t pos = seg_a; pos < seg_b;) {
     const int64_t tile = pos / nz;
     const int zs = (int)(pos - tile * nz);
     const int ze = (int)min((int64_t)nz, zs + (seg_b - pos));
     pos += ze - zs;
     const int x0 = (int)(tile % p.tiles_x) * TL::BX, y0 = (int)(tile / p.tiles_x) * TL::BY;
-    entries = burgers_segment<T, Z, D, VISC, MODE>(&tmap, p, x0, y0, zs, ze, entries);
+    entries = burgers_segment<T, Z, D, VISC, MODE>(&tmap, p, x0, y0, zs, ze, entries, kmax);
     if (entries == kPipeAborted) return;
   }
+  burgers_flush_max(kmax, p.maxabs_key);
 }
 
 // One instance of a batched Burgers stage: the tensor map of its stage input and the stage's
@@ -609,8 +626,10 @@ burgers_batch_kernel(const BurgersBatchInst<T>* __restrict__ inst, int n_inst, i
     const int x0 = (int)(tile % p.tiles_x) * TL::BX, y0 = (int)(tile / p.tiles_x) * TL::BY;
     const CUtensorMap* tm = &inst[i].tmap;
     if (tma && threadIdx.x == 0) tma_prefetch_desc(tm);
-    entries = burgers_segment<T, Z, D, VISC, MODE>(tm, p, x0, y0, zs, ze, entries);
+    typename KeyOf<T>::type kmax = 0;
+    entries = burgers_segment<T, Z, D, VISC, MODE>(tm, p, x0, y0, zs, ze, entries, kmax);
     if (entries == kPipeAborted) return;
+    burgers_flush_max(kmax, p.maxabs_key);
   }
 }
 
