@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "work_split.h"
+
 namespace adv {
 
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // 2 s
@@ -41,6 +43,30 @@ __device__ __forceinline__ bool adv_in_range(long long i, long long n, int* stat
 #else
 #define ADV_IN_RANGE(i, n, status) true
 #endif
+
+// ------------------------------------------------------------------------- work split
+// CTA b's share [begin, end) of the (tile, plane) pairs (work_split.h): where shares are never cut tile by
+// tile, and in general.
+__device__ __forceinline__ void split_range_whole(const WorkSplit& w, unsigned b, int64_t* begin, int64_t* end) {
+  const unsigned k0 = min((unsigned)((uint64_t)b * w.ratio >> 31), w.extra);
+  const unsigned k1 = min((unsigned)((uint64_t)(b + 1) * w.ratio >> 31), w.extra);
+  *begin = w.each * b + k0;
+  *end = w.each * (b + 1) + k1;
+}
+__device__ __forceinline__ void split_range(const WorkSplit& w, unsigned b, int nz, int64_t* begin, int64_t* end) {
+  int64_t base = 0;
+  if (w.parts != w.ctas) {  // tile by tile
+    const unsigned tile = b / w.parts;
+    b -= tile * w.parts;
+    base = (int64_t)tile * nz;
+  }
+  *begin = base + w.each * b + (b < w.extra ? b : w.extra);
+  *end = *begin + w.each + (b < w.extra ? 1 : 0);
+}
+// n / d for n >= 0, in 32 bits where n allows it.
+__device__ __forceinline__ int64_t div_units(int64_t n, int d) {
+  return n <= 0xffffffffll ? (int64_t)((unsigned)n / (unsigned)d) : n / d;
+}
 
 // ------------------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {

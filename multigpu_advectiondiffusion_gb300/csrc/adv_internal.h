@@ -9,6 +9,7 @@
 #include <string>
 
 #include "../../include/advdiff.h"
+#include "work_split.h"
 
 namespace adv {
 
@@ -81,6 +82,7 @@ struct HeatLaunch {
   int warps = 8;                 // warps per CTA
   int lanes = 32;                // lanes per row (16: two rows per warp); tile lanes*vector x (32*warps/lanes)*rows
   int tiles_x = 0, tiles_y = 0;  // x-y tiles; the grid is one wave of CTAs sharing the tile-planes
+  WorkSplit split;
   dim3 grid, block;
   size_t smem = 0;
   CUtensorMap tmap_in;  // tensor map of u_in (re-encoded when the pointer changes)
@@ -121,6 +123,7 @@ struct BurgersLaunch {
   int mode = 0;  // BurgersMode: the kernel's load path and problem class
   int occ = 0;  // resident CTAs per SM of the stage kernel (before any tuning cap)
   int tiles_x = 0, tiles_y = 0;  // 32 x 16 column tiles; the grid is one wave sharing the tile-planes
+  WorkSplit split;
   dim3 grid, block;
   size_t smem = 0;
   CUtensorMap tmap_in;

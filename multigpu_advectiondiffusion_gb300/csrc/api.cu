@@ -132,10 +132,11 @@ adv_status burgers_prepare(const adv_burgers_desc& d, const void* u_in, BurgersL
     min_share = std::max(1, tp.b);
   }
   const int64_t wave = (int64_t)di.sms * occ;
-  const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>(total >= 48 * wave ? 2 * wave : wave, total / min_share));
+  L->split = work_split((int64_t)tiles_x * tiles_y, d.nz, total >= 48 * wave ? 2 * wave : wave, min_share,
+                        d.dtype == ADV_F32 ? 3.0 : 0.6);
   L->tiles_x = tiles_x;
   L->tiles_y = tiles_y;
-  L->grid = dim3((unsigned)ctas, 1, 1);
+  L->grid = dim3(L->split.ctas, 1, 1);
   std::memset(&L->tmap_in, 0, sizeof(L->tmap_in));
   if (L->tma) {
     EncodeTiledFn enc = encode_tiled_fn();

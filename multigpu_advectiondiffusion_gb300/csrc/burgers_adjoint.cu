@@ -74,6 +74,7 @@ struct AdjArgs {
   T* acc_out;       // accumulated adjoint of u^n (stages 3, 2); may equal acc_in
   int nx, ny, nz, stage;
   int tiles_x, tiles_y;
+  WorkSplit split;  // of the (tile, plane) pairs over the CTAs
   int vec_ok;  // outputs and acc_in: pairs of nodes aligned for one access
   T dt, rdx, rdy, rdz;
   int* status;
@@ -197,15 +198,16 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) burgers_adjoint_k
     h_dst = part + rp * XS + c;
   }
   auto split = [](V u, V& fp, V& fm) { lf_split2(u, vabs(u), fp, fm); };
-  const int64_t total = (int64_t)a.tiles_x * a.tiles_y * nz;
-  const int64_t seg_a = total * blockIdx.x / gridDim.x, seg_b = total * (blockIdx.x + 1) / gridDim.x;
+  int64_t seg_a, seg_b;
+  split_range(a.split, blockIdx.x, nz, &seg_a, &seg_b);
 
   for (int64_t pos = seg_a; pos < seg_b;) {
-    const int64_t tile = pos / nz;
+    const int64_t tile = div_units(pos, nz);
     const int zs = (int)(pos - tile * nz);
     const int ze = (int)min((int64_t)nz, zs + (seg_b - pos));
     pos += ze - zs;
-    const int x0 = (int)(tile % a.tiles_x) * TL::BX, y0 = (int)(tile / a.tiles_x) * TL::BY;
+    const int64_t ty = div_units(tile, a.tiles_x);
+    const int x0 = (int)(tile - ty * a.tiles_x) * TL::BX, y0 = (int)ty * TL::BY;
     const int Q = (ze - zs) + 10;  // planes zs-5 .. ze+4
     __syncthreads();  // the previous segment's copies have all been issued, its planes read
     for (int e = tid; e < TL::PLANE; e += TL::NT) {
@@ -444,12 +446,11 @@ adv_status adjoint_stage_t(const adv_burgers_desc& d, int stage, const void* v, 
   int occ = 0;
   ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 256, smem));
   occ = std::max(occ, 1);
-  const int64_t units = (int64_t)a.tiles_x * a.tiles_y * d.nz;
   // one wave of equal shares (128^3: 91.7 us per stage, two waves 96, four 112: a segment streams ten extra
   // planes), at least two planes each (48^3: 16.8 us, four 23.1, eight 35.6)
-  const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>((int64_t)di.sms * occ, units / 2));
+  a.split = work_split((int64_t)a.tiles_x * a.tiles_y, d.nz, (int64_t)di.sms * occ, 2, 6.0);
   void* args[] = {&a};
-  ADV_CUDA_TRY(cudaLaunchKernel(k, dim3((unsigned)ctas), dim3(256), args, smem, s));
+  ADV_CUDA_TRY(cudaLaunchKernel(k, dim3(a.split.ctas), dim3(256), args, smem, s));
   count_launches(1);
   return ADV_OK;
 }

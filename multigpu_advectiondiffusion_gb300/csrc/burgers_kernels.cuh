@@ -48,6 +48,7 @@ struct BurgersParams {
   int periodic;  // 1: periodic wrap; 0: the reference's frozen outer 3 layers
   int bug_b2;
   int tiles_x, tiles_y;
+  WorkSplit split;  // of the (tile, plane) pairs over the CTAs of a single-grid launch
   int tma;
   int un_is_uin;
   int vec_ok;  // u_n and u_out: pairs of nodes aligned for one access
@@ -559,17 +560,18 @@ burgers_stage_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_cons
   // Balanced split: the (tile, z-plane) pairs, tile-major, are cut into gridDim.x equal
   // contiguous ranges (several waves of CTAs); a range crossing a tile boundary becomes segments.
   const int nz = p.nz;
-  const int64_t total = (int64_t)p.tiles_x * p.tiles_y * nz;
-  const int64_t seg_a = total * blockIdx.x / gridDim.x, seg_b = total * (blockIdx.x + 1) / gridDim.x;
+  int64_t seg_a, seg_b;
+  split_range(p.split, blockIdx.x, nz, &seg_a, &seg_b);
   burgers_cta_init<T>(&tmap, p.tma != 0);
   unsigned entries = 0;
   typename KeyOf<T>::type kmax = 0;
   for (int64_t pos = seg_a; pos < seg_b;) {
-    const int64_t tile = pos / nz;
+    const int64_t tile = div_units(pos, nz);
     const int zs = (int)(pos - tile * nz);
     const int ze = (int)min((int64_t)nz, zs + (seg_b - pos));
     pos += ze - zs;
-    const int x0 = (int)(tile % p.tiles_x) * TL::BX, y0 = (int)(tile / p.tiles_x) * TL::BY;
+    const int64_t ty = div_units(tile, p.tiles_x);
+    const int x0 = (int)(tile - ty * p.tiles_x) * TL::BX, y0 = (int)ty * TL::BY;
     entries = burgers_segment<T, Z, D, VISC, MODE>(&tmap, p, x0, y0, zs, ze, entries, kmax);
     if (entries == kPipeAborted) return;
   }
@@ -617,13 +619,14 @@ burgers_batch_kernel(const BurgersBatchInst<T>* __restrict__ inst, int n_inst, i
     const BurgersParams<T>& p = ps;
     const int64_t local = pos - inst[i].unit_begin;
     const int64_t inst_end = i + 1 < n_inst ? inst[i + 1].unit_begin : total_units;
-    const int64_t tile = local / p.nz;
+    const int64_t tile = div_units(local, p.nz);
     const int zs = (int)(local - tile * p.nz);
     const int64_t stop = min(seg_b, inst_end);
     const int ze = (int)min((int64_t)p.nz, zs + (stop - pos));
     pos += ze - zs;
     if (p.active && *p.active == 0) continue;
-    const int x0 = (int)(tile % p.tiles_x) * TL::BX, y0 = (int)(tile / p.tiles_x) * TL::BY;
+    const int64_t ty = div_units(tile, p.tiles_x);
+    const int x0 = (int)(tile - ty * p.tiles_x) * TL::BX, y0 = (int)ty * TL::BY;
     const CUtensorMap* tm = &inst[i].tmap;
     if (tma && threadIdx.x == 0) tma_prefetch_desc(tm);
     typename KeyOf<T>::type kmax = 0;

@@ -40,6 +40,7 @@ BurgersParams<T> burgers_params(const adv_burgers_desc& d, const BurgersLaunch& 
   p.bug_b2 = d.bug_b2;
   p.tiles_x = L.tiles_x;
   p.tiles_y = L.tiles_y;
+  p.split = L.split;
   p.tma = L.tma ? 1 : 0;
   p.un_is_uin = a.u_n == a.u_in ? 1 : 0;
   const uintptr_t pair = 2 * sizeof(T);

@@ -17,6 +17,7 @@ HeatParams<T> heat_params(const adv_heat_desc& d, const HeatLaunch& L, int stage
   p.frozen = d.frozen; p.zero_boundary = d.zero_boundary; p.stage = stage;
   p.tiles_x = L.tiles_x;
   p.tiles_y = L.tiles_y;
+  p.split = L.split;
   p.vec_ok = (((uintptr_t)u_out % 16) == 0 && ((int64_t)d.nx * sizeof(T)) % 16 == 0) ? 1 : 0;
   p.kx = (T)d.kx; p.ky = (T)d.ky; p.kz = (T)d.kz; p.dt = (T)d.dt;
   p.status = device_status_ptr();

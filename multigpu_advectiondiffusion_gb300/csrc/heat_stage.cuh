@@ -89,6 +89,7 @@ struct HeatParams {
   int nx, ny, nz;
   int frozen, zero_boundary, stage;
   int tiles_x, tiles_y;
+  WorkSplit split;  // of the (tile, plane) pairs over the CTAs of a single-grid launch
   int vec_ok;  // output rows 16-byte aligned: vector stores
   T kx, ky, kz, dt;
   int* status;  // device status word
@@ -593,8 +594,8 @@ heat_stage_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
   const int tid = threadIdx.y * C::TX + threadIdx.x;
   // Balanced split: the (tile, z-plane) pairs, tile-major, are cut into gridDim.x equal
   // contiguous ranges; a range that crosses a tile boundary becomes several segments.
-  const int64_t total = (int64_t)p.tiles_x * p.tiles_y * p.nz;
-  const int64_t seg_a = total * blockIdx.x / gridDim.x, seg_b = total * (blockIdx.x + 1) / gridDim.x;
+  int64_t seg_a, seg_b;
+  split_range_whole(p.split, blockIdx.x, &seg_a, &seg_b);
   if (tid == 0) {
     if (TMA) {
       for (int s = 0; s < C::NS; ++s) mbar_init(&bars[s], 1);
@@ -606,11 +607,12 @@ heat_stage_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
   __syncthreads();
   HeatPipe pipe{0, 0, 0u};
   for (int64_t pos = seg_a; pos < seg_b;) {
-    const int64_t tile = pos / p.nz;
+    const int64_t tile = div_units(pos, p.nz);
     const int zs = (int)(pos - tile * p.nz);
     const int ze = (int)min((int64_t)p.nz, zs + (seg_b - pos));
     pos += ze - zs;
-    const int x0 = (int)(tile % p.tiles_x) * C::BX, y0 = (int)(tile / p.tiles_x) * C::BY;
+    const int64_t trow = div_units(tile, p.tiles_x);
+    const int x0 = (int)(tile - trow * p.tiles_x) * C::BX, y0 = (int)trow * C::BY;
     pipe = heat_segment<T, ORDER, NDIM, TMA, STAGE, ROWS, WARPS, LANES, CONTRACT, HOOK, NODES>(&tmap, p, x0, y0, zs, ze, pipe);
     if (pipe.s_issue < 0) return;
   }
@@ -652,12 +654,13 @@ __device__ __forceinline__ void heat_batch_share(const HeatBatchInst<T>* __restr
     const HeatParams<T> p = inst[i].p[slot];  // a copy: registers, not reloads from the table
     const int64_t local = pos - inst[i].unit_begin;
     const int64_t inst_end = i + 1 < n_inst ? inst[i + 1].unit_begin : u0 + units;
-    const int64_t tile = local / p.nz;
+    const int64_t tile = div_units(local, p.nz);
     const int zs = (int)(local - tile * p.nz);
     const int64_t stop = min(seg_b, inst_end);
     const int ze = (int)min((int64_t)p.nz, zs + (stop - pos));
     pos += ze - zs;
-    const int x0 = (int)(tile % p.tiles_x) * C::BX, y0 = (int)(tile / p.tiles_x) * C::BY;
+    const int64_t trow = div_units(tile, p.tiles_x);
+    const int x0 = (int)(tile - trow * p.tiles_x) * C::BX, y0 = (int)trow * C::BY;
     const CUtensorMap* tm = &inst[i].tmap[slot];
     if (TMA && tid == 0) tma_prefetch_desc(tm);
     pipe = heat_segment<T, ORDER, 3, TMA, STAGE, ROWS, WARPS, LANES>(tm, p, x0, y0, zs, ze, pipe);

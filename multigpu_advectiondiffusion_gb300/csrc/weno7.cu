@@ -192,6 +192,7 @@ struct W7Params {
   float* out;  // the new state, or R(u)
   float* r;    // 2N-storage register; null: R(u) alone
   int nx, ny, nz, tiles_x, tiles_y;
+  WorkSplit split;  // of the (tile, plane) pairs over the CTAs
   int stage;
   int vec_ok;  // out and r: pairs of nodes aligned for one access
   float rhx, rhy, rhz;
@@ -277,14 +278,15 @@ __global__ void __launch_bounds__(256, 3) weno7_fused_kernel(const __grid_consta
   const int l_src = l_x ? lane * XS + TL::BX : YP + TL::BY * PX + (lane - TL::BY / 2);
   unsigned n = 0;  // stream entries so far (slot n % NS)
 
-  const int64_t total = (int64_t)p.tiles_x * p.tiles_y * nz;
-  const int64_t seg_a = total * blockIdx.x / gridDim.x, seg_b = total * (blockIdx.x + 1) / gridDim.x;
+  int64_t seg_a, seg_b;
+  split_range(p.split, blockIdx.x, nz, &seg_a, &seg_b);
   for (int64_t pos = seg_a; pos < seg_b;) {
-    const int64_t tile = pos / nz;
+    const int64_t tile = div_units(pos, nz);
     const int zs = (int)(pos - tile * nz);
     const int ze = (int)min((int64_t)nz, zs + (seg_b - pos));
     pos += ze - zs;
-    const int x0 = (int)(tile % p.tiles_x) * TL::BX, y0 = (int)(tile / p.tiles_x) * TL::BY;
+    const int64_t ty = div_units(tile, p.tiles_x);
+    const int x0 = (int)(tile - ty * p.tiles_x) * TL::BX, y0 = (int)ty * TL::BY;
     const int Q = (ze - zs) + 2 * lag;
     for (int e = tid; e < TL::PLANE; e += TL::NT) {  // (each thread reads back only what it wrote)
       const int r = e / SW, c = e - r * SW;
@@ -562,9 +564,8 @@ adv_status weno7_fused(const adv_weno7_desc& d, const float* u, float* out, floa
   int occ = 0;
   ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, weno7_fused_kernel, W7Tile::NT, W7Tile::SMEM));
   // one wave of equal shares, at least two planes each (a segment streams eight more)
-  const int64_t units = (int64_t)p.tiles_x * p.tiles_y * d.nz;
-  const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>((int64_t)di.sms * std::max(occ, 1), d.nz == 1 ? units : units / 2));
-  weno7_fused_kernel<<<(unsigned)ctas, W7Tile::NT, W7Tile::SMEM, s>>>(p);
+  p.split = work_split((int64_t)p.tiles_x * p.tiles_y, d.nz, (int64_t)di.sms * std::max(occ, 1), d.nz == 1 ? 1 : 2, 4.0);
+  weno7_fused_kernel<<<p.split.ctas, W7Tile::NT, W7Tile::SMEM, s>>>(p);
   ADV_CUDA_TRY(cudaGetLastError());
   if (count) count_launches(1);
   return ADV_OK;

@@ -1,0 +1,51 @@
+"""How a stage's (tile, plane) pairs are shared among CTAs never shows in its result: every pair once, at
+sizes that take each form of the split (tile by tile, one range, the longer shares first or spread)."""
+import numpy as np
+import pytest
+
+from multigpu_advectiondiffusion_gb300 import _native as N
+from multigpu_advectiondiffusion_gb300.solvers import BurgersConfig, HeatConfig, burgers_stage, heat_stage
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("size", [(224, 232, 240), (233, 233, 233), (256, 256, 193)])
+def test_heat_stage_on_both_sides_of_the_l2(cuda, oracle, size):
+    import torch
+    cfg = HeatConfig(3, *size, 2, 1, True, 0.03, 0.02, 0.01, 0.5)
+    u = np.random.default_rng(5).standard_normal(cfg.numel).astype(np.float32)
+    a = torch.from_numpy(u).to(cuda)
+    out = torch.full_like(a, float("nan"))
+    heat_stage(cfg, 1, a, a, out)
+    np.testing.assert_array_equal(out.cpu().numpy().view(np.uint8), oracle.heat_stage(cfg, 1, u, u).view(np.uint8))
+
+
+@pytest.mark.parametrize("size", [(96, 96, 96), (128, 112, 101), (250, 200, 1), (40, 33, 64), (97, 65, 300)])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_burgers_stage_of_a_rolled_state_is_the_rolled_stage(cuda, size, dtype):
+    """On a periodic grid a shift along z moves every share's edges to other planes; each node's operations
+    stay the same, so the states and the maximum agree bit for bit."""
+    import torch
+    nx, ny, nz = size
+    if nz == 1:
+        cfg = BurgersConfig.reference_2d(2.0, 2.0, nx, ny)
+        shifts = (0,)
+    else:
+        cfg = BurgersConfig(nx, ny, nz, 2.0 / nx, 2.0 / ny, 2.0 / nz, N.ADV_WENO5_Z, N.ADV_LF_GLOBAL, N.ADV_BC_PERIODIC)
+        shifts = (0, 1, nz // 3)
+    u = np.random.default_rng(6).uniform(-1, 1, (nz, ny, nx)).astype(dtype)
+    bits, real = (torch.int64, torch.float64) if dtype == np.float64 else (torch.int32, torch.float32)
+    key = torch.zeros(1, dtype=bits, device=cuda)
+    want = None
+    for k in shifts:
+        a = torch.from_numpy(np.ascontiguousarray(np.roll(u, k, 0)).ravel()).to(cuda)
+        out = torch.full_like(a, float("nan"))
+        key.zero_()
+        burgers_stage(cfg, 1, a, a, out, 1e-3, 1.0, maxabs_key=key)
+        got = np.roll(out.cpu().numpy().reshape(nz, ny, nx), -k, 0)
+        assert np.isfinite(got).all()
+        top = key.view(real).item()
+        if nz > 1:
+            assert top == np.abs(got).max()
+        want = got if want is None else want
+        np.testing.assert_array_equal(got, want)
