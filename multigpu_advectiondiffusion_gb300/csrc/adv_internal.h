@@ -118,6 +118,19 @@ adv_status heat2_launch(const adv_heat_desc& d, const HeatLaunch& L, const void*
 int heat_tune_variant(const adv_heat_desc& d);
 
 // --------------------------------------------------------------- Burgers launchers
+// What a second segment costs a Burgers share, in planes (work_split.h): FP32 pays for its halo planes' loads
+// and latency, the FP64 stage waits for its pipe all the same.
+inline double burgers_restart(int dtype) { return dtype == ADV_F32 ? 3.0 : 0.6; }
+
+// Waves of CTAs for a Burgers stage of `units` (tile, plane) pairs, `wave` CTAs resident: one, so that no last
+// wave is nearly empty, but more where each CTA streams many planes: the cost of a pair varies (ragged and
+// edge tiles) and the later waves even it out. us per stage with 1 / 2 / 3 / 4 waves: 48 planes a CTA (224^3)
+// 150.8 / 151.9 / 157 / 157, 72 (256^3) 219 / 216 / 223 / 217, 74 (400 x 406 x 100) 234 / 229 / 228 / 236,
+// 140 (320^3) 416 / 405 / 398 / 396.
+inline int64_t burgers_waves(int64_t units, int64_t wave) {
+  return units >= 120 * wave ? 3 : units >= 60 * wave ? 2 : 1;
+}
+
 struct BurgersLaunch {
   bool tma = false;
   int mode = 0;  // BurgersMode: the kernel's load path and problem class

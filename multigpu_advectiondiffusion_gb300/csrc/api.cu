@@ -122,8 +122,7 @@ adv_status burgers_prepare(const adv_burgers_desc& d, const void* u_in, BurgersL
   // nearly empty (FP64 121 x 101 x 97: 339 CTAs of 8 planes on 304 resident ones ran 3293 us a stage,
   // 304 run 2646; FP32 128^3: 46.2 -> 41.3), also when that leaves fewer than 8 planes each (FP32 64^3
   // 24.6 -> 14.7, 61 x 53 x 47 22.1 -> 12.8: a segment's six extra planes cost less than idle SMs), but
-  // at least 2 planes in 3D. Two waves from 48 planes a CTA on: the cost of a (tile, plane) pair varies
-  // (edge tiles patch their halo) and the second wave evens it out (256^3: 242 -> 234; four: 237).
+  // at least 2 planes in 3D. More waves for long shares: burgers_waves.
   const int64_t total = (int64_t)tiles_x * tiles_y * d.nz;
   int64_t min_share = d.nz == 1 ? 1 : 2;
   const TuneParams tp = tune_lookup(TUNE_BURGERS, burgers_tune_variant(d), d.nx, d.ny, d.nz);
@@ -132,8 +131,8 @@ adv_status burgers_prepare(const adv_burgers_desc& d, const void* u_in, BurgersL
     min_share = std::max(1, tp.b);
   }
   const int64_t wave = (int64_t)di.sms * occ;
-  L->split = work_split((int64_t)tiles_x * tiles_y, d.nz, total >= 48 * wave ? 2 * wave : wave, min_share,
-                        d.dtype == ADV_F32 ? 3.0 : 0.6);
+  L->split = work_split((int64_t)tiles_x * tiles_y, d.nz, burgers_waves(total, wave) * wave, min_share,
+                        burgers_restart(d.dtype));
   L->tiles_x = tiles_x;
   L->tiles_y = tiles_y;
   L->grid = dim3(L->split.ctas, 1, 1);

@@ -330,10 +330,11 @@ __device__ __forceinline__ unsigned burgers_segment(const CUtensorMap* tmap, con
     }
     return z;
   };
-  // Periodic edge tile: the TMA box zero-fills what lies outside the domain. The elements to
-  // patch with their wrapped neighbours are listed once per segment (CTA-uniform branch), so a
-  // plane's patch is one load and one store per listed element. Element copies (cp.async) take every
-  // element's place in its plane from the same list, so a plane's staging has no index arithmetic.
+  // Periodic edge tile: the TMA box zero-fills what lies outside the domain. The three layers there that
+  // a face of the domain's cells reads are listed once per segment (CTA-uniform branch), and each plane
+  // copies their wrapped neighbours over the zeros, asynchronously: nothing reads them before the barrier
+  // one plane later. Element copies (cp.async) take every element's place in its plane from the same
+  // list, so a plane's staging has no index arithmetic.
   BurgersPatch* patch = burgers_patch();
   if (!tma) {
     for (int e = tid; e < TL::PLANE; e += TL::NT) {
@@ -350,7 +351,7 @@ __device__ __forceinline__ unsigned burgers_segment(const CUtensorMap* tmap, con
     for (int e = tid; e < TL::PLANE; e += TL::NT) {
       const int r = e / SW, c = e - r * SW;
       const int gx = x0 - TL::PADX + c, gy = y0 - R + r;
-      if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) {
+      if ((gx < 0 || gx >= nx || gy < 0 || gy >= ny) && gx >= -R && gx < nx + R && gy >= -R && gy < ny + R) {
         const int k = atomicAdd(&patch->n, 1);
         patch->slot[k] = (uint16_t)e;
         patch->src[k] = (int64_t)wrapi(gy, ny) * nx + wrapi(gx, nx);
@@ -402,15 +403,20 @@ __device__ __forceinline__ unsigned burgers_segment(const CUtensorMap* tmap, con
     if (tma) {
       if (!wait(q)) *abort_flag = 1;  // every lane waits (converged)
       if (edge) {
-        // the listed elements of plane q take their wrapped neighbours; outside this thread's own
-        // columns they are read only by the split three planes later (2D: after this barrier)
+        // the listed elements of plane q take their wrapped neighbours; they are read only from the
+        // second plane after this one on (2D: after this barrier)
         const size_t zo = (size_t)plane_z(q) * sxy;
         for (int k = tid; k < patch->n; k += TL::NT) {
           const size_t gs = zo + (size_t)patch->src[k];
           const int e = patch->slot[k];
-          if (ADV_IN_RANGE(gs, sxy * nz, p.status) && ADV_IN_RANGE(e, TL::PLANE, p.status)) plq[e] = p.uin[gs];
+          if (ADV_IN_RANGE(gs, sxy * nz, p.status) && ADV_IN_RANGE(e, TL::PLANE, p.status))
+            cp_async_zfill<sizeof(T)>(plq + e, p.uin + gs, true);
         }
-        if (twod) __syncthreads();
+        cp_async_commit();
+        if (twod) {
+          cp_async_wait<0>();
+          __syncthreads();
+        }
       }
     } else {
       cp_async_wait<TL::P>();
@@ -463,6 +469,7 @@ __device__ __forceinline__ unsigned burgers_segment(const CUtensorMap* tmap, con
       split(uq, fp, fm);
       fz = line.push(fp, fm, uc, u2, q >= 2 * R - 1);
     }
+    if (tma && edge) cp_async_wait<1>();  // this thread's patch of plane q - 1
     __syncthreads();  // f+- in place; every read of the output plane's slot is done
     if (tma && *abort_flag != 0) {
       // A wait expired: let the copies already issued (planes q+1 .. q+P) land before returning.
@@ -542,6 +549,7 @@ __device__ __forceinline__ unsigned burgers_segment(const CUtensorMap* tmap, con
     if (VISC) { ua = ub; ub = uc; }
     uc = u2;
   }
+  if (tma && edge) cp_async_wait<0>();
   return n0 + (unsigned)Q;
 }
 
