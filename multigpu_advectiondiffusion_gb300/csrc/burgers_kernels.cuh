@@ -560,17 +560,15 @@ constexpr int burgers_min_ctas() {
   return sizeof(T) == 4 ? 3 : 2;
 }
 
+// CTA b's share of one grid's stage (work_split.h); a share crossing a tile boundary becomes segments.
 template <class T, bool Z, class D, bool VISC, int MODE>
-__global__ void __launch_bounds__(256, burgers_min_ctas<T>())
-burgers_stage_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ BurgersParams<T> p) {
+__device__ __forceinline__ void burgers_share(const CUtensorMap* tmap, const BurgersParams<T>& p, unsigned b) {
   using TL = BurgersTile;
   if (p.active && *p.active == 0) return;
-  // Balanced split: the (tile, z-plane) pairs, tile-major, are cut into gridDim.x equal
-  // contiguous ranges (several waves of CTAs); a range crossing a tile boundary becomes segments.
   const int nz = p.nz;
   int64_t seg_a, seg_b;
-  split_range(p.split, blockIdx.x, nz, &seg_a, &seg_b);
-  burgers_cta_init<T>(&tmap, p.tma != 0);
+  split_range(p.split, b, nz, &seg_a, &seg_b);
+  burgers_cta_init<T>(tmap, p.tma != 0);
   unsigned entries = 0;
   typename KeyOf<T>::type kmax = 0;
   for (int64_t pos = seg_a; pos < seg_b;) {
@@ -580,10 +578,16 @@ burgers_stage_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_cons
     pos += ze - zs;
     const int64_t ty = div_units(tile, p.tiles_x);
     const int x0 = (int)(tile - ty * p.tiles_x) * TL::BX, y0 = (int)ty * TL::BY;
-    entries = burgers_segment<T, Z, D, VISC, MODE>(&tmap, p, x0, y0, zs, ze, entries, kmax);
+    entries = burgers_segment<T, Z, D, VISC, MODE>(tmap, p, x0, y0, zs, ze, entries, kmax);
     if (entries == kPipeAborted) return;
   }
   burgers_flush_max(kmax, p.maxabs_key);
+}
+
+template <class T, bool Z, class D, bool VISC, int MODE>
+__global__ void __launch_bounds__(256, burgers_min_ctas<T>())
+burgers_stage_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ BurgersParams<T> p) {
+  burgers_share<T, Z, D, VISC, MODE>(&tmap, p, blockIdx.x);
 }
 
 // One instance of a batched Burgers stage: the tensor map of its stage input and the stage's
@@ -596,7 +600,7 @@ struct alignas(64) BurgersBatchInst {
   int64_t pad[7];
 };
 
-// Batched stage over many instances: the units (instance, tile, z-plane) of all instances,
+// Batched stage over more instances than a BurgersGroup holds: the units (instance, tile, z-plane) of all instances,
 // instance-major then tile-major, are cut into gridDim.x equal contiguous ranges. Instances
 // whose active flag is 0 are skipped (the choice is per segment, so uniform over the CTA).
 template <class T, bool Z, class D, bool VISC, int MODE>
@@ -642,6 +646,33 @@ burgers_batch_kernel(const BurgersBatchInst<T>* __restrict__ inst, int n_inst, i
     if (entries == kPipeAborted) return;
     burgers_flush_max(kmax, p.maxabs_key);
   }
+}
+
+// A stage of up to MAX instances, each with CTAs [cta_begin[i], cta_begin[i + 1]) of its own (the host shares
+// them out so that no instance's longest share stands out). The instances' parameters are the kernel's own:
+// read from the constant bank like a single grid's, they cost no registers, where the table of
+// burgers_batch_kernel, staged in shared memory and read again after every barrier, spilled 120-180 bytes per
+// thread (us per stage of one 160^3 member: 83 in a batch, 68 in a group, 68 alone).
+template <class T>
+struct BurgersGroup {
+  static constexpr int MAX = 64;
+  const CUtensorMap* tmap;  // instance i's, i * stride bytes on
+  size_t stride;
+  int n;
+  unsigned cta_begin[MAX];
+  BurgersParams<T> p[MAX];
+};
+
+template <class T, bool Z, class D, bool VISC, int MODE>
+__global__ void __launch_bounds__(256, burgers_min_ctas<T>())
+burgers_group_kernel(const __grid_constant__ BurgersGroup<T> g) {
+  int i = 0, hi = g.n - 1;
+  while (i < hi) {
+    const int mid = (i + hi + 1) / 2;
+    if (g.cta_begin[mid] <= blockIdx.x) i = mid; else hi = mid - 1;
+  }
+  const CUtensorMap* tm = reinterpret_cast<const CUtensorMap*>(reinterpret_cast<const char*>(g.tmap) + i * g.stride);
+  burgers_share<T, Z, D, VISC, MODE>(tm, g.p[i], blockIdx.x - g.cta_begin[i]);
 }
 
 }  // namespace adv

@@ -1,12 +1,12 @@
 // ensemble.cu -- batched ensembles (adv_ensemble_* in advdiff.h): many independent 3D heat and
 // Burgers problems of uneven size advanced by one CUDA graph.
 //
-// Each member contributes its (tile, z-plane) units to one flat range per kind; a batched stage
-// launch cuts that range into equal contiguous shares, one per CTA (two waves of CTAs for heat,
-// one for Burgers), so small members neither leave SMs idle nor pay a launch each
-// (heat_batch_kernel, burgers_batch_kernel). The
-// device tables hold, per member and per stage slot, the stage parameters and the tensor map of
-// the stage input. A run is one graph with two while-nodes that run concurrently: the heat loop
+// A stage of all members of a kind is one launch, so small members neither leave SMs idle nor pay a launch
+// each. Heat members, and Burgers members beyond BurgersGroup::MAX, contribute their (tile, z-plane) units to
+// one flat range that is cut into equal contiguous shares, one per CTA (two waves of CTAs for heat, one for
+// Burgers: heat_batch_kernel, burgers_batch_kernel). Up to MAX Burgers members get CTAs of their own
+// (burgers_group_kernel): 16 heat + 8 Burgers members, 20 steps: 17.9 -> 15.8 ms. The device tables hold, per
+// member and per stage slot, the stage parameters and the tensor map of the stage input. A run is one graph with two while-nodes that run concurrently: the heat loop
 // (a device counter) and the Burgers loop (per-member dt, Lax-Friedrichs constant and stop test,
 // the same device code as adv_burgers_run).
 #include <algorithm>
@@ -24,6 +24,8 @@ void* heat_batch_kernel_for(int dtype, int order, bool tma, int stage_kind, int 
 void* heat_batch_mixed_kernel_for(int stage_kind);
 template <class T>
 void* burgers_batch_kernel_for(const adv_burgers_desc& d, int mode);
+template <class T>
+void* burgers_group_kernel_for(const adv_burgers_desc& d, int mode);
 size_t burgers_smem_f32();
 size_t burgers_smem_f64();
 }  // namespace adv
@@ -58,6 +60,7 @@ struct adv_ensemble {
   int burg_ctas = 0;
   size_t burg_smem = 0;
   void* burg_k = nullptr;
+  std::vector<unsigned char> burg_group[3];  // the stages' BurgersGroup (few members), else empty
   BurgersLoopState* states = nullptr;
   std::vector<BurgersLoopState> h_states;
   // loop control (device)
@@ -193,6 +196,62 @@ adv_status build_burgers_tables(adv_ensemble* e, std::vector<unsigned char> (&by
   return ADV_OK;
 }
 
+// CTAs of their own for each member of a group, at most `most` in all, so that the longest share of any is
+// as short as they allow; returns their number. A member never gets fewer than one or shorter shares than a
+// single run's.
+template <class T>
+int build_burgers_group(adv_ensemble* e, const std::vector<unsigned char> (&bytes)[3], int64_t most) {
+  const int n = e->n_burg;
+  const double restart = burgers_restart(e->burg_dtype);
+  struct Need {
+    int64_t tiles, nz, min_share;
+  };
+  std::vector<Need> need((size_t)n);
+  int64_t longest = 1;
+  for (int i = 0; i < n; ++i) {
+    const adv_burgers_desc& d = e->burg[(size_t)i].desc;
+    need[(size_t)i] = {(int64_t)((d.nx + 31) / 32) * ((d.ny + 15) / 16), d.nz, d.nz == 1 ? 1 : 2};
+    longest = std::max(longest, need[(size_t)i].tiles * d.nz);
+  }
+  // the fewest CTAs whose shares of a member cost at most `planes`: tile by tile, or of the whole
+  auto ctas = [&](const Need& m, double planes) -> int64_t {
+    const int64_t total = m.tiles * m.nz;
+    const int64_t whole = (int64_t)std::floor(planes - 2 * restart), part = (int64_t)std::floor(planes - restart);
+    int64_t c = std::max<int64_t>(1, total / m.min_share);
+    if (whole >= 1) c = std::min(c, (total + whole - 1) / whole);
+    if (part >= 1) c = std::min(c, m.tiles * ((m.nz + part - 1) / part));
+    return std::max<int64_t>(c, 1);
+  };
+  int64_t lo = 0, hi = longest + 8;  // planes: too few, enough (one CTA each)
+  while (hi - lo > 1) {
+    const int64_t mid = (lo + hi) / 2;
+    int64_t sum = 0;
+    for (const Need& m : need) sum += ctas(m, (double)mid);
+    (sum <= most ? hi : lo) = mid;
+  }
+  std::vector<BurgersGroup<T>> g(3);
+  unsigned begin = 0;
+  for (int i = 0; i < n; ++i) {
+    const Need& m = need[(size_t)i];
+    const WorkSplit w = work_split(m.tiles, (int)m.nz, ctas(m, (double)hi), m.min_share, restart);
+    for (int s = 0; s < 3; ++s) {
+      const BurgersBatchInst<T>* tab = reinterpret_cast<const BurgersBatchInst<T>*>(bytes[s].data());
+      g[(size_t)s].cta_begin[i] = begin;
+      g[(size_t)s].p[i] = tab[i].p;
+      g[(size_t)s].p[i].split = w;
+    }
+    begin += w.ctas;
+  }
+  for (int s = 0; s < 3; ++s) {
+    g[(size_t)s].tmap = &static_cast<const BurgersBatchInst<T>*>(e->burg_tab[s])->tmap;
+    g[(size_t)s].stride = sizeof(BurgersBatchInst<T>);
+    g[(size_t)s].n = n;
+    e->burg_group[s].resize(sizeof(BurgersGroup<T>));
+    std::memcpy(e->burg_group[s].data(), &g[(size_t)s], sizeof(BurgersGroup<T>));
+  }
+  return (int)begin;
+}
+
 int one_wave_ctas(void* kernel, int threads, size_t smem, int sms, int64_t units, adv_status* st) {
   int occ = 0;
   cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem);
@@ -230,6 +289,7 @@ adv_status launch_burgers_stage(adv_ensemble* e, int stage, cudaStream_t s) {
   int64_t units = e->burg_units;
   int tma = e->burg_tma ? 1 : 0;
   void* args[] = {&tab, &n, &units, &tma};
+  if (!e->burg_group[stage - 1].empty()) args[0] = e->burg_group[stage - 1].data();
   ADV_CUDA_TRY(cudaLaunchKernel(e->burg_k, dim3((unsigned)e->burg_ctas), dim3(256, 1, 1), args, e->burg_smem, s));
   count_launches(1);
   return ADV_OK;
@@ -418,15 +478,30 @@ adv_status create_impl(const adv_heat_member* heat, int n_heat, int scheme, cons
     int mode = e->burg_tma ? BURGERS_3D_TMA : BURGERS_3D_COPY;
     for (int i = 0; i < n_burgers; ++i)
       if (burgers[i].desc.nz == 1) mode = BURGERS_ANY;
-    e->burg_k = e->burg_dtype == ADV_F32 ? burgers_batch_kernel_for<float>(burgers[0].desc, mode)
-                                         : burgers_batch_kernel_for<double>(burgers[0].desc, mode);
+    const bool f32 = e->burg_dtype == ADV_F32;
+    const bool group = n_burgers <= BurgersGroup<float>::MAX;
+    if (group) e->burg_k = f32 ? burgers_group_kernel_for<float>(burgers[0].desc, mode)
+                               : burgers_group_kernel_for<double>(burgers[0].desc, mode);
+    else e->burg_k = f32 ? burgers_batch_kernel_for<float>(burgers[0].desc, mode)
+                         : burgers_batch_kernel_for<double>(burgers[0].desc, mode);
     if (!e->burg_k) return set_error(ADV_ERR_UNSUPPORTED, "ensemble: no batched Burgers kernel");
     e->burg_smem = e->burg_dtype == ADV_F32 ? burgers_smem_f32() : burgers_smem_f64();
     ADV_CUDA_TRY(cudaFuncSetAttribute(e->burg_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->burg_smem));
-    // one wave of equal shares (16 heat + 8 Burgers members, 20 steps: 17.97 ms with one wave, 18.65 with
-    // two, 18.85 with four, 20.82 with eight)
+    // one wave of equal shares (20 steps of 16 heat + 8 Burgers members in this form: 17.97 ms with one wave,
+    // 18.65 with two, 18.85 with four, 20.82 with eight)
     e->burg_ctas = one_wave_ctas(e->burg_k, 256, e->burg_smem, e->sms, e->burg_units, &st);
     if (st != ADV_OK) return st;
+    if (group) {
+      int occ = 0;
+      ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, e->burg_k, 256, e->burg_smem));
+      // one wave, three where each CTA would stream 60 planes or more (members of uneven size vary more than
+      // one grid's tiles). us per 10 steps with 1 / 2 / 3 / 4 waves: 16 x 64^3 (18 planes a CTA) 2481 / 2394 /
+      // 2635 / 2677, 200^3 + 3 x 24^3 (40) 4140 / 4276 / 4213 / 4264, 4 x 160^3 (70) 6759 / 6789 / 6661 / 6730,
+      // 16 x 128^3 (144) 13609 / 13092 / 13140 / 13013
+      const int64_t wave = (int64_t)e->sms * std::max(occ, 1);
+      const int64_t most = (e->burg_units >= 60 * wave ? 3 : 1) * wave;
+      e->burg_ctas = f32 ? build_burgers_group<float>(e, bytes, most) : build_burgers_group<double>(e, bytes, most);
+    }
     e->h_states.resize((size_t)n_burgers);
   }
   return ADV_OK;
