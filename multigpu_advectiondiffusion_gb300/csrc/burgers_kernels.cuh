@@ -15,17 +15,19 @@
 //     share is computed once per cell), advanced by plane q;
 //   * the 33x16 x-faces and 32x17 y-faces are reconstructed by all threads, two at a time;
 //   * L = -(dF/dx + dG/dy + dH/dz) (+ viscous O4 term), the SSP-RK3 combine, the store and a
-//     warp-shuffle max|u_out| reduction (one atomicMax per warp) for the next stage's
+//     warp-shuffle max|u_out| reduction (one atomicMax per CTA) for the next stage's
 //     Lax-Friedrichs constant and time step all happen in the same pass.
 // Two barriers per plane: the one after the split also releases the ring slot of the output plane
 // (nothing reads it later), the one after the faces hands them to their cells.
 // Every node is read from HBM once per stage and written once. Bound by issue: at 256^3 FP32 WENO5-Z
-// a plane takes 612 issue slots per pair of cells, 280 of them paired FP32 instructions (832 and 290
+// a plane takes 561 issue slots per pair of cells, half of them paired FP32 instructions (832 and 290
 // before neighbouring faces shared their differences, pairs were loaded instead of packed, and the six
-// quotients per cell went through the paired correction of vnquot): 334 -> 234 us per stage back to
-// back, 50.3 -> 71.8 Gcell-stage/s; the FMA pipe is 55% busy. A 2D problem (nz == 1) streams its one
+// quotients per cell went through the paired correction of vnquot): 334 -> 215 us per stage back to
+// back, 50.3 -> 78.0 Gcell-stage/s; the FMA pipe is 57% busy, 58% of the issue slots are used. A 2D problem (nz == 1) streams its one
 // plane alone: no z faces, no z halo (1000 x 900 FP32: 61 -> 14.5 us per stage against streaming the
-// plane seven times).
+// plane seven times). FP64 is bound by its pipe (78% busy at 128 x 112 x 101): warps whose faces no updated
+// node reads reconstruct none, and the faces left over are one value per lane of two warps
+// (121 x 101 x 97: 2378 -> 2086 us per stage, 64 x 53 x 60: 519 -> 409).
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -289,6 +291,14 @@ __device__ __forceinline__ unsigned burgers_segment(const CUtensorMap* tmap, con
   const bool upd0 = in0 && yok && (per || (x >= FR && x < nx - FR));
   const bool upd1 = in1 && yok && (per || (x + 1 >= FR && x + 1 < nx - FR));
   const bool vec = p.vec_ok && in1;
+  // FP64: what this warp reconstructs. Faces no updated node reads (frozen rows, rows and tiles past the
+  // domain) are left out; a warp's x- and z-faces serve its own two rows, its y-faces the row below them as
+  // well. (FP32, bound by issue and latency, lost 2-4% to the extra predicates.)
+  const bool all = sizeof(T) == 4;
+  const int yw0 = y0 + 2 * warp;
+  const bool cols = all || per || (x0 + TL::BX > FR && x0 < nx - FR);
+  const bool need = all || (cols && yw0 + 1 >= FR && yw0 < ny - FR);
+  const bool need_y = all || (cols && yw0 + 1 >= FR && yw0 - 1 < ny - FR);
   // Operand places of this thread's share of the splits and faces.
   T* const xw = reinterpret_cast<T*>(part + warp * XS + 2 * cp + R) + (row & 1);  // its cells, x layout
   V* const yw = part + YP + R * PX + tid;                                        // its cells, y layout
@@ -446,7 +456,8 @@ __device__ __forceinline__ unsigned burgers_segment(const CUtensorMap* tmap, con
         const V ym2 = *reinterpret_cast<const V*>(r0 - 2 * SW), ym1 = *reinterpret_cast<const V*>(r0 - SW);
         const V yp1 = *reinterpret_cast<const V*>(r0 + SW), yp2 = *reinterpret_cast<const V*>(r0 + 2 * SW);
         auto o4 = [](T m2, T m1, T c, T p1, T p2) {
-          return sub_rn(add_rn(sub_rn(add_rn(-m2, mul_rn(T(16), m1)), mul_rn(T(30), c)), mul_rn(T(16), p1)), p2);
+          // (products by 16 are exact)
+          return sub_rn(fma_rn_(T(16), p1, sub_rn(fma_rn_(T(16), m1, -m2), mul_rn(T(30), c))), p2);
         };
         V vz = vc<V>(0);
         if (!twod) {
@@ -467,7 +478,7 @@ __device__ __forceinline__ unsigned burgers_segment(const CUtensorMap* tmap, con
       u2 = *reinterpret_cast<const V*>(slot(q - 2) + own);  // (before plane 2: a stale slot, not used)
       V fp, fm;
       split(uq, fp, fm);
-      fz = line.push(fp, fm, uc, u2, q >= 2 * R - 1);
+      fz = line.push(fp, fm, uc, u2, need && q >= 2 * R - 1);
     }
     if (tma && edge) cp_async_wait<1>();  // this thread's patch of plane q - 1
     __syncthreads();  // f+- in place; every read of the output plane's slot is done
@@ -494,12 +505,33 @@ __device__ __forceinline__ unsigned burgers_segment(const CUtensorMap* tmap, con
           const V* const m = a + PART;
           return F::f(a[0], a[st], a[2 * st], a[3 * st], a[4 * st], m[st], m[2 * st], m[3 * st], m[4 * st], m[5 * st]);
         };
-        const V fx = face(xr, 1);
-        fxS[(2 * warp) * TL::XF + lane] = fx.x;
-        fxS[(2 * warp + 1) * TL::XF + lane] = fx.y;
-        const V fym = face(yr, PX);
-        fyS[tid] = fym;
-        if (warp == (q & 7) && lane < TL::BY / 2 + PX) {
+        if (need) {
+          const V fx = face(xr, 1);
+          fxS[(2 * warp) * TL::XF + lane] = fx.x;
+          fxS[(2 * warp + 1) * TL::XF + lane] = fx.y;
+        }
+        V fym;
+        if (need_y) {
+          fym = face(yr, PX);
+          fyS[tid] = fym;
+        } else {
+          fym = vc<V>(0);
+        }
+        if constexpr (EXACT) {
+          // one value per lane of two warps: the FP64 pipe is each scheduler's own, and a warp's extra
+          // work is waited for by all
+          const int e = ((q & 7) == warp) ? lane : ((q + 1) & 7) == warp ? 32 + lane : TL::BY + TL::BX;
+          if (cols && e < TL::BY + TL::BX) {
+            const bool ex = e < TL::BY;
+            const int i = ex ? e : e - TL::BY, st = ex ? 2 : 2 * PX;
+            const T* const a = reinterpret_cast<const T*>(part + (ex ? (i / 2) * XS + TL::BX : YP + TL::BY * PX + i / 2)) + (i & 1);
+            const T* const m = a + 2 * PART;
+            const T f = weno_face_ref<Z, T>(a[0], a[st], a[2 * st], a[3 * st], a[4 * st], m[st], m[2 * st], m[3 * st],
+                                            m[4 * st], m[5 * st]);
+            if (ex) fxS[i * TL::XF + TL::BX] = f;
+            else reinterpret_cast<T*>(fyS + TL::BY * PX)[i] = f;
+          }
+        } else if (warp == (q & 7) && cols && lane < TL::BY / 2 + PX) {
           const V f = face(part + l_src, l_st);
           if (l_x) {
             fxS[(2 * lane) * TL::XF + TL::BX] = f.x;
