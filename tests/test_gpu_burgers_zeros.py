@@ -1,0 +1,53 @@
+"""FP64 Burgers stages over constant, zero, subnormal and tiny states and over tiles with columns and rows past
+the domain or in the frozen layers, bit for bit against the oracle: the divisions' numerators reach zero
+there, and whole warps have no face to reconstruct."""
+import numpy as np
+import pytest
+
+from multigpu_advectiondiffusion_gb300 import _native as N
+from multigpu_advectiondiffusion_gb300.solvers import BurgersConfig, burgers_stage
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(36, 20, 9), (33, 35, 8), (97, 98, 7), (35, 16, 10), (34, 19, 9), (32, 51, 7), (40, 50, 1)]
+
+
+@pytest.mark.parametrize("size", SIZES)
+@pytest.mark.parametrize("state", ["zero", "constant", "half", "tiny", "subnormal", "steps"])
+@pytest.mark.parametrize("bc,weno,C", [(N.ADV_BC_PERIODIC, N.ADV_WENO5_Z, 0.0), (N.ADV_BC_FROZEN, N.ADV_WENO5_Z, 1e-2),
+                                       (N.ADV_BC_FROZEN, N.ADV_WENO5_JS, 0.0)])
+def test_stage_over_zero_numerators(cuda, oracle, size, state, bc, weno, C):
+    import torch
+    nx, ny, nz = size
+    if nz == 1:
+        if bc == N.ADV_BC_PERIODIC:
+            pytest.skip("2D grids are frozen")
+        cfg = BurgersConfig.reference_2d(2.0, 2.0, nx, ny)
+    else:
+        cfg = BurgersConfig(nx, ny, nz, 2.0 / nx, 2.0 / ny, 2.0 / nz, weno, N.ADV_LF_LOCAL, bc)
+        cfg.C = C
+    rng = np.random.default_rng(4)
+    u = rng.uniform(-1, 1, (nz, ny, nx))
+    if state == "zero":
+        u[:] = 0.0
+        u[:, :, : nx // 3] = -0.0
+    elif state == "constant":
+        u[:] = 0.7
+    elif state == "half":
+        u[:, :, nx // 2:] = 0.0
+        u[:, ny // 2:, :] = -0.25
+    elif state == "tiny":
+        u *= 1e-60
+    elif state == "subnormal":
+        u *= 1e-310
+    else:
+        u = np.round(2 * u) / 2
+    u = np.ascontiguousarray(u).ravel()
+    un = rng.permutation(u)
+    for stage in (1, 3):
+        base = u if stage == 1 else un
+        a, b = (torch.from_numpy(v).to(cuda) for v in (u, base))
+        out = torch.full_like(a, float("nan"))
+        burgers_stage(cfg, stage, a, b, out, 1e-3, float(np.abs(u).max()))
+        np.testing.assert_array_equal(out.cpu().numpy().view(np.uint8),
+                                      oracle.burgers_stage(cfg, stage, u, base, 1e-3).view(np.uint8))
