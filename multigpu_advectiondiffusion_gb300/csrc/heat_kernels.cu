@@ -111,7 +111,10 @@ adv_status heat_prepare(const adv_heat_desc& d, const void* u_in, HeatLaunch* L,
       if (!k) return set_error(ADV_ERR_UNSUPPORTED, "heat: no kernel for this configuration");
       ADV_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     }
-    void* k0 = pick_kernel(d, L->tma, 1, *L);
+    // The wave is counted by stage 1's kernel, which forward Euler runs alone. FP64 O4 in 3D, an SSP-RK3 scheme's:
+    // by stage 3's, which takes the most registers; stages of more CTAs than fit end with a second, nearly
+    // empty wave (us per step, before -> after: 201 x 199 x 200 1248 -> 1143, 208 x 160 x 150 711 -> 657).
+    void* k0 = pick_kernel(d, L->tma, d.dtype == ADV_F64 && d.order == 4 && d.ndim == 3 ? 3 : 1, *L);
     ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k0, 32 * L->warps, smem));
     occ = std::max(occ, 1);
     L->occ = occ;

@@ -328,6 +328,11 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
   const bool warp_x_ends = __all_sync(0xffffffffu, (xkeep & ~(1u | (1u << (VX - 1)))) == 0);
   const bool warp_rows_clean = __all_sync(0xffffffffu, rowkeep == 0);
   const bool warp_inside = __all_sync(0xffffffffu, inside == ALL);
+  // FP64 waits for its pipe: a warp without an updated node (rows past the grid, frozen layers) leaves the
+  // stencil out (us per O4 SSP-RK3 step with this and five CTAs per SM: 65 x 61 x 57 56.8 -> 51.8, 129^3
+  // 389 -> 360, 201 x 199 x 200 1220 -> 1143)
+  constexpr unsigned ROWS_ALL = (1u << RY) - 1u, XS_ALL = (1u << VX) - 1u;
+  const bool warp_work = sizeof(T) == 4 || __any_sync(0xffffffffu, rowkeep != ROWS_ALL && xkeep != XS_ALL);
   bool row_ok[RY];
 #pragma unroll
   for (int r = 0; r < RY; ++r) row_ok[r] = ya + r < ny;
@@ -450,6 +455,11 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
             res[r][e] = v.x;
             res[r + DR][e + DE] = v.y;
           }
+      } else if (sizeof(T) == 8 && !(warp_work && zin)) {
+#pragma unroll
+      for (int r = 0; r < RY; ++r)
+#pragma unroll
+        for (int e = 0; e < VX; ++e) res[r][e] = WS(RZ)[r][e];
       } else {
 #pragma unroll
       for (int r = 0; r < RY; ++r)
@@ -575,10 +585,11 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
   return HeatPipe{s_issue, s_wait, parity};
 }
 
-// Resident CTAs per SM the register budget is sized for.
+// Resident CTAs per SM the register budget is sized for. (FP64: five; stage 3 took 110 registers under four,
+// and its fifth CTA ran alone.)
 template <class T, int ORDER, int ROWS, int WARPS, int NODES = 16 / (int)sizeof(T)>
 constexpr int heat_min_ctas() {
-  if (NODES == 1) return sizeof(T) == 8 ? 4 : ORDER == 2 ? 5 : 3;
+  if (NODES == 1) return sizeof(T) == 8 ? 5 : ORDER == 2 ? 5 : 3;
   return ROWS > 2 ? 16 / WARPS : (ORDER == 2 ? 4 : (sizeof(T) == 4 ? 3 : 2));
 }
 
