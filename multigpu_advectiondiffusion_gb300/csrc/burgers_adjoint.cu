@@ -18,13 +18,16 @@
 // planes behind). Per streamed plane p each thread advances its columns' f+- windows and differentiates
 // the z-faces p-3+1/2, pushing the partials into per-column accumulators for cells p-5..p; cell p-5 is
 // then complete in z. For that plane f+- go to shared memory in two layouts (pairs of rows for the
-// x-faces, pairs of columns for the y-faces, as in the forward stage: an operand pair is one load), the
-// 37 x 16 x-faces and 32 x 21 y-faces of the tile are differentiated two at a time into shared memory
-// (structure of arrays), each cell gathers its ten partials per axis, and the stage output is written.
+// x-faces, pairs of columns for the y-faces, as in the forward stage: an operand pair is one load), and the
+// 37 x 16 x-faces and 32 x 21 y-faces of the tile are differentiated two at a time in one go: an x-face's
+// partials go to its warp's cells by shuffles, a y-face's through shared memory (structure of arrays), and the
+// 120 pairs past the tile to four warps, one per scheduler, others each plane. Then each cell gathers its ten
+// partials per axis, and the stage output is written; three barriers per plane.
 // Every face is differentiated once per pass. Bound by issue, as the forward stage: 128^3 FP32 WENO5-Z
-// 146.6 -> 91.7 us per stage back to back, FP64 64^3 1326 -> 630, against one face per thread with its two
+// 146.6 -> 84.4 us per stage back to back, FP64 64^3 1326 -> 591, against one face per thread with its two
 // sides packed into a pair, the weights' full form (about 125 paired instructions a side against 84) and
-// an index division per staged element.
+// an index division per staged element; with the x- and y-faces in turn, each with its own faces past the
+// tile waited for, five barriers: 89.9 and 629.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -47,9 +50,10 @@ struct AdjTile {
   static constexpr int PADL = 4, SWL = BX + 2 * PADL;    // lam: column 0 holds x0 - 4
   static constexpr int SHL = BY + 2 * HL, PLANEL = SWL * SHL;
   static constexpr int NS = 8, NSL = 6;                  // ring slots: v p-5 .. p+2, lam p-5 .. p
-  static constexpr int FX = BX + 5, NFX = FX * BY / 2;   // x-faces i+1/2, i = -3 .. 33, per pair of rows
-  static constexpr int FY = BY + 5, NFY = FY * PX;       // y-faces, pairs of columns
-  static constexpr int NF = NFY > NFX ? NFY : NFX;
+  static constexpr int FY = BY + 5, NF = FY * PX;        // y-faces j+1/2, j = -3 .. 17, pairs of columns
+  // x-faces i+1/2, i = -3 .. 33, per pair of rows: lane l's is i = l - 3, the last five go through shared
+  // memory, each part behind five zeros
+  static constexpr int EX = 10, NEX = 10 * EX;
   static constexpr int XS = BX + 2 * H;                  // x-face operands per pair of rows: cells x0-5 .. x0+36
 };
 
@@ -60,9 +64,9 @@ struct AdjSmem {
   static constexpr int SLOTL = ((TL::PLANEL * (int)sizeof(T) + 127) / 128 * 128) / (int)sizeof(T);
   static constexpr size_t RING = (size_t)(TL::NS * SLOT + TL::NSL * SLOTL) * sizeof(T);
   static constexpr int PART = TL::BY / 2 * TL::XS + TL::SH * TL::PX;            // pairs of one split part
-  static constexpr size_t FB = (size_t)10 * TL::NF * 2 * sizeof(T);             // face partials (SoA)
+  static constexpr size_t FB = (size_t)(10 * TL::NF + TL::BY / 2 * TL::NEX) * 2 * sizeof(T);  // face partials (SoA)
   static constexpr size_t JX = (size_t)TL::BX * TL::BY * sizeof(T);             // x part of J^T lam per cell
-  static constexpr size_t TOTAL = RING + (size_t)2 * PART * 2 * sizeof(T) + FB + JX + TL::PLANE * sizeof(int64_t);
+  static constexpr size_t TOTAL = RING + (size_t)2 * PART * 2 * sizeof(T) + FB + JX + TL::PLANE * sizeof(uint32_t);
 };
 
 template <class T>
@@ -171,9 +175,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) burgers_adjoint_k
   T* const ring = reinterpret_cast<T*>(smem_raw);
   T* const ringl = ring + TL::NS * SM::SLOT;
   V* const part = reinterpret_cast<V*>(smem_raw + SM::RING);  // f+; f- follows PART pairs later
-  V* const FB = part + 2 * PART;                              // [10][NF]: P0..P4, M0..M4
-  T* const jx = reinterpret_cast<T*>(FB + 10 * NF);           // [BY][BX]
-  int64_t* const src = reinterpret_cast<int64_t*>(jx + TL::BX * TL::BY);  // in-plane offsets of v's staged elements
+  V* const FB = part + 2 * PART;                              // y: [10][NF]: P0..P4, M0..M4
+  V* const FE = FB + 10 * NF;                                 // x: [BY/2][10][EX], the last five faces
+  T* const jx = reinterpret_cast<T*>(FE + TL::BY / 2 * TL::NEX);  // [BY][BX], a warp's rows its own
+  uint32_t* const src = reinterpret_cast<uint32_t*>(jx + TL::BX * TL::BY);  // in-plane offsets of v's staged elements
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cp = tid & (PX - 1), row = tid / PX;
@@ -198,6 +203,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) burgers_adjoint_k
     h_dst = part + rp * XS + c;
   }
   auto split = [](V u, V& fp, V& fm) { lf_split2(u, vabs(u), fp, fm); };
+  for (int e = tid; e < TL::BY / 2 * TL::NEX; e += TL::NT)
+    if (e % TL::EX < 5) FE[e] = vc<V>(0);
   int64_t seg_a, seg_b;
   split_range(a.split, blockIdx.x, nz, &seg_a, &seg_b);
 
@@ -212,7 +219,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) burgers_adjoint_k
     __syncthreads();  // the previous segment's copies have all been issued, its planes read
     for (int e = tid; e < TL::PLANE; e += TL::NT) {
       const int r = e / SW, c = e - r * SW;
-      src[e] = (int64_t)wrap(y0 - H + r, ny) * nx + wrap(x0 - TL::PADX + c, nx);
+      src[e] = (uint32_t)((int64_t)wrap(y0 - H + r, ny) * nx + wrap(x0 - TL::PADX + c, nx));
     }
     __syncthreads();
     // stream entry q: v of plane zs-5+q and lam of the plane two before it
@@ -229,7 +236,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) burgers_adjoint_k
 #pragma unroll 2
           for (int e = tid; e < TL::PLANEL; e += TL::NT) {
             const int r = e / SWL, c = e - r * SWL;
-            const int64_t o = src[(r + H - TL::HL) * SW + c + TL::PADX - TL::PADL];
+            const uint32_t o = src[(r + H - TL::HL) * SW + c + TL::PADX - TL::PADL];
             cp_async_zfill<sizeof(T)>(dl + e, pl + o, ADV_IN_RANGE(pl + o - a.lam, sxy * nz, a.status));
           }
         }
@@ -294,55 +301,70 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) burgers_adjoint_k
       }
       if (out) {
         __syncthreads();  // f+- in place
-        // one face pair: operands at p (f+; f- PART later) with stride st, partials into FB[.][f]
-        auto face = [&](const V* p, int st, V psi, int f) {
-          V g[5];
+        // one face pair: operands at p (f+; f- PART later) with stride st
+        auto face = [&](const V* p, int st, V psi, V (&g)[5], V (&h)[5]) {
           side_rev<Z>(p[0], p[st], p[2 * st], p[3 * st], p[4 * st], psi, g);
-#pragma unroll
-          for (int k = 0; k < 5; ++k) FB[k * NF + f] = g[k];
           const V* const m = p + PART;
-          side_rev<Z>(m[5 * st], m[4 * st], m[3 * st], m[2 * st], m[st], psi, g);
-#pragma unroll
-          for (int k = 0; k < 5; ++k) FB[(5 + k) * NF + f] = g[4 - k];
+          side_rev<Z>(m[5 * st], m[4 * st], m[3 * st], m[2 * st], m[st], psi, h);
         };
-        // x-faces: f = 37 rp + i + 3; rows 2 rp, 2 rp + 1
-        auto xface = [&](int rp, int fi) {
-          const T* const l = lo + (2 * rp + TL::HL) * SWL + TL::PADL + fi - 3;  // lam of cell i, both rows
+        V sx, tx;  // x part of J^T lam from the f+ and f- partials: rows 2 warp, 2 warp + 1 of column `lane`
+        {
+          const T* const l = lo + (2 * warp + TL::HL) * SWL + TL::PADL + lane - 3;  // lam of cell lane - 3, both rows
           const V psi = vmul(V{a.rdx, a.rdx}, vsub(V{l[1], l[SWL + 1]}, V{l[0], l[SWL]}));
-          face(part + rp * XS + fi, 1, psi, rp * TL::FX + fi);
-        };
-        xface(warp, lane);
-        {  // the five faces past lane 31 of every row pair: 40, in two warps (others each plane)
-          const int e = ((warp - q) & 7) * 32 + lane;
-          if (e < 5 * (TL::BY / 2)) xface(e / 5, 32 + e % 5);
+          V g[5], h[5];
+          face(part + warp * XS + lane, 1, psi, g, h);
+          auto from = [&](V w, int d) {  // lane + d's, where the warp has it
+            const V v = {__shfl_down_sync(0xffffffffu, w.x, d), __shfl_down_sync(0xffffffffu, w.y, d)};
+            return lane + d < 32 ? v : vc<V>(0);
+          };
+          sx = vadd(from(g[2], 3), vadd(vadd(from(g[4], 1), from(g[3], 2)), vadd(from(g[1], 4), from(g[0], 5))));
+          tx = vadd(from(h[3], 3), vadd(vadd(h[0], from(h[1], 1)), vadd(from(h[2], 2), from(h[4], 4))));
+        }
+        {  // y-faces: f = 16 (j + 3) + column pair
+          const T* const l = lo + (row - 3 + TL::HL) * SWL + TL::PADL + 2 * cp;  // lam of row j
+          const V psi = vmul(V{a.rdy, a.rdy}, vsub(*reinterpret_cast<const V*>(l + SWL), *reinterpret_cast<const V*>(l)));
+          V g[5], h[5];
+          face(part + YP + tid, PX, psi, g, h);
+#pragma unroll
+          for (int k = 0; k < 5; ++k) {
+            FB[k * NF + tid] = g[k];
+            FB[(5 + k) * NF + tid] = h[4 - k];
+          }
+        }
+        // the faces left over, 5 x 8 in x and 5 x 16 in y: 30 for each of four warps in turn, one per scheduler
+        const int e = ((warp - q) & 7) * 30 + lane;
+        if (lane < 30 && e < 5 * (TL::BY / 2) + 5 * PX) {
+          const bool ex = e < 5 * (TL::BY / 2);
+          const int ey = e - 5 * (TL::BY / 2), r = ex ? e / 5 : TL::BY + ey / PX, c = ex ? 32 + e % 5 : ey % PX;
+          const T* const l = lo + (ex ? (2 * r + TL::HL) * SWL + TL::PADL + c - 3 : (r - 3 + TL::HL) * SWL + TL::PADL + 2 * c);
+          const V psi = vmul(ex ? V{a.rdx, a.rdx} : V{a.rdy, a.rdy},
+                             vsub(V{ex ? l[1] : l[SWL], l[SWL + 1]}, V{l[0], ex ? l[SWL] : l[1]}));
+          V g[5], h[5];
+          face(part + (ex ? r * XS + c : YP + r * PX + c), ex ? 1 : PX, psi, g, h);
+          V* const d = ex ? FE + r * TL::NEX + 5 + c - 32 : FB + r * PX + c;
+          const int ds = ex ? TL::EX : NF;
+#pragma unroll
+          for (int k = 0; k < 5; ++k) {
+            d[k * ds] = g[k];
+            d[(5 + k) * ds] = h[4 - k];
+          }
         }
         __syncthreads();
         {
-          // x part of J^T lam: rows 2 warp, 2 warp + 1 of column `lane`
-          const V* const P = FB + warp * TL::FX + lane + 3;
-          V sp = vadd(P[2 * NF], vadd(vadd(P[4 * NF - 2], P[3 * NF - 1]), vadd(P[NF + 1], P[2])));
-          const V* const M = P + 5 * NF;
-          V sm = vadd(M[NF], vadd(vadd(M[4 * NF - 3], M[3 * NF - 2]), vadd(M[2 * NF - 1], M[1])));
+          if (lane >= 27) {
+            const V* const P = FE + warp * TL::NEX + 5 + lane - 32;
+            const V* const M = P + 5 * TL::EX;
+            sx = vadd(sx, vadd(vadd(P[2 * TL::EX + 3], P[4 * TL::EX + 1]), vadd(vadd(P[3 * TL::EX + 2], P[TL::EX + 4]), P[5])));
+            tx = vadd(tx, vadd(vadd(M[TL::EX + 3], M[3 * TL::EX + 1]), vadd(M[2 * TL::EX + 2], M[4])));
+          }
           const T* const uu = vo + (2 * warp + H) * SW + TL::PADX + lane;
           const V u = {uu[0], uu[SW]};
           const V hu = vmul(vc<V>(0.5), u), au = vabs(u);
-          const V j = vfma(vadd(hu, au), sp, vmul(vsub(hu, au), sm));
+          const V j = vfma(vadd(hu, au), sx, vmul(vsub(hu, au), tx));
           jx[(2 * warp) * TL::BX + lane] = j.x;
           jx[(2 * warp + 1) * TL::BX + lane] = j.y;
         }
-        __syncthreads();
-        // y-faces: f = 16 (j + 3) + column pair
-        auto yface = [&](int fj, int c) {
-          const T* const l = lo + (fj - 3 + TL::HL) * SWL + TL::PADL + 2 * c;  // lam of row j
-          const V psi = vmul(V{a.rdy, a.rdy}, vsub(*reinterpret_cast<const V*>(l + SWL), *reinterpret_cast<const V*>(l)));
-          face(part + YP + fj * PX + c, PX, psi, fj * PX + c);
-        };
-        yface(row, cp);
-        {  // the five rows of faces past row 15: 80, in three warps
-          const int e = ((warp - q - 3) & 7) * 32 + lane;
-          if (e < 5 * PX) yface(TL::BY + e / PX, e % PX);
-        }
-        __syncthreads();
+        __syncwarp();
         const int ko = wrap(zs - 10 + q, nz);
         const V* const P = FB + (row + 3) * PX + cp;
         const V sp = vadd(accP[0], vadd(P[2 * NF], vadd(vadd(P[4 * NF - 2 * PX], P[3 * NF - PX]), vadd(P[NF + PX], P[2 * PX]))));
@@ -446,7 +468,7 @@ adv_status adjoint_stage_t(const adv_burgers_desc& d, int stage, const void* v, 
   int occ = 0;
   ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 256, smem));
   occ = std::max(occ, 1);
-  // one wave of equal shares (128^3: 91.7 us per stage, two waves 96, four 112: a segment streams ten extra
+  // one wave of equal shares (128^3: 92 us per stage, two waves 96, four 112: a segment streams ten extra
   // planes), at least two planes each (48^3: 16.8 us, four 23.1, eight 35.6)
   a.split = work_split((int64_t)a.tiles_x * a.tiles_y, d.nz, (int64_t)di.sms * occ, 2, 6.0);
   void* args[] = {&a};
