@@ -83,6 +83,7 @@ struct HeatLaunch {
   int lanes = 32;                // lanes per row (16: two rows per warp); tile lanes*vector x (32*warps/lanes)*rows
   int tiles_x = 0, tiles_y = 0;  // x-y tiles; the grid is one wave of CTAs sharing the tile-planes
   WorkSplit split;
+  bool down = false;  // the shares are walked downwards in z (heat_prepare_back)
   dim3 grid, block;
   size_t smem = 0;
   CUtensorMap tmap_in;  // tensor map of u_in (re-encoded when the pointer changes)
@@ -95,6 +96,7 @@ struct HeatLaunch {
 // rows: rows per thread of a batched kernel's tile (2 or 4), lanes: lanes per row (32 or 16); 0 = the
 // single-grid stage kernel, its tile the library's choice.
 adv_status heat_prepare(const adv_heat_desc& d, const void* u_in, HeatLaunch* L, int rows = 0, int lanes = 0);
+adv_status heat_prepare_back(const adv_heat_desc& d, const void* u_in, HeatLaunch* L);
 // Lanes per row of the 4-row FP32 tile for rows of nx nodes: 16 (64-wide tiles) where 128-wide
 // tiles leave clearly more lanes idle, else 32.
 int heat_row_lanes(int nx);

@@ -441,7 +441,7 @@ adv_status adv_heat_run(const adv_heat_desc* d, int time_scheme, int64_t nsteps,
   } else if (time_scheme == ADV_EULER) {
     HeatLaunch La, Lb;
     if ((st = heat_prepare(*d, u, &La)) != ADV_OK) return st;
-    if ((st = heat_prepare(*d, w1, &Lb)) != ADV_OK) return st;
+    if ((st = heat_prepare_back(*d, w1, &Lb)) != ADV_OK) return st;
     // Ping-pong u -> w1 -> u; a chunk of 2*C steps is captured once and replayed.
     const int64_t pairs = nsteps / 2;
     const int64_t C = std::min<int64_t>(pairs, 32);

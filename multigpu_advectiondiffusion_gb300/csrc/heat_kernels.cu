@@ -73,6 +73,12 @@ static double tile_use(int nx, int bx) { return (double)nx / ((double)((nx + bx 
 // rows of 16 lanes (tile 64 wide) where they waste clearly fewer lanes than rows of 32
 int heat_row_lanes(int nx) { return tile_use(nx, 64) > tile_use(nx, 128) + 0.02 ? 16 : 32; }
 
+// A stage's two states beyond what stays in the 129 MB L2 from one stage to the next.
+static bool heat_leaves_l2(const adv_heat_desc& d) {
+  const size_t nz = d.ndim == 3 ? d.nz : 1;
+  return (size_t)d.nx * d.ny * nz * (d.dtype == ADV_F32 ? 8 : 16) > ((size_t)96 << 20);
+}
+
 adv_status heat_prepare(const adv_heat_desc& d, const void* u_in, HeatLaunch* L, int rows, int lanes) {
   DeviceInfo di;
   adv_status st = device_info(&di);
@@ -134,7 +140,7 @@ adv_status heat_prepare(const adv_heat_desc& d, const void* u_in, HeatLaunch* L,
   L->split = work_split((int64_t)tiles_x * tiles_y, nz, (int64_t)di.sms * occ, min_share, 0.0);
   // FP32 states that leave the L2 between stages are bound by HBM and run 1-3% faster with the longer shares
   // spread (us per step: 256^3 20.9 against 21.5, 320^3 54.0 against 55.6, 512^3 218 against 222)
-  if (d.dtype == ADV_F32 && (size_t)d.nx * d.ny * nz * 8 > ((size_t)96 << 20))
+  if (d.dtype == ADV_F32 && heat_leaves_l2(d))
     L->split.ratio = (unsigned)((((uint64_t)L->split.extra << 31) + L->split.ctas - 1) / L->split.ctas);
   L->tiles_x = tiles_x;
   L->tiles_y = tiles_y;
@@ -217,12 +223,25 @@ adv_status heat2_launch(const adv_heat_desc& d, const HeatLaunch& L, const void*
   return ADV_OK;
 }
 
+void* heat_down_kernel_f32(int lanes);
+// Forward Euler's second state: where the states leave the L2, its stage walks every share downwards in z
+// and so begins with the planes that the stage before wrote last (us per step, before -> after: 256^3 20.74 ->
+// 20.50, 288^3 46.5 -> 45.3, 320^3 54.5 -> 50.1, 384^3 96.4 -> 94.0, 512^3 219.8 -> 218.0; with states that fit
+// it is 1-3% slower).
+adv_status heat_prepare_back(const adv_heat_desc& d, const void* u_in, HeatLaunch* L) {
+  adv_status st = heat_prepare(d, u_in, L);
+  if (st != ADV_OK || !(d.dtype == ADV_F32 && L->tma && L->rows == 4 && L->warps == 4) || !heat_leaves_l2(d)) return st;
+  L->down = true;
+  ADV_CUDA_TRY(cudaFuncSetAttribute(heat_down_kernel_f32(L->lanes), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->smem));
+  return ADV_OK;
+}
+
 template <class T>
 static adv_status heat_launch_t(const adv_heat_desc& d, const HeatLaunch& L, int stage, const void* u_in,
                                 const void* u_n, void* u_out, cudaStream_t s) {
   HeatParams<T> p = heat_params<T>(d, L, stage, u_in, u_n, u_out);
   const int stage_kind = (stage == 1 && u_n != u_in) ? 0 : stage;
-  void* k = pick_kernel(d, L.tma, stage_kind, L);
+  void* k = L.down && stage_kind == 1 ? heat_down_kernel_f32(L.lanes) : pick_kernel(d, L.tma, stage_kind, L);
   void* args[] = {const_cast<CUtensorMap*>(&L.tmap_in), &p};
   ADV_CUDA_TRY(cudaLaunchKernel(k, L.grid, L.block, args, L.smem, s));
   count_launches(1);

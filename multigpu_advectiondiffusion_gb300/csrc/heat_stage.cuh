@@ -205,9 +205,9 @@ __device__ __forceinline__ int* heat_abort_flag() {
 // STAGE: 1 = stage 1 / forward Euler with u_n == u_in (u_n not read); 2, 3 = RK stages;
 // 0 = stage taken at run time with a separate u_n. Returns the pipeline state for the next
 // segment (by value, so it stays in registers), with s_issue = -1 if a wait timed out (the CTA
-// must then return).
+// must then return). DOWN: the planes in descending order.
 template <class T, int ORDER, int NDIM, bool TMA, int STAGE, int ROWS = 2, int WARPS = 8, int LANES = 32,
-          bool CONTRACT = false, bool HOOK = false, int NODES = 16 / (int)sizeof(T)>
+          bool CONTRACT = false, bool HOOK = false, int NODES = 16 / (int)sizeof(T), bool DOWN = false>
 __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const HeatParams<T>& p, int x0, int y0, int zs,
                                              int ze, HeatPipe pipe) {
   using C = HeatTile<T, ORDER, NDIM, ROWS, WARPS, LANES, NODES>;
@@ -234,11 +234,12 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
   const int F = p.frozen;
   T w[2 * RZ + 1][RY][VX];  // register window along z (w[RZ] = centre plane), re-primed per segment
   const int Q = (ze - zs) + 2 * RZ;  // planes streamed for this segment
-  const int p0 = zs - RZ;            // z of stream entry 0
+  const int p0 = DOWN ? ze - 1 + RZ : zs - RZ;  // z of stream entry 0
+  constexpr int DZ = DOWN ? -1 : 1;             // .. and from one entry to the next
 
   auto issue = [&](int q) {
     T* dst = ring + s_issue * C::SLOT_ELEMS;
-    const int z = p0 + q;
+    const int z = p0 + DZ * q;
     if (TMA) {
       if (tid == 0 && (!HOOK || z != p.withheld_plane)) {
         mbar_arrive_expect_tx(&bars[s_issue], C::PLANE_BYTES);
@@ -339,7 +340,8 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
   const bool vec_rows = (VX == 1 || p.vec_ok) && xb + VX <= nx;
   // every lane stores whole vectors of existing rows: one uniform branch instead of one per row
   const bool warp_vec_store = __all_sync(0xffffffffu, vec_rows && ya + RY - 1 < ny);
-  T* obase = p.out + (size_t)zs * sxy + (size_t)ya * nx + xb;  // output row pointer, plane zs
+  // output row pointer, the first output plane
+  T* obase = p.out + (size_t)(DOWN ? ze - 1 : zs) * sxy + (size_t)ya * nx + xb;
 
   // The z window is a ring of NW = 2 RZ + 1 plane slots: after ROT pushes, logical plane sl
   // (0 = oldest) sits in slot (sl + ROT) % NW. With the plane loop unrolled NW times (O2 in 3D)
@@ -349,6 +351,7 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
   auto plane_step = [&](auto rot, int q) -> bool {
     constexpr int ROT = decltype(rot)::value;
     auto WS = [&](int sl) -> T (&)[RY][VX] { return w[(sl + ROT) % NW]; };
+    auto WZ = [&](int sl) -> T (&)[RY][VX] { return w[((DOWN ? NW - 1 - sl : sl) + ROT) % NW]; };  // ascending in z
     // ---- wait for plane q
     bool ok = true;
     if (TMA) {
@@ -375,7 +378,7 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
     }
 
     if (q >= 2 * RZ && !warp_abort) {
-      const int z = p0 + q - RZ;  // output plane (stream entry q - RZ)
+      const int z = p0 + DZ * (q - RZ);  // output plane (stream entry q - RZ)
       const T* row0 = ring + s_cent * C::SLOT_ELEMS + (RY * ty + R) * SW + C::PADX + tx * VX;
       // x-neighbourhood of the thread's rows: xr[r][j] holds x = xb - R + j.
       T xr[RY][VX + 2 * R];
@@ -434,7 +437,7 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
           for (int e = 0; e < VX; e += 1 + DE) {
             auto X = [&](int j) { return make_float2(xr[r][e + j], xr[r + DR][e + DE + j]); };
             auto Y = [&](int j) { return make_float2(yv[r + j][e], yv[r + DR + j][e + DE]); };
-            auto W = [&](int j) { return make_float2(WS(j)[r][e], WS(j)[r + DR][e + DE]); };
+            auto W = [&](int j) { return make_float2(WZ(j)[r][e], WZ(j)[r + DR][e + DE]); };
             const float2 c = W(RZ);
             const float2 L = lap<float2, ORDER, NDIM, true>(
                 X(R - O1), X(R - 1), c, X(R + 1), X(R + O1), Y(R - O1), Y(R - 1), Y(R + 1), Y(R + O1),
@@ -442,7 +445,7 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
                 W(RZ + (RZ >= 2 ? 2 : 0)), kx2, ky2, kz2);
             float2 un = c;
             if (STAGE != 1) {
-              const size_t off = (size_t)(q - 2 * RZ) * sxy + (size_t)r * nx + e;
+              const size_t off = (DOWN ? -(size_t)(q - 2 * RZ) : (size_t)(q - 2 * RZ)) * sxy + (size_t)r * nx + e;
               const T* src = p.un + (obase - p.out) + off;
               const T* src1 = src + (DR ? (size_t)nx : (size_t)1);
               const bool i0 = (warp_inside || ((inside >> (r * VX + e)) & 1u)) &&
@@ -469,11 +472,11 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
           const T L = lap<T, ORDER, NDIM, FAST>(
               xr[r][R + e - (R >= 2 ? 2 : 1)], xr[r][R + e - 1], c, xr[r][R + e + 1], xr[r][R + e + (R >= 2 ? 2 : 1)],
               yv[R + r - (R >= 2 ? 2 : 1)][e], yv[R + r - 1][e], yv[R + r + 1][e], yv[R + r + (R >= 2 ? 2 : 1)][e],
-              WS(RZ >= 2 ? RZ - 2 : 0)[r][e], WS(RZ >= 1 ? RZ - 1 : 0)[r][e], WS(RZ + (RZ >= 1 ? 1 : 0))[r][e],
-              WS(RZ + (RZ >= 2 ? 2 : 0))[r][e], kx, ky, kz);
+              WZ(RZ >= 2 ? RZ - 2 : 0)[r][e], WZ(RZ >= 1 ? RZ - 1 : 0)[r][e], WZ(RZ + (RZ >= 1 ? 1 : 0))[r][e],
+              WZ(RZ + (RZ >= 2 ? 2 : 0))[r][e], kx, ky, kz);
           T un = c;
           if (STAGE != 1) {
-            const size_t off = (size_t)(q - 2 * RZ) * sxy + (size_t)r * nx + e;
+            const size_t off = (DOWN ? -(size_t)(q - 2 * RZ) : (size_t)(q - 2 * RZ)) * sxy + (size_t)r * nx + e;
             un = ((warp_inside || ((inside >> (r * VX + e)) & 1u)) &&
                   ADV_IN_RANGE((obase - p.out) + off, sxy * nz, p.status))
                      ? p.un[(obase - p.out) + off]
@@ -516,7 +519,7 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
                 res[r][e] = (p.zero_boundary && ((edge >> (r * VX + e)) & 1u)) ? T(0) : WS(RZ)[r][e];
         }
       }
-      T* dst0 = obase + (size_t)(q - 2 * RZ) * sxy;
+      T* dst0 = DOWN ? obase - (size_t)(q - 2 * RZ) * sxy : obase + (size_t)(q - 2 * RZ) * sxy;
       if (warp_vec_store) {
 #pragma unroll
         for (int r = 0; r < RY; ++r) {
@@ -550,7 +553,7 @@ __device__ __forceinline__ HeatPipe heat_segment(const CUtensorMap* tmap, const 
       // the planes prefetched after it.
       if (TMA && tid == 0) {
         const int s_q = s_wait == 0 ? C::NS - 1 : s_wait - 1;
-        if (!HOOK || p0 + q != p.withheld_plane) mbar_wait_bounded(&bars[s_q], ((parity >> s_q) & 1u) ^ 1u, p.status);
+        if (!HOOK || p0 + DZ * q != p.withheld_plane) mbar_wait_bounded(&bars[s_q], ((parity >> s_q) & 1u) ^ 1u, p.status);
         int s = s_wait;
         for (int m = q + 1; m < Q && m <= q + C::P; ++m) {
           mbar_wait_bounded(&bars[s], (parity >> s) & 1u, p.status);
@@ -596,7 +599,7 @@ constexpr int heat_min_ctas() {
 // HOOK: the failure-path test's variant (adv_test_heat_stage_withheld); every other launch runs the
 // kernels without it.
 template <class T, int ORDER, int NDIM, bool TMA, int STAGE, int ROWS = 2, int WARPS = 8, int LANES = 32,
-          bool CONTRACT = false, bool HOOK = false, int NODES = 16 / (int)sizeof(T)>
+          bool CONTRACT = false, bool HOOK = false, int NODES = 16 / (int)sizeof(T), bool DOWN = false>
 __global__ void __launch_bounds__(32 * WARPS, heat_min_ctas<T, ORDER, ROWS, WARPS, NODES>())
 heat_stage_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ HeatParams<T> p) {
   using C = HeatTile<T, ORDER, NDIM, ROWS, WARPS, LANES, NODES>;
@@ -604,7 +607,7 @@ heat_stage_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
   int& abort_flag = *heat_abort_flag();
   const int tid = threadIdx.y * C::TX + threadIdx.x;
   // Balanced split: the (tile, z-plane) pairs, tile-major, are cut into gridDim.x equal
-  // contiguous ranges; a range that crosses a tile boundary becomes several segments.
+  // contiguous ranges; a range that crosses a tile boundary becomes several segments (DOWN: the last first).
   int64_t seg_a, seg_b;
   split_range_whole(p.split, blockIdx.x, &seg_a, &seg_b);
   if (tid == 0) {
@@ -617,15 +620,28 @@ heat_stage_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
   }
   __syncthreads();
   HeatPipe pipe{0, 0, 0u};
-  for (int64_t pos = seg_a; pos < seg_b;) {
-    const int64_t tile = div_units(pos, p.nz);
-    const int zs = (int)(pos - tile * p.nz);
-    const int ze = (int)min((int64_t)p.nz, zs + (seg_b - pos));
-    pos += ze - zs;
-    const int64_t trow = div_units(tile, p.tiles_x);
-    const int x0 = (int)(tile - trow * p.tiles_x) * C::BX, y0 = (int)trow * C::BY;
-    pipe = heat_segment<T, ORDER, NDIM, TMA, STAGE, ROWS, WARPS, LANES, CONTRACT, HOOK, NODES>(&tmap, p, x0, y0, zs, ze, pipe);
-    if (pipe.s_issue < 0) return;
+  if constexpr (DOWN) {
+    for (int64_t pos = seg_b; pos > seg_a;) {
+      const int64_t tile = div_units(pos - 1, p.nz);
+      const int ze = (int)(pos - tile * p.nz);
+      const int zs = (int)max((int64_t)0, ze - (pos - seg_a));
+      pos -= ze - zs;
+      const int64_t trow = div_units(tile, p.tiles_x);
+      const int x0 = (int)(tile - trow * p.tiles_x) * C::BX, y0 = (int)trow * C::BY;
+      pipe = heat_segment<T, ORDER, NDIM, TMA, STAGE, ROWS, WARPS, LANES, CONTRACT, HOOK, NODES, true>(&tmap, p, x0, y0, zs, ze, pipe);
+      if (pipe.s_issue < 0) return;
+    }
+  } else {
+    for (int64_t pos = seg_a; pos < seg_b;) {
+      const int64_t tile = div_units(pos, p.nz);
+      const int zs = (int)(pos - tile * p.nz);
+      const int ze = (int)min((int64_t)p.nz, zs + (seg_b - pos));
+      pos += ze - zs;
+      const int64_t trow = div_units(tile, p.tiles_x);
+      const int x0 = (int)(tile - trow * p.tiles_x) * C::BX, y0 = (int)trow * C::BY;
+      pipe = heat_segment<T, ORDER, NDIM, TMA, STAGE, ROWS, WARPS, LANES, CONTRACT, HOOK, NODES>(&tmap, p, x0, y0, zs, ze, pipe);
+      if (pipe.s_issue < 0) return;
+    }
   }
 }
 

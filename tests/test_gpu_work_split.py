@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from multigpu_advectiondiffusion_gb300 import _native as N
-from multigpu_advectiondiffusion_gb300.solvers import BurgersConfig, HeatConfig, burgers_stage, heat_stage
+from multigpu_advectiondiffusion_gb300.solvers import BurgersConfig, HeatConfig, burgers_stage, heat_run, heat_stage
 
 pytestmark = pytest.mark.gpu
 
@@ -18,6 +18,20 @@ def test_heat_stage_on_both_sides_of_the_l2(cuda, oracle, size):
     out = torch.full_like(a, float("nan"))
     heat_stage(cfg, 1, a, a, out)
     np.testing.assert_array_equal(out.cpu().numpy().view(np.uint8), oracle.heat_stage(cfg, 1, u, u).view(np.uint8))
+
+
+@pytest.mark.parametrize("size", [(128, 300, 340), (320, 199, 201), (256, 192, 270)])
+@pytest.mark.parametrize("frozen,zero", [(1, True), (2, False)])
+def test_euler_steps_of_a_state_beyond_the_l2(cuda, oracle, size, frozen, zero):
+    """Every second step walks its shares downwards in z (tiles of both widths, ragged rows)."""
+    import torch
+    cfg = HeatConfig(3, *size, 2, frozen, zero, 0.03, 0.02, 0.01, 0.5, N.ADV_EULER)
+    u = np.random.default_rng(7).standard_normal(cfg.numel).astype(np.float32)
+    a = torch.from_numpy(u).to(cuda)
+    heat_run(cfg, a, 3)
+    for _ in range(3):
+        u = oracle.heat_stage(cfg, 1, u, u)
+    np.testing.assert_array_equal(a.cpu().numpy().view(np.uint8), u.view(np.uint8))
 
 
 @pytest.mark.parametrize("size", [(96, 96, 96), (128, 112, 101), (250, 200, 1), (40, 33, 64), (97, 65, 300)])
