@@ -70,6 +70,13 @@ void tune_store(int kind, int variant, int nx, int ny, int nz, TuneParams p);
 void tune_clear();
 void graph_cache_clear();  // cached CUDA graphs hold launch shapes: drop them when tuning changes
 
+// Unique id of the calling thread's current CUDA context (0 if none is current), through the driver entry
+// points the runtime exposes (no -lcuda link). A context made after a cudaDeviceReset has a new one.
+unsigned long long current_context_id();
+// Lets `kernel` take `smem` bytes of dynamic shared memory and, with occ, tells how many of its CTAs of
+// `threads` threads an SM holds.
+adv_status kernel_setup(const void* kernel, int threads, size_t smem, int* occ);
+
 // ------------------------------------------------------------------ heat launchers
 // "No plane withheld": below every plane a stream can visit (halo planes reach z = -2).
 constexpr int kNoWithheldPlane = -2147483647 - 1;

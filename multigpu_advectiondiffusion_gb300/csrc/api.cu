@@ -61,6 +61,40 @@ adv_status device_info(DeviceInfo* out) {
   return ADV_OK;
 }
 
+// The runtime takes about 0.5 us to set a kernel's attribute and 1 us to compute its occupancy, several of each
+// per stage call, so what was set and found is kept per (context, kernel) in a fixed table; an entry that
+// another one needs the place of is set and computed again on its next use.
+adv_status kernel_setup(const void* kernel, int threads, size_t smem, int* occ) {
+  struct Entry {
+    unsigned long long ctx;
+    const void* kernel;
+    size_t smem;
+    int threads, occ;  // occ 0: not asked for yet
+  };
+  static std::mutex mu;
+  static Entry table[1024];
+  const unsigned long long ctx = current_context_id();
+  Entry* const e = &table[(((uintptr_t)kernel >> 4) * 2654435761u + ctx * 40503u) % 1024];
+  if (ctx != 0) {
+    std::lock_guard<std::mutex> lk(mu);
+    if (e->ctx == ctx && e->kernel == kernel && e->smem == smem && e->threads == threads && (!occ || e->occ > 0)) {
+      if (occ) *occ = e->occ;
+      return ADV_OK;
+    }
+  }
+  if (smem > 0) ADV_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int n = 0;
+  if (occ) {
+    ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem));
+    *occ = n = std::max(n, 1);
+  }
+  if (ctx != 0) {
+    std::lock_guard<std::mutex> lk(mu);
+    *e = Entry{ctx, kernel, smem, threads, n};
+  }
+  return ADV_OK;
+}
+
 EncodeTiledFn encode_tiled_fn() {
   static EncodeTiledFn fn = nullptr;
   static std::once_flag once;
@@ -113,10 +147,8 @@ adv_status burgers_prepare(const adv_burgers_desc& d, const void* u_in, BurgersL
   L->mode = d.nz == 1 ? 2 : aligned ? 0 : 1;  // BurgersMode
   void* k = d.dtype == ADV_F32 ? burgers_kernel_for<float>(d, L->mode) : burgers_kernel_for<double>(d, L->mode);
   if (!k) return set_error(ADV_ERR_UNSUPPORTED, "burgers: no kernel for this configuration");
-  ADV_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->smem));
   int occ = 0;
-  ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 256, L->smem));
-  occ = std::max(occ, 1);
+  if ((st = kernel_setup(k, 256, L->smem, &occ)) != ADV_OK) return st;
   L->occ = occ;
   // CTAs with equal shares of the (tile, plane) pairs: one wave of them, so that no last wave is
   // nearly empty (FP64 121 x 101 x 97: 339 CTAs of 8 planes on 304 resident ones ran 3293 us a stage,

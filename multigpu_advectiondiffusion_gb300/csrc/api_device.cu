@@ -14,11 +14,16 @@ namespace adv {
 __device__ int g_status_word[1];
 
 int* device_status_ptr() {
-  // The address of a __device__ symbol is per device; resolve it each call (cheap) so the
-  // pointer always belongs to the current device.
+  // The address of a __device__ symbol is per context; each thread keeps that of the one it last asked for.
+  static thread_local unsigned long long last_ctx = 0;
+  static thread_local int* last = nullptr;
+  const unsigned long long ctx = current_context_id();
+  if (ctx != 0 && ctx == last_ctx) return last;
   void* p = nullptr;
   if (cudaGetSymbolAddress(&p, g_status_word) != cudaSuccess) return nullptr;
-  return static_cast<int*>(p);
+  last_ctx = current_context_id();
+  last = static_cast<int*>(p);
+  return last;
 }
 
 adv_status read_and_clear_device_status(cudaStream_t s) {

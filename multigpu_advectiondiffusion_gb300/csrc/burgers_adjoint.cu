@@ -464,10 +464,8 @@ adv_status adjoint_stage_t(const adv_burgers_desc& d, int stage, const void* v, 
   a.rdx = (T)(1.0 / d.dx); a.rdy = (T)(1.0 / d.dy); a.rdz = (T)(1.0 / d.dz);
   void* k = adjoint_kernel(d);
   const size_t smem = AdjSmem<T>::TOTAL;
-  ADV_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int occ = 0;
-  ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 256, smem));
-  occ = std::max(occ, 1);
+  if ((st = kernel_setup(k, 256, smem, &occ)) != ADV_OK) return st;
   // one wave of equal shares (128^3: 92 us per stage, two waves 96, four 112: a segment streams ten extra
   // planes), at least two planes each (48^3: 16.8 us, four 23.1, eight 35.6)
   a.split = work_split((int64_t)a.tiles_x * a.tiles_y, d.nz, (int64_t)di.sms * occ, 2, 6.0);

@@ -112,17 +112,15 @@ adv_status heat_prepare(const adv_heat_desc& d, const void* u_in, HeatLaunch* L,
   int occ = 1;
   L->occ = 0;
   if (rows == 0) {  // (with explicit rows the caller runs a batched kernel of its own over this tile)
-    for (int sk = 0; sk <= 3; ++sk) {
-      void* k = pick_kernel(d, L->tma, sk, *L);
-      if (!k) return set_error(ADV_ERR_UNSUPPORTED, "heat: no kernel for this configuration");
-      ADV_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    }
     // The wave is counted by stage 1's kernel, which forward Euler runs alone. FP64 O4 in 3D, an SSP-RK3 scheme's:
     // by stage 3's, which takes the most registers; stages of more CTAs than fit end with a second, nearly
     // empty wave (us per step, before -> after: 201 x 199 x 200 1248 -> 1143, 208 x 160 x 150 711 -> 657).
-    void* k0 = pick_kernel(d, L->tma, d.dtype == ADV_F64 && d.order == 4 && d.ndim == 3 ? 3 : 1, *L);
-    ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k0, 32 * L->warps, smem));
-    occ = std::max(occ, 1);
+    const int counted = d.dtype == ADV_F64 && d.order == 4 && d.ndim == 3 ? 3 : 1;
+    for (int sk = 0; sk <= 3; ++sk) {
+      void* k = pick_kernel(d, L->tma, sk, *L);
+      if (!k) return set_error(ADV_ERR_UNSUPPORTED, "heat: no kernel for this configuration");
+      if ((st = kernel_setup(k, 32 * L->warps, smem, sk == counted ? &occ : nullptr)) != ADV_OK) return st;
+    }
     L->occ = occ;
   }
   // One wave: every CTA resident at once, each with an equal share of the (tile, plane) pairs (or what
@@ -184,10 +182,8 @@ adv_status heat2_prepare(const adv_heat_desc& d, const void* u_in, HeatLaunch* L
   constexpr int BX = 128, BY = 16, SW = 136, SHU = 20;
   void* k = heat_twostep_kernel_ptr();
   const size_t smem = heat_twostep_smem();
-  ADV_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int occ = 0;
-  ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 128, smem));
-  occ = std::max(occ, 1);
+  if ((st = kernel_setup(k, 128, smem, &occ)) != ADV_OK) return st;
   L->tma = true;
   L->occ = occ;
   L->rows = 4;
@@ -232,8 +228,7 @@ adv_status heat_prepare_back(const adv_heat_desc& d, const void* u_in, HeatLaunc
   adv_status st = heat_prepare(d, u_in, L);
   if (st != ADV_OK || !(d.dtype == ADV_F32 && L->tma && L->rows == 4 && L->warps == 4) || !heat_leaves_l2(d)) return st;
   L->down = true;
-  ADV_CUDA_TRY(cudaFuncSetAttribute(heat_down_kernel_f32(L->lanes), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->smem));
-  return ADV_OK;
+  return kernel_setup(heat_down_kernel_f32(L->lanes), 32 * L->warps, L->smem, nullptr);
 }
 
 template <class T>

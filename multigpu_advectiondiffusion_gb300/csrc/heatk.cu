@@ -544,7 +544,7 @@ void heatk_shape(const adv_heatk_desc& d, int kind, const void* kernel, int lx, 
   DeviceInfo di;
   const int sms = device_info(&di) == ADV_OK ? di.sms : 152;
   int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, lx * 8, 0) != cudaSuccess || occ < 1) occ = 4;
+  if (kernel_setup(kernel, lx * 8, 0, &occ) != ADV_OK) occ = 4;
   const int64_t tiles = (int64_t)((d.nx + bx - 1) / bx) * ((d.ny + by - 1) / by);
   const int64_t chunks = std::max<int64_t>(1, std::min<int64_t>(d.nz, (int64_t)sms * occ / tiles));
   *zc = (int)((d.nz + chunks - 1) / chunks);

@@ -13,9 +13,7 @@ namespace adv {
 // Scratch of adv_heat_run_noalloc. Every GPU that loads this library holds it until exit.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[ADV_NOALLOC_SCRATCH_BYTES];
 
-// Unique id of the calling thread's current CUDA context (0 if none is current), through the
-// driver entry points the runtime exposes (no -lcuda link).
-static unsigned long long current_context_id() {
+unsigned long long current_context_id() {
   typedef CUresult (*GetCurrentFn)(CUcontext*);
   typedef CUresult (*GetIdFn)(CUcontext, unsigned long long*);
   static GetCurrentFn get_current = nullptr;

@@ -560,11 +560,10 @@ adv_status weno7_fused(const adv_weno7_desc& d, const float* u, float* out, floa
   p.maxkey = static_cast<unsigned*>(maxkey);
   p.active = active;
   p.status = device_status_ptr();
-  ADV_CUDA_TRY(cudaFuncSetAttribute(weno7_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)W7Tile::SMEM));
   int occ = 0;
-  ADV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, weno7_fused_kernel, W7Tile::NT, W7Tile::SMEM));
+  if ((st = kernel_setup(reinterpret_cast<const void*>(&weno7_fused_kernel), W7Tile::NT, W7Tile::SMEM, &occ)) != ADV_OK) return st;
   // one wave of equal shares, at least two planes each (a segment streams eight more)
-  p.split = work_split((int64_t)p.tiles_x * p.tiles_y, d.nz, (int64_t)di.sms * std::max(occ, 1), d.nz == 1 ? 1 : 2, 4.0);
+  p.split = work_split((int64_t)p.tiles_x * p.tiles_y, d.nz, (int64_t)di.sms * occ, d.nz == 1 ? 1 : 2, 4.0);
   weno7_fused_kernel<<<p.split.ctas, W7Tile::NT, W7Tile::SMEM, s>>>(p);
   ADV_CUDA_TRY(cudaGetLastError());
   if (count) count_launches(1);

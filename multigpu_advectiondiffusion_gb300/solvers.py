@@ -37,12 +37,14 @@ def _fields(numel: int, *ts) -> int:
     past it (an FP64 state in an FP32 buffer of the same length included)."""
     first = ts[0]
     code = _dtype_code(first)
+    dtype, device = first.dtype, first.device
     for t in ts:
         _ptr(t)
-        if t.dtype != first.dtype:
-            raise ValueError(f"fields of one call must share a dtype: {first.dtype} and {t.dtype}")
-        if t.device != first.device:
-            raise ValueError(f"fields of one call must share a device: {first.device} and {t.device}")
+        if t is not first:
+            if t.dtype != dtype:
+                raise ValueError(f"fields of one call must share a dtype: {dtype} and {t.dtype}")
+            if t.device != device:
+                raise ValueError(f"fields of one call must share a device: {device} and {t.device}")
         if t.numel() < numel:
             raise ValueError(f"a field has {t.numel()} elements; the grid has {numel}")
     return code
@@ -54,9 +56,13 @@ def _stream(stream, like):
     `with torch.cuda.stream(...)`); None (the default stream) without CUDA."""
     if stream is not None:
         return N.stream_handle(stream)
-    import torch
-    if getattr(like, "is_cuda", False) and torch.cuda.is_available():
-        return torch.cuda.current_stream(like.device).cuda_stream or None
+    if getattr(like, "is_cuda", False):
+        import torch
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        if raw is not None and torch.cuda.is_initialized():
+            return raw(like.device.index) or None  # (0.3 us; with the stream object below 3 us)
+        if torch.cuda.is_available():
+            return torch.cuda.current_stream(like.device).cuda_stream or None
     return None
 
 
