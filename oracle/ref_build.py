@@ -177,9 +177,9 @@ def build_mains() -> list[Path]:
 
 
 def reference_dir() -> Path | None:
-    """The reference checkout to build from: $ADV_REFERENCE_DIR, else /root/reference; None if absent."""
+    """The reference checkout to build from: $ADV_REFERENCE_DIR, else /root/reference; None if absent or empty."""
     p = Path(os.environ.get("ADV_REFERENCE_DIR", "/root/reference"))
-    return p if p.is_dir() else None
+    return p if p.is_dir() and any(p.iterdir()) else None
 
 
 def main(argv=None) -> None:
