@@ -143,6 +143,7 @@ inline int64_t burgers_waves(int64_t units, int64_t wave) {
 struct BurgersLaunch {
   bool tma = false;
   int mode = 0;  // BurgersMode: the kernel's load path and problem class
+  bool differentiated = false;  // the forms that gradients follow (Candidates in weno.cuh)
   int occ = 0;  // resident CTAs per SM of the stage kernel (before any tuning cap)
   int tiles_x = 0, tiles_y = 0;  // 32 x 16 column tiles; the grid is one wave sharing the tile-planes
   WorkSplit split;
@@ -152,7 +153,8 @@ struct BurgersLaunch {
 };
 adv_status burgers_validate(const adv_burgers_desc* d);
 int burgers_tune_variant(const adv_burgers_desc& d);
-adv_status burgers_prepare(const adv_burgers_desc& d, const void* u_in, BurgersLaunch* L);
+// differentiated: a stage of a forward run that the adjoint sweeps back through.
+adv_status burgers_prepare(const adv_burgers_desc& d, const void* u_in, BurgersLaunch* L, bool differentiated = false);
 // Stage launch arguments. The Lax-Friedrichs constant and dt come from the host values unless
 // a device source is given (used by the graph-resident time loop).
 struct BurgersStageArgs {

@@ -24,7 +24,7 @@ adv_status burgers_launch_f64(const adv_burgers_desc& d, const BurgersLaunch& L,
 size_t burgers_smem_f32();
 size_t burgers_smem_f64();
 template <class T>
-void* burgers_kernel_for(const adv_burgers_desc& d, int mode);
+void* burgers_kernel_for(const adv_burgers_desc& d, int mode, bool differentiated);
 
 // ---------------------------------------------------------------------------- errors
 static thread_local std::string g_last_error;
@@ -133,7 +133,7 @@ int burgers_tune_variant(const adv_burgers_desc& d) {
   return d.dtype * 1000 + d.weno * 100 + d.div * 10 + visc;
 }
 
-adv_status burgers_prepare(const adv_burgers_desc& d, const void* u_in, BurgersLaunch* L) {
+adv_status burgers_prepare(const adv_burgers_desc& d, const void* u_in, BurgersLaunch* L, bool differentiated) {
   DeviceInfo di;
   adv_status st = device_info(&di);
   if (st != ADV_OK) return st;
@@ -145,7 +145,8 @@ adv_status burgers_prepare(const adv_burgers_desc& d, const void* u_in, BurgersL
   const int tiles_x = (d.nx + 31) / 32, tiles_y = (d.ny + 15) / 16;
   L->smem = d.dtype == ADV_F32 ? burgers_smem_f32() : burgers_smem_f64();
   L->mode = d.nz == 1 ? 2 : aligned ? 0 : 1;  // BurgersMode
-  void* k = d.dtype == ADV_F32 ? burgers_kernel_for<float>(d, L->mode) : burgers_kernel_for<double>(d, L->mode);
+  L->differentiated = differentiated;
+  void* k = d.dtype == ADV_F32 ? burgers_kernel_for<float>(d, L->mode, differentiated) : burgers_kernel_for<double>(d, L->mode, differentiated);
   if (!k) return set_error(ADV_ERR_UNSUPPORTED, "burgers: no kernel for this configuration");
   int occ = 0;
   if ((st = kernel_setup(k, 256, L->smem, &occ)) != ADV_OK) return st;

@@ -108,12 +108,10 @@ __device__ __forceinline__ double sgn_mul(double d, double t) { return d > 0.0 ?
 // bars of e and b carry a factor 2).
 template <bool Z, class V>
 __device__ __forceinline__ void side_rev(V a, V b, V c, V d, V e, V psi, V (&g)[5]) {
-  const V A = vsub(b, a), B = vsub(c, b), C = vsub(d, c), E = vsub(e, d);
-  const V t0 = vsub(B, A), t1 = vsub(C, B), t2 = vsub(E, C);
-  const V s0 = vfma(vc<V>(2), B, t0), s1 = vadd(B, C), s2 = vfma(vc<V>(-2), C, t2);
-  const V K = vc<V>(13.0 / 3.0), eps = vc<V>(4e-6);
-  const V k0 = vmul(K, t0), k1 = vmul(K, t1), k2 = vmul(K, t2);
-  const V b0 = vfma(k0, t0, vfma(s0, s0, eps)), b1 = vfma(k1, t1, vfma(s1, s1, eps)), b2 = vfma(k2, t2, vfma(s2, s2, eps));
+  V t[3], s[3], k[3], w[3];  // (the forward run's own indicators: see Candidates in weno.cuh)
+  weno_indicators(a, b, c, d, e, t, s, k, w);
+  const V t0 = t[0], t1 = t[1], t2 = t[2], s0 = s[0], s1 = s[1], s2 = s[2], k0 = k[0], k1 = k[1], k2 = k[2];
+  const V b0 = w[0], b1 = w[1], b2 = w[2];
   const V p12 = vmul(b1, b2), p02 = vmul(b0, b2), p01 = vmul(b0, b1);
   const V da = vsub(t1, t0), db = vsub(t2, t1);
   V e0, e1, e2, d02, tau;
@@ -504,13 +502,13 @@ adv_status forward_step(const adv_burgers_desc& d, const void* un, void* u1, voi
   BurgersLaunch L;
   BurgersStageArgs a{};
   a.dt_host = dt;
-  adv_status st = burgers_prepare(d, un, &L);
+  adv_status st = burgers_prepare(d, un, &L, true);
   a.stage = 1; a.u_in = un; a.u_n = un; a.u_out = u1;
   if (st == ADV_OK) st = burgers_launch(d, L, a, s);
-  if (st == ADV_OK) st = burgers_prepare(d, u1, &L);
+  if (st == ADV_OK) st = burgers_prepare(d, u1, &L, true);
   a.stage = 2; a.u_in = u1; a.u_n = un; a.u_out = u2;
   if (st == ADV_OK) st = burgers_launch(d, L, a, s);
-  if (st == ADV_OK) st = burgers_prepare(d, u2, &L);
+  if (st == ADV_OK) st = burgers_prepare(d, u2, &L, true);
   a.stage = 3; a.u_in = u2; a.u_n = un; a.u_out = unext;
   if (st == ADV_OK) st = burgers_launch(d, L, a, s);
   return st;
@@ -612,10 +610,10 @@ adv_status adv_burgers_backward(const adv_burgers_desc* d, double dt, int64_t ns
         BurgersLaunch L;
         BurgersStageArgs a{};
         a.dt_host = dt;
-        if ((st = burgers_prepare(*d, un(r), &L)) != ADV_OK) return st;
+        if ((st = burgers_prepare(*d, un(r), &L, true)) != ADV_OK) return st;
         a.stage = 1; a.u_in = un(r); a.u_n = un(r); a.u_out = u1(r);
         if ((st = burgers_launch(*d, L, a, s)) != ADV_OK) return st;
-        if ((st = burgers_prepare(*d, u1(r), &L)) != ADV_OK) return st;
+        if ((st = burgers_prepare(*d, u1(r), &L, true)) != ADV_OK) return st;
         a.stage = 2; a.u_in = u1(r); a.u_n = un(r); a.u_out = u2(r);
         if ((st = burgers_launch(*d, L, a, s)) != ADV_OK) return st;
       }

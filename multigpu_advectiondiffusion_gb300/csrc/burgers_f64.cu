@@ -6,7 +6,7 @@
 namespace adv {
 
 template <>
-void* burgers_kernel_for<double>(const adv_burgers_desc& d, int mode) {
+void* burgers_kernel_for<double>(const adv_burgers_desc& d, int mode, bool) {
 #define K(Z, D, V, M) reinterpret_cast<void*>(&burgers_stage_kernel<double, Z, D, V, M>)
   ADV_BURGERS_PICK(d, mode, double, K);
 #undef K

@@ -149,6 +149,32 @@ struct Face<double, Z, double> {
   };
 };
 
+// The candidates' weighted mean (weno.cuh): a z-face from the last four cells of each part and the newest.
+template <class D>
+struct Face<float, true, Candidates<D>> {
+  using V = float2;
+  __device__ __forceinline__ static V f(V p0, V p1, V p2, V p3, V p4, V m0, V m1, V m2, V m3, V m4) {
+    return weno_face_mean<D>(p0, p1, p2, p3, p4, m0, m1, m2, m3, m4);
+  }
+  __device__ __forceinline__ static void split(V u, V a, V& fp, V& fm) { lf_split2(u, a, fp, fm); }
+  struct Line {
+    V p[5], m[4];  // f+ one plane behind f-
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+      for (int i = 0; i < 5; ++i) p[i] = vc<V>(0);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) m[i] = vc<V>(0);
+    }
+    __device__ __forceinline__ V push(V fp, V fm, V, V, bool want) {
+      V r = vc<V>(0);
+      if (want) r = f(p[0], p[1], p[2], p[3], p[4], m[0], m[1], m[2], m[3], fm);
+      p[0] = p[1]; p[1] = p[2]; p[2] = p[3]; p[3] = p[4]; p[4] = fp;
+      m[0] = m[1]; m[1] = m[2]; m[2] = m[3]; m[3] = fm;
+      return r;
+    }
+  };
+};
+
 // Stream entries a CTA has waited for so far (entry n lives in slot n % NS and is that slot's phase
 // n / NS); kPipeAborted after a wait that timed out.
 constexpr unsigned kPipeAborted = 0xffffffffu;
@@ -254,8 +280,8 @@ __device__ __forceinline__ double2 combine2(int stage, double2 un, double2 u, do
   return make_double2(stage_combine<double>(stage, un.x, u.x, dt, L.x), stage_combine<double>(stage, un.y, u.y, dt, L.y));
 }
 __device__ __forceinline__ float2 combine2(int stage, float2 un, float2 u, float dt, float2 L) {
-  const float2 dL = vmul(make_float2(dt, dt), L);
-  if (stage == 2) return vadd(vmul(vc<float2>(0.75), un), vmul(vc<float2>(0.25), vadd(u, dL)));
+  const float2 dL = vmul_alone(make_float2(dt, dt), L);
+  if (stage == 2) return vadd(vmul_alone(vc<float2>(0.75), un), vmul(vc<float2>(0.25), vadd(u, dL)));  // (u/4 is exact)
   if (stage == 3) return div3(vfma(vc<float2>(2), vadd(u, dL), un));
   return vadd(un, dL);
 }
@@ -573,6 +599,9 @@ __device__ __forceinline__ unsigned burgers_segment(const CUtensorMap* tmap, con
                           div_by(sub_rn(fzp, fzm), p.dz, p.rdz));
           };
           L = {rhs(fx0.x, fx1.x, fym.x, fyp.x, fz_prev.x, fz.x), rhs(fx0.y, fx1.y, fym.y, fyp.y, fz_prev.y, fz.y)};
+        } else if constexpr (IsCandidates<D>::value) {
+          L = vfma(vsub(fz_prev, fz), V{p.rdz, p.rdz},
+                   vfma(vsub(fx0, fx1), V{p.rdx, p.rdx}, vmul(vsub(fym, fyp), V{p.rdy, p.rdy})));
         } else {
           L = vfma(vsub(fz_prev, fz), V{p.rdz, p.rdz},
                    vfma(vsub(fym, fyp), V{p.rdy, p.rdy}, vmul(vsub(fx0, fx1), V{p.rdx, p.rdx})));

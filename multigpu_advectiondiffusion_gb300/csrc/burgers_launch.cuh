@@ -7,7 +7,7 @@
 namespace adv {
 
 template <class T>
-void* burgers_kernel_for(const adv_burgers_desc& d, int mode);
+void* burgers_kernel_for(const adv_burgers_desc& d, int mode, bool differentiated);
 
 // The kernel of a scheme and mode among all instantiations of K<Z, D, VISC, MODE>. FP32 divides alike
 // for ADV_DIV_F32 and ADV_DIV_F64 (an FP64 quotient rounded to FP32 is the correctly rounded one).
@@ -64,7 +64,7 @@ template <class T>
 adv_status burgers_launch_t(const adv_burgers_desc& d, const BurgersLaunch& L, const BurgersStageArgs& a,
                             cudaStream_t s) {
   BurgersParams<T> p = burgers_params<T>(d, L, a);
-  void* k = burgers_kernel_for<T>(d, L.mode);
+  void* k = burgers_kernel_for<T>(d, L.mode, L.differentiated);
   if (!k) return set_error(ADV_ERR_UNSUPPORTED, "burgers: no kernel for this configuration");
   void* args[] = {const_cast<CUtensorMap*>(&L.tmap_in), &p};
   ADV_CUDA_TRY(cudaLaunchKernel(k, L.grid, L.block, args, L.smem, s));
