@@ -935,10 +935,10 @@ def bench_weno7(args, world, rank, dev, stream, flush, lib):
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
     fp32_peak = sms * 128 * 2 * 2070.0 * 1e6 / 1e12
     flops = WENO7_FLOPS_PER_CELL_STAGE * cfg.numel / stage_s / 1e12
-    roofline = {"bound": "hbm", "kernel": "weno7_face_fast_kernel + weno7_residual_kernel (3 axes per stage)",
+    roofline = {"bound": "hbm", "kernel": "weno7_fused_kernel",
                 "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
                 "traffic": None, "algorithmic_bytes_per_launch": 16 * cfg.numel, "avg_launch_us": stage_s * 1e6,
-                "launch": "one LSRK stage (six kernels)"}
+                "launch": "one LSRK stage"}
     roofline_alu = {"bound": "fp32", "achieved": flops, "peak": fp32_peak, "unit": "TFLOP/s",
                     "frac": flops / fp32_peak, "flops_per_cell_stage": WENO7_FLOPS_PER_CELL_STAGE,
                     "peak_source": f"nominal: {sms} SMs x 128 FP32 lanes x 2 flop x 2070 MHz"}
@@ -1169,7 +1169,9 @@ def main():
     if heat:
         launches_per_step = max(1, launched // max(1, args.steps))
         bytes_per_launch = 8 * cfg.numel
-        if launches_per_step * 2 <= inner:  # the tuner chose two Euler steps per launch
+        if args.workload == "heat2d" and launches_per_step * 2 <= inner:
+            kernel = "heat2d_multi_kernel (several forward-Euler steps per launch)"
+        elif launches_per_step * 2 <= inner:  # the tuner chose two Euler steps per launch
             kernel = "heat_twostep_kernel (two forward-Euler steps per launch)"
     else:
         launches_per_step = inner * 3
