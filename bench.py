@@ -285,11 +285,10 @@ def cpu_baseline_heat(cfg, u0, nsteps: int, budget_s: float) -> dict:
 
 
 # FP32 flops per cell-stage of the fused WENO5-Z stage, counting an FFMA2 as 4 flops, an FADD2,
-# FMUL2 or FFMA as 2 and an FADD or FMUL as 1, from the ncu instruction mix of the
-# reciprocal-division form at 256^3 (stage 1): FFMA2 81.2, FADD2 18.5, FMUL2 37.3, FFMA 6.6,
-# FADD 5.3, FMUL 10.1 per cell = 465.0. The division counts as the reciprocal form's operations
-# whichever division is run.
-BURGERS_FLOPS_PER_CELL_STAGE = 465.0
+# FMUL2 or FFMA as 2 and an FADD or FMUL as 1, from the ncu instruction mix at 256^3 (stage 1):
+# FFMA2 63.29, FADD2 36.07, FMUL2 35.05, FMUL 1.0 per cell = 396.4 (the correctly rounded quotient's
+# operations among them).
+BURGERS_FLOPS_PER_CELL_STAGE = 396.4
 
 ENSEMBLE_SEED = 2024
 ENSEMBLE_STEPS = 500
@@ -876,11 +875,9 @@ def weno7_config(world: int) -> dict:
 
 
 # FP32 flops per cell-stage of the WENO7 right-hand side, counted from the ncu instruction mix of
-# adv_weno7_rhs at 256^3 (FP32 state: the tiled face kernels with paired instructions and
-# reciprocal-based weights). Per cell: FFMA2 153 x 4 + FADD2 21 x 2 + FMUL2 96 x 2 + FFMA 22.3 x 2
-# + FADD 11.0 + FMUL 50.6 = 952.25. (The prototype's own operand order, which the FP64 state
-# keeps, counted 1949: FFMA 495 x 2 + FADD 401 + FMUL 558.)
-WENO7_FLOPS_PER_CELL_STAGE = 952.25
+# adv_weno7_rhs at 256^3 (FP32 state: the fused stage). Per cell: FFMA2 81.57 x 4 + FADD2 81.82 x 2
+# + FMUL2 66.0 x 2 = 621.9.
+WENO7_FLOPS_PER_CELL_STAGE = 621.9
 
 
 def bench_weno7(args, world, rank, dev, stream, flush, lib):
