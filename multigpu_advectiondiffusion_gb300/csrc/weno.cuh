@@ -254,10 +254,11 @@ __device__ __forceinline__ float weno_ref_tau(float t) { return t; }
 __device__ __forceinline__ double weno_ref_tau(double t) {
   return __double2hiint(t) < (1023 - 100) << 20 ? __hiloint2double((1023 - 100) << 20, 0) : t;
 }
-// ... and zero over a positive sum is the same zero.
+// ... and zero over a positive finite sum is the same zero. (Over any other it is not: from |u| of about 1e39 on
+// every WENO5-JS weight underflows to 0, and 0/0 has to come out as NaN.)
 __device__ __forceinline__ float weno_ref_quot(float n, float d) { return div_rn(n, d); }
 __device__ __forceinline__ double weno_ref_quot(double n, double d) {
-  const bool zero = ((__double2hiint(n) << 1) | __double2loint(n)) == 0;
+  const bool zero = ((__double2hiint(n) << 1) | __double2loint(n)) == 0 && (unsigned)__double2hiint(d) - 1u < 0x7fefffffu;
   const double q = div_rn(zero ? 1.0 : n, d);
   return zero ? n : q;
 }

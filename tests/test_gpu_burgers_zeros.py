@@ -51,3 +51,24 @@ def test_stage_over_zero_numerators(cuda, oracle, size, state, bc, weno, C):
         burgers_stage(cfg, stage, a, b, out, 1e-3, float(np.abs(u).max()))
         np.testing.assert_array_equal(out.cpu().numpy().view(np.uint8),
                                       oracle.burgers_stage(cfg, stage, u, base, 1e-3).view(np.uint8))
+
+
+@pytest.mark.parametrize("size", [(36, 20, 9), (35, 16, 10), (40, 50, 1)])
+@pytest.mark.parametrize("scale", [1e38, 1e39, 1e60])
+def test_js_weights_that_all_underflow(cuda, oracle, size, scale):
+    """From |u| of about 1e39 on, every (eps + beta)^2 overflows, the weights are 0 and a side is 0/0: NaN, as in
+    the scheme as written (constant lines, whose indicators vanish, stay finite)."""
+    import torch
+    nx, ny, nz = size
+    cfg = BurgersConfig.reference_2d(2.0, 2.0, nx, ny) if nz == 1 else BurgersConfig(
+        nx, ny, nz, 2.0 / nx, 2.0 / ny, 2.0 / nz, N.ADV_WENO5_JS, N.ADV_LF_LOCAL, N.ADV_BC_PERIODIC)
+    cfg.weno, cfg.C = N.ADV_WENO5_JS, 0.0
+    u = scale * np.random.default_rng(4).uniform(-1, 1, (nz, ny, nx))
+    u[:, : ny // 2] = 0.25 * scale
+    u = u.ravel()
+    want = oracle.burgers_stage(cfg, 1, u, u, 1e-3 / scale)
+    assert np.isnan(want).any() == (scale > 1e38) and np.isfinite(want).any()
+    a = torch.from_numpy(u).to(cuda)
+    out = torch.zeros_like(a)
+    burgers_stage(cfg, 1, a, a, out, 1e-3 / scale, scale)
+    np.testing.assert_array_equal(out.cpu().numpy(), want)
