@@ -249,10 +249,11 @@ __device__ __forceinline__ T weno_ref_k(T a, T b, T c) {
 // a tile's columns past the domain) takes its warp along: with it kept away, a stage of 121 x 101 x 97, whose
 // last tiles hold seven such columns, takes 1740 us instead of 2086, periodic 120^3 2510 instead of 3397,
 // 128^3 2389 instead of 2447. Neither operation changes a result: beside an indicator of at least eps, a tau
-// below 2^-100 leaves 1 + tau / (B + eps) at exactly 1 ...
+// below 2^-100 leaves 1 + tau / (B + eps) at exactly 1 (unsigned: the NaN of two infinite indicators, which the
+// absolute value may leave with its sign, is not below it) ...
 __device__ __forceinline__ float weno_ref_tau(float t) { return t; }
 __device__ __forceinline__ double weno_ref_tau(double t) {
-  return __double2hiint(t) < (1023 - 100) << 20 ? __hiloint2double((1023 - 100) << 20, 0) : t;
+  return (unsigned)__double2hiint(t) < (1023u - 100u) << 20 ? __hiloint2double((1023 - 100) << 20, 0) : t;
 }
 // ... and zero over a positive finite sum is the same zero. (Over any other it is not: from |u| of about 1e39 on
 // every WENO5-JS weight underflows to 0, and 0/0 has to come out as NaN.)

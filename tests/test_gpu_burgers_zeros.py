@@ -72,3 +72,23 @@ def test_js_weights_that_all_underflow(cuda, oracle, size, scale):
     out = torch.zeros_like(a)
     burgers_stage(cfg, 1, a, a, out, 1e-3 / scale, scale)
     np.testing.assert_array_equal(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("size", [(36, 20, 9), (35, 16, 10), (33, 35, 8)])
+@pytest.mark.parametrize("scale", [1e77, 2e77, 1e78, 1e100])
+def test_z_indicators_that_are_all_infinite(cuda, oracle, size, scale):
+    """tau = |beta0 - beta2| of two infinite indicators is NaN, and so is the side: NaN wherever the scheme as
+    written gives one. (3D: on a 2D grid the oracle also reconstructs the equal z-faces, whose rounding overflows
+    at this scale; the stage leaves them out.)"""
+    import torch
+    nx, ny, nz = size
+    cfg = BurgersConfig(nx, ny, nz, 2.0 / nx, 2.0 / ny, 2.0 / nz, N.ADV_WENO5_Z, N.ADV_LF_LOCAL, N.ADV_BC_PERIODIC)
+    u = scale * np.random.default_rng(4).uniform(-1, 1, (nz, ny, nx))
+    u[:, : ny // 2] = 0.25 * scale
+    u = u.ravel()
+    want = oracle.burgers_stage(cfg, 1, u, u, 1e-3 / scale)
+    assert np.isnan(want).any()
+    a = torch.from_numpy(u).to(cuda)
+    out = torch.zeros_like(a)
+    burgers_stage(cfg, 1, a, a, out, 1e-3 / scale, scale)
+    assert np.isnan(out.cpu().numpy())[np.isnan(want)].all()
