@@ -230,8 +230,8 @@ struct WenoLine {
 
 // ---------------------------------------------------------- reference literal form
 // Operand order of kernels.cu:142-192 / :92-140 (and of the CPU oracle), every operation rounded on
-// its own. Products by powers of two are exact (short of overflow; the quarter of C*C only ever meets
-// eps = 1e-6 or a tau of the same size), so they go into fused multiply-adds without changing a bit:
+// its own. Products by powers of two are exact (short of overflow; the quarter of C*C: weno_ref_beta), so
+// they go into fused multiply-adds without changing a bit:
 // 52 operations and four divisions per side instead of 66 and four. FP64 is bound by its pipe (two lanes
 // per SM and cycle), so a stage's time follows this count.
 // RECIP: the normalisation of SingleGPU/Burgers3d_WENO5_SharedMem/kernels.cu:51-198, which takes
@@ -243,6 +243,22 @@ template <class T>
 __device__ __forceinline__ T weno_ref_k(T a, T b, T c) {
   const T A = add_rn(fma_rn_(T(-2), b, a), c);
   return mul_rn(mul_rn(T(13. / 12.), A), A);
+}
+
+// The three indicators K + C^2/4 from their triples' shares and first differences, (1/4 C) C rounded twice as
+// written. FP64 fuses the exact quarter of C^2 instead (what a subnormal C^2 loses only ever meets eps = 1e-6 or a
+// tau of the same size), except where C^2 overflows and a quarter of it need not.
+__device__ __forceinline__ void weno_ref_beta(const float (&K)[3], const float (&C)[3], float (&B)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) B[i] = add_rn(K[i], mul_rn(mul_rn(0.25f, C[i]), C[i]));
+}
+__device__ __forceinline__ void weno_ref_beta(const double (&K)[3], const double (&C)[3], double (&B)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) B[i] = fma_rn_(0.25, mul_rn(C[i], C[i]), K[i]);
+  if (max(max(__double2hiint(B[0]), __double2hiint(B[1])), __double2hiint(B[2])) >= 0x7ff00000) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) B[i] = add_rn(K[i], mul_rn(mul_rn(0.25, C[i]), C[i]));
+  }
 }
 
 // A compiled FP64 division leaves its short form for a numerator of zero, and one such lane (a constant state,
@@ -271,8 +287,9 @@ __device__ __forceinline__ T weno_side_ref(T a, T b, T c, T d, T e, T K0, T K1, 
   const T eps = T(1e-6);
   const T c3 = mul_rn(T(3), c);
   const T C0 = add_rn(fma_rn_(T(-4), b, a), c3), C1 = sub_rn(b, d), C2 = add_rn(fma_rn_(T(-4), d, c3), e);
-  const T B0 = fma_rn_(T(0.25), mul_rn(C0, C0), K0), B1 = fma_rn_(T(0.25), mul_rn(C1, C1), K1),
-          B2 = fma_rn_(T(0.25), mul_rn(C2, C2), K2);
+  T B[3];
+  weno_ref_beta({K0, K1, K2}, {C0, C1, C2}, B);
+  const T B0 = B[0], B1 = B[1], B2 = B[2];
   const T d0 = T(PLUS ? 1. / 10. : 3. / 10.), d1 = T(6. / 10.), d2 = T(PLUS ? 3. / 10. : 1. / 10.);
   T a0, a1, a2;
   if (Z) {

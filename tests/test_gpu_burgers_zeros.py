@@ -92,3 +92,31 @@ def test_z_indicators_that_are_all_infinite(cuda, oracle, size, scale):
     out = torch.zeros_like(a)
     burgers_stage(cfg, 1, a, a, out, 1e-3 / scale, scale)
     assert np.isnan(out.cpu().numpy())[np.isnan(want)].all()
+
+
+@pytest.mark.parametrize("size", [(36, 20, 9), (35, 16, 10), (33, 35, 8)])
+@pytest.mark.parametrize("scale", [6.5e76, 8e76, 1.1e77])
+def test_indicators_whose_first_difference_squared_overflows(cuda, oracle, size, scale):
+    """C^2 beyond the largest number where C^2/4 is not: finite indicators, finite results."""
+    import torch
+    nx, ny, nz = size
+    cfg = BurgersConfig(nx, ny, nz, 2.0 / nx, 2.0 / ny, 2.0 / nz, N.ADV_WENO5_Z, N.ADV_LF_LOCAL, N.ADV_BC_PERIODIC)
+    u = scale * np.random.default_rng(4).uniform(-1, 1, nx * ny * nz)
+    want = oracle.burgers_stage(cfg, 1, u, u, 1e-3 / scale)
+    assert np.isfinite(want).any()
+    a = torch.from_numpy(u).to(cuda)
+    out = torch.zeros_like(a)
+    burgers_stage(cfg, 1, a, a, out, 1e-3 / scale, scale)
+    np.testing.assert_array_equal(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("dtype,scale", [(np.float64, 7e76), (np.float32, 2.6e9)])
+def test_sweep_where_the_first_difference_squared_overflows(cuda, native, oracle, dtype, scale):
+    import torch
+    u = (scale * np.random.default_rng(4).uniform(-1, 1, (9, 9, 40))).astype(dtype)
+    want = oracle.burgers_sweep_all(0, True, u, 0.1, np.zeros_like(u))
+    a = torch.from_numpy(u.ravel()).to(cuda)
+    L = torch.zeros_like(a)
+    assert native.adv_ref_burgers_sweep_all(N.ADV_F64 if dtype == np.float64 else N.ADV_F32, 0, N.ADV_WENO5_Z, 40, 40, 9,
+                                            9, 0.1, a.data_ptr(), L.data_ptr(), None) == N.ADV_OK
+    np.testing.assert_array_equal(L.cpu().numpy().reshape(u.shape), want)
