@@ -35,6 +35,7 @@
 #include "adv_device.cuh"
 #include "adv_internal.h"
 #include "adv_math.cuh"
+#include "heatk_rows.h"
 #include "nvtx_range.h"
 
 namespace adv {
@@ -139,14 +140,13 @@ __device__ __forceinline__ void stv(T* p, const VN<T, N>& v) {
 
 // A thread's nodes and what its neighbours are. LX: threads per block row.
 template <class T, int VX, int RY, int LX>
-struct HeatKThread {
+struct HeatKThread : HeatKRows<RY> {
+  using HeatKRows<RY>::dr;
   static constexpr int N = RY * VX;
   int x, y, z0, z1;
   int nx, ny, nz;
   int64_t sz;
   int64_t first;     // offset of its first node in the grid's first plane (clamped to the grid)
-  int dr[RY];        // its rows' offsets from the first (rows past the grid: the last one) ..
-  int above, below;  // .. and those of the rows y-1 and y+RY (clamped to its own first / last)
   bool ok[RY];       // the row is on the grid (and so are all VX nodes)
   int left, right;   // offsets of the nodes x-1 and x+VX (clamped)
   int tx;
@@ -162,12 +162,8 @@ struct HeatKThread {
     const int xc = min(x, nx - VX), yc = min(y, ny - 1);  // threads past the grid read its last nodes (shuffles)
     first = (int64_t)yc * nx + xc;
 #pragma unroll
-    for (int r = 0; r < RY; ++r) {
-      ok[r] = any && y + r < ny;
-      dr[r] = (min(yc + r, ny - 1) - yc) * nx;
-    }
-    above = yc > 0 ? -nx : 0;
-    below = (min(yc + RY, ny - 1) - yc) * nx;
+    for (int r = 0; r < RY; ++r) ok[r] = any && y + r < ny;
+    this->set(yc, nx, ny);
     left = xc > 0 ? -1 : 0;
     right = xc + VX < nx ? VX : VX - 1;
     return any;
