@@ -121,10 +121,11 @@ struct W7Geom {
 };
 
 // Face kernel of axis AX: for every node (the face i+1/2 on its right along AX) the two parts'
-// reconstructions into hp / hn.
+// reconstructions into hp / hn. active (may be null): 0 in a step past the run's end, which computes nothing.
 template <class T, int AX>
 __global__ void __launch_bounds__(256) weno7_face_kernel(const T* __restrict__ u, T* __restrict__ hp,
-                                                         T* __restrict__ hn, W7Geom g) {
+                                                         T* __restrict__ hn, W7Geom g, const int* active) {
+  if (active && *active == 0) return;
   const int64_t stride = AX == 0 ? 1 : AX == 1 ? (int64_t)g.nx : (int64_t)g.nx * g.ny;
   const int N = AX == 0 ? g.nx : AX == 1 ? g.ny : g.nz;
   for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < g.n; o += (int64_t)gridDim.x * blockDim.x) {
@@ -429,8 +430,8 @@ __global__ void __launch_bounds__(256, 3) weno7_fused_kernel(const __grid_consta
 }
 
 template <class T, int AX>
-void weno7_face_launch(const T* u, T* hp, T* hn, const W7Geom& g, int grid, cudaStream_t s) {
-  weno7_face_kernel<T, AX><<<grid, 256, 0, s>>>(u, hp, hn, g);
+void weno7_face_launch(const T* u, T* hp, T* hn, const W7Geom& g, const int* active, int grid, cudaStream_t s) {
+  weno7_face_kernel<T, AX><<<grid, 256, 0, s>>>(u, hp, hn, g, active);
 }
 
 // Residual kernel of axis AX: res_i = (((hp_i + hn_i) - hp_{i-1}) - hn_{i-1}) / h (0 for the face
@@ -582,14 +583,14 @@ adv_status weno7_stage64(const adv_weno7_desc& d, double* u, const W7Work& w, in
   double* acc = reinterpret_cast<double*>(w.acc);
   double* r = reinterpret_cast<double*>(w.r);
   K* mk = static_cast<K*>(maxkey);
-  weno7_face_launch<double, 0>(u, hp, hn, g, grid, s);
+  weno7_face_launch<double, 0>(u, hp, hn, g, active, grid, s);
   weno7_residual_launch<double, 0, true, false>(hp, hn, acc, r, u, g, d.dx, stage, dt_dev, mk, active, grid, s);
-  weno7_face_launch<double, 1>(u, hp, hn, g, grid, s);
+  weno7_face_launch<double, 1>(u, hp, hn, g, active, grid, s);
   if (nd == 2) {
     weno7_residual_launch<double, 1, false, true>(hp, hn, acc, r, u, g, d.dy, stage, dt_dev, mk, active, grid, s);
   } else {
     weno7_residual_launch<double, 1, false, false>(hp, hn, acc, r, u, g, d.dy, stage, dt_dev, mk, active, grid, s);
-    weno7_face_launch<double, 2>(u, hp, hn, g, grid, s);
+    weno7_face_launch<double, 2>(u, hp, hn, g, active, grid, s);
     weno7_residual_launch<double, 2, false, true>(hp, hn, acc, r, u, g, d.dz, stage, dt_dev, mk, active, grid, s);
   }
   ADV_CUDA_TRY(cudaGetLastError());
@@ -616,12 +617,12 @@ adv_status weno7_rhs64(const adv_weno7_desc& d, const double* u, double* L, cons
   const int nd = weno7_ndim(d);
   double* hp = reinterpret_cast<double*>(w.hp);
   double* hn = reinterpret_cast<double*>(w.hn);
-  weno7_face_launch<double, 0>(u, hp, hn, g, grid, s);
+  weno7_face_launch<double, 0>(u, hp, hn, g, nullptr, grid, s);
   weno7_residual_launch<double, 0, true, false>(hp, hn, L, nullptr, nullptr, g, d.dx, 0, nullptr, nullptr, nullptr, grid, s);
-  weno7_face_launch<double, 1>(u, hp, hn, g, grid, s);
+  weno7_face_launch<double, 1>(u, hp, hn, g, nullptr, grid, s);
   weno7_residual_launch<double, 1, false, false>(hp, hn, L, nullptr, nullptr, g, d.dy, 0, nullptr, nullptr, nullptr, grid, s);
   if (nd == 3) {
-    weno7_face_launch<double, 2>(u, hp, hn, g, grid, s);
+    weno7_face_launch<double, 2>(u, hp, hn, g, nullptr, grid, s);
     weno7_residual_launch<double, 2, false, false>(hp, hn, L, nullptr, nullptr, g, d.dz, 0, nullptr, nullptr, nullptr, grid, s);
   }
   ADV_CUDA_TRY(cudaGetLastError());
@@ -688,9 +689,12 @@ adv_status adv_weno7_run(const adv_weno7_desc* d, void* u, void* workspace, doub
   };
   const int64_t launched_per_step = 1 + 5 * weno7_stage_launches(*d);
   bool graph_ran = false;
-  // A run of a few steps at most: its launches, predicated on the loop state, cost less than capturing
-  // and instantiating a graph (about 0.2 ms).
-  if (max_steps > 0 && max_steps <= 8 && tEnd > 0.0) {
+  // A run of a few launches at most: they cost less queued one by one, predicated on the loop state, than captured
+  // and instantiated as a graph (about 0.1 ms; then 3 us less a step in FP32, 60 us in FP64 3D). us directly / as a
+  // graph: FP32 24^3 (six launches a step) 1 step 138 / 229, 4 370 / 420, 8 676 / 679; FP64 (31) 1 step
+  // 981 / 1081, 3 2812 / 2775.
+  const bool direct = max_steps > 0 && max_steps <= 48 / launched_per_step;
+  if (direct && tEnd > 0.0) {
     for (int64_t i = 0; i < max_steps; ++i)
       if ((st = body(s, 0, 0)) != ADV_OK) return st;
   } else if (max_steps > 0 && tEnd > 0.0) {
@@ -746,6 +750,7 @@ adv_status adv_weno7_run(const adv_weno7_desc* d, void* u, void* workspace, doub
   ADV_CUDA_TRY(cudaMemcpyAsync(&h, w.st, sizeof(h), cudaMemcpyDeviceToHost, s));
   ADV_CUDA_TRY(cudaStreamSynchronize(s));
   if (graph_ran) count_launches(launched_per_step * h.step);  // (the host loop counted its own)
+  else if (direct && tEnd > 0.0) count_launches(launched_per_step * (h.step - max_steps));  // steps past the end: none
   if (t_out) *t_out = h.t;
   if (steps_out) *steps_out = h.step;
   return read_and_clear_device_status(s);
