@@ -327,7 +327,8 @@ adv_status adv_autotune_heat(const adv_heat_desc* d, const void* u, void* stream
   const int nz = d->ndim == 3 ? d->nz : 1;
   const size_t bytes = (size_t)d->nx * d->ny * nz * (d->dtype == ADV_F32 ? 4 : 8);
   // Time stages the way a run issues them: each launch reads the previous launch's output
-  // (two scratch arrays, the first a copy of u; u itself is not modified).
+  // (two scratch arrays, the first a copy of u; u itself is not modified), every second one with
+  // adv_heat_run's launch of its second state (heat_prepare_back).
   Scratch tmp(s), tmp2(s);
   if ((st = tmp.alloc(bytes)) != ADV_OK) return st;
   if ((st = tmp2.alloc(bytes)) != ADV_OK) return st;
@@ -348,7 +349,7 @@ adv_status adv_autotune_heat(const adv_heat_desc* d, const void* u, void* stream
   int flip = 0;
   auto prep = [&]() {
     adv_status r = heat_prepare(*d, tmp2.p, &La);
-    return r == ADV_OK ? heat_prepare(*d, tmp.p, &Lb) : r;
+    return r == ADV_OK ? heat_prepare_back(*d, tmp.p, &Lb) : r;
   };
   auto run = [&]() {
     flip ^= 1;

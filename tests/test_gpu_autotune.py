@@ -81,3 +81,29 @@ def test_autotune_rejects_bad_descriptor(cuda, native):
     r = N.TuneResult()
     bad = N.HeatDesc(4, 8, 8, 8, N.ADV_F32, 2, 1, 1, 1.0, 1.0, 1.0, 0.1)
     assert native.adv_autotune_heat(N.C.byref(bad), None, None, N.C.byref(r)) == N.ADV_ERR_INVALID_ARG
+
+
+def test_heat_tuner_times_what_a_run_launches(cuda, native):
+    """Beyond the L2 every second Euler step runs a kernel that walks the other way, 8-10% faster; the tuner's choices
+    (shapes, one or two steps per launch) hold only if it times a run's own launches: its default shape takes what an
+    untuned run takes per step, but for the launches queued one by one (2 us of 61; with the first kernel alone 70)."""
+    import torch
+    cfg = HeatConfig(3, 352, 352, 300, 2, 1, True, 0.03, 0.02, 0.01, 0.5, N.ADV_EULER)
+    u = torch.rand(cfg.numel, dtype=torch.float32, device=cuda)
+    steps = 64
+
+    def run_us():
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        heat_run(cfg, u, steps)
+        b.record()
+        b.synchronize()
+        return 1e3 * a.elapsed_time(b) / steps
+
+    ratios = []
+    for _ in range(3):
+        autotune_clear()
+        untuned = min(run_us() for _ in range(4))
+        ratios.append(autotune_heat(cfg, u)["default_us"] / untuned)
+    autotune_clear()
+    assert min(ratios) < 1.10, ratios
