@@ -53,9 +53,9 @@ typedef enum adv_time { ADV_EULER = 0, ADV_SSPRK3 = 1 } adv_time;
 typedef enum adv_weno { ADV_WENO5_JS = 0, ADV_WENO5_Z = 1 } adv_weno;
 typedef enum adv_lf { ADV_LF_LOCAL = 0, ADV_LF_GLOBAL = 1 } adv_lf;
 typedef enum adv_bc { ADV_BC_FROZEN = 0, ADV_BC_PERIODIC = 1 } adv_bc;
-/* Division of the WENO weights when the state is FP32 (one division per face side):
- * F32 = IEEE FP32 division, F64 = the division in FP64, FAST = FP32 reciprocal-based division
- * (at most 2 ulp). An FP64 state uses the reference's own operand order and its four FP64
+/* Division of the WENO weights when the state is FP32 (one division per face side): F32 and F64
+ * give the correctly rounded FP32 quotient (an FP64 division rounded to FP32 is the same number, so
+ * the two share their kernels), FAST a reciprocal-based one (at most 2 ulp). An FP64 state uses the reference's own operand order and its four FP64
  * divisions per side (bit-exact) with F32 or F64, and with FAST the common-denominator form:
  * one FP64 division per side, fused multiply-adds, flux differences times 1/h (a few ulps from
  * the reference's rounding). */

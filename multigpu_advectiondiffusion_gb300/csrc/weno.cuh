@@ -77,14 +77,15 @@ __device__ __forceinline__ float rcp_approx(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-// Negated quotient -num / den of the weight sums (den > 0 and far from the subnormals: at least
-// (4e-6)^3). FP32: FastDiv multiplies by the reciprocal approximation; otherwise one Newton step on
-// the reciprocal and one residual correction of the quotient in fused multiply-adds (Markstein,
-// IBM J. Res. Dev. 34 (1990) 111-119), which returns the correctly rounded quotient -- what an
-// FP64 division rounded to FP32 also returns, so both division kinds of an FP32 state share it.
-// Compiled IEEE divisions took about 10 issue slots per quotient, six quotients per cell; this
-// takes 3.5 in paired instructions. (Negated: the reciprocal of -den makes both corrections plain
-// multiply-adds.)
+// Negated quotient -num / den of the weight sums (den at least 6.4e-16 with WENO5-Z, 10 (4e-6)^3, and 2.5e-21 with JS,
+// 10 (4e-6)^4: far from the subnormals). FP32: FastDiv multiplies by the reciprocal approximation; otherwise one
+// Newton step on the reciprocal and one residual correction of the quotient in fused multiply-adds (Markstein,
+// IBM J. Res. Dev. 34 (1990) 111-119). The quotient is correctly rounded where the residual is exact (|num| from
+// 2^-102 on) -- what an FP64 division rounded to FP32 also returns, so both division kinds of an FP32 state share
+// it: the reciprocal is the correctly rounded one for each of the 2^23 significands, which leaves only quotients
+// within 2^-22 ulp of a tie in question, and all of those come out right (both compared on the GPU by
+// tests/test_gpu_quotients.py). 3.5 issue slots per quotient in paired instructions; compiled IEEE divisions take about
+// 10, six quotients per cell. (Negated: the reciprocal of -den makes both corrections plain multiply-adds.)
 template <class D>
 __device__ __forceinline__ float2 vnquot(float2 num, float2 den) {
   const float2 r0 = make_float2(rcp_approx(-den.x), rcp_approx(-den.y));
