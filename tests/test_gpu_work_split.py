@@ -63,3 +63,28 @@ def test_burgers_stage_of_a_rolled_state_is_the_rolled_stage(cuda, size, dtype):
             assert top == np.abs(got).max()
         want = got if want is None else want
         np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("size", [(250, 200, 1), (1000, 90, 1), (33, 17, 1)])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("periodic", [True, False])
+def test_burgers_2d_stage_and_maximum(cuda, oracle, size, dtype, periodic):
+    """One plane: FP64 equals the oracle bit for bit, FP32 the FP32 oracle within 4e-7 of the maximum (two units of a state's
+    rounding and four faces' at dt = h/20), and the key is the maximum of what was written."""
+    import torch
+    nx, ny, nz = size
+    cfg = BurgersConfig(nx, ny, nz, 0.01, 0.01, 0.01, N.ADV_WENO5_Z, N.ADV_LF_GLOBAL, N.ADV_BC_PERIODIC) if periodic else \
+        BurgersConfig.reference_2d(0.01 * (nx - 1), 0.01 * (ny - 1), nx, ny)
+    rng = np.random.default_rng(8)
+    u, un = (rng.uniform(-1, 1, cfg.numel).astype(dtype) for _ in range(2))
+    bits, real = (torch.int64, torch.float64) if dtype == np.float64 else (torch.int32, torch.float32)
+    key = torch.zeros(1, dtype=bits, device=cuda)
+    a, b = (torch.from_numpy(v).to(cuda) for v in (u, un))
+    out = torch.full_like(a, float("nan"))
+    burgers_stage(cfg, 3, a, b, out, 5e-4, float(np.abs(u).max()), maxabs_key=key)
+    got, want = out.cpu().numpy(), oracle.burgers_stage(cfg, 3, u, un, 5e-4)
+    if dtype == np.float64:
+        np.testing.assert_array_equal(got, want)
+    else:
+        assert np.abs(got - want).max() <= 4e-7 * np.abs(want).max()
+    assert key.view(real).item() == np.abs(got).max()
