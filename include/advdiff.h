@@ -55,10 +55,10 @@ typedef enum adv_lf { ADV_LF_LOCAL = 0, ADV_LF_GLOBAL = 1 } adv_lf;
 typedef enum adv_bc { ADV_BC_FROZEN = 0, ADV_BC_PERIODIC = 1 } adv_bc;
 /* Division of the WENO weights when the state is FP32 (one division per face side): F32 and F64
  * give the correctly rounded FP32 quotient (an FP64 division rounded to FP32 is the same number, so
- * the two share their kernels), FAST a reciprocal-based one (at most 2 ulp). An FP64 state uses the reference's own operand order and its four FP64
- * divisions per side (bit-exact) with F32 or F64, and with FAST the common-denominator form:
- * one FP64 division per side, fused multiply-adds, flux differences times 1/h (a few ulps from
- * the reference's rounding). */
+ * the two share their kernels), FAST a reciprocal-based one (at most 2 ulp). An FP64 state uses
+ * the reference's own operand order and its four FP64 divisions per side (bit-exact) with F32 or
+ * F64, and with FAST the common-denominator form: one FP64 division per side, fused
+ * multiply-adds, flux differences times 1/h (a few ulps from the reference's rounding). */
 typedef enum adv_div { ADV_DIV_F32 = 0, ADV_DIV_F64 = 1, ADV_DIV_FAST = 2 } adv_div;
 /* Burgers time-step rule. FIXED: dt = min(CFL*dx/1, 0.9/(2C sum 1/h^2)) as the reference driver
  * (SingleGPU/Burgers3d_WENO5/main.cpp:130-133); MAXU: dt = CFL*dx/max|u^n| computed on the
@@ -282,6 +282,12 @@ adv_status adv_heatk_backward(const adv_heatk_desc* d, const void* k, int64_t ns
 /* --------------------------------------------------------------- Burgers discrete adjoint
  * Exact transpose of the fixed-dt SSP-RK3 step of the periodic, local Lax-Friedrichs, inviscid
  * scheme (WENO5-JS or WENO5-Z; FP32 or FP64 state; other schemes return ADV_ERR_UNSUPPORTED).
+ * WENO5-Z has a kink where two smoothness indicators are equal; there the rounding decides which
+ * side's derivative is taken. For an FP32 state with ADV_DIV_F32 or _F64 adv_burgers_forward
+ * computes the indicators with the adjoint's own operations, so the two decide alike; states
+ * from adv_burgers_stage or adv_burgers_run, and any with ADV_DIV_FAST, come from a faster form
+ * that rounds differently (the same to a few ulps), and single entries of their gradients differ
+ * from adv_burgers_forward's by what such a decision moves, neither being the closer to FP64.
  * No counterpart in the reference. adv_burgers_adjoint_step turns lam = dJ/du^{n+1} into
  * dJ/du^n given the step's stage inputs u^n, u1, u2; `work` holds 3 arrays. The forward run
  * stores u every `interval` steps; the backward run recomputes each interval (its stage inputs)

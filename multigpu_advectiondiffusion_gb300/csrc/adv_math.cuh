@@ -17,7 +17,9 @@ __device__ __forceinline__ double div_rn(double a, double b) { return __ddiv_rn(
 
 // Two FP32 lanes at once with Blackwell's paired instructions (FADD2 / FMUL2 / FFMA2): each lane
 // is rounded exactly as the scalar operation, so packed code gives the scalar results bit for
-// bit. a - b is issued as fma(b, -1, a) (one rounding of the exact difference).
+// bit (as long as no paired product goes into a paired sum: the compiler fuses the two, which it
+// does not do to the scalar ones). a - b is issued as fma(b, -1, a) (one rounding of the exact
+// difference).
 __device__ __forceinline__ float2 add_rn(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 sub_rn(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
 __device__ __forceinline__ float2 mul_rn(float2 a, float2 b) { return __fmul2_rn(a, b); }

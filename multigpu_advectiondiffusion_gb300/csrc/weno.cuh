@@ -34,7 +34,9 @@ __device__ __forceinline__ void lf_split(T u, T a, T& fp, T& fm) {
 // ------------------------------------------------------------------ two values at once
 // A pair of values: float2 operations are Blackwell's paired FP32 instructions (FFMA2 / FADD2 /
 // FMUL2: one instruction, each lane rounded like the scalar operation), double2 operations two
-// scalar ones. Every operation is explicit, so the single-grid and the batched kernels round alike.
+// scalar ones. Every operation is explicit, but the compiler fuses a paired product into a paired sum that takes it
+// (vmul_alone keeps one apart). The single-grid and the batched kernels round alike all the same: the only products
+// that their stages add are by powers of two, which are exact.
 template <class T> struct Vec2;
 template <> struct Vec2<float> { using type = float2; };
 template <> struct Vec2<double> { using type = double2; };
@@ -159,13 +161,13 @@ __device__ __forceinline__ V weno_face2(V p0, V p1, V p2, V p3, V p4, V m0, V m1
   return vfma(vc<V>(0.5), vadd(qp, qm), lin);
 }
 
-// WENO-Z of FP32 states in forward runs that an adjoint sweep follows. tau = |b0 - b2| has a kink, so a gradient
-// jumps where the rounding of a state or of an indicator decides the sign of b0 - b2: the forms above, in such a
-// run, moved single entries by up to 5e-3 of the gradient's rms at 24^3 .. 64^3 (either side's error against FP64
-// is as large). These runs therefore weigh the candidates q_k/6 = c + t_k/12 + { s0/4 | s1/4 | -s2/4 } themselves,
-// operation for operation as gradients have always been taken, and the adjoint takes the same indicators: ten steps at
-// 24^3 .. 128^3 give the states of the first such kernels bit for bit and their gradients to 3e-5 of the rms, for 1.8%
-// of a gradient's time (128^3: 3790 -> 3860 us; 6490 with those kernels). D: the quotient's kind.
+// WENO-Z of FP32 states in forward runs that an adjoint sweep follows (adv_burgers_forward). tau = |b0 - b2| has a
+// kink, so a gradient jumps where the rounding of a state or of an indicator decides the sign of b0 - b2: two forms of
+// the same run differ in single entries by up to 5e-3 of the gradient's rms at 24^3 .. 64^3, either of them as far from
+// FP64. These runs and the adjoint take one form, and the same indicators: the candidates q_k/6 = c + t_k/12 +
+// { s0/4 | s1/4 | -s2/4 } themselves, weighed (128^3: 1.8% of a gradient's 3860 us). Their sum of weights adds
+// products that must not be fused into it; tests/test_gpu_burgers_gradient_form.py holds the states to the separately
+// rounded operations. D: the quotient's kind.
 template <class D>
 struct Candidates {};
 template <class D> struct IsCandidates : std::false_type {};

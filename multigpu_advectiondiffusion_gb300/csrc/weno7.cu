@@ -39,9 +39,6 @@
 #include "nvtx_range.h"
 #include "weno.cuh"
 
-#ifndef W7OCC
-#define W7OCC 3
-#endif
 namespace adv {
 namespace {
 
@@ -173,7 +170,7 @@ __global__ void __launch_bounds__(256) weno7_face_kernel(const T* __restrict__ u
 // Layout as the WENO5 stage (burgers_kernels.cuh): 32 x 16 columns per CTA, two adjacent in x per
 // thread; planes with a halo of 4 stream through an 8-slot ring (cp.async from a list of the clamped
 // in-plane offsets); f+- of the output plane go to shared memory in pairs of rows (x-faces) and of
-// columns (y-faces); z-faces come from register windows; two barriers per plane. Bound by the FMA pipe
+// columns (y-faces); z-faces come from register windows; three barriers per plane (copies landed, parts split, faces done). Bound by the FMA pipe
 // and the barriers (pipe 54% busy, 459 paired FP32 instructions of 922 per pair of cells): right-hand side
 // 256^3 383 us with two CTAs per SM, 371 with three; a run of 3 steps at 160^3 2556 -> 1743 us against
 // six face and residual launches per stage.
