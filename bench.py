@@ -469,7 +469,7 @@ def bench_ensemble(args, world, rank, dev, stream, flush, lib):
             "data": "synthetic (seeded sizes, diffusivities and Philox4x32-10 initial conditions)",
             "config": ensemble_config(world),
             "shape": {"heat_cells": heat_cells, "burgers_cells": burg_cells, **shape},
-            "roofline": {"bound": "hbm", "kernel": f"burgers_batch_kernel<float,Z,{ENSEMBLE_DIV} div>", "achieved": achieved,
+            "roofline": {"bound": "hbm", "kernel": f"burgers_group_kernel<float,Z,{ENSEMBLE_DIV} div>", "achieved": achieved,
                          "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
                          "traffic": _traffic("ensemble"), "algorithmic_bytes_per_launch": bytes_per_launch,
                          "avg_launch_us": launch_ms * 1e3},

@@ -27,7 +27,7 @@
 // plane alone: no z faces, no z halo (1000 x 900 FP32: 61 -> 14.5 us per stage against streaming the
 // plane seven times). FP64 is bound by its pipe (78% busy at 128 x 112 x 101): warps whose faces no updated
 // node reads reconstruct none, and the faces left over are one value per lane of two warps
-// (121 x 101 x 97: 2378 -> 2086 us per stage, 64 x 53 x 60: 519 -> 409).
+// (121 x 101 x 97: 2378 -> 2086 us per stage, 64 x 53 x 60: 519 -> 409; 1714 and 386 with weno_ref_quot).
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>

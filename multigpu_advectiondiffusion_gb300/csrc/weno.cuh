@@ -266,7 +266,7 @@ __device__ __forceinline__ void weno_ref_beta(const double (&K)[3], const double
 
 // A compiled FP64 division leaves its short form for a numerator of zero, and one such lane (a constant state,
 // a tile's columns past the domain) takes its warp along: with it kept away, a stage of 121 x 101 x 97, whose
-// last tiles hold seven such columns, takes 1740 us instead of 2086, periodic 120^3 2510 instead of 3397,
+// last tiles hold seven such columns, took 1740 us instead of 2086 (1714 now), periodic 120^3 2510 instead of 3397,
 // 128^3 2389 instead of 2447. Neither operation changes a result: beside an indicator of at least eps, a tau
 // below 2^-100 leaves 1 + tau / (B + eps) at exactly 1 (unsigned: the NaN of two infinite indicators, which the
 // absolute value may leave with its sign, is not below it) ...

@@ -9,8 +9,8 @@ heat3d: the 3D O2 forward-Euler stage on an n^3 FP32 grid (ping-pong between two
 heat3d2: the same problem through adv_heat_run, whose launches each advance two Euler steps
 (2 x launches time steps).
 burgers3d: the periodic WENO5-Z global-Lax-Friedrichs SSP-RK3 stage 1 on an n^3 FP32 grid.
-weno7: the WENO7 prototype scheme's right-hand side (adv_weno7_rhs: a face and a residual kernel
-per axis) on the prototype's Gaussian at n^3 FP32.
+weno7: the WENO7 prototype scheme's right-hand side (adv_weno7_rhs: one fused launch; FP64 a face
+and a residual kernel per axis) on the prototype's Gaussian at n^3.
 Inputs are the seeded initial conditions of the benchmark workloads, generated on the host.
 """
 from __future__ import annotations
